@@ -43,6 +43,7 @@ adamw_matrix_kernel(float* const* __restrict__ w_ptrs, const float* const* __res
                     float* const* __restrict__ m_ptrs, float* const* __restrict__ v_ptrs, int rows, int cols,
                     bf16* __restrict__ dst, bf16* __restrict__ dstT, const AdamwScalars a)
 {
+    pdl_wait();
     __shared__ float tile[32][33];
     const int e = blockIdx.z;
     float* w = w_ptrs[e];
@@ -78,6 +79,7 @@ __global__ void __launch_bounds__(256)
 adamw_flat_kernel(float* const* __restrict__ w_ptrs, const float* const* __restrict__ g_ptrs,
                   float* const* __restrict__ m_ptrs, float* const* __restrict__ v_ptrs, int len, const AdamwScalars a)
 {
+    pdl_wait();
     const int e = blockIdx.y;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= len) return;
@@ -105,26 +107,26 @@ int launch_adamw(mgpt_moe_layer* L, float lr, float beta1, float beta2, float ep
     const bool bf = d.mode == MGPT_MOE_BF16;
     if (L->experts_bound) {
         dim3 gCH((d.H + 31) / 32, (d.C + 31) / 32, E), gHC((d.C + 31) / 32, (d.H + 31) / 32, E);
-        adamw_matrix_kernel<<<gCH, 256, 0, st>>>((float* const*)L->master.Wg, (const float* const*)L->master.gWg,
+        MGPT_CUDA(launch_pdl(adamw_matrix_kernel, gCH, 256, 0, st, (float* const*)L->master.Wg, (const float* const*)L->master.gWg,
                                                  (float* const*)T(0), (float* const*)T(6), d.C, d.H,
-                                                 bf ? L->sWg : nullptr, bf ? L->sWgT : nullptr, a);
+                                                 bf ? L->sWg : nullptr, bf ? L->sWgT : nullptr, a));
         MGPT_LAUNCHED("adamw_matrix_kernel<Wg>");
-        adamw_matrix_kernel<<<gCH, 256, 0, st>>>((float* const*)L->master.Wu, (const float* const*)L->master.gWu,
+        MGPT_CUDA(launch_pdl(adamw_matrix_kernel, gCH, 256, 0, st, (float* const*)L->master.Wu, (const float* const*)L->master.gWu,
                                                  (float* const*)T(1), (float* const*)T(7), d.C, d.H,
-                                                 bf ? L->sWu : nullptr, bf ? L->sWuT : nullptr, a);
+                                                 bf ? L->sWu : nullptr, bf ? L->sWuT : nullptr, a));
         MGPT_LAUNCHED("adamw_matrix_kernel<Wu>");
-        adamw_matrix_kernel<<<gHC, 256, 0, st>>>((float* const*)L->master.Wd, (const float* const*)L->master.gWd,
+        MGPT_CUDA(launch_pdl(adamw_matrix_kernel, gHC, 256, 0, st, (float* const*)L->master.Wd, (const float* const*)L->master.gWd,
                                                  (float* const*)T(2), (float* const*)T(8), d.H, d.C,
-                                                 bf ? L->sWd : nullptr, bf ? L->sWdT : nullptr, a);
+                                                 bf ? L->sWd : nullptr, bf ? L->sWdT : nullptr, a));
         MGPT_LAUNCHED("adamw_matrix_kernel<Wd>");
-        adamw_flat_kernel<<<dim3((d.H + 255) / 256, E), 256, 0, st>>>((float* const*)L->master.bg, (const float* const*)L->master.gbg,
-                                                                      (float* const*)T(3), (float* const*)T(9), d.H, a);
+        MGPT_CUDA(launch_pdl(adamw_flat_kernel, dim3((d.H + 255) / 256, E), 256, 0, st, (float* const*)L->master.bg, (const float* const*)L->master.gbg,
+                                                                      (float* const*)T(3), (float* const*)T(9), d.H, a));
         MGPT_LAUNCHED("adamw_flat_kernel<bg>");
-        adamw_flat_kernel<<<dim3((d.H + 255) / 256, E), 256, 0, st>>>((float* const*)L->master.bu, (const float* const*)L->master.gbu,
-                                                                      (float* const*)T(4), (float* const*)T(10), d.H, a);
+        MGPT_CUDA(launch_pdl(adamw_flat_kernel, dim3((d.H + 255) / 256, E), 256, 0, st, (float* const*)L->master.bu, (const float* const*)L->master.gbu,
+                                                                      (float* const*)T(4), (float* const*)T(10), d.H, a));
         MGPT_LAUNCHED("adamw_flat_kernel<bu>");
-        adamw_flat_kernel<<<dim3((d.C + 255) / 256, E), 256, 0, st>>>((float* const*)L->master.bd, (const float* const*)L->master.gbd,
-                                                                      (float* const*)T(5), (float* const*)T(11), d.C, a);
+        MGPT_CUDA(launch_pdl(adamw_flat_kernel, dim3((d.C + 255) / 256, E), 256, 0, st, (float* const*)L->master.bd, (const float* const*)L->master.gbd,
+                                                                      (float* const*)T(5), (float* const*)T(11), d.C, a));
         MGPT_LAUNCHED("adamw_flat_kernel<bd>");
     }
     if (L->router_bound) {
@@ -133,9 +135,9 @@ int launch_adamw(mgpt_moe_layer* L, float lr, float beta1, float beta2, float ep
         const float* const* rg = (const float* const*)T(13);
         float* const* rm = (float* const*)T(14);
         float* const* rv = (float* const*)T(15);
-        adamw_flat_kernel<<<dim3((d.C * E + 255) / 256, 1), 256, 0, st>>>(rw, rg, rm, rv, d.C * E, a);
+        MGPT_CUDA(launch_pdl(adamw_flat_kernel, dim3((d.C * E + 255) / 256, 1), 256, 0, st, rw, rg, rm, rv, d.C * E, a));
         MGPT_LAUNCHED("adamw_flat_kernel<Wr>");
-        adamw_flat_kernel<<<dim3((E + 255) / 256, 1), 256, 0, st>>>(rw + 1, rg + 1, rm + 1, rv + 1, E, a);
+        MGPT_CUDA(launch_pdl(adamw_flat_kernel, dim3((E + 255) / 256, 1), 256, 0, st, rw + 1, rg + 1, rm + 1, rv + 1, E, a));
         MGPT_LAUNCHED("adamw_flat_kernel<br>");
     }
     cudaError_t err = cudaGetLastError();

@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(256)
 block_rmsnorm_fwd_kernel(const TIo* __restrict__ x, const float* __restrict__ scale, float eps, int N, int C,
                          TIo* __restrict__ out, float* __restrict__ rs)
 {
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int tok = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (tok >= N) return;
@@ -51,6 +52,7 @@ block_bwd_kernel(const TIo* __restrict__ x1, const float* __restrict__ scale, co
                  const TIo* __restrict__ g_in, const TIo* __restrict__ dout, int N, int C, TIo* __restrict__ d_x1,
                  float* __restrict__ d_scale)
 {
+    pdl_wait();
     extern __shared__ float part[];                 // [C]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int c = threadIdx.x; c < C; c += blockDim.x) part[c] = 0.0f;
@@ -126,11 +128,11 @@ int mgpt_moe_block_forward(mgpt_moe_layer* L, const void* x1, const float* rms_s
     char* ws = (char*)workspace;
     const int grid = (n_tokens + 7) / 8;
     if (io == MGPT_MOE_IO_F32)
-        block_rmsnorm_fwd_kernel<float><<<grid, 256, 0, st>>>((const float*)x1, rms_scale, eps, n_tokens, L->d.C,
-                                                              (float*)(ws + b.ln2), (float*)(ws + b.rs));
+        MGPT_CUDA(launch_pdl(block_rmsnorm_fwd_kernel<float>, grid, 256, 0, st, (const float*)x1, rms_scale, eps, n_tokens, L->d.C,
+                                                              (float*)(ws + b.ln2), (float*)(ws + b.rs)));
     else
-        block_rmsnorm_fwd_kernel<bf16><<<grid, 256, 0, st>>>((const bf16*)x1, rms_scale, eps, n_tokens, L->d.C,
-                                                             (bf16*)(ws + b.ln2), (float*)(ws + b.rs));
+        MGPT_CUDA(launch_pdl(block_rmsnorm_fwd_kernel<bf16>, grid, 256, 0, st, (const bf16*)x1, rms_scale, eps, n_tokens, L->d.C,
+                                                             (bf16*)(ws + b.ln2), (float*)(ws + b.rs)));
     MGPT_LAUNCHED("block_rmsnorm_fwd_kernel");
     // x2 = x1 + moe(ln2): the skip connection rides on the combine write
     return mgpt_moe_forward_residual(L, ws + b.ln2, x1, x2, n_tokens, io, ws + b.moe, ws_bytes - b.moe, stream);
@@ -158,13 +160,13 @@ int mgpt_moe_block_backward(mgpt_moe_layer* L, const void* x1, const float* rms_
     const size_t sm = (size_t)L->d.C * sizeof(float);
     if (sm > 48 * 1024) return fail(MGPT_MOE_EINVAL, "embed_dim above 12288 is not supported by the block glue");
     if (io == MGPT_MOE_IO_F32)
-        block_bwd_kernel<float><<<grid, 256, sm, st>>>((const float*)x1, rms_scale, (const float*)(ws + b.rs),
+        MGPT_CUDA(launch_pdl(block_bwd_kernel<float>, grid, 256, sm, st, (const float*)x1, rms_scale, (const float*)(ws + b.rs),
                                                        (const float*)(ws + b.d_in), (const float*)dout, n, L->d.C,
-                                                       (float*)d_x1, d_rms_scale);
+                                                       (float*)d_x1, d_rms_scale));
     else
-        block_bwd_kernel<bf16><<<grid, 256, sm, st>>>((const bf16*)x1, rms_scale, (const float*)(ws + b.rs),
+        MGPT_CUDA(launch_pdl(block_bwd_kernel<bf16>, grid, 256, sm, st, (const bf16*)x1, rms_scale, (const float*)(ws + b.rs),
                                                       (const bf16*)(ws + b.d_in), (const bf16*)dout, n, L->d.C,
-                                                      (bf16*)d_x1, d_rms_scale);
+                                                      (bf16*)d_x1, d_rms_scale));
     MGPT_LAUNCHED("block_bwd_kernel");
     return 0;
 }

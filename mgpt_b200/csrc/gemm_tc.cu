@@ -454,17 +454,15 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
                const __grid_constant__ CUtensorMap tmD2, const RowsP p)
 {
     extern __shared__ uint8_t smem_raw[];
-    const int total_items = (MODE == MODE_DX ? p.fixed_tiles : *p.n_tiles) * p.n_col_tiles;
-    if ((int)blockIdx.x >= total_items) {                // whole CTA leaves before any barrier or TMEM use
-        if (threadIdx.x == 0) sched_finish(p.sched);
-        return;
-    }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int COLS_PER_ITEM = MODE == MODE_GATEUP ? BN / 2 : BN;
     const int kb_per_item = (MODE == MODE_DXG ? 2 : 1) * p.kblocks;
 
     const Pipe pipe = carve(smem_raw);
     const uint32_t tmem_base = cta_setup(pipe, warp);
+    pdl_wait();                                         // the setup above overlaps the end of the kernel before
+    // a CTA beyond the last item publishes "no work" to its own queue and leaves through the teardown
+    const int total_items = (MODE == MODE_DX ? p.fixed_tiles : *p.n_tiles) * p.n_col_tiles;
 
     if (warp == 0) {
         if (lane == 0) {
@@ -628,13 +626,9 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant_
     extern __shared__ uint8_t smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int total_items = p.total_items;
-    if ((int)blockIdx.x >= total_items) {
-        if (threadIdx.x == 0) sched_finish(p.sched);
-        return;
-    }
-
     const Pipe pipe = carve(smem_raw);
     const uint32_t tmem_base = cta_setup(pipe, warp, CS_WARPS);
+    pdl_wait();
     constexpr uint32_t BOX = 64 * BK * 2;      // one {64 MN elements, 64 rows} box = 8 KiB
 
     if (warp == 0) {
@@ -1083,9 +1077,9 @@ int launch_rows(mgpt_moe_layer* L, TcState* s, const Workspace& w, const RowsP& 
     const int budget = grid_sms(L, s);
     if (s->max_pairs > 0 && p.pairs) {
         const int pairs = imin(imin(s->max_pairs, budget / 2), w.max_tiles * p.n_col_tiles);
-        tc_rows_pair_kernel<MODE><<<2 * (pairs > 0 ? pairs : 1), TC_THREADS, SMEM_BYTES, st>>>(a0, a1, b0, b1, d0, d1, d2, p);
+        MGPT_CUDA(launch_pdl(tc_rows_pair_kernel<MODE>, 2 * (pairs > 0 ? pairs : 1), TC_THREADS, SMEM_BYTES, st, a0, a1, b0, b1, d0, d1, d2, p));
     } else {
-        tc_rows_kernel<MODE><<<imin(budget, w.max_tiles * p.n_col_tiles), TC_THREADS, SMEM_BYTES, st>>>(a0, a1, b0, b1, d0, d1, d2, p);
+        MGPT_CUDA(launch_pdl(tc_rows_kernel<MODE>, imin(budget, w.max_tiles * p.n_col_tiles), TC_THREADS, SMEM_BYTES, st, a0, a1, b0, b1, d0, d1, d2, p));
     }
     MGPT_LAUNCHED(what);
     return 0;
@@ -1189,11 +1183,11 @@ int tc_experts_backward(mgpt_moe_layer* L, const Workspace& w, char* ws, cudaStr
     }
     g.block_loads = s->blocks_ok ? 1 : 0;
     if (g.block_loads)
-        tc_wgrad_kernel<<<imin(grid_sms(L, s), items), WG_THREADS, SMEM_BYTES, st>>>(s->dG_b2, s->Xg_b4, s->dU_b2, s->Xg_b4,
-                                                                           s->Hh_b2, s->dYg_b4, g);
+        MGPT_CUDA(launch_pdl(tc_wgrad_kernel, imin(grid_sms(L, s), items), WG_THREADS, SMEM_BYTES, st, s->dG_b2, s->Xg_b4, s->dU_b2, s->Xg_b4,
+                                                                           s->Hh_b2, s->dYg_b4, g));
     else
-        tc_wgrad_kernel<<<imin(grid_sms(L, s), items), WG_THREADS, SMEM_BYTES, st>>>(s->dG_t, s->Xg_t, s->dU_t, s->Xg_t, s->Hh_t,
-                                                                           s->dYg_t, g);
+        MGPT_CUDA(launch_pdl(tc_wgrad_kernel, imin(grid_sms(L, s), items), WG_THREADS, SMEM_BYTES, st, s->dG_t, s->Xg_t, s->dU_t, s->Xg_t, s->Hh_t,
+                                                                           s->dYg_t, g));
     MGPT_LAUNCHED("tc_wgrad_kernel");
     L->stage_end(ST_WGRAD, st);
     return 0;
@@ -1220,8 +1214,7 @@ int tc_router_dx(mgpt_moe_layer* L, const Workspace& w, char* ws, const void* dX
     p.fixed_tiles = cdiv(w.n_tokens, BM); p.n_valid_rows = w.n_tokens;
     p.gather_src = (const bf16*)dXg; p.gather_pos = pos; p.gather_k = d.k;
     p.sched = s->sched + 10;
-    tc_rows_kernel<MODE_DX><<<imin(grid_sms(L, s), p.fixed_tiles * p.n_col_tiles), TC_THREADS, SMEM_BYTES, st>>>(
-        mA, mA, mB, mB, mD, mD, mD, p);
+    MGPT_CUDA(launch_pdl(tc_rows_kernel<MODE_DX>, imin(grid_sms(L, s), p.fixed_tiles * p.n_col_tiles), TC_THREADS, SMEM_BYTES, st, mA, mA, mB, mB, mD, mD, mD, p));
     MGPT_LAUNCHED("tc_rows_kernel<dx>");
     return 0;
 }
@@ -1248,7 +1241,7 @@ int tc_router_wgrad(mgpt_moe_layer* L, const Workspace& w, char* ws, const void*
     q.n_groups = chunks; q.uniform_rows = rows; q.single_grad = L->p_grad[0]; q.item_begin = 0;
     g.total_items = chunks * per_chunk;
     g.sched = s->sched + 12;
-    tc_wgrad_kernel<<<imin(grid_sms(L, s), g.total_items), WG_THREADS, SMEM_BYTES, st>>>(mA, mB, mA, mB, mA, mB, g);
+    MGPT_CUDA(launch_pdl(tc_wgrad_kernel, imin(grid_sms(L, s), g.total_items), WG_THREADS, SMEM_BYTES, st, mA, mB, mA, mB, mA, mB, g));
     MGPT_LAUNCHED("tc_wgrad_kernel<Wr>");
     return 0;
 }
@@ -1258,6 +1251,7 @@ int tc_router_wgrad(mgpt_moe_layer* L, const Workspace& w, char* ws, const void*
 __global__ void bounded_wait_selftest_kernel(int32_t* status)
 {
     __shared__ __align__(8) uint64_t bar;
+    pdl_wait();
     if (threadIdx.x == 0) {
         mbar_init(smem_u32(&bar), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1267,7 +1261,7 @@ __global__ void bounded_wait_selftest_kernel(int32_t* status)
 
 int tc_selftest_bounded_wait(mgpt_moe_layer* L, cudaStream_t st)
 {
-    bounded_wait_selftest_kernel<<<1, 32, 0, st>>>(L->d_status);
+    MGPT_CUDA(launch_pdl(bounded_wait_selftest_kernel, 1, 32, 0, st, L->d_status));
     MGPT_LAUNCHED("bounded_wait_selftest_kernel");
     L->last_stream = st;
     return 0;

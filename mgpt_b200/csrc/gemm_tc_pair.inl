@@ -112,6 +112,7 @@ tc_rows_pair_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_const
                     const __grid_constant__ CUtensorMap tmD2, const RowsP p)
 {
     extern __shared__ uint8_t smem_raw[];
+    pdl_wait();
     const uint32_t rank = cluster_ctarank();
     const int pair = blockIdx.x >> 1, grid_pairs = gridDim.x >> 1;
     const int total_items = *p.n_pairs * p.n_col_tiles;

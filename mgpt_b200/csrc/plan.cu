@@ -36,6 +36,7 @@ template <> __device__ __forceinline__ bf16 from_f32<bf16>(float v) { return __f
 __global__ void __launch_bounds__(PLAN_BLOCK)
 plan_count_kernel(const int32_t* __restrict__ top_idx, int R, int E, int32_t* __restrict__ blk_cnt)
 {
+    pdl_wait();
     __shared__ int cnt[MAX_EXPERTS];
     if (threadIdx.x < E) cnt[threadIdx.x] = 0;
     __syncthreads();
@@ -56,6 +57,7 @@ plan_scan_kernel(int32_t* __restrict__ blk_cnt, int n_blocks, int E,
                  int32_t* __restrict__ n_tiles, int max_tiles, int32_t* __restrict__ status,
                  int32_t* __restrict__ sticky, int32_t* __restrict__ pairs, int32_t* __restrict__ n_pairs)
 {
+    pdl_wait();
     __shared__ int tot[MAX_EXPERTS];
     __shared__ int poff[MAX_EXPERTS + 1];
     __shared__ int pair0[MAX_EXPERTS + 1];
@@ -117,6 +119,7 @@ plan_assign_kernel(const int32_t* __restrict__ top_idx, int R, int E,
                    int32_t* __restrict__ map, int32_t* __restrict__ pos, int32_t* __restrict__ row_src,
                    int32_t* __restrict__ slot_of, int32_t* __restrict__ status, int32_t* __restrict__ sticky)
 {
+    pdl_wait();
     __shared__ int warp_cnt[PLAN_BLOCK / 32][MAX_EXPERTS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < (PLAN_BLOCK / 32) * MAX_EXPERTS; i += PLAN_BLOCK) (&warp_cnt[0][0])[i] = 0;
@@ -161,6 +164,7 @@ plan_small_kernel(const int32_t* __restrict__ top_idx, int R, int E, int32_t* __
                   int32_t* __restrict__ row_src, int32_t* __restrict__ slot_of, int32_t* __restrict__ status,
                   int32_t* __restrict__ sticky, int32_t* __restrict__ pairs, int32_t* __restrict__ n_pairs)
 {
+    pdl_wait();
     __shared__ int warp_cnt[PLAN_BLOCK / 32][MAX_EXPERTS];
     __shared__ int tot[MAX_EXPERTS], off[MAX_EXPERTS + 1], poff[MAX_EXPERTS + 1], pair0[MAX_EXPERTS + 1];
     __shared__ int bad;
@@ -234,6 +238,7 @@ __global__ void __launch_bounds__(256)
 dispatch_rows_kernel(const TIn* __restrict__ x, const int32_t* __restrict__ row_src,
                      const int32_t* __restrict__ n_tiles, int fixed_rows, int C, int k, TAct* __restrict__ Xg)
 {
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     // rows in use: all tiles of the plan, or a count the host already knows
@@ -301,6 +306,7 @@ __global__ void __launch_bounds__(256, 8)
 combine_fwd_kernel(const TAct* __restrict__ Yg, const int32_t* __restrict__ pos, const float* __restrict__ top_p,
                    int N, int C, int k, const TIo* __restrict__ residual, TIo* __restrict__ y)
 {
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int tok = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (tok >= N) return;
@@ -347,6 +353,7 @@ combine_bwd_kernel(const TIo* __restrict__ dy, const TAct* __restrict__ Yg, cons
                    const float* __restrict__ top_p, const int32_t* __restrict__ n_tiles, int fixed_rows, int C, int k,
                    TAct* __restrict__ dYg, float* __restrict__ d_top_p)
 {
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (p >= (fixed_rows >= 0 ? fixed_rows : *n_tiles * ROW_TILE)) return;
@@ -392,6 +399,7 @@ struct BiasGradArgs {
 template <typename TAct>
 __global__ void __launch_bounds__(256) bias_grad_kernel(BiasGradArgs a)
 {
+    pdl_wait();
     __shared__ float red[8][256 + 8];
     const int tile = blockIdx.x, which = blockIdx.z;
     if (tile >= *a.n_tiles) return;
@@ -442,19 +450,19 @@ int run_plan(const int32_t* top_idx, int R, int E, int32_t* counts, int32_t* off
 {
     const int plan_blocks = R > 0 ? (R + PLAN_BLOCK - 1) / PLAN_BLOCK : 1;
     if (R <= PLAN_BLOCK) {
-        plan_small_kernel<<<1, PLAN_BLOCK, 0, st>>>(top_idx, R, E, counts, offsets, padded_offsets, tile_expert, n_tiles,
-                                                    max_tiles, map, pos, row_src, slot_of, status, sticky, pairs, n_pairs);
+        MGPT_CUDA(launch_pdl(plan_small_kernel, 1, PLAN_BLOCK, 0, st, top_idx, R, E, counts, offsets, padded_offsets, tile_expert, n_tiles,
+                                                    max_tiles, map, pos, row_src, slot_of, status, sticky, pairs, n_pairs));
         MGPT_LAUNCHED("plan_small_kernel");
         return 0;
     }
     (void)row_cap;      // rows beyond the plan's tiles are never read; padding rows are marked by plan_assign_kernel
-    plan_count_kernel<<<plan_blocks, PLAN_BLOCK, 0, st>>>(top_idx, R, E, blk);
+    MGPT_CUDA(launch_pdl(plan_count_kernel, plan_blocks, PLAN_BLOCK, 0, st, top_idx, R, E, blk));
     MGPT_LAUNCHED("plan_count_kernel");
-    plan_scan_kernel<<<1, MAX_EXPERTS, 0, st>>>(blk, plan_blocks, E, counts, offsets, padded_offsets, tile_expert,
-                                                n_tiles, max_tiles, status, sticky, pairs, n_pairs);
+    MGPT_CUDA(launch_pdl(plan_scan_kernel, 1, MAX_EXPERTS, 0, st, blk, plan_blocks, E, counts, offsets, padded_offsets, tile_expert,
+                                                n_tiles, max_tiles, status, sticky, pairs, n_pairs));
     MGPT_LAUNCHED("plan_scan_kernel");
-    plan_assign_kernel<<<plan_blocks, PLAN_BLOCK, 0, st>>>(top_idx, R, E, blk, counts, offsets, padded_offsets, map, pos,
-                                                           row_src, slot_of, status, sticky);
+    MGPT_CUDA(launch_pdl(plan_assign_kernel, plan_blocks, PLAN_BLOCK, 0, st, top_idx, R, E, blk, counts, offsets, padded_offsets, map, pos,
+                                                           row_src, slot_of, status, sticky));
     MGPT_LAUNCHED("plan_assign_kernel");
     return 0;
 }
@@ -476,11 +484,11 @@ int gather_rows(const void* src, int src_io, const int32_t* row_src, const int32
     const int grid = (grid_rows + 7) / 8;
     if (act_bytes == 4) {
         if (src_io != MGPT_MOE_IO_F32) return fail(MGPT_MOE_EINVAL, "FP32 mode takes FP32 rows");
-        dispatch_rows_kernel<float, float><<<grid, 256, 0, st>>>((const float*)src, row_src, n_tiles, rows, C, k, (float*)dst);
+        MGPT_CUDA(launch_pdl(dispatch_rows_kernel<float, float>, grid, 256, 0, st, (const float*)src, row_src, n_tiles, rows, C, k, (float*)dst));
     } else if (src_io == MGPT_MOE_IO_F32) {
-        dispatch_rows_kernel<float, bf16><<<grid, 256, 0, st>>>((const float*)src, row_src, n_tiles, rows, C, k, (bf16*)dst);
+        MGPT_CUDA(launch_pdl(dispatch_rows_kernel<float, bf16>, grid, 256, 0, st, (const float*)src, row_src, n_tiles, rows, C, k, (bf16*)dst));
     } else {
-        dispatch_rows_kernel<bf16, bf16><<<grid, 256, 0, st>>>((const bf16*)src, row_src, n_tiles, rows, C, k, (bf16*)dst);
+        MGPT_CUDA(launch_pdl(dispatch_rows_kernel<bf16, bf16>, grid, 256, 0, st, (const bf16*)src, row_src, n_tiles, rows, C, k, (bf16*)dst));
     }
     MGPT_LAUNCHED("dispatch_rows_kernel");
     return 0;
@@ -501,11 +509,11 @@ int combine_rows(const void* rows, const int32_t* pos, const float* top_p, int N
 #define MGPT_COMBINE(KK)                                                                                                  \
     do {                                                                                                                  \
         if (act_bytes == 4)                                                                                               \
-            combine_fwd_kernel<float, float, KK><<<grid, 256, 0, st>>>((const float*)rows, pos, top_p, N, C, k, (const float*)residual, (float*)y); \
+            MGPT_CUDA(launch_pdl(combine_fwd_kernel<float, float, KK>, grid, 256, 0, st, (const float*)rows, pos, top_p, N, C, k, (const float*)residual, (float*)y)); \
         else if (io == MGPT_MOE_IO_F32)                                                                                   \
-            combine_fwd_kernel<bf16, float, KK><<<grid, 256, 0, st>>>((const bf16*)rows, pos, top_p, N, C, k, (const float*)residual, (float*)y); \
+            MGPT_CUDA(launch_pdl(combine_fwd_kernel<bf16, float, KK>, grid, 256, 0, st, (const bf16*)rows, pos, top_p, N, C, k, (const float*)residual, (float*)y)); \
         else                                                                                                              \
-            combine_fwd_kernel<bf16, bf16, KK><<<grid, 256, 0, st>>>((const bf16*)rows, pos, top_p, N, C, k, (const bf16*)residual, (bf16*)y);   \
+            MGPT_CUDA(launch_pdl(combine_fwd_kernel<bf16, bf16, KK>, grid, 256, 0, st, (const bf16*)rows, pos, top_p, N, C, k, (const bf16*)residual, (bf16*)y));   \
     } while (0)
     if (k <= 1) MGPT_COMBINE(1);
     else if (k <= 2) MGPT_COMBINE(2);
@@ -530,14 +538,14 @@ int combine_rows_backward(const void* dy, int io, const void* rows, const int32_
     if (grid_rows <= 0) return 0;
     const int grid = (grid_rows + 7) / 8;
     if (act_bytes == 4)
-        combine_bwd_kernel<float, float><<<grid, 256, 0, st>>>((const float*)dy, (const float*)rows, row_src, top_p,
-                                                               n_tiles, n_rows, C, k, (float*)d_rows, d_top_p);
+        MGPT_CUDA(launch_pdl(combine_bwd_kernel<float, float>, grid, 256, 0, st, (const float*)dy, (const float*)rows, row_src, top_p,
+                                                               n_tiles, n_rows, C, k, (float*)d_rows, d_top_p));
     else if (io == MGPT_MOE_IO_F32)
-        combine_bwd_kernel<bf16, float><<<grid, 256, 0, st>>>((const float*)dy, (const bf16*)rows, row_src, top_p,
-                                                              n_tiles, n_rows, C, k, (bf16*)d_rows, d_top_p);
+        MGPT_CUDA(launch_pdl(combine_bwd_kernel<bf16, float>, grid, 256, 0, st, (const float*)dy, (const bf16*)rows, row_src, top_p,
+                                                              n_tiles, n_rows, C, k, (bf16*)d_rows, d_top_p));
     else
-        combine_bwd_kernel<bf16, bf16><<<grid, 256, 0, st>>>((const bf16*)dy, (const bf16*)rows, row_src, top_p,
-                                                             n_tiles, n_rows, C, k, (bf16*)d_rows, d_top_p);
+        MGPT_CUDA(launch_pdl(combine_bwd_kernel<bf16, bf16>, grid, 256, 0, st, (const bf16*)dy, (const bf16*)rows, row_src, top_p,
+                                                             n_tiles, n_rows, C, k, (bf16*)d_rows, d_top_p));
     MGPT_LAUNCHED("combine_bwd_kernel");
     return 0;
 }
@@ -560,8 +568,8 @@ int launch_bias_grads(const mgpt_moe_layer* L, const Workspace& w, char* ws, cud
     a.n_tiles = (const int32_t*)(ws + w.n_tiles);
     const int mc = d.C > d.H ? d.C : d.H;
     dim3 grid(w.max_tiles, (mc + 255) / 256, 3);
-    if (w.act_bytes == 4) bias_grad_kernel<float><<<grid, 256, 0, st>>>(a);
-    else bias_grad_kernel<bf16><<<grid, 256, 0, st>>>(a);
+    if (w.act_bytes == 4) MGPT_CUDA(launch_pdl(bias_grad_kernel<float>, grid, 256, 0, st, a));
+    else MGPT_CUDA(launch_pdl(bias_grad_kernel<bf16>, grid, 256, 0, st, a));
     MGPT_LAUNCHED("bias_grad_kernel");
     return 0;
 }
@@ -576,6 +584,7 @@ segment_tiles_kernel(const int32_t* __restrict__ seg_counts, int n_src, int E, i
                      int32_t* __restrict__ status, int32_t* __restrict__ sticky,
                      int32_t* __restrict__ pairs, int32_t* __restrict__ n_pairs)
 {
+    pdl_wait();
     __shared__ int first_tile[MAX_SEGMENTS + 1];     // in arrival order (s, e)
     __shared__ int first_item[MAX_SEGMENTS];         // in processing order (e, s)
     __shared__ int pair0[MAX_EXPERTS + 1];
@@ -638,11 +647,11 @@ int launch_segment_tiles(const Dims& d, const Workspace& w, char* ws, const int3
                          int32_t* sticky)
 {
     if (n_src * d.E > MAX_SEGMENTS) return fail(MGPT_MOE_EINVAL, "sources x local experts must not exceed 4096");
-    segment_tiles_kernel<<<1, 256, 0, st>>>(seg_counts, n_src, d.E, (int32_t*)(ws + w.counts),
+    MGPT_CUDA(launch_pdl(segment_tiles_kernel, 1, 256, 0, st, seg_counts, n_src, d.E, (int32_t*)(ws + w.counts),
                                             (int32_t*)(ws + w.tile_expert), (int32_t*)(ws + w.tile_order),
                                             (int32_t*)(ws + w.n_tiles), w.max_tiles, (int32_t*)(ws + w.seg),
                                             (int32_t*)(ws + w.status), sticky, (int32_t*)(ws + w.pairs),
-                                            (int32_t*)(ws + w.n_pairs));
+                                            (int32_t*)(ws + w.n_pairs)));
     MGPT_LAUNCHED("segment_tiles_kernel");
     return 0;
 }

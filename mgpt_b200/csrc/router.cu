@@ -124,6 +124,7 @@ router_fwd_kernel(const TIn* __restrict__ x, const float* __restrict__ Wr, const
                   int32_t* __restrict__ top_idx, float* __restrict__ top_p,
                   const int32_t* __restrict__ list, const int32_t* __restrict__ list_count)
 {
+    pdl_wait();
     constexpr int SUB = 32 / EL;                    // tokens per warp pass
     constexpr int TOK_W = TPW * SUB;                // tokens per warp
     constexpr int TOK = R_WARPS * TOK_W;            // tokens per CTA
@@ -285,6 +286,7 @@ router_list_kernel(const TIn* __restrict__ x, const float* __restrict__ Wr, cons
                    int32_t* __restrict__ top_idx, float* __restrict__ top_p,
                    const int32_t* __restrict__ list, const int32_t* __restrict__ list_count)
 {
+    pdl_wait();
     constexpr int TOK = R_WARPS * TPW, WCOLS = 32 * EPL, THREADS = R_WARPS * 32;
     constexpr int ST = EPL <= 2 ? 4 : 2;            // stages: 36 KiB of static shared memory at most
     constexpr int XV = 16 / sizeof(TIn);            // elements per 16-byte piece
@@ -381,6 +383,7 @@ router_dlogits_kernel(const float* __restrict__ probs, const int32_t* __restrict
                       int N, int E, int k, float alpha, float* __restrict__ dlogits,
                       bf16* __restrict__ dl16, int E8, float* __restrict__ gbr)
 {
+    pdl_wait();
     __shared__ float bred[8][EPL * 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned full = 0xffffffffu;
@@ -451,6 +454,7 @@ __global__ void __launch_bounds__(256)
 router_dx_kernel(const TAct* __restrict__ dXg, const int32_t* __restrict__ pos, const float* __restrict__ dlogits,
                  const float* __restrict__ Wr, int N, int C, int E, int k, int chunk, TIo* __restrict__ dx)
 {
+    pdl_wait();
     extern __shared__ __align__(16) float sm_dx[];
     const int wstride = chunk + 4;                      // padded row: transposed staging without 32-way conflicts
     float* wt = sm_dx;                                  // [E][chunk+4]  (Wr^T of this channel chunk)
@@ -553,6 +557,7 @@ __global__ void __launch_bounds__(256)
 router_wgrad_partial_kernel(const TIo* __restrict__ x, const float* __restrict__ dlogits, int N, int C, int E,
                             int tok_per_chunk, float* __restrict__ part, float* __restrict__ partb)
 {
+    pdl_wait();
     const int E4 = (E + 3) / 4;                         // expert groups of 4
     const int cg_per_cta = 256 / E4;                    // channel groups of 4 handled by this CTA
     const int eg = threadIdx.x % E4, cgi = threadIdx.x / E4;
@@ -612,6 +617,7 @@ __global__ void __launch_bounds__(256)
 router_wgrad_reduce_kernel(const float* __restrict__ part, const float* __restrict__ partb, int n_chunks, int CE, int E,
                            float* __restrict__ gWr, float* __restrict__ gbr)
 {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < CE) {
         float s = 0.0f;
@@ -634,9 +640,9 @@ int router_fwd_launch(const TIn* x, const float* Wr, const float* br, int N, int
     const int grid = (N + TOK - 1) / TOK;
     const bool fast = C % R_CK == 0 && E == EPL * EL && ((uintptr_t)x & 15) == 0 && ((uintptr_t)Wr & 15) == 0;
     if (fast)
-        router_fwd_kernel<TIn, EL, EPL, TPW, true><<<grid, R_WARPS * 32, 0, st>>>(x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, list, list_count);
+        MGPT_CUDA(launch_pdl(router_fwd_kernel<TIn, EL, EPL, TPW, true>, grid, R_WARPS * 32, 0, st, x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, list, list_count));
     else
-        router_fwd_kernel<TIn, EL, EPL, TPW, false><<<grid, R_WARPS * 32, 0, st>>>(x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, list, list_count);
+        MGPT_CUDA(launch_pdl(router_fwd_kernel<TIn, EL, EPL, TPW, false>, grid, R_WARPS * 32, 0, st, x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, list, list_count));
     MGPT_LAUNCHED("router_fwd_kernel");
     return 0;
 }
@@ -652,9 +658,9 @@ int router_fwd_dispatch(const TIn* x, const float* Wr, const float* br, int N, i
         ((uintptr_t)Wr & 15) == 0) {
         // the chunks through the cp.async ring: with a handful of CTAs, nothing else hides the loads of a chunk
         const int grid = (N + R_WARPS - 1) / R_WARPS;
-        if (E == 32) router_list_kernel<TIn, 1, 1><<<grid, R_WARPS * 32, 0, st>>>(x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, nullptr, nullptr);
-        else if (E == 64) router_list_kernel<TIn, 2, 1><<<grid, R_WARPS * 32, 0, st>>>(x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, nullptr, nullptr);
-        else router_list_kernel<TIn, 4, 1><<<grid, R_WARPS * 32, 0, st>>>(x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, nullptr, nullptr);
+        if (E == 32) MGPT_CUDA(launch_pdl(router_list_kernel<TIn, 1, 1>, grid, R_WARPS * 32, 0, st, x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, nullptr, nullptr));
+        else if (E == 64) MGPT_CUDA(launch_pdl(router_list_kernel<TIn, 2, 1>, grid, R_WARPS * 32, 0, st, x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, nullptr, nullptr));
+        else MGPT_CUDA(launch_pdl(router_list_kernel<TIn, 4, 1>, grid, R_WARPS * 32, 0, st, x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, nullptr, nullptr));
         MGPT_LAUNCHED("router_list_kernel<decode>");
         return 0;
     }
@@ -669,9 +675,9 @@ int router_fwd_dispatch(const TIn* x, const float* Wr, const float* br, int N, i
     // CTAs (16 tokens) so that the few thousand listed tokens still spread over every SM.
     if (list && C % R_CK == 0 && E % 32 == 0 && E <= 128 && E != 96 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)Wr & 15) == 0) {
         const int grid = (N + 15) / 16;
-        if (E == 32) router_list_kernel<TIn, 1, 4><<<grid, R_WARPS * 32, 0, st>>>(x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, list, list_count);
-        else if (E == 64) router_list_kernel<TIn, 2, 4><<<grid, R_WARPS * 32, 0, st>>>(x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, list, list_count);
-        else router_list_kernel<TIn, 4, 4><<<grid, R_WARPS * 32, 0, st>>>(x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, list, list_count);
+        if (E == 32) MGPT_CUDA(launch_pdl(router_list_kernel<TIn, 1, 4>, grid, R_WARPS * 32, 0, st, x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, list, list_count));
+        else if (E == 64) MGPT_CUDA(launch_pdl(router_list_kernel<TIn, 2, 4>, grid, R_WARPS * 32, 0, st, x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, list, list_count));
+        else MGPT_CUDA(launch_pdl(router_list_kernel<TIn, 4, 4>, grid, R_WARPS * 32, 0, st, x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, list, list_count));
         MGPT_LAUNCHED("router_list_kernel");
         return 0;
     }
@@ -721,9 +727,9 @@ int launch_router_bwd(mgpt_moe_layer* L, const Workspace& w, char* ws, const voi
         const int grid = min((N + 7) / 8, 1184);
         bf16* dl16 = tc ? (bf16*)(ws + w.dl16) : nullptr;
         float* gbr = tc_wgrad ? L->p_grad[1] : nullptr;
-        if (E <= 32) router_dlogits_kernel<1><<<grid, 256, 0, st>>>(probs, top_idx, dtp, counts, N, E, k, d.alpha, dl, dl16, E8, gbr);
-        else if (E <= 64) router_dlogits_kernel<2><<<grid, 256, 0, st>>>(probs, top_idx, dtp, counts, N, E, k, d.alpha, dl, dl16, E8, gbr);
-        else router_dlogits_kernel<4><<<grid, 256, 0, st>>>(probs, top_idx, dtp, counts, N, E, k, d.alpha, dl, dl16, E8, gbr);
+        if (E <= 32) MGPT_CUDA(launch_pdl(router_dlogits_kernel<1>, grid, 256, 0, st, probs, top_idx, dtp, counts, N, E, k, d.alpha, dl, dl16, E8, gbr));
+        else if (E <= 64) MGPT_CUDA(launch_pdl(router_dlogits_kernel<2>, grid, 256, 0, st, probs, top_idx, dtp, counts, N, E, k, d.alpha, dl, dl16, E8, gbr));
+        else MGPT_CUDA(launch_pdl(router_dlogits_kernel<4>, grid, 256, 0, st, probs, top_idx, dtp, counts, N, E, k, d.alpha, dl, dl16, E8, gbr));
         MGPT_LAUNCHED("router_dlogits_kernel");
     }
     if (tc) {
@@ -741,11 +747,11 @@ int launch_router_bwd(mgpt_moe_layer* L, const Workspace& w, char* ws, const voi
             L->router_dx_attr = true;
         }
         if (w.act_bytes == 4) {
-            router_dx_kernel<float, float><<<grid, 256, sm, st>>>((const float*)dXg, pos, dl, Wr, N, C, E, k, chunk, (float*)dx);
+            MGPT_CUDA(launch_pdl(router_dx_kernel<float, float>, grid, 256, sm, st, (const float*)dXg, pos, dl, Wr, N, C, E, k, chunk, (float*)dx));
         } else if (io == MGPT_MOE_IO_F32) {
-            router_dx_kernel<bf16, float><<<grid, 256, sm, st>>>((const bf16*)dXg, pos, dl, Wr, N, C, E, k, chunk, (float*)dx);
+            MGPT_CUDA(launch_pdl(router_dx_kernel<bf16, float>, grid, 256, sm, st, (const bf16*)dXg, pos, dl, Wr, N, C, E, k, chunk, (float*)dx));
         } else {
-            router_dx_kernel<bf16, bf16><<<grid, 256, sm, st>>>((const bf16*)dXg, pos, dl, Wr, N, C, E, k, chunk, (bf16*)dx);
+            MGPT_CUDA(launch_pdl(router_dx_kernel<bf16, bf16>, grid, 256, sm, st, (const bf16*)dXg, pos, dl, Wr, N, C, E, k, chunk, (bf16*)dx));
         }
         MGPT_LAUNCHED("router_dx_kernel");
     }
@@ -759,12 +765,12 @@ int launch_router_bwd(mgpt_moe_layer* L, const Workspace& w, char* ws, const voi
         const int tpc = (N + w.rw_chunks - 1) / w.rw_chunks;
         dim3 grid(cblocks, w.rw_chunks);
         if (io == MGPT_MOE_IO_F32)
-            router_wgrad_partial_kernel<float><<<grid, 256, 0, st>>>((const float*)x, dl, N, C, E, tpc, part, partb);
+            MGPT_CUDA(launch_pdl(router_wgrad_partial_kernel<float>, grid, 256, 0, st, (const float*)x, dl, N, C, E, tpc, part, partb));
         else
-            router_wgrad_partial_kernel<bf16><<<grid, 256, 0, st>>>((const bf16*)x, dl, N, C, E, tpc, part, partb);
+            MGPT_CUDA(launch_pdl(router_wgrad_partial_kernel<bf16>, grid, 256, 0, st, (const bf16*)x, dl, N, C, E, tpc, part, partb));
         MGPT_LAUNCHED("router_wgrad_partial_kernel");
-        router_wgrad_reduce_kernel<<<(C * E + 255) / 256, 256, 0, st>>>(part, partb, w.rw_chunks, C * E, E,
-                                                                      L->p_grad[0], L->p_grad[1]);
+        MGPT_CUDA(launch_pdl(router_wgrad_reduce_kernel, (C * E + 255) / 256, 256, 0, st, part, partb, w.rw_chunks, C * E, E,
+                                                                      L->p_grad[0], L->p_grad[1]));
         MGPT_LAUNCHED("router_wgrad_reduce_kernel");
     }
     return 0;

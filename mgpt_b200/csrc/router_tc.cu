@@ -63,8 +63,6 @@ tc_router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     constexpr int STAGES = Cfg::STAGES;
     extern __shared__ uint8_t smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if ((int)blockIdx.x >= p.n_tiles) return;
-
     const uint32_t base = smem_u32(smem_raw);
     const uint32_t pad = (1024u - (base & 1023u)) & 1023u;
     uint8_t* tiles = smem_raw + pad;
@@ -95,6 +93,7 @@ tc_router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     tc_fence_after();
     uint32_t tmem_base;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
+    pdl_wait();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -314,6 +313,7 @@ router_pieces_kernel(const float* __restrict__ Wr, const float* __restrict__ br,
                      bf16* __restrict__ out, float* __restrict__ rstat)
 {
     __shared__ float red[8];
+    pdl_wait();
     const int e = blockIdx.x;
     float ss = 0.0f;
     for (int c = threadIdx.x; c < C; c += blockDim.x) {
@@ -347,7 +347,7 @@ int launch_rt(const CUtensorMap& mx, const CUtensorMap& mw, const RtP& p, int gr
         MGPT_CUDA(cudaFuncSetAttribute(tc_router_fwd_kernel<NE>, cudaFuncAttributeMaxDynamicSharedMemorySize, RtCfg<NE>::SMEM));
         *attr_done = true;
     }
-    tc_router_fwd_kernel<NE><<<grid, RT_THREADS, RtCfg<NE>::SMEM, st>>>(mx, mw, p);
+    MGPT_CUDA(launch_pdl(tc_router_fwd_kernel<NE>, grid, RT_THREADS, RtCfg<NE>::SMEM, st, mx, mw, p));
     MGPT_LAUNCHED("tc_router_fwd_kernel");
     return 0;
 }
@@ -360,7 +360,7 @@ int launch_router_pieces(mgpt_moe_layer* L, cudaStream_t st)
     const Dims& d = L->d;
     if (!L->sWrT2 || !L->router_bound) return 0;
     MGPT_CUDA(cudaMemsetAsync(L->d_rstat, 0, 2 * sizeof(float), st));
-    router_pieces_kernel<<<d.E, 256, 0, st>>>(L->p_data[0], L->p_data[1], d.C, d.E, L->router_ne, L->sWrT2, L->d_rstat);
+    MGPT_CUDA(launch_pdl(router_pieces_kernel, d.E, 256, 0, st, L->p_data[0], L->p_data[1], d.C, d.E, L->router_ne, L->sWrT2, L->d_rstat));
     MGPT_LAUNCHED("router_pieces_kernel");
     return 0;
 }

@@ -17,6 +17,7 @@ __global__ void __launch_bounds__(256)
 shadow_kernel(const void* const* __restrict__ src_ptrs, int rows, int cols,
               bf16* __restrict__ dst, bf16* __restrict__ dstT)
 {
+    pdl_wait();
     __shared__ float tile[32][33];
     const int e = blockIdx.z;
     const float* src = (const float*)src_ptrs[e];
@@ -43,6 +44,7 @@ shadow_kernel(const void* const* __restrict__ src_ptrs, int rows, int cols,
 __global__ void __launch_bounds__(256)
 router_shadow_kernel(const float* __restrict__ Wr, int C, int E, int E8, bf16* __restrict__ out)
 {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= C * E8) return;
     const int c = i / E8, e = i % E8;
@@ -57,7 +59,7 @@ int launch_sync_router_only(mgpt_moe_layer* L, cudaStream_t st)
     const Dims& d = L->d;
     if (d.mode == MGPT_MOE_BF16 && L->router_bound) {
         const int E8 = (d.E + 7) / 8 * 8;
-        router_shadow_kernel<<<(d.C * E8 + 255) / 256, 256, 0, st>>>(L->p_data[0], d.C, d.E, E8, L->sWr);
+        MGPT_CUDA(launch_pdl(router_shadow_kernel, (d.C * E8 + 255) / 256, 256, 0, st, L->p_data[0], d.C, d.E, E8, L->sWr));
         MGPT_LAUNCHED("router_shadow_kernel");
         MGPT_TRY(launch_router_pieces(L, st));
     }
@@ -71,7 +73,7 @@ int launch_sync_weights(mgpt_moe_layer* L, cudaStream_t st)
     if (d.mode != MGPT_MOE_BF16) return 0;
     if (L->router_bound) {
         const int E8 = (d.E + 7) / 8 * 8;
-        router_shadow_kernel<<<(d.C * E8 + 255) / 256, 256, 0, st>>>(L->p_data[0], d.C, d.E, E8, L->sWr);
+        MGPT_CUDA(launch_pdl(router_shadow_kernel, (d.C * E8 + 255) / 256, 256, 0, st, L->p_data[0], d.C, d.E, E8, L->sWr));
         MGPT_LAUNCHED("router_shadow_kernel");
         MGPT_TRY(launch_router_pieces(L, st));
     }
@@ -80,11 +82,11 @@ int launch_sync_weights(mgpt_moe_layer* L, cudaStream_t st)
         return 0;
     }
     dim3 gCH((d.H + 31) / 32, (d.C + 31) / 32, d.E), gHC((d.C + 31) / 32, (d.H + 31) / 32, d.E);
-    shadow_kernel<<<gCH, 256, 0, st>>>(L->master.Wg, d.C, d.H, L->sWg, L->sWgT);
+    MGPT_CUDA(launch_pdl(shadow_kernel, gCH, 256, 0, st, L->master.Wg, d.C, d.H, L->sWg, L->sWgT));
     MGPT_LAUNCHED("shadow_kernel<Wg>");
-    shadow_kernel<<<gCH, 256, 0, st>>>(L->master.Wu, d.C, d.H, L->sWu, L->sWuT);
+    MGPT_CUDA(launch_pdl(shadow_kernel, gCH, 256, 0, st, L->master.Wu, d.C, d.H, L->sWu, L->sWuT));
     MGPT_LAUNCHED("shadow_kernel<Wu>");
-    shadow_kernel<<<gHC, 256, 0, st>>>(L->master.Wd, d.H, d.C, L->sWd, L->sWdT);
+    MGPT_CUDA(launch_pdl(shadow_kernel, gHC, 256, 0, st, L->master.Wd, d.H, d.C, L->sWd, L->sWdT));
     MGPT_LAUNCHED("shadow_kernel<Wd>");
     L->shadows_fresh = true;
     return 0;
