@@ -85,7 +85,7 @@ Workspace make_workspace(const Dims& d, int n_tokens, int kind)
         const int e4 = (d.E + 3) / 4, ch_per_cta = (256 / e4) * 4;
         const int cblocks = (d.C + ch_per_cta - 1) / ch_per_cta;
         int chunks = 1184 / (cblocks > 0 ? cblocks : 1);
-        if (chunks > 64) chunks = 64;
+        if (chunks > 128) chunks = 128;
         if (chunks > n_tokens) chunks = n_tokens;
         if (chunks < 1) chunks = 1;
         w.rw_chunks = chunks;
@@ -262,12 +262,14 @@ int mgpt_moe_bind_params(mgpt_moe_layer* L, float* const* data, float* const* gr
     const bool router = data[0] != nullptr && data[1] != nullptr;
     const bool experts = n == L->n_params;
     if (!router && !experts) return fail(MGPT_MOE_EINVAL, "null parameter pointer");
+    L->masters_aligned = true;
     for (int i = 0; i < L->n_params; ++i) {
         const bool want = i < 2 ? router : experts;
         if (want && !data[i]) return fail(MGPT_MOE_EINVAL, "null parameter pointer");
         if (want && grad && !grad[i]) return fail(MGPT_MOE_EINVAL, "null gradient pointer");
         L->p_data[i] = want ? data[i] : nullptr;
         L->p_grad[i] = (want && grad) ? grad[i] : nullptr;
+        if (i >= 2 && (((uintptr_t)L->p_data[i] | (uintptr_t)L->p_grad[i]) & 15)) L->masters_aligned = false;
     }
     L->has_grad = grad != nullptr;
     L->router_bound = router;
@@ -591,7 +593,7 @@ int mgpt_moe_backward(mgpt_moe_layer* L, const void* x, const void* dy, void* dx
     L->stage_end(ST_ROUTER_BWD, st);
     if (L->dx_ready_event) MGPT_CUDA(cudaEventRecord(L->dx_ready_event, st));
     if (use_tc(L)) MGPT_TRY(tc_experts_backward(L, w, ws, st, 2));
-    if (L->has_grad && !(use_tc(L) && tc_fused_bias_grads(L->d))) {      // else the tensor-core weight-gradient kernel sums the bias gradients itself
+    if (L->has_grad && use_tc(L) && !tc_fused_bias_grads(L->d)) {      // the other weight-gradient kernels sum the bias gradients themselves
         L->stage_begin(ST_BIAS_GRAD, st);
         MGPT_TRY(launch_bias_grads(L, w, ws, st));
         L->stage_end(ST_BIAS_GRAD, st);

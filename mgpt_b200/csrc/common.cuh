@@ -153,12 +153,13 @@ struct mgpt_moe_layer {
     std::vector<float*> p_data, p_grad;      // host copies of the bound pointers
     bool bound = false, has_grad = false, shadows_fresh = false;
     bool router_bound = false, experts_bound = false;
+    bool masters_aligned = false;            // every bound expert tensor (data and gradient) starts on a 16-byte boundary
 
     // Error bits of every kernel of this layer since the last mgpt_moe_check_status (device word, zero at create)
     // and the pinned host word they are read into.
     int32_t* d_status = nullptr;
     int32_t* h_status = nullptr;
-    bool router_dx_attr = false;             // shared-memory opt-in of router_dx_kernel done on this layer's device
+    bool router_dx_attr[2] = {};             // shared-memory opt-in of router_dx_kernel (1 / 4 tokens per thread) done on this layer's device
     bool router_tc_attr = false;             // the same for tc_router_fwd_kernel
 
     // device tables: pointers to FP32 masters / grads per expert

@@ -12,47 +12,104 @@ namespace mgpt {
 
 namespace {
 
+// One CTA: a 64 x 64 output tile, 128 threads per K group, 8 rows x 4 columns per thread; operands go through two
+// shared-memory buffers of 16 k each, the next one loaded into registers with 16-byte accesses while this one is worked
+// on.  What bounds these products at the reference's default size (2048 routed rows, C = 128, H = 512) is not the
+// 0.13-0.27 GFMA but how many warps are in flight and how long one CTA's k loop is: the products over H with C = 128
+// columns are 72 tiles for 148 SMs.  KS groups of 128 threads therefore split a tile's k loop and are added up, in
+// order, through shared memory (KS by split_k below).  One 64 x 64 tile per 256 threads with scalar loads and nothing in
+// flight between two barriers took 49 / 74 / 25 / 73 us for gate-up / down / dHh / dXg and 27 us for each weight
+// gradient there.
 constexpr int TM = 64, TN = 64, TK = 16;
+constexpr int GT = 128;                       // threads per K group
+constexpr int SROW = TM + 4;                  // padded row of a staged operand (floats)
+constexpr int OPER = TK * SROW;               // one staged operand
 
-__device__ __forceinline__ float to_f32(float v) { return v; }
-__device__ __forceinline__ float to_f32(bf16 v) { return __bfloat162float(v); }
 template <typename T> __device__ __forceinline__ T from_f32(float v);
 template <> __device__ __forceinline__ float from_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ bf16 from_f32<bf16>(float v) { return __float2bfloat16(v); }
 
-// acc[4][4] += A(m0.., 0..K) * B(0..K, n0..) with element (m,k) of A at A[m*sAm + k*sAk]
-// and (k,n) of B at B[k*sBk + n*sBn]; out-of-range rows/cols read as zero.
-template <typename TA, typename TB>
-__device__ __forceinline__ void tile_mac(const TA* __restrict__ A, long sAm, long sAk, int m0, int M,
-                                         const TB* __restrict__ B, long sBk, long sBn, int n0, int N,
-                                         int K, float (&acc)[4][4], float (*As)[TM + 4], float (*Bs)[TN + 4])
+// four consecutive elements (VEC: the address is aligned to four elements)
+template <bool VEC> __device__ __forceinline__ float4 load4(const float* p)
 {
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    for (int k0 = 0; k0 < K; k0 += TK) {
+    if constexpr (VEC) return *reinterpret_cast<const float4*>(p);
+    else return make_float4(p[0], p[1], p[2], p[3]);
+}
+template <bool VEC> __device__ __forceinline__ float4 load4(const bf16* p)
+{
+    const uint2 u = *reinterpret_cast<const uint2*>(p);       // the library's own buffers: always aligned
+    return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
+                       __uint_as_float(u.y & 0xffff0000u));
+}
+__device__ __forceinline__ float round_to(float v, float) { return v; }
+__device__ __forceinline__ float round_to(float v, bf16) { return __bfloat162float(__float2bfloat16(v)); }
+__device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void store4(bf16* p, float4 v)
+{
+    __nv_bfloat162 h0 = __floats2bfloat162_rn(v.x, v.y), h1 = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t*>(&h0), *reinterpret_cast<uint32_t*>(&h1));
+}
+__device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(GT) : "memory"); }
+
+// A staged operand is [TK][SROW]: element (k, m) at k*SROW + m.  Thread t of a group fetches two pieces of four
+// elements: along k for a matrix whose k is contiguous (KMAJOR), along m otherwise; out of range reads as zero.
+template <typename T, bool KMAJOR, bool VEC>
+__device__ __forceinline__ void fetch(const T* __restrict__ P, long ld, int m0, int M, int k0, int K, int t, float4 (&r)[2])
+{
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int idx = tid + i * 256;
-            int m, k;
-            if (sAk == 1) { k = idx % TK; m = idx / TK; } else { m = idx % TM; k = idx / TM; }
-            const int gm = m0 + m, gk = k0 + k;
-            As[k][m] = (gm < M && gk < K) ? to_f32(A[gm * sAm + gk * sAk]) : 0.0f;
-            int n, kb;
-            if (sBk == 1) { kb = idx % TK; n = idx / TK; } else { n = idx % TN; kb = idx / TN; }
-            const int gn = n0 + n, gkb = k0 + kb;
-            Bs[kb][n] = (gn < N && gkb < K) ? to_f32(B[gkb * sBk + gn * sBn]) : 0.0f;
+    for (int i = 0; i < 2; ++i) {
+        const int m = m0 + (KMAJOR ? (t >> 2) + 32 * i : (t & 15) * 4);
+        const int k = k0 + (KMAJOR ? (t & 3) * 4 : (t >> 4) + 8 * i);
+        r[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (m < M && k < K) r[i] = load4<VEC>(KMAJOR ? P + (long)m * ld + k : P + (long)k * ld + m);
+    }
+}
+template <bool KMAJOR>
+__device__ __forceinline__ void put(float* S, int t, const float4 (&r)[2])
+{
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        if (KMAJOR) {
+            float* d = S + (t & 3) * 4 * SROW + (t >> 2) + 32 * i;
+            d[0] = r[i].x; d[SROW] = r[i].y; d[2 * SROW] = r[i].z; d[3 * SROW] = r[i].w;
+        } else {
+            *reinterpret_cast<float4*>(S + ((t >> 4) + 8 * i) * SROW + (t & 15) * 4) = r[i];
         }
+    }
+}
+// acc[8][4] += rows ty*8.. x columns tx*4.. over the TK staged k
+__device__ __forceinline__ void mac(const float* As, const float* Bs, int ty, int tx, float (&acc)[8][4])
+{
+#pragma unroll
+    for (int k = 0; k < TK; ++k) {
+        const float4 a0 = *reinterpret_cast<const float4*>(As + k * SROW + ty * 8);
+        const float4 a1 = *reinterpret_cast<const float4*>(As + k * SROW + ty * 8 + 4);
+        const float4 b = *reinterpret_cast<const float4*>(Bs + k * SROW + tx * 4);
+        const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+    }
+}
+// The groups' sums, added to group 0's in group order.  S: shared memory of 64*64 floats per group beyond the first.
+template <int KS>
+__device__ __forceinline__ void fold(float* S, int group, int t, float (&acc)[8][4])
+{
+    if constexpr (KS > 1) {
+        __syncthreads();                      // every group is done with its operand buffers
+        float4* mine = reinterpret_cast<float4*>(S) + (group - 1) * 1024;
+        if (group > 0)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) mine[i * GT + t] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
         __syncthreads();
+        if (group == 0)
+            for (int g = 1; g < KS; ++g)
 #pragma unroll
-        for (int k = 0; k < TK; ++k) {
-            const float4 a = *reinterpret_cast<const float4*>(&As[k][ty * 4]);
-            const float4 b = *reinterpret_cast<const float4*>(&Bs[k][tx * 4]);
-            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-        }
-        __syncthreads();
+                for (int i = 0; i < 8; ++i) {
+                    const float4 v = reinterpret_cast<const float4*>(S)[(g - 1) * 1024 + i * GT + t];
+                    acc[i][0] += v.x; acc[i][1] += v.y; acc[i][2] += v.z; acc[i][3] += v.w;
+                }
     }
 }
 
@@ -65,112 +122,271 @@ struct RowsArgs {
     void* D; void* D2; void* D3;               // outputs [rows, Nout]
     const void* G; const void* U;              // saved pre-activations (EPI_DHH)
     const int32_t* tile_expert; const int32_t* n_tiles;
+    // real rows of an expert and its first row: 64-row pieces of a tile that hold padding only are left out (nothing
+    // reads them: the weight gradients below stop at the last real row).  Null where rows come in segments.
+    const int32_t* counts; const int32_t* padded_offsets;
     int K, Nout;
 };
 
-template <typename TAct, typename TW, int EPI>
-__global__ void __launch_bounds__(256) simt_rows_kernel(RowsArgs a)
+template <int EPI, int KS> constexpr size_t rows_smem()
 {
-    __shared__ __align__(16) float As[TK][TM + 4];
-    __shared__ __align__(16) float Bs[TK][TN + 4];
+    constexpr size_t ops = (size_t)KS * 2 * (EPI == EPI_GATEUP ? 3 : 2) * OPER * sizeof(float);
+    constexpr size_t red = (size_t)(KS - 1) * (EPI == EPI_GATEUP ? 2 : 1) * TM * TN * sizeof(float);
+    return ops > red ? ops : red;
+}
+
+template <typename TAct, typename TW, int EPI, int KS, bool VEC>
+__global__ void __launch_bounds__(GT * KS) simt_rows_kernel(RowsArgs a)
+{
+    extern __shared__ __align__(16) float sm[];
+    pdl_wait();
+    constexpr bool BK_MAJOR = EPI == EPI_DHH || EPI == EPI_DXG;      // B(k, n) at n*K + k
+    constexpr int NOP = EPI == EPI_GATEUP ? 3 : 2;
     const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
     const int rows = *a.n_tiles * ROW_TILE;
     if (m0 >= rows) return;
     const int e = a.tile_expert[m0 / ROW_TILE];
+    if (a.counts && m0 - a.padded_offsets[e] >= a.counts[e]) return;
+    const int group = threadIdx.x / GT, t = threadIdx.x % GT;
+    const int tx = t & 15, ty = t >> 4;
     const int K = a.K, N = a.Nout;
-    const TAct* A = (const TAct*)a.A;
-    const TW* B = (const TW*)a.B[e];
-    float acc[4][4] = {}, acc2[4][4] = {};
-    if (EPI == EPI_GATEUP) {           // B = Wg, B2 = Wu, both [K=C, N=H] row-major
-        tile_mac(A, (long)K, 1L, m0, rows, B, (long)N, 1L, n0, N, K, acc, As, Bs);
-        tile_mac(A, (long)K, 1L, m0, rows, (const TW*)a.B2[e], (long)N, 1L, n0, N, K, acc2, As, Bs);
-    } else if (EPI == EPI_DOWN) {      // B = Wd [K=H, N=C]
-        tile_mac(A, (long)K, 1L, m0, rows, B, (long)N, 1L, n0, N, K, acc, As, Bs);
-    } else if (EPI == EPI_DHH) {       // B(k=c, n=h) = Wd[h*C + c]
-        tile_mac(A, (long)K, 1L, m0, rows, B, 1L, (long)K, n0, N, K, acc, As, Bs);
-    } else {                           // dXg = dG*Wg^T + dU*Wu^T ; B(k=h, n=c) = W[c*H + h]
-        tile_mac(A, (long)K, 1L, m0, rows, B, 1L, (long)K, n0, N, K, acc, As, Bs);
-        tile_mac((const TAct*)a.A2, (long)K, 1L, m0, rows, (const TW*)a.B2[e], 1L, (long)K, n0, N, K, acc, As, Bs);
+    float* S = sm + (size_t)group * 2 * NOP * OPER;
+    float acc[8][4] = {}, acc2[8][4] = {};
+    // this group's steps of TK; EPI_DXG runs through dG*Wg^T and then dU*Wu^T
+    const int per = (K + TK - 1) / TK, steps = EPI == EPI_DXG ? 2 * per : per;
+    const int s0 = (int)((long)steps * group / KS), s1 = (int)((long)steps * (group + 1) / KS);
+    const TW *B1 = (const TW*)a.B[e], *B2 = NOP == 3 || EPI == EPI_DXG ? (const TW*)a.B2[e] : nullptr;
+    float4 ra[2], rb[2], rc[2];
+    auto gload = [&](int s) {
+        const bool second = EPI == EPI_DXG && s >= per;
+        const int k0 = (second ? s - per : s) * TK;
+        fetch<TAct, true, true>((const TAct*)(second ? a.A2 : a.A), K, m0, rows, k0, K, t, ra);
+        fetch<TW, BK_MAJOR, VEC>(second ? B2 : B1, BK_MAJOR ? K : N, n0, N, k0, K, t, rb);
+        if (NOP == 3) fetch<TW, BK_MAJOR, VEC>(B2, N, n0, N, k0, K, t, rc);
+    };
+    auto sstore = [&](int buf) {
+        float* d = S + buf * NOP * OPER;
+        put<true>(d, t, ra);
+        put<BK_MAJOR>(d + OPER, t, rb);
+        if (NOP == 3) put<BK_MAJOR>(d + 2 * OPER, t, rc);
+    };
+    if (s0 < s1) {
+        gload(s0);
+        sstore(0);
     }
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + ty * 4 + i;
-        if (m >= rows) continue;
+    group_sync(group);
+    for (int s = s0; s < s1; ++s) {
+        const int buf = (s - s0) & 1;
+        if (s + 1 < s1) gload(s + 1);
+        const float* c = S + buf * NOP * OPER;
+        mac(c, c + OPER, ty, tx, acc);
+        if (NOP == 3) mac(c, c + 2 * OPER, ty, tx, acc2);
+        if (s + 1 < s1) sstore(buf ^ 1);
+        group_sync(group);
+    }
+    fold<KS>(sm, group, t, acc);
+    if (NOP == 3) fold<KS>(sm + (KS - 1) * TM * TN, group, t, acc2);
+    const int n = n0 + tx * 4;
+    if (group > 0 || n >= N) return;
+    float b1[4] = {}, b2[4] = {};
+    if (EPI == EPI_GATEUP || EPI == EPI_DOWN)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx * 4 + j;
-            if (n >= N) continue;
-            const size_t o = (size_t)m * N + n;
+            b1[j] = a.bias[e][n + j];
+            if (EPI == EPI_GATEUP) b2[j] = a.bias2[e][n + j];
+        }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const size_t o = (size_t)(m0 + ty * 8 + i) * N + n;
+        float d[4], d2[4], d3[4];
+        float4 g4, u4;
+        if (EPI == EPI_DHH) {
+            g4 = load4<true>((const TAct*)a.G + o);
+            u4 = load4<true>((const TAct*)a.U + o);
+        }
+        const float gs[4] = {g4.x, g4.y, g4.z, g4.w}, us[4] = {u4.x, u4.y, u4.z, u4.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
             if (EPI == EPI_GATEUP) {
-                // layers/SwiGLU.cpp:32-40, utils/Tensor.cpp:1997-2002
-                const float g = acc[i][j] + a.bias[e][n], u = acc2[i][j] + a.bias2[e][n];
-                // downstream stages read the stored (rounded) values, so round first
-                const TAct gs = from_f32<TAct>(g), us = from_f32<TAct>(u);
-                const float gr = to_f32(gs), ur = to_f32(us);
-                ((TAct*)a.D)[o] = gs;
-                ((TAct*)a.D2)[o] = us;
-                ((TAct*)a.D3)[o] = from_f32<TAct>((gr / (1.0f + expf(-gr))) * ur);
+                // layers/SwiGLU.cpp:32-40, utils/Tensor.cpp:1997-2002; downstream stages read the stored (rounded)
+                // values, so round first
+                d[j] = round_to(acc[i][j] + b1[j], TAct());
+                d2[j] = round_to(acc2[i][j] + b2[j], TAct());
+                d3[j] = __fdiv_rn(d[j], 1.0f + expf(-d[j])) * d2[j];
             } else if (EPI == EPI_DOWN) {
-                ((TAct*)a.D)[o] = from_f32<TAct>(acc[i][j] + a.bias[e][n]);
+                d[j] = acc[i][j] + b1[j];
             } else if (EPI == EPI_DHH) {
                 // utils/Tensor.cpp:2020-2027
-                const float dd = acc[i][j];
-                const float g = to_f32(((const TAct*)a.G)[o]), u = to_f32(((const TAct*)a.U)[o]);
+                const float dd = acc[i][j], g = gs[j], u = us[j];
                 const float sig = 1.0f / (1.0f + expf(-g));
-                ((TAct*)a.D)[o] = from_f32<TAct>((dd * u) * (sig * (1.0f + g * (1.0f - sig))));   // dG
-                ((TAct*)a.D2)[o] = from_f32<TAct>(dd * (g * sig));                                 // dU
+                d[j] = (dd * u) * (sig * (1.0f + g * (1.0f - sig)));      // dG
+                d2[j] = dd * (g * sig);                                   // dU
             } else {
-                ((TAct*)a.D)[o] = from_f32<TAct>(acc[i][j]);
+                d[j] = acc[i][j];
             }
         }
+        store4((TAct*)a.D + o, make_float4(d[0], d[1], d[2], d[3]));
+        if (EPI == EPI_GATEUP || EPI == EPI_DHH) store4((TAct*)a.D2 + o, make_float4(d2[0], d2[1], d2[2], d2[3]));
+        if (EPI == EPI_GATEUP) store4((TAct*)a.D3 + o, make_float4(d3[0], d3[1], d3[2], d3[3]));
     }
 }
 
-// grad[e][m,n] += sum over the expert's rows p of A[p,m] * B[p,n]
-// (layers/LinearLayer.cpp:60-66: dW = X^T * dOut, accumulated like Tensor::add_grad).
+// grad[e][m,n] += sum over the expert's rows p of A[p,m] * B[p,n], and the bias gradient that is the column sum of B
+// (layers/LinearLayer.cpp:56-66: dW = X^T * dOut, db = sum of dOut, accumulated like Tensor::add_grad).  One launch for
+// the three weights of every expert: gWg = Xg^T dG, gWu = Xg^T dU, gWd = Hh^T dYg.
 struct WgradArgs {
-    const void* A; int lda;      // [rows, M]
-    const void* B; int ldb;      // [rows, N]
-    float* const* grad;          // per expert [M, N]
+    const void* Xg; const void* Hh; const void* dG; const void* dU; const void* dYg;
+    float* const* grad[3];       // per expert: gWg, gWu [C,H], gWd [H,C]
+    float* const* gb[3];         // per expert: gbg, gbu [H], gbd [C]
     const int32_t* padded_offsets;
-    int M, N;
+    const int32_t* counts;       // real rows per expert; null: every row of the padded segment is summed (zeros add nothing)
+    int C, H;
     const int32_t* seg;          // [E][n_seg][2] {first row, rows} when an expert's rows come in several segments
     int n_seg;
 };
 
-template <typename TAct>
-__global__ void __launch_bounds__(256) simt_wgrad_kernel(WgradArgs a)
+template <int KS> constexpr size_t wgrad_smem()
 {
-    __shared__ __align__(16) float As[TK][TM + 4];
-    __shared__ __align__(16) float Bs[TK][TN + 4];
-    const int e = blockIdx.z;
-    const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
-    float acc[4][4] = {};
+    constexpr size_t ops = (size_t)KS * 4 * OPER * sizeof(float);
+    constexpr size_t red = ((size_t)(KS - 1) * TM * TN + KS * TN) * sizeof(float);
+    return ops > red ? ops : red;
+}
+
+template <typename TAct, int KS, bool VEC>
+__global__ void __launch_bounds__(GT * KS) simt_wgrad_kernel(WgradArgs a)
+{
+    extern __shared__ __align__(16) float sm[];
+    pdl_wait();
+    const int e = blockIdx.y / 3, which = blockIdx.y % 3;
+    const int M = which == 2 ? a.H : a.C, N = which == 2 ? a.C : a.H;
+    const int mt = (M + TM - 1) / TM, m0 = blockIdx.x % mt * TM, n0 = blockIdx.x / mt * TN;
+    const TAct* A = (const TAct*)(which == 2 ? a.Hh : a.Xg);
+    const TAct* B = (const TAct*)(which == 0 ? a.dG : which == 1 ? a.dU : a.dYg);
+    const int group = threadIdx.x / GT, t = threadIdx.x % GT;
+    const int tx = t & 15, ty = t >> 4;
+    const bool bias = m0 == 0;                 // this CTA also sums its columns of B
+    float* S = sm + (size_t)group * 4 * OPER;
+    float acc[8][4] = {}, bs[4] = {};
     const int nseg = a.n_seg > 0 ? a.n_seg : 1;
     int total = 0;
     for (int sgi = 0; sgi < nseg; ++sgi) {
         const int r0 = a.n_seg > 0 ? a.seg[(e * a.n_seg + sgi) * 2] : a.padded_offsets[e];
-        const int len = a.n_seg > 0 ? a.seg[(e * a.n_seg + sgi) * 2 + 1] : a.padded_offsets[e + 1] - r0;
+        const int len = a.n_seg > 0 ? a.seg[(e * a.n_seg + sgi) * 2 + 1] : a.counts ? a.counts[e] : a.padded_offsets[e + 1] - r0;
         if (len <= 0) continue;               // uniform over the CTA
         total += len;
-        const TAct* A = (const TAct*)a.A + (size_t)r0 * a.lda;
-        const TAct* B = (const TAct*)a.B + (size_t)r0 * a.ldb;
-        tile_mac(A, 1L, (long)a.lda, m0, a.M, B, (long)a.ldb, 1L, n0, a.N, len, acc, As, Bs);
-    }
-    if (total == 0) return;
-    float* g = a.grad[e];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+        const int steps = (len + TK - 1) / TK;
+        const int s0 = (int)((long)steps * group / KS), s1 = (int)((long)steps * (group + 1) / KS);
+        const TAct *As = A + (size_t)r0 * M, *Bs = B + (size_t)r0 * N;
+        float4 ra[2], rb[2];
+        auto gload = [&](int s) {
+            fetch<TAct, false, true>(As, M, m0, M, s * TK, len, t, ra);
+            fetch<TAct, false, true>(Bs, N, n0, N, s * TK, len, t, rb);
+        };
+        auto sstore = [&](int buf) {
+            put<false>(S + buf * 2 * OPER, t, ra);
+            put<false>(S + buf * 2 * OPER + OPER, t, rb);
+        };
+        if (s0 < s1) {
+            gload(s0);
+            sstore(0);
+        }
+        group_sync(group);
+        for (int s = s0; s < s1; ++s) {
+            const int buf = (s - s0) & 1;
+            if (s + 1 < s1) gload(s + 1);
+            const float* c = S + buf * 2 * OPER;
+            mac(c, c + OPER, ty, tx, acc);
+            if (bias && ty == 0)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + ty * 4 + i;
-        if (m >= a.M) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx * 4 + j;
-            if (n < a.N) g[(size_t)m * a.N + n] += acc[i][j];
+                for (int k = 0; k < TK; ++k) {
+                    const float4 b = *reinterpret_cast<const float4*>(c + OPER + k * SROW + tx * 4);
+                    bs[0] += b.x; bs[1] += b.y; bs[2] += b.z; bs[3] += b.w;
+                }
+            if (s + 1 < s1) sstore(buf ^ 1);
+            group_sync(group);
         }
     }
+    if (total == 0) return;
+    fold<KS>(sm, group, t, acc);
+    const int n = n0 + tx * 4;
+    if (bias) {
+        float* sb = sm + (KS - 1) * TM * TN;
+        if (KS == 1) __syncthreads();         // (more groups: fold has waited for the last reads of the operand buffers)
+        if (ty == 0) *reinterpret_cast<float4*>(sb + group * TN + tx * 4) = make_float4(bs[0], bs[1], bs[2], bs[3]);
+        __syncthreads();
+        if (threadIdx.x < TN && n0 + (int)threadIdx.x < N) {
+            float v = 0.0f;
+            for (int g = 0; g < KS; ++g) v += sb[g * TN + threadIdx.x];
+            a.gb[which][e][n0 + threadIdx.x] += v;
+        }
+    }
+    if (group > 0 || n >= N) return;
+    float* g = a.grad[which][e];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int m = m0 + ty * 8 + i;
+        if (m >= M) break;
+        float* p = g + (size_t)m * N + n;
+        if (VEC) {
+            float4 v = *reinterpret_cast<const float4*>(p);
+            v.x += acc[i][0]; v.y += acc[i][1]; v.z += acc[i][2]; v.w += acc[i][3];
+            *reinterpret_cast<float4*>(p) = v;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) p[j] += acc[i][j];
+        }
+    }
+}
+
+// K groups per tile: enough that ~8 warps (four per group) fall to every SM, at most four, and no group with less than
+// two steps.
+int split_k(int tiles, int k)
+{
+    int ks = tiles * 4 < 400 ? 4 : tiles * 4 < 800 ? 2 : 1;
+    while (ks > 1 && k < ks * 2 * TK) ks /= 2;
+    return ks;
+}
+
+template <typename TAct, typename TW, int EPI, int KS>
+int launch_rows_ks(const mgpt_moe_layer* L, const RowsArgs& a, dim3 grid, cudaStream_t st)
+{
+    constexpr size_t smem = rows_smem<EPI, KS>();
+    auto* kernel = L->masters_aligned ? simt_rows_kernel<TAct, TW, EPI, KS, true> : simt_rows_kernel<TAct, TW, EPI, KS, false>;
+    if (smem > 48 * 1024) MGPT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MGPT_CUDA(launch_pdl(kernel, grid, GT * KS, smem, st, a));
+    return 0;
+}
+template <typename TAct, typename TW, int EPI>
+int launch_rows(const mgpt_moe_layer* L, const Workspace& w, const RowsArgs& a, cudaStream_t st, const char* what)
+{
+    const int cols = (a.Nout + TN - 1) / TN;
+    // tiles with real rows: about R/64 and half a tile per expert
+    const int ks = split_k((w.R / TM + (L->d.E + 1) / 2) * cols, EPI == EPI_DXG ? 2 * a.K : a.K);
+    const dim3 grid(w.row_cap / TM, cols);
+    if (ks == 4) MGPT_TRY((launch_rows_ks<TAct, TW, EPI, 4>(L, a, grid, st)));
+    else if (ks == 2) MGPT_TRY((launch_rows_ks<TAct, TW, EPI, 2>(L, a, grid, st)));
+    else MGPT_TRY((launch_rows_ks<TAct, TW, EPI, 1>(L, a, grid, st)));
+    MGPT_LAUNCHED(what);
+    return 0;
+}
+template <typename TAct, int KS>
+int launch_wgrad_ks(const mgpt_moe_layer* L, const WgradArgs& a, dim3 grid, cudaStream_t st)
+{
+    constexpr size_t smem = wgrad_smem<KS>();
+    auto* kernel = L->masters_aligned ? simt_wgrad_kernel<TAct, KS, true> : simt_wgrad_kernel<TAct, KS, false>;
+    if (smem > 48 * 1024) MGPT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MGPT_CUDA(launch_pdl(kernel, grid, GT * KS, smem, st, a));
+    return 0;
+}
+
+// Real rows per expert and the start of its segment, for the kernels that leave padding out: in FP32 mode, where an
+// expert's rows are one padded segment.  (With BF16 data these products are the cross-check of the tensor-core ones and
+// compute the padding rows as those do.)
+void rows_of_experts(const mgpt_moe_layer* L, const Workspace& w, char* ws, const int32_t*& counts, const int32_t*& padded_offsets)
+{
+    if (w.act_bytes != 4 || L->n_seg > 0) return;
+    counts = (const int32_t*)(ws + w.counts);
+    padded_offsets = (const int32_t*)(ws + w.padded_offsets);
 }
 
 template <typename TAct, typename TW>
@@ -180,18 +396,17 @@ int experts_forward_t(mgpt_moe_layer* L, const ExpertPtrs& P, const Workspace& w
     RowsArgs a = {};
     a.tile_expert = (const int32_t*)(ws + w.tile_expert);
     a.n_tiles = (const int32_t*)(ws + w.n_tiles);
+    rows_of_experts(L, w, ws, a.counts, a.padded_offsets);
     // gate/up + SwiGLU
     a.A = buf_Xg(L, w, ws); a.B = P.Wg; a.B2 = P.Wu; a.bias = P.bg; a.bias2 = P.bu;
     a.D = ws + w.G; a.D2 = ws + w.U; a.D3 = ws + w.Hh; a.K = d.C; a.Nout = d.H;
     L->stage_begin(ST_GATEUP, st);
-    simt_rows_kernel<TAct, TW, EPI_GATEUP><<<dim3(w.row_cap / TM, (d.H + TN - 1) / TN), 256, 0, st>>>(a);
-    MGPT_LAUNCHED("simt_rows_kernel<gateup>");
+    MGPT_TRY((launch_rows<TAct, TW, EPI_GATEUP>(L, w, a, st, "simt_rows_kernel<gateup>")));
     L->stage_end(ST_GATEUP, st);
     // down
     a.A = ws + w.Hh; a.B = P.Wd; a.bias = P.bd; a.D = buf_Yg(L, w, ws); a.K = d.H; a.Nout = d.C;
     L->stage_begin(ST_DOWN, st);
-    simt_rows_kernel<TAct, TW, EPI_DOWN><<<dim3(w.row_cap / TM, (d.C + TN - 1) / TN), 256, 0, st>>>(a);
-    MGPT_LAUNCHED("simt_rows_kernel<down>");
+    MGPT_TRY((launch_rows<TAct, TW, EPI_DOWN>(L, w, a, st, "simt_rows_kernel<down>")));
     L->stage_end(ST_DOWN, st);
     return 0;
 }
@@ -203,39 +418,36 @@ int experts_backward_t(mgpt_moe_layer* L, const ExpertPtrs& P, const Workspace& 
     RowsArgs a = {};
     a.tile_expert = (const int32_t*)(ws + w.tile_expert);
     a.n_tiles = (const int32_t*)(ws + w.n_tiles);
+    rows_of_experts(L, w, ws, a.counts, a.padded_offsets);
     // dHh = dYg * Wd^T, fused SwiGLU backward -> dG, dU
     a.A = buf_dYg(L, w, ws); a.B = P.Wd; a.G = ws + w.G; a.U = ws + w.U; a.D = ws + w.dG; a.D2 = ws + w.dU;
     a.K = d.C; a.Nout = d.H;
     L->stage_begin(ST_DHH, st);
-    simt_rows_kernel<TAct, TW, EPI_DHH><<<dim3(w.row_cap / TM, (d.H + TN - 1) / TN), 256, 0, st>>>(a);
-    MGPT_LAUNCHED("simt_rows_kernel<dhh>");
+    MGPT_TRY((launch_rows<TAct, TW, EPI_DHH>(L, w, a, st, "simt_rows_kernel<dhh>")));
     L->stage_end(ST_DHH, st);
     // dXg = dG * Wg^T + dU * Wu^T
     a.A = ws + w.dG; a.A2 = ws + w.dU; a.B = P.Wg; a.B2 = P.Wu; a.D = buf_dXg(L, w, ws); a.K = d.H; a.Nout = d.C;
     L->stage_begin(ST_DXG, st);
-    simt_rows_kernel<TAct, TW, EPI_DXG><<<dim3(w.row_cap / TM, (d.C + TN - 1) / TN), 256, 0, st>>>(a);
-    MGPT_LAUNCHED("simt_rows_kernel<dxg>");
+    MGPT_TRY((launch_rows<TAct, TW, EPI_DXG>(L, w, a, st, "simt_rows_kernel<dxg>")));
     L->stage_end(ST_DXG, st);
     if (!L->has_grad) return 0;
     L->stage_begin(ST_WGRAD, st);
-    const int32_t* poff = (const int32_t*)(ws + w.padded_offsets);
     WgradArgs g = {};
-    g.padded_offsets = poff;
+    g.Xg = buf_Xg(L, w, ws); g.Hh = ws + w.Hh; g.dG = ws + w.dG; g.dU = ws + w.dU; g.dYg = buf_dYg(L, w, ws);
+    g.grad[0] = L->master.gWg; g.grad[1] = L->master.gWu; g.grad[2] = L->master.gWd;
+    g.gb[0] = L->master.gbg; g.gb[1] = L->master.gbu; g.gb[2] = L->master.gbd;
+    g.padded_offsets = (const int32_t*)(ws + w.padded_offsets);
+    const int32_t* ignored = nullptr;
+    rows_of_experts(L, w, ws, g.counts, ignored);
+    g.C = d.C; g.H = d.H;
     g.seg = (const int32_t*)(ws + w.seg); g.n_seg = L->n_seg;
-    // dWg += Xg^T dG ; dWu += Xg^T dU   [C,H]
-    g.A = buf_Xg(L, w, ws); g.lda = d.C; g.M = d.C; g.N = d.H; g.ldb = d.H;
-    dim3 gCH((d.C + TM - 1) / TM, (d.H + TN - 1) / TN, d.E);
-    g.B = ws + w.dG; g.grad = L->master.gWg;
-    simt_wgrad_kernel<TAct><<<gCH, 256, 0, st>>>(g);
-    MGPT_LAUNCHED("simt_wgrad_kernel<Wg>");
-    g.B = ws + w.dU; g.grad = L->master.gWu;
-    simt_wgrad_kernel<TAct><<<gCH, 256, 0, st>>>(g);
-    MGPT_LAUNCHED("simt_wgrad_kernel<Wu>");
-    // dWd += Hh^T dYg   [H,C]
-    g.A = ws + w.Hh; g.lda = d.H; g.M = d.H; g.B = buf_dYg(L, w, ws); g.ldb = d.C; g.N = d.C; g.grad = L->master.gWd;
-    dim3 gHC((d.H + TM - 1) / TM, (d.C + TN - 1) / TN, d.E);
-    simt_wgrad_kernel<TAct><<<gHC, 256, 0, st>>>(g);
-    MGPT_LAUNCHED("simt_wgrad_kernel<Wd>");
+    const int per = ((d.C + TM - 1) / TM) * ((d.H + TM - 1) / TM);
+    const dim3 grid(per, 3 * d.E);
+    const int ks = split_k(per * 3 * d.E, w.R / d.E);
+    if (ks == 4) MGPT_TRY((launch_wgrad_ks<TAct, 4>(L, g, grid, st)));
+    else if (ks == 2) MGPT_TRY((launch_wgrad_ks<TAct, 2>(L, g, grid, st)));
+    else MGPT_TRY((launch_wgrad_ks<TAct, 1>(L, g, grid, st)));
+    MGPT_LAUNCHED("simt_wgrad_kernel");
     L->stage_end(ST_WGRAD, st);
     return 0;
 }

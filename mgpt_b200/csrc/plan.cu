@@ -396,7 +396,6 @@ struct BiasGradArgs {
     const int32_t* n_tiles;
 };
 
-template <typename TAct>
 __global__ void __launch_bounds__(256) bias_grad_kernel(BiasGradArgs a)
 {
     pdl_wait();
@@ -408,22 +407,16 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(BiasGradArgs a)
     const int c = blockIdx.y * 256 + tx * 8;
     float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (c < cols) {
-        const TAct* base = (const TAct*)a.M[which] + (size_t)tile * ROW_TILE * cols + c;
+        const bf16* base = (const bf16*)a.M[which] + (size_t)tile * ROW_TILE * cols + c;
 #pragma unroll 4
         for (int r = ty; r < ROW_TILE; r += 8) {
-            const TAct* p = base + (size_t)r * cols;
-            if constexpr (sizeof(TAct) == 2) {
-                const uint4 u = *reinterpret_cast<const uint4*>(p);
-                const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+            const bf16* p = base + (size_t)r * cols;
+            const uint4 u = *reinterpret_cast<const uint4*>(p);
+            const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    s[2 * i] += __uint_as_float(w[i] << 16);
-                    s[2 * i + 1] += __uint_as_float(w[i] & 0xffff0000u);
-                }
-            } else {
-                const float4 f0 = *reinterpret_cast<const float4*>(p), f1 = *reinterpret_cast<const float4*>(p + 4);
-                s[0] += f0.x; s[1] += f0.y; s[2] += f0.z; s[3] += f0.w;
-                s[4] += f1.x; s[5] += f1.y; s[6] += f1.z; s[7] += f1.w;
+            for (int i = 0; i < 4; ++i) {
+                s[2 * i] += __uint_as_float(w[i] << 16);
+                s[2 * i + 1] += __uint_as_float(w[i] & 0xffff0000u);
             }
         }
     }
@@ -568,8 +561,7 @@ int launch_bias_grads(const mgpt_moe_layer* L, const Workspace& w, char* ws, cud
     a.n_tiles = (const int32_t*)(ws + w.n_tiles);
     const int mc = d.C > d.H ? d.C : d.H;
     dim3 grid(w.max_tiles, (mc + 255) / 256, 3);
-    if (w.act_bytes == 4) MGPT_CUDA(launch_pdl(bias_grad_kernel<float>, grid, 256, 0, st, a));
-    else MGPT_CUDA(launch_pdl(bias_grad_kernel<bf16>, grid, 256, 0, st, a));
+    MGPT_CUDA(launch_pdl(bias_grad_kernel, grid, 256, 0, st, a));
     MGPT_LAUNCHED("bias_grad_kernel");
     return 0;
 }

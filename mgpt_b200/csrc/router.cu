@@ -445,31 +445,50 @@ router_dlogits_kernel(const float* __restrict__ probs, const int32_t* __restrict
 // dx[tok,:] = sum_j dXg[pos(tok,j),:] (ascending slot order, as the reference's
 // scatter-add visits them, utils/Tensor.cpp:1451-1458) + dlogits[tok,:] * Wr^T
 // (layers/LinearLayer.cpp:68-69, layers/MoELayer.cpp:217).
-// One CTA: DX_TOK tokens x one channel chunk (8192/E_pad channels, Wr^T of the chunk in shared
-// memory); a thread owns 8 consecutive channels and uses 16-byte accesses.
-constexpr int DX_TOK = 64;
-constexpr int DX_WS_FLOATS = 8192;
-template <typename TAct, typename TIo>
+// One CTA: 64 channels of 32*TPT tokens, a thread owns 8 consecutive channels of TPT tokens; Wr^T of the channels and
+// dlogits^T of the tokens in shared memory.  TPT = 4 where that still gives every SM two CTAs (the products are then 32
+// multiply-adds per three 16-byte shared-memory reads), else 1.  (Whole rows of 64 tokens per CTA left most SMs idle:
+// 25 us at 1024 tokens, C = 128, E = 8 and 30 us at 5003 tokens, C = 512, E = 16.)
+constexpr int DX_CH = 64;
+template <typename TAct> __device__ __forceinline__ void add_row8(float (&s)[8], const TAct* r)
+{
+    if constexpr (sizeof(TAct) == 2) {
+        const uint4 u = *reinterpret_cast<const uint4*>(r);
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            s[2 * i] = __fadd_rn(s[2 * i], __uint_as_float(w[i] << 16));
+            s[2 * i + 1] = __fadd_rn(s[2 * i + 1], __uint_as_float(w[i] & 0xffff0000u));
+        }
+    } else {
+        const float4 a = *reinterpret_cast<const float4*>(r), b = *reinterpret_cast<const float4*>(r + 4);
+        s[0] = __fadd_rn(s[0], a.x); s[1] = __fadd_rn(s[1], a.y); s[2] = __fadd_rn(s[2], a.z); s[3] = __fadd_rn(s[3], a.w);
+        s[4] = __fadd_rn(s[4], b.x); s[5] = __fadd_rn(s[5], b.y); s[6] = __fadd_rn(s[6], b.z); s[7] = __fadd_rn(s[7], b.w);
+    }
+}
+template <int TPT> constexpr size_t dx_smem(int E) { return (size_t)E * (DX_CH + 4 + 32 * TPT) * sizeof(float); }
+
+template <typename TAct, typename TIo, int TPT>
 __global__ void __launch_bounds__(256)
 router_dx_kernel(const TAct* __restrict__ dXg, const int32_t* __restrict__ pos, const float* __restrict__ dlogits,
-                 const float* __restrict__ Wr, int N, int C, int E, int k, int chunk, TIo* __restrict__ dx)
+                 const float* __restrict__ Wr, int N, int C, int E, int k, TIo* __restrict__ dx)
 {
     pdl_wait();
+    constexpr int TOK = 32 * TPT, WS = DX_CH + 4;       // padded row: transposed staging without 32-way conflicts
     extern __shared__ __align__(16) float sm_dx[];
-    const int wstride = chunk + 4;                      // padded row: transposed staging without 32-way conflicts
-    float* wt = sm_dx;                                  // [E][chunk+4]  (Wr^T of this channel chunk)
-    float* dlT = sm_dx + DX_WS_FLOATS + 4 * MAX_EXPERTS;   // [E][DX_TOK]  (dlogits^T of this token tile)
-    __shared__ int spos[DX_TOK][MAX_TOPK];
-    const int tok0 = blockIdx.x * DX_TOK, c_base = blockIdx.y * chunk;
-    for (int i = threadIdx.x; i < chunk * E; i += blockDim.x) {
+    float* wt = sm_dx;                                  // [E][DX_CH+4]  (Wr^T of these channels)
+    float* dlT = sm_dx + E * WS;                        // [E][TOK]  (dlogits^T of these tokens)
+    __shared__ int spos[TOK][MAX_TOPK];
+    const int tok0 = blockIdx.x * TOK, c_base = blockIdx.y * DX_CH;
+    for (int i = threadIdx.x; i < DX_CH * E; i += blockDim.x) {
         const int c = i / E, e = i % E;
-        wt[e * wstride + c] = (c_base + c < C) ? Wr[(size_t)(c_base + c) * E + e] : 0.0f;
+        wt[e * WS + c] = (c_base + c < C) ? Wr[(size_t)c_base * E + i] : 0.0f;
     }
-    for (int i = threadIdx.x; i < DX_TOK * E; i += blockDim.x) {
+    for (int i = threadIdx.x; i < TOK * E; i += blockDim.x) {
         const int t = i / E, e = i % E;
-        dlT[e * DX_TOK + t] = (tok0 + t < N) ? dlogits[(size_t)(tok0 + t) * E + e] : 0.0f;
+        dlT[e * TOK + t] = (tok0 + t < N) ? dlogits[(size_t)tok0 * E + i] : 0.0f;
     }
-    if (threadIdx.x < DX_TOK) {
+    if (threadIdx.x < TOK) {
         const int tok = tok0 + threadIdx.x;
         int v[MAX_TOPK];
 #pragma unroll
@@ -487,63 +506,50 @@ router_dx_kernel(const TAct* __restrict__ dXg, const int32_t* __restrict__ pos, 
         for (int j = 0; j < MAX_TOPK; ++j) spos[threadIdx.x][j] = v[j];
     }
     __syncthreads();
-    const int groups = chunk / 8;                       // 8-channel groups in the chunk
-    const int g = threadIdx.x % groups, ql = threadIdx.x / groups, qstep = blockDim.x / groups;
+    const int g = threadIdx.x & 7, tl0 = (threadIdx.x >> 3) * TPT;
     const int c = c_base + g * 8;
     if (c >= C) return;
-    for (int tq = ql; tq < DX_TOK / 4; tq += qstep) {    // a thread owns 8 channels of 4 consecutive tokens
-        if (tok0 + tq * 4 >= N) break;
-        float acc[4][8];
+    float acc[TPT][8];
 #pragma unroll
-        for (int t = 0; t < 4; ++t)
+    for (int t = 0; t < TPT; ++t)
 #pragma unroll
-            for (int i = 0; i < 8; ++i) acc[t][i] = 0.0f;
-        for (int e = 0; e < E; ++e) {
-            const float4 d = *reinterpret_cast<const float4*>(&dlT[e * DX_TOK + tq * 4]);
-            const float4 w0 = *reinterpret_cast<const float4*>(&wt[e * wstride + g * 8]);
-            const float4 w1 = *reinterpret_cast<const float4*>(&wt[e * wstride + g * 8 + 4]);
-            const float dv[4] = {d.x, d.y, d.z, d.w};
-            const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-#pragma unroll
-            for (int t = 0; t < 4; ++t)
-#pragma unroll
-                for (int i = 0; i < 8; ++i) acc[t][i] = fmaf(dv[t], wv[i], acc[t][i]);
+        for (int i = 0; i < 8; ++i) acc[t][i] = 0.0f;
+#pragma unroll 4
+    for (int e = 0; e < E; ++e) {
+        const float4 w0 = *reinterpret_cast<const float4*>(&wt[e * WS + g * 8]);
+        const float4 w1 = *reinterpret_cast<const float4*>(&wt[e * WS + g * 8 + 4]);
+        const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+        float dv[TPT];
+        if constexpr (TPT == 4) {
+            const float4 d = *reinterpret_cast<const float4*>(&dlT[e * TOK + tl0]);
+            dv[0] = d.x; dv[1] = d.y; dv[2] = d.z; dv[3] = d.w;
+        } else {
+            dv[0] = dlT[e * TOK + tl0];
         }
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            const int tl = tq * 4 + t, tok = tok0 + tl;
-            if (tok >= N) break;
-            float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            for (int j = 0; j < k; ++j) {
-                const TAct* r = dXg + (size_t)spos[tl][j] * C + c;
-                if constexpr (sizeof(TAct) == 2) {
-                    const uint4 u = *reinterpret_cast<const uint4*>(r);
-                    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+        for (int t = 0; t < TPT; ++t)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        s[2 * i] = __fadd_rn(s[2 * i], __uint_as_float(w[i] << 16));
-                        s[2 * i + 1] = __fadd_rn(s[2 * i + 1], __uint_as_float(w[i] & 0xffff0000u));
-                    }
-                } else {
-                    const float4 a = *reinterpret_cast<const float4*>(r), b = *reinterpret_cast<const float4*>(r + 4);
-                    s[0] = __fadd_rn(s[0], a.x); s[1] = __fadd_rn(s[1], a.y); s[2] = __fadd_rn(s[2], a.z); s[3] = __fadd_rn(s[3], a.w);
-                    s[4] = __fadd_rn(s[4], b.x); s[5] = __fadd_rn(s[5], b.y); s[6] = __fadd_rn(s[6], b.z); s[7] = __fadd_rn(s[7], b.w);
-                }
-            }
+            for (int i = 0; i < 8; ++i) acc[t][i] = fmaf(dv[t], wv[i], acc[t][i]);
+    }
 #pragma unroll
-            for (int i = 0; i < 8; ++i) s[i] = __fadd_rn(s[i], acc[t][i]);
-            TIo* o = dx + (size_t)tok * C + c;
-            if constexpr (sizeof(TIo) == 4) {
-                *reinterpret_cast<float4*>(o) = make_float4(s[0], s[1], s[2], s[3]);
-                *reinterpret_cast<float4*>(o + 4) = make_float4(s[4], s[5], s[6], s[7]);
-            } else {
-                uint4 u;
-                __nv_bfloat162 h0 = __floats2bfloat162_rn(s[0], s[1]), h1 = __floats2bfloat162_rn(s[2], s[3]);
-                __nv_bfloat162 h2 = __floats2bfloat162_rn(s[4], s[5]), h3 = __floats2bfloat162_rn(s[6], s[7]);
-                u.x = *reinterpret_cast<uint32_t*>(&h0); u.y = *reinterpret_cast<uint32_t*>(&h1);
-                u.z = *reinterpret_cast<uint32_t*>(&h2); u.w = *reinterpret_cast<uint32_t*>(&h3);
-                *reinterpret_cast<uint4*>(o) = u;
-            }
+    for (int t = 0; t < TPT; ++t) {
+        const int tl = tl0 + t, tok = tok0 + tl;
+        if (tok >= N) break;
+        float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        for (int j = 0; j < k; ++j) add_row8(s, dXg + (size_t)spos[tl][j] * C + c);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s[i] = __fadd_rn(s[i], acc[t][i]);
+        TIo* o = dx + (size_t)tok * C + c;
+        if constexpr (sizeof(TIo) == 4) {
+            *reinterpret_cast<float4*>(o) = make_float4(s[0], s[1], s[2], s[3]);
+            *reinterpret_cast<float4*>(o + 4) = make_float4(s[4], s[5], s[6], s[7]);
+        } else {
+            uint4 u;
+            __nv_bfloat162 h0 = __floats2bfloat162_rn(s[0], s[1]), h1 = __floats2bfloat162_rn(s[2], s[3]);
+            __nv_bfloat162 h2 = __floats2bfloat162_rn(s[4], s[5]), h3 = __floats2bfloat162_rn(s[6], s[7]);
+            u.x = *reinterpret_cast<uint32_t*>(&h0); u.y = *reinterpret_cast<uint32_t*>(&h1);
+            u.z = *reinterpret_cast<uint32_t*>(&h2); u.w = *reinterpret_cast<uint32_t*>(&h3);
+            *reinterpret_cast<uint4*>(o) = u;
         }
     }
 }
@@ -567,7 +573,8 @@ router_wgrad_partial_kernel(const TIo* __restrict__ x, const float* __restrict__
     const bool c_ok = c < C;
     float acc[4][4] = {};
     float bs[4] = {0, 0, 0, 0};
-    constexpr int UN = 4;                               // tokens in flight per thread
+    constexpr int UN = 8;                               // tokens in flight per thread
+    const bool e_vec = (E & 3) == 0;                    // dlogits in 16-byte pieces
     for (int tb = t0; tb < t1; tb += UN) {
         float xv[UN][4], dv[UN][4];
 #pragma unroll
@@ -586,8 +593,13 @@ router_wgrad_partial_kernel(const TIo* __restrict__ x, const float* __restrict__
                     xv[u][0] = f.x; xv[u][1] = f.y; xv[u][2] = f.z; xv[u][3] = f.w;
                 }
             }
+            if (e_vec) {
+                const float4 f = ok ? *reinterpret_cast<const float4*>(dlogits + (size_t)tok * E + e0) : make_float4(0, 0, 0, 0);
+                dv[u][0] = f.x; dv[u][1] = f.y; dv[u][2] = f.z; dv[u][3] = f.w;
+            } else {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) dv[u][j] = (ok && e0 + j < E) ? dlogits[(size_t)tok * E + e0 + j] : 0.0f;
+                for (int j = 0; j < 4; ++j) dv[u][j] = (ok && e0 + j < E) ? dlogits[(size_t)tok * E + e0 + j] : 0.0f;
+            }
         }
 #pragma unroll
         for (int u = 0; u < UN; ++u) {
@@ -613,21 +625,31 @@ router_wgrad_partial_kernel(const TIo* __restrict__ x, const float* __restrict__
             if (e0 + j < E) partb[(size_t)blockIdx.y * E + e0 + j] = bs[j];
 }
 
+// 32 elements per CTA, the chunks shared out over 8 threads per element (one thread per element walked up to 64 chunks
+// one after another: 6 us for 1024 elements)
 __global__ void __launch_bounds__(256)
 router_wgrad_reduce_kernel(const float* __restrict__ part, const float* __restrict__ partb, int n_chunks, int CE, int E,
                            float* __restrict__ gWr, float* __restrict__ gbr)
 {
     pdl_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < CE) {
-        float s = 0.0f;
-        for (int ch = 0; ch < n_chunks; ++ch) s += part[(size_t)ch * CE + i];
-        gWr[i] += s;
-    }
-    if (i < E) {
-        float s = 0.0f;
-        for (int ch = 0; ch < n_chunks; ++ch) s += partb[(size_t)ch * E + i];
-        gbr[i] += s;
+    __shared__ float red[8][32];
+    const int x = threadIdx.x & 31, slice = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + x;                  // elements CE .. CE+E-1 are the bias gradient
+    const bool bias = i >= CE;
+    const float* src = bias ? partb + (i - CE) : part + i;
+    const size_t stride = bias ? E : CE;
+    float s = 0.0f;
+    if (i < CE + E)
+#pragma unroll 8
+        for (int ch = slice; ch < n_chunks; ch += 8) s += src[(size_t)ch * stride];
+    red[slice][x] = s;
+    __syncthreads();
+    if (slice == 0 && i < CE + E) {
+        float t = 0.0f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) t += red[w][x];
+        if (bias) gbr[i - CE] += t;
+        else gWr[i] += t;
     }
 }
 
@@ -705,6 +727,28 @@ int launch_router_fwd(const void* x, int io, const float* Wr, const float* br, i
     return router_fwd_dispatch((const bf16*)x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, st, list, list_count);
 }
 
+template <int TPT>
+static int launch_router_dx(mgpt_moe_layer* L, const void* dXg, size_t act_bytes, int io, const int32_t* pos, const float* dl,
+                            const float* Wr, int N, int C, int E, int k, void* dx, cudaStream_t st)
+{
+    const dim3 grid((N + 32 * TPT - 1) / (32 * TPT), (C + DX_CH - 1) / DX_CH);
+    const size_t sm = dx_smem<TPT>(E);
+    if (!L->router_dx_attr[TPT == 4]) {             // a per-device attribute: one opt-in per layer (layers live on one device)
+        const int most = (int)dx_smem<TPT>(MAX_EXPERTS);
+        MGPT_CUDA(cudaFuncSetAttribute(router_dx_kernel<float, float, TPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        MGPT_CUDA(cudaFuncSetAttribute(router_dx_kernel<bf16, float, TPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        MGPT_CUDA(cudaFuncSetAttribute(router_dx_kernel<bf16, bf16, TPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        L->router_dx_attr[TPT == 4] = true;
+    }
+    if (act_bytes == 4)
+        MGPT_CUDA(launch_pdl(router_dx_kernel<float, float, TPT>, grid, 256, sm, st, (const float*)dXg, pos, dl, Wr, N, C, E, k, (float*)dx));
+    else if (io == MGPT_MOE_IO_F32)
+        MGPT_CUDA(launch_pdl(router_dx_kernel<bf16, float, TPT>, grid, 256, sm, st, (const bf16*)dXg, pos, dl, Wr, N, C, E, k, (float*)dx));
+    else
+        MGPT_CUDA(launch_pdl(router_dx_kernel<bf16, bf16, TPT>, grid, 256, sm, st, (const bf16*)dXg, pos, dl, Wr, N, C, E, k, (bf16*)dx));
+    return 0;
+}
+
 int launch_router_bwd(mgpt_moe_layer* L, const Workspace& w, char* ws, const void* x, int io,
                       void* dx, cudaStream_t st, const void* dXg_rows, const int32_t* pos_rows)
 {
@@ -735,24 +779,9 @@ int launch_router_bwd(mgpt_moe_layer* L, const Workspace& w, char* ws, const voi
     if (tc) {
         MGPT_TRY(tc_router_dx(L, w, ws, dXg, pos, dx, st));
     } else {
-        int epad = 8;
-        while (epad < E) epad <<= 1;
-        const int chunk = DX_WS_FLOATS / epad;                 // channels per CTA (multiple of 8)
-        dim3 grid((N + DX_TOK - 1) / DX_TOK, (C + chunk - 1) / chunk);
-        const size_t sm = (size_t)(DX_WS_FLOATS + 4 * MAX_EXPERTS + DX_TOK * E) * sizeof(float);
-        if (!L->router_dx_attr) {                   // a per-device attribute: one opt-in per layer (layers live on one device)
-            MGPT_CUDA(cudaFuncSetAttribute(router_dx_kernel<float, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024));
-            MGPT_CUDA(cudaFuncSetAttribute(router_dx_kernel<bf16, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024));
-            MGPT_CUDA(cudaFuncSetAttribute(router_dx_kernel<bf16, bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024));
-            L->router_dx_attr = true;
-        }
-        if (w.act_bytes == 4) {
-            MGPT_CUDA(launch_pdl(router_dx_kernel<float, float>, grid, 256, sm, st, (const float*)dXg, pos, dl, Wr, N, C, E, k, chunk, (float*)dx));
-        } else if (io == MGPT_MOE_IO_F32) {
-            MGPT_CUDA(launch_pdl(router_dx_kernel<bf16, float>, grid, 256, sm, st, (const bf16*)dXg, pos, dl, Wr, N, C, E, k, chunk, (float*)dx));
-        } else {
-            MGPT_CUDA(launch_pdl(router_dx_kernel<bf16, bf16>, grid, 256, sm, st, (const bf16*)dXg, pos, dl, Wr, N, C, E, k, chunk, (bf16*)dx));
-        }
+        const int cols = (C + DX_CH - 1) / DX_CH;
+        if ((N + 127) / 128 * cols >= 2 * 148) MGPT_TRY(launch_router_dx<4>(L, dXg, w.act_bytes, io, pos, dl, Wr, N, C, E, k, dx, st));
+        else MGPT_TRY(launch_router_dx<1>(L, dXg, w.act_bytes, io, pos, dl, Wr, N, C, E, k, dx, st));
         MGPT_LAUNCHED("router_dx_kernel");
     }
     if (tc_wgrad) {
@@ -769,7 +798,7 @@ int launch_router_bwd(mgpt_moe_layer* L, const Workspace& w, char* ws, const voi
         else
             MGPT_CUDA(launch_pdl(router_wgrad_partial_kernel<bf16>, grid, 256, 0, st, (const bf16*)x, dl, N, C, E, tpc, part, partb));
         MGPT_LAUNCHED("router_wgrad_partial_kernel");
-        MGPT_CUDA(launch_pdl(router_wgrad_reduce_kernel, (C * E + 255) / 256, 256, 0, st, part, partb, w.rw_chunks, C * E, E,
+        MGPT_CUDA(launch_pdl(router_wgrad_reduce_kernel, (C * E + E + 31) / 32, 256, 0, st, part, partb, w.rw_chunks, C * E, E,
                                                                       L->p_grad[0], L->p_grad[1]));
         MGPT_LAUNCHED("router_wgrad_reduce_kernel");
     }

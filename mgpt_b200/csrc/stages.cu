@@ -213,7 +213,7 @@ static int experts_backward_impl(mgpt_moe_layer* L, const void* d_out_rows, void
     } else if (phase & 1) {
         MGPT_TRY(simt_experts_backward(L, w, ws, st));     // the CUDA-core path computes both kinds in one go
     }
-    if ((phase & 2) && L->has_grad && !(tc && tc_fused_bias_grads(d))) {      // else the tensor-core weight-gradient kernel sums them itself
+    if ((phase & 2) && L->has_grad && tc && !tc_fused_bias_grads(d)) {      // the other weight-gradient kernels sum them themselves
         L->stage_begin(ST_BIAS_GRAD, st);
         MGPT_TRY(launch_bias_grads(L, w, ws, st));
         L->stage_end(ST_BIAS_GRAD, st);
