@@ -63,8 +63,6 @@ Workspace make_workspace(const Dims& d, int n_tokens, int kind)
     w.map = take(N * k * 4);
     w.pos = take(N * k * 4);
     w.row_src = take(rc * 4);
-    w.pairs = take((size_t)w.max_tiles * 8);           // part of the plan: inside the range save_routing copies
-    w.n_pairs = take(4);
     w.blk_cnt = take((size_t)w.plan_blocks * E * 4);
     w.slot = take(N * k * 4);
     w.seg = take(E * MAX_SOURCES * 2 * 4);
@@ -188,17 +186,21 @@ int mgpt_moe_create(const mgpt_moe_config* cfg, mgpt_moe_layer** out)
             }
         }
         const size_t n = (size_t)E * C * H;
-        bf16** s[6] = {&L->sWg, &L->sWu, &L->sWd, &L->sWgT, &L->sWuT, &L->sWdT};
-        // the transposed copies are tile-major with zero padding up to whole 128 x 64 blocks
-        const size_t ns[6] = {n, n, n, E * tile_major_elems(H, C), E * tile_major_elems(H, C), E * tile_major_elems(C, H)};
-        for (int i = 0; i < 6; ++i) {
+        // as stored for the CUDA-core products, else transposed and tile-major with zero padding up to whole 128 x 64 blocks
+        const bool tm = cfg->gemm_impl == 0;
+        // (the copies of Wg and Wu in one piece, so that one TMA load brings a block of each)
+        const size_t eCH = tm ? E * tile_major_elems(H, C) : n, eHC = tm ? E * tile_major_elems(C, H) : n;
+        bf16** s[2] = {tm ? &L->sWgT : &L->sWg, tm ? &L->sWdT : &L->sWd};
+        const size_t ns[2] = {2 * eCH, eHC};
+        for (int i = 0; i < 2; ++i) {
             e = cudaMalloc(s[i], ns[i] * sizeof(bf16));
-            if (e == cudaSuccess && i >= 3) e = cudaMemset(*s[i], 0, ns[i] * sizeof(bf16));
+            if (e == cudaSuccess && tm) e = cudaMemset(*s[i], 0, ns[i] * sizeof(bf16));
             if (e != cudaSuccess) {
                 mgpt_moe_destroy(L);
-                return cuda_fail(e, "cudaMalloc(shadows)");
+                return cuda_fail(e, "cudaMalloc(weight copies)");
             }
         }
+        (tm ? L->sWuT : L->sWu) = *s[0] + eCH;
         e = cudaDeviceSynchronize();
         if (e != cudaSuccess) {
             mgpt_moe_destroy(L);
@@ -218,8 +220,8 @@ void mgpt_moe_destroy(mgpt_moe_layer* L)
     cudaFree(L->d_opt);
     cudaFree(L->d_status);
     if (L->h_status) cudaFreeHost(L->h_status);
-    cudaFree(L->sWg); cudaFree(L->sWu); cudaFree(L->sWd);
-    cudaFree(L->sWgT); cudaFree(L->sWuT); cudaFree(L->sWdT);
+    cudaFree(L->sWg); cudaFree(L->sWd);             // (sWu, sWuT lie behind sWg, sWgT)
+    cudaFree(L->sWgT); cudaFree(L->sWdT);
     cudaFree(L->sWr);
     cudaFree(L->sWrT2);
     cudaFree(L->d_rstat);
@@ -308,6 +310,7 @@ int mgpt_moe_bind_optimizer_state(mgpt_moe_layer* L, float* const* m, float* con
     const int E = L->d.E, S = E < 2 ? 2 : E;
     if (!L->d_opt) MGPT_CUDA(cudaMalloc(&L->d_opt, (size_t)16 * S * sizeof(void*)));
     std::vector<void*> h((size_t)16 * S, nullptr);
+    L->opt_aligned = true;
     for (int e = 0; e < E && L->experts_bound; ++e) {
         const int b = 2 + 6 * e;
         const int order[6] = {b + 0, b + 2, b + 4, b + 1, b + 3, b + 5};      // Wg Wu Wd bg bu bd
@@ -315,6 +318,7 @@ int mgpt_moe_bind_optimizer_state(mgpt_moe_layer* L, float* const* m, float* con
             if (!m[order[j]] || !v[order[j]]) return fail(MGPT_MOE_EINVAL, "null optimiser-state pointer");
             h[(size_t)j * S + e] = m[order[j]];
             h[(size_t)(6 + j) * S + e] = v[order[j]];
+            if (((uintptr_t)m[order[j]] | (uintptr_t)v[order[j]]) & 15) L->opt_aligned = false;
         }
     }
     if (L->router_bound) {
@@ -452,8 +456,7 @@ int mgpt_moe_selftest_bounded_wait(mgpt_moe_layer* L, mgpt_stream_t stream)
 }
 
 // Routing results and plan of one forward: the workspace bytes from probs up to (not including) the plan's
-// scratch -- probs, top_idx, top_p, counts, offsets, padded_offsets, tile_expert, n_tiles, status, map, pos, row_src,
-// pairs, n_pairs.
+// scratch -- probs, top_idx, top_p, counts, offsets, padded_offsets, tile_expert, n_tiles, status, map, pos, row_src.
 static size_t routing_begin(const Workspace& w) { return w.probs; }
 static size_t routing_end(const Workspace& w) { return w.blk_cnt; }
 

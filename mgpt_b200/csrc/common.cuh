@@ -98,7 +98,6 @@ struct Workspace {
     // plan
     size_t counts, offsets, padded_offsets, tile_expert, n_tiles, status;
     size_t map, pos, row_src, blk_cnt, slot, seg, tile_order;
-    size_t pairs, n_pairs;      // row tiles two by two within an expert ({first, second or -1}), in processing order
     // forward activations (kept for backward)
     size_t Xg, G, U, Hh, Yg;
     // backward temporaries
@@ -166,12 +165,13 @@ struct mgpt_moe_layer {
     void* d_tables = nullptr;                // one allocation holding all tables
     void* d_opt = nullptr;                   // optimiser-state tables (m, v per tensor kind; router w, g, m, v)
     bool opt_bound = false;
+    bool opt_aligned = false;                // every bound expert moment buffer starts on a 16-byte boundary
     mgpt::ExpertPtrs master;                 // W pointers -> FP32 masters
     mgpt::ExpertPtrs shadow;                 // W pointers -> BF16 shadows (BF16 mode)
 
-    // BF16 shadows, contiguous over experts (BF16 mode only)
-    mgpt::bf16 *sWg = nullptr, *sWu = nullptr, *sWd = nullptr;      // [E][C][H],[E][C][H],[E][H][C]
-    mgpt::bf16 *sWgT = nullptr, *sWuT = nullptr, *sWdT = nullptr;   // transposed copies ([H,C],[H,C],[C,H] per expert), tile-major: see tile_major_index
+    // BF16 copies, contiguous over experts (BF16 mode only): one of the two forms
+    mgpt::bf16 *sWg = nullptr, *sWu = nullptr, *sWd = nullptr;      // gemm_impl 1: as stored, [E][C][H],[E][C][H],[E][H][C]
+    mgpt::bf16 *sWgT = nullptr, *sWuT = nullptr, *sWdT = nullptr;   // gemm_impl 0: transposed ([H,C],[H,C],[C,H] per expert), tile-major: see tile_major_index
     mgpt::bf16* sWr = nullptr;                                      // router weight [C][E8], E8 = E rounded up to 8
     mgpt::bf16* sWrT2 = nullptr;     // router weight transposed and split in two BF16 pieces: [2][NE][C], Wr^T ~ hi + mid
     float* d_rstat = nullptr;        // {max_e ||Wr[:,e]||_2, max_e |br[e]|}, slightly inflated (screened router's error bound)
@@ -238,7 +238,6 @@ int launch_router_fwd(const void* x, int io, const float* Wr, const float* br, i
 // routing the first pass cannot prove
 bool tc_router_usable(const mgpt_moe_layer* L, const void* x, int io, int n_tokens);
 int tc_router_fwd(mgpt_moe_layer* L, const Workspace& w, char* ws, const void* x, cudaStream_t st);
-int launch_router_pieces(mgpt_moe_layer* L, cudaStream_t st);
 int router_tc_ne(int E);
 int launch_router_bwd(mgpt_moe_layer* L, const Workspace& w, char* ws, const void* x, int io,
                       void* dx, cudaStream_t st, const void* dXg_rows = nullptr, const int32_t* pos_rows = nullptr);
@@ -262,7 +261,7 @@ int combine_rows_backward(const void* dy, int io, const void* rows, const int32_
 int run_plan(const int32_t* top_idx, int R, int E, int32_t* counts, int32_t* offsets, int32_t* padded_offsets,
              int32_t* tile_expert, int32_t* n_tiles, int max_tiles, int32_t* map, int32_t* pos,
              int32_t* row_src, int row_cap, int32_t* status, int32_t* blk, cudaStream_t st, int32_t* slot_of,
-             int32_t* sticky, int32_t* pairs, int32_t* n_pairs);
+             int32_t* sticky);
 
 // gemm_simt.cu
 int simt_experts_forward(mgpt_moe_layer* L, const Workspace& w, char* ws, cudaStream_t st);
@@ -276,7 +275,6 @@ bool tc_fused_bias_grads(const Dims& d);
 int tc_selftest_bounded_wait(mgpt_moe_layer* L, cudaStream_t st);
 void tc_destroy(mgpt_moe_layer* L);
 void host_pipe_destroy(mgpt_moe_layer* L);          // frees the staging of mgpt_moe_step_host_async (waits for steps in flight)
-int launch_sync_router_only(mgpt_moe_layer* L, cudaStream_t st);
 int launch_adamw(mgpt_moe_layer* L, float lr, float beta1, float beta2, float eps, float weight_decay, int t,
                  cudaStream_t st, float grad_clip = 0.0f, int skip_nonfinite = 0);
 int tc_router_dx(mgpt_moe_layer* L, const Workspace& w, char* ws, const void* dXg, const int32_t* pos, void* dx,
@@ -285,5 +283,7 @@ int tc_router_wgrad(mgpt_moe_layer* L, const Workspace& w, char* ws, const void*
 
 // weights.cu
 int launch_sync_weights(mgpt_moe_layer* L, cudaStream_t st);
+int launch_router_copies(mgpt_moe_layer* L, bool stat_clear, cudaStream_t st);
+int launch_weight_copies(mgpt_moe_layer* L, cudaStream_t st);      // adamw.cu
 
 }  // namespace mgpt

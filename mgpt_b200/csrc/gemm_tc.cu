@@ -22,9 +22,6 @@
 // Every wait on an mbarrier is bounded; a wait that runs out sets a bit in the
 // workspace status word and the CTA leaves through its normal teardown
 // (TMEM is released), so a fault in a descriptor cannot hang the device.
-#include <cstdio>
-#include <cstdlib>
-
 #include "tc_common.cuh"
 
 namespace mgpt {
@@ -36,6 +33,7 @@ constexpr uint32_t A_BYTES = BM * BK * 2;            // 16 KiB
 constexpr uint32_t B_BYTES = BN * BK * 2;            // 32 KiB
 constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;  // 48 KiB
 constexpr uint32_t HALF_B = B_BYTES / 2;
+constexpr uint32_t BOX_BYTES = 64 * BK * 2;          // one {64 MN elements, 64 reduction rows} box of an MN-major operand: 8 KiB
 constexpr int EPI_WARPS = 16;                        // four per TMEM lane quarter
 constexpr uint32_t STAGING_BYTES = 2048;             // per epilogue warp: 32 rows x 64 B
 constexpr uint32_t TMEM_COLS = 2 * BN;               // two accumulators
@@ -184,11 +182,10 @@ __device__ __forceinline__ int sched_consume(const Pipe& pipe, uint32_t n, int32
 }
 __device__ __forceinline__ void sched_release(const Pipe& pipe, uint32_t n) { mbar_arrive(pipe.sched_empty(n % SCHED_Q)); }
 // Once per CTA of the grid, by the producer thread after its last fetch (also CTAs that leave without fetching).
-// `n`: how many callers there are (every CTA of the grid, or every pair's leader)
-__device__ __forceinline__ void sched_finish(int32_t* counter, int n = -1)
+__device__ __forceinline__ void sched_finish(int32_t* counter)
 {
     __threadfence();
-    if (atomicAdd(counter + 1, 1) == (n < 0 ? (int)gridDim.x : n) - 1) {
+    if (atomicAdd(counter + 1, 1) == (int)gridDim.x - 1) {
         counter[0] = 0;
         counter[1] = 0;
         __threadfence();
@@ -196,15 +193,11 @@ __device__ __forceinline__ void sched_finish(int32_t* counter, int n = -1)
 }
 
 // Epilogue warp -> accumulator buffer is free again (all its tcgen05.ld of this tile are done).
-// bar: a barrier of this CTA, or -- remote -- the shared::cluster address of a barrier of the pair's leader CTA.
-__device__ __forceinline__ void release_acc(uint32_t bar, int lane, bool remote = false)
+__device__ __forceinline__ void release_acc(uint32_t bar, int lane)
 {
     tc_fence_before();
     __syncwarp();
-    if (lane == 0) {
-        if (remote) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-        else mbar_arrive(bar);
-    }
+    if (lane == 0) mbar_arrive(bar);
 }
 
 // Writes this thread's row of a [32 rows x 32 bf16] tile into the warp's staging tile in the
@@ -275,45 +268,36 @@ struct RowsP {
     const int32_t* tile_expert;
     const int32_t* tile_order;  // optional: i-th row tile to work on (expert-major order over scattered tiles)
     const int32_t* n_tiles;
-    const int32_t* pairs;       // pair kernel: {first tile, second tile or -1} per pair, in processing order
-    const int32_t* n_pairs;
     int32_t* status;
     int32_t* sched;         // {next item, finished CTAs}, both zero between launches
     int kblocks;            // k-blocks (of 64) per operand pair
     int n_out;              // output columns (H or C)
     int n_col_tiles;        // column tiles per row tile
-    int b_rows_per_expert;  // rows of one expert in the B tensor map (= n_out)
     bf16 *G, *U;            // P and Q (see the gate/up epilogue) in the blocked layout (written by MODE_GATEUP, read by MODE_DHH)
     const float* const* bias0;
     const float* const* bias1;
     // MODE_DX only: row tiles are token tiles (no experts); the epilogue adds the expert rows of each token
     int fixed_tiles;            // number of 128-token tiles
     int n_valid_rows;           // tokens
-    // MODE_GATEUP / MODE_DOWN: the B operand is a tile-major weight copy (common.cuh): its map is [blocks * 128 rows,
-    // 64 columns]; block (expert e, row block rb, column block kb) starts at row ((e * b_row_blocks + rb) * b_kb + kb) * 128
-    int b_row_blocks, b_kb;
+    // The B operand (MODE_DX apart) is a tile-major weight copy (common.cuh): block (expert e, row block rb, column block
+    // cb) is block (e * b_row_blocks + rb) * b_col_blocks + cb of the copy.
+    // MODE_GATEUP / MODE_DOWN: rows are output columns, block columns the reduction (whole blocks of 128 rows, K-major);
+    // MODE_DHH / MODE_DXG: rows are the reduction, block columns output columns (half blocks of 64 rows, MN-major).
+    int b_row_blocks, b_col_blocks;
     const bf16* gather_src;     // dXg rows [*, n_out]
     const int32_t* gather_pos;  // [tokens, gather_k] row of dXg for (token, j)
     int gather_k;
 };
 
 // The epilogue of one work item for one of the 16 epilogue warps: TMEM lane quarter q (rows q*32..+31 of the row
-// tile), column group h.  acc_empty_bar is where "this warp has read the accumulator" is signalled: a barrier of
-// this CTA, or (remote) of the leader CTA of a pair.  store = false: the tile is a stand-in (a pair's missing
-// second tile): the accumulator is released and nothing is written.  False: a bounded wait ran out.
+// tile), column group h.  False: a bounded wait ran out.
 template <int MODE>
-__device__ __forceinline__ bool rows_epilogue(const RowsP& p, uint32_t acc_full_bar, uint32_t acc_empty_bar, bool remote,
+__device__ __forceinline__ bool rows_epilogue(const RowsP& p, uint32_t acc_full_bar, uint32_t acc_empty_bar,
                                               uint32_t tmem_base, uint32_t buf, uint32_t t, int row_tile, int n0, int e,
                                               int q, int h, int lane, uint8_t* stage, const CUtensorMap* tmD0,
-                                              const CUtensorMap* tmD1, const CUtensorMap* tmD2, bool store)
+                                              const CUtensorMap* tmD1, const CUtensorMap* tmD2)
 {
     const int row_w = row_tile * BM + q * 32;           // first row of this warp
-    if (!store) {
-        if (!mbar_wait(acc_full_bar, (t >> 1) & 1, p.status, ERR_ACC_WAIT)) return false;
-        tc_fence_after();
-        release_acc(acc_empty_bar, lane, remote);
-        return true;
-    }
     // MODE_DHH: the saved G and U of this item come from HBM.  Unit 0's pieces are requested before the wait
     // for the accumulator, unit 1's while unit 0 is worked on, so their latency hides behind other work.
     uint32_t gq[2][16], uq[2][16];
@@ -333,7 +317,7 @@ __device__ __forceinline__ bool rows_epilogue(const RowsP& p, uint32_t acc_full_
         tmem_ld32(t_lane + h * 32, a);
         tmem_ld32(t_lane + BN / 2 + h * 32, b);
         tmem_ld_wait();
-        release_acc(acc_empty_bar, lane, remote);
+        release_acc(acc_empty_bar, lane);
         if (n < p.n_out) {
             // What backward needs of G and U is not the values themselves but
             //   Q = silu(G)                       (dU = dHh * Q)
@@ -378,7 +362,7 @@ __device__ __forceinline__ bool rows_epilogue(const RowsP& p, uint32_t acc_full_
             float v[32];
             tmem_ld32(t_lane + h * 64 + un * 32, v);
             tmem_ld_wait();
-            if (un == 1) release_acc(acc_empty_bar, lane, remote);
+            if (un == 1) release_acc(acc_empty_bar, lane);
             if (n >= p.n_out) continue;                      // warp-uniform
             uint32_t pk[16];
             if (MODE == MODE_DOWN) {
@@ -456,6 +440,7 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
     extern __shared__ uint8_t smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int COLS_PER_ITEM = MODE == MODE_GATEUP ? BN / 2 : BN;
+    constexpr bool DATA_GRAD = MODE == MODE_DHH || MODE == MODE_DXG;
     const int kb_per_item = (MODE == MODE_DXG ? 2 : 1) * p.kblocks;
 
     const Pipe pipe = carve(smem_raw);
@@ -473,8 +458,8 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
             for (uint32_t nf = 1; ok && item >= 0; ++nf) {
                 const int row_i = item / p.n_col_tiles, n0 = (item % p.n_col_tiles) * COLS_PER_ITEM;
                 const int row_tile = p.tile_order ? p.tile_order[row_i] : row_i;
-                const int brow = (MODE == MODE_DX ? 0 : p.tile_expert[row_tile] * p.b_rows_per_expert) + n0;
                 const int row0 = row_tile * BM;
+                const int e_rows = MODE == MODE_DX ? 0 : p.tile_expert[row_tile] * p.b_row_blocks;      // row blocks before this expert's
                 for (int kb = 0; kb < kb_per_item; ++kb, ++it) {
                     const int s = it % STAGES;
                     if (it >= STAGES && !mbar_wait(pipe.empty(s), ((it / STAGES) - 1) & 1, p.status, ERR_EMPTY_WAIT)) {
@@ -486,18 +471,18 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
                     const bool second = MODE == MODE_DXG && kb >= p.kblocks;
                     const int kx = (second ? kb - p.kblocks : kb) * BK;
                     tma_load_2d(a_dst, second ? &tmA1 : &tmA0, kx, row0, pipe.full(s));
-                    if (MODE == MODE_GATEUP) {
-                        const int y = ((p.tile_expert[row_tile] * p.b_row_blocks + (n0 >> 7)) * p.b_kb + kb) * 128;
-                        tma_load_2d(b_dst, &tmB0, 0, y, pipe.full(s));
-                        tma_load_2d(b_dst + HALF_B, &tmB1, 0, y, pipe.full(s));
-                    } else if (MODE == MODE_DOWN) {
-                        const int y = ((p.tile_expert[row_tile] * p.b_row_blocks + (n0 >> 7)) * p.b_kb + kb) * 128;
-                        tma_load_2d(b_dst, &tmB0, 0, y, pipe.full(s));
-                        tma_load_2d(b_dst + HALF_B, &tmB0, 0, y + p.b_kb * 128, pipe.full(s));
+                    // One load for the whole 32 KiB of B: a k-block of two loads costs the producer ~500 cycles, one of five
+                    // (B in 8 KiB pieces) made dXg 14 % slower
+                    if (MODE == MODE_GATEUP) {             // gate block and up block of the same hidden units
+                        tma_load_4d(b_dst, &tmB0, 0, 0, (e_rows + (n0 >> 7)) * p.b_col_blocks + kb, 0, pipe.full(s));
+                    } else if (MODE == MODE_DOWN) {        // two row blocks
+                        tma_load_4d(b_dst, &tmB0, 0, 0, kb, e_rows + (n0 >> 7), pipe.full(s));
+                    } else if (DATA_GRAD) {
+                        // four half blocks side by side (past the last column block: columns that are not computed)
+                        tma_load_3d(b_dst, second ? &tmB1 : &tmB0, 0, kx & 64, (e_rows + (kx >> 7)) * p.b_col_blocks + (n0 >> 6), pipe.full(s));
                     } else {
-                        const CUtensorMap* mb = second ? &tmB1 : &tmB0;
-                        tma_load_2d(b_dst, mb, kx, brow, pipe.full(s));
-                        tma_load_2d(b_dst + HALF_B, mb, kx, brow + BN / 2, pipe.full(s));
+                        tma_load_2d(b_dst, &tmB0, kx, n0, pipe.full(s));
+                        tma_load_2d(b_dst + HALF_B, &tmB0, kx, n0 + BN / 2, pipe.full(s));
                     }
                 }
                 // the next item is claimed as late as possible (the ring is full by now, so the round trip to the
@@ -510,7 +495,6 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc(BM, BN, 0, 0);
             uint32_t it = 0, t = 0;
             bool ok = true;
             for (; ok; ++t) {
@@ -521,6 +505,9 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
                 if (t >= 2 && !mbar_wait(pipe.acc_empty(buf), ((t >> 1) - 1) & 1, p.status, ERR_ACC_WAIT)) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * BN;
+                // a narrower product where the last item of a row tile has fewer columns
+                const int ncols = DATA_GRAD ? min(BN, 64 * p.b_col_blocks - (item % p.n_col_tiles) * BN) : BN;
+                const uint32_t idesc = make_idesc(BM, ncols, 0, DATA_GRAD ? 1 : 0);
                 for (int kb = 0; kb < kb_per_item; ++kb, ++it) {
                     const int s = it % STAGES;
                     if (!mbar_wait(pipe.full(s), (it / STAGES) & 1, p.status, ERR_FULL_WAIT)) {
@@ -532,7 +519,8 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
 #pragma unroll
                     for (int k = 0; k < BK / 16; ++k) {
                         const uint64_t ad = make_desc(a_addr + k * 32, 16, 1024);
-                        const uint64_t bd = make_desc(b_addr + k * 32, 16, 1024);
+                        // MN-major: 16 reduction rows = two 8-row groups (1 KiB each), 64-column blocks BOX_BYTES apart
+                        const uint64_t bd = DATA_GRAD ? make_desc(b_addr + k * 2048, BOX_BYTES, 1024) : make_desc(b_addr + k * 32, 16, 1024);
                         umma_bf16(d_tmem, ad, bd, idesc, (kb > 0 || k > 0) ? 1u : 0u);
                     }
                     umma_commit(pipe.empty(s));           // frees the stage once these MMAs have read it
@@ -553,16 +541,14 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
             const int row_i = item / p.n_col_tiles, n0 = (item % p.n_col_tiles) * COLS_PER_ITEM;
             const int row_tile = p.tile_order ? p.tile_order[row_i] : row_i;
             const int e = MODE == MODE_DX ? 0 : p.tile_expert[row_tile];
-            if (!rows_epilogue<MODE>(p, pipe.acc_full(buf), pipe.acc_empty(buf), false, tmem_base, buf, t, row_tile, n0, e, q, h,
-                                     lane, stage, &tmD0, &tmD1, &tmD2, true))
+            if (!rows_epilogue<MODE>(p, pipe.acc_full(buf), pipe.acc_empty(buf), tmem_base, buf, t, row_tile, n0, e, q, h,
+                                     lane, stage, &tmD0, &tmD1, &tmD2))
                 break;
         }
         if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // stores landed before exit
     }
     cta_teardown(tmem_base, warp);
 }
-
-#include "gemm_tc_pair.inl"
 
 // ---- weight gradients: grad[e][M,N] += A_e^T * B_e over the expert's rows ---------
 // One weight-gradient problem: grad[e][M,N] += A_e^T * B_e over the rows of "expert" e.
@@ -629,7 +615,7 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant_
     const Pipe pipe = carve(smem_raw);
     const uint32_t tmem_base = cta_setup(pipe, warp, CS_WARPS);
     pdl_wait();
-    constexpr uint32_t BOX = 64 * BK * 2;      // one {64 MN elements, 64 rows} box = 8 KiB
+    constexpr uint32_t BOX = BOX_BYTES;
 
     if (warp == 0) {
         if (lane == 0) {
@@ -942,7 +928,26 @@ bool make_map_blocks(CUtensorMap* m, const void* base, uint64_t rows, uint64_t c
     return r == CUDA_SUCCESS;
 }
 
+// A tile-major weight copy as {64 columns, 128 rows, n2 blocks at stride2 elements, n3 at stride3}, box {64, rows, b2, b3}.
+static int make_map_weights(CUtensorMap* m, const void* base, uint64_t n2, uint64_t stride2, uint64_t n3, uint64_t stride3,
+                            uint32_t rows, uint32_t b2, uint32_t b3)
+{
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return fail(MGPT_MOE_ECUDA, "cuTensorMapEncodeTiled is not available from this driver");
+    cuuint64_t dims[4] = {64, 128, n2, n3};
+    cuuint64_t strides[3] = {64 * sizeof(bf16), stride2 * sizeof(bf16), stride3 * sizeof(bf16)};
+    cuuint32_t box[4] = {64, rows, b2, b3};
+    cuuint32_t estr[4] = {1, 1, 1, 1};
+    CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, n3 ? 4 : 3, const_cast<void*>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(MGPT_MOE_ECUDA, "cuTensorMapEncodeTiled failed (code " + std::to_string((int)r) + ")");
+    return 0;
+}
+
 namespace {
+
+int cdiv(int a, int b) { return (a + b - 1) / b; }
 
 struct TcState {
     const void* ws = nullptr;
@@ -950,10 +955,12 @@ struct TcState {
     int n_tokens = -1;
     bool attr_set = false;
     int sms = 0;
-    int max_pairs = 0;           // CTA pairs (clusters of two) that can be resident at once; 0 = pair kernels off
     int32_t* sched = nullptr;    // device: one {next item, finished CTAs} pair per kind of launch, zero between launches
     // K-major operand loads (box 64 x 128 rows)
-    CUtensorMap Xg, Hh, dYg, dG, dU, WgT, WuT, WdT, Wg, Wu, Wd;
+    CUtensorMap Xg, Hh, dYg, dG, dU;
+    // weight copies: two whole blocks (gate and up; two row blocks of Wd) per load
+    CUtensorMap WguT, WdT;
+    CUtensorMap Wg_h, Wu_h, Wd_h;      // the same weight copies in half blocks (box 64 columns x 64 rows x 4 blocks)
     // reduction-over-rows operand loads (box 64 x 64 rows)
     CUtensorMap Xg_t, Hh_t, dYg_t, dG_t, dU_t;
     // the same operands by column blocks (one load per operand tile): A side {64, 64 rows, 2}, B side {64, 64 rows, 4}
@@ -978,13 +985,14 @@ int prepare(mgpt_moe_layer* L, const Workspace& w, char* ws)
     MGPT_TRY(make_map(&s->dYg, dyg, rc, C, 128));
     MGPT_TRY(make_map(&s->dG, ws + w.dG, rc, H, 128));
     MGPT_TRY(make_map(&s->dU, ws + w.dU, rc, H, 128));
-    // tile-major copies: one 16 KiB block per (128 rows, 64 columns), seen as a tall matrix of 64 columns
-    MGPT_TRY(make_map(&s->WgT, L->sWgT, E * tile_major_elems(d.H, d.C) / 64, 64, 128));
-    MGPT_TRY(make_map(&s->WuT, L->sWuT, E * tile_major_elems(d.H, d.C) / 64, 64, 128));
-    MGPT_TRY(make_map(&s->WdT, L->sWdT, E * tile_major_elems(d.C, d.H) / 64, 64, 128));
-    MGPT_TRY(make_map(&s->Wg, L->sWg, E * C, H, 128));
-    MGPT_TRY(make_map(&s->Wu, L->sWu, E * C, H, 128));
-    MGPT_TRY(make_map(&s->Wd, L->sWd, E * H, C, 128));
+    // tile-major weight copies, 16 KiB (8192 elements) per block
+    const uint64_t BLK = 128 * 64, eCH = E * tile_major_elems(d.H, d.C), eHC = E * tile_major_elems(d.C, d.H);
+    const uint64_t cb = cdiv(d.H, 64);
+    MGPT_TRY(make_map_weights(&s->WguT, L->sWgT, eCH / BLK, BLK, 2, eCH, 128, 1, 2));            // Wu's copy follows Wg's
+    MGPT_TRY(make_map_weights(&s->WdT, L->sWdT, cb, BLK, eHC / BLK / cb, cb * BLK, 128, 1, 2));
+    MGPT_TRY(make_map_weights(&s->Wg_h, L->sWgT, eCH / BLK, BLK, 0, 0, 64, BN / 64, 1));
+    MGPT_TRY(make_map_weights(&s->Wu_h, L->sWuT, eCH / BLK, BLK, 0, 0, 64, BN / 64, 1));
+    MGPT_TRY(make_map_weights(&s->Wd_h, L->sWdT, eHC / BLK, BLK, 0, 0, 64, BN / 64, 1));
     MGPT_TRY(make_map(&s->Xg_t, xg, rc, C, 64));
     MGPT_TRY(make_map(&s->Hh_t, ws + w.Hh, rc, H, 64));
     MGPT_TRY(make_map(&s->dYg_t, dyg, rc, C, 64));
@@ -1016,35 +1024,6 @@ int prepare_attrs(mgpt_moe_layer* L)
         MGPT_CUDA(cudaFuncSetAttribute(tc_rows_kernel<MODE_DX>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
         MGPT_CUDA(cudaFuncSetAttribute(tc_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
         MGPT_CUDA(cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, L->device));
-        MGPT_CUDA(cudaFuncSetAttribute(tc_rows_pair_kernel<MODE_GATEUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        MGPT_CUDA(cudaFuncSetAttribute(tc_rows_pair_kernel<MODE_DOWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        MGPT_CUDA(cudaFuncSetAttribute(tc_rows_pair_kernel<MODE_DHH>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        MGPT_CUDA(cudaFuncSetAttribute(tc_rows_pair_kernel<MODE_DXG>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        {
-            // The CTA-pair kernels (gemm_tc_pair.inl) are opt-in, MGPT_MOE_CTA_PAIRS=1 in the environment: measured on
-            // B200 they match the single-CTA kernels at the 64-expert shapes (both sit at ~82-90 % of what cuBLAS
-            // sustains under the 1 kW power cap) and lose a little on small shapes.  How many clusters of two CTAs
-            // fit on the device at once is asked of the driver (SMs pair up within a GPC).
-            const char* env = getenv("MGPT_MOE_CTA_PAIRS");
-            s->max_pairs = 0;
-            if (env && env[0] == '1') {
-                cudaLaunchConfig_t cfg = {};
-                cfg.gridDim = dim3(2 * (unsigned)s->sms, 1, 1);
-                cfg.blockDim = dim3(TC_THREADS, 1, 1);
-                cfg.dynamicSmemBytes = SMEM_BYTES;
-                cudaLaunchAttribute at[1];
-                at[0].id = cudaLaunchAttributeClusterDimension;
-                at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-                cfg.attrs = at;
-                cfg.numAttrs = 1;
-                int n = 0;
-                if (cudaOccupancyMaxActiveClusters(&n, tc_rows_pair_kernel<MODE_DOWN>, &cfg) == cudaSuccess && n > 0)
-                    s->max_pairs = n;
-                else
-                    cudaGetLastError();       // no pairs on this device: the single-CTA kernels stay
-            }
-            if (getenv("MGPT_MOE_VERBOSE")) fprintf(stderr, "mgpt_moe: %d SMs, %d resident CTA pairs\n", s->sms, s->max_pairs);
-        }
         // the work-item counters must read zero before the first launch on any stream: allocate and clear them
         // here, at layer creation, and wait for the clear (nothing orders the legacy stream with a caller's
         // non-blocking stream)
@@ -1056,7 +1035,6 @@ int prepare_attrs(mgpt_moe_layer* L)
     return 0;
 }
 
-int cdiv(int a, int b) { return (a + b - 1) / b; }
 int imin(int a, int b) { return a < b ? a : b; }
 // persistent CTAs to launch: every SM, or the caller's budget when other kernels must stay resident beside these
 int grid_sms(const mgpt_moe_layer* L, const TcState* s) { return L->sm_budget > 0 ? imin(L->sm_budget, s->sms) : s->sms; }
@@ -1068,19 +1046,14 @@ int grid_sms(const mgpt_moe_layer* L, const TcState* s) { return L->sm_budget > 
 bool tc_fused_bias_grads(const Dims& d) { return cdiv(d.H, BM) >= 2; }
 
 namespace {
-// One of the four token-major products: on CTA pairs where the device takes them, else one CTA per tile.
+// One of the four token-major products.
 template <int MODE>
 int launch_rows(mgpt_moe_layer* L, TcState* s, const Workspace& w, const RowsP& p, const CUtensorMap& a0, const CUtensorMap& a1,
                 const CUtensorMap& b0, const CUtensorMap& b1, const CUtensorMap& d0, const CUtensorMap& d1,
                 const CUtensorMap& d2, cudaStream_t st, const char* what)
 {
-    const int budget = grid_sms(L, s);
-    if (s->max_pairs > 0 && p.pairs) {
-        const int pairs = imin(imin(s->max_pairs, budget / 2), w.max_tiles * p.n_col_tiles);
-        MGPT_CUDA(launch_pdl(tc_rows_pair_kernel<MODE>, 2 * (pairs > 0 ? pairs : 1), TC_THREADS, SMEM_BYTES, st, a0, a1, b0, b1, d0, d1, d2, p));
-    } else {
-        MGPT_CUDA(launch_pdl(tc_rows_kernel<MODE>, imin(budget, w.max_tiles * p.n_col_tiles), TC_THREADS, SMEM_BYTES, st, a0, a1, b0, b1, d0, d1, d2, p));
-    }
+    MGPT_CUDA(launch_pdl(tc_rows_kernel<MODE>, imin(grid_sms(L, s), w.max_tiles * p.n_col_tiles), TC_THREADS, SMEM_BYTES, st, a0, a1,
+                         b0, b1, d0, d1, d2, p));
     MGPT_LAUNCHED(what);
     return 0;
 }
@@ -1095,22 +1068,20 @@ int tc_experts_forward(mgpt_moe_layer* L, const Workspace& w, char* ws, cudaStre
     p.tile_expert = (const int32_t*)(ws + w.tile_expert);
     p.tile_order = L->n_seg > 0 ? (const int32_t*)(ws + w.tile_order) : nullptr;
     p.n_tiles = (const int32_t*)(ws + w.n_tiles);
-    p.pairs = (const int32_t*)(ws + w.pairs);
-    p.n_pairs = (const int32_t*)(ws + w.n_pairs);
     p.status = L->d_status;
     // gate/up + SwiGLU: K = C, 128 hidden units per item
-    p.kblocks = cdiv(d.C, BK); p.n_out = d.H; p.b_rows_per_expert = d.H; p.n_col_tiles = cdiv(d.H, BN / 2);
-    p.b_row_blocks = cdiv(d.H, 128); p.b_kb = cdiv(d.C, BK);
+    p.kblocks = cdiv(d.C, BK); p.n_out = d.H; p.n_col_tiles = cdiv(d.H, BN / 2);
+    p.b_row_blocks = cdiv(d.H, 128); p.b_col_blocks = cdiv(d.C, BK);
     p.bias0 = L->master.bg; p.bias1 = L->master.bu;
     p.G = w.inference ? nullptr : (bf16*)(ws + w.G);
     p.U = w.inference ? nullptr : (bf16*)(ws + w.U);
     L->stage_begin(ST_GATEUP, st);
     p.sched = s->sched + 0;
-    MGPT_TRY(launch_rows<MODE_GATEUP>(L, s, w, p, s->Xg, s->Xg, s->WgT, s->WuT, s->Hh_s, s->Hh_s, s->Hh_s, st, "tc_rows<gateup>"));
+    MGPT_TRY(launch_rows<MODE_GATEUP>(L, s, w, p, s->Xg, s->Xg, s->WguT, s->WguT, s->Hh_s, s->Hh_s, s->Hh_s, st, "tc_rows<gateup>"));
     L->stage_end(ST_GATEUP, st);
     // down: K = H
-    p.kblocks = cdiv(d.H, BK); p.n_out = d.C; p.b_rows_per_expert = d.C; p.n_col_tiles = cdiv(d.C, BN);
-    p.b_row_blocks = cdiv(d.C, 128); p.b_kb = cdiv(d.H, BK);
+    p.kblocks = cdiv(d.H, BK); p.n_out = d.C; p.n_col_tiles = cdiv(d.C, BN);
+    p.b_row_blocks = cdiv(d.C, 128); p.b_col_blocks = cdiv(d.H, BK);
     p.bias0 = L->master.bd; p.bias1 = nullptr;
     L->stage_begin(ST_DOWN, st);
     p.sched = s->sched + 2;
@@ -1130,21 +1101,21 @@ int tc_experts_backward(mgpt_moe_layer* L, const Workspace& w, char* ws, cudaStr
     p.tile_expert = (const int32_t*)(ws + w.tile_expert);
     p.tile_order = L->n_seg > 0 ? (const int32_t*)(ws + w.tile_order) : nullptr;
     p.n_tiles = (const int32_t*)(ws + w.n_tiles);
-    p.pairs = (const int32_t*)(ws + w.pairs);
-    p.n_pairs = (const int32_t*)(ws + w.n_pairs);
     p.status = L->d_status;
     // dHh = dYg * Wd^T  (K = C), SwiGLU backward in the epilogue
-    p.kblocks = cdiv(d.C, BK); p.n_out = d.H; p.b_rows_per_expert = d.H; p.n_col_tiles = cdiv(d.H, BN);
+    p.kblocks = cdiv(d.C, BK); p.n_out = d.H; p.n_col_tiles = cdiv(d.H, BN);
+    p.b_row_blocks = cdiv(d.C, 128); p.b_col_blocks = cdiv(d.H, BK);
     p.G = (bf16*)(ws + w.G); p.U = (bf16*)(ws + w.U);
     L->stage_begin(ST_DHH, st);
     p.sched = s->sched + 4;
-    MGPT_TRY(launch_rows<MODE_DHH>(L, s, w, p, s->dYg, s->dYg, s->Wd, s->Wd, s->dG_s, s->dU_s, s->dU_s, st, "tc_rows<dhh>"));
+    MGPT_TRY(launch_rows<MODE_DHH>(L, s, w, p, s->dYg, s->dYg, s->Wd_h, s->Wd_h, s->dG_s, s->dU_s, s->dU_s, st, "tc_rows<dhh>"));
     L->stage_end(ST_DHH, st);
     // dXg = dG * Wg^T + dU * Wu^T  (K = 2H)
-    p.kblocks = cdiv(d.H, BK); p.n_out = d.C; p.b_rows_per_expert = d.C; p.n_col_tiles = cdiv(d.C, BN);
+    p.kblocks = cdiv(d.H, BK); p.n_out = d.C; p.n_col_tiles = cdiv(d.C, BN);
+    p.b_row_blocks = cdiv(d.H, 128); p.b_col_blocks = cdiv(d.C, BK);
     L->stage_begin(ST_DXG, st);
     p.sched = s->sched + 6;
-    MGPT_TRY(launch_rows<MODE_DXG>(L, s, w, p, s->dG, s->dU, s->Wg, s->Wu, s->dXg_s, s->dXg_s, s->dXg_s, st, "tc_rows<dxg>"));
+    MGPT_TRY(launch_rows<MODE_DXG>(L, s, w, p, s->dG, s->dU, s->Wg_h, s->Wu_h, s->dXg_s, s->dXg_s, s->dXg_s, st, "tc_rows<dxg>"));
     L->stage_end(ST_DXG, st);
     }
     if (!L->has_grad || !(phase & 2)) return 0;
@@ -1210,7 +1181,7 @@ int tc_router_dx(mgpt_moe_layer* L, const Workspace& w, char* ws, const void* dX
     p.n_tiles = (const int32_t*)(ws + w.n_tiles);
     p.tile_expert = (const int32_t*)(ws + w.tile_expert);
     p.status = L->d_status;
-    p.kblocks = cdiv(E8, BK); p.n_out = d.C; p.b_rows_per_expert = 0; p.n_col_tiles = cdiv(d.C, BN);
+    p.kblocks = cdiv(E8, BK); p.n_out = d.C; p.n_col_tiles = cdiv(d.C, BN);
     p.fixed_tiles = cdiv(w.n_tokens, BM); p.n_valid_rows = w.n_tokens;
     p.gather_src = (const bf16*)dXg; p.gather_pos = pos; p.gather_k = d.k;
     p.sched = s->sched + 10;

@@ -306,38 +306,6 @@ tc_router_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     }
 }
 
-// Wr [C,E] fp32 -> transposed BF16 pieces [2][NE][C] (hi = bf16(w), mid = bf16(w - hi)) and the largest column
-// norm / bias magnitude, for the error bound.  One block per expert row of the output.
-__global__ void __launch_bounds__(256)
-router_pieces_kernel(const float* __restrict__ Wr, const float* __restrict__ br, int C, int E, int NE,
-                     bf16* __restrict__ out, float* __restrict__ rstat)
-{
-    __shared__ float red[8];
-    pdl_wait();
-    const int e = blockIdx.x;
-    float ss = 0.0f;
-    for (int c = threadIdx.x; c < C; c += blockDim.x) {
-        const float w = Wr[(size_t)c * E + e];
-        const bf16 hi = __float2bfloat16(w);
-        const bf16 mid = __float2bfloat16(w - __bfloat162float(hi));
-        out[(size_t)e * C + c] = hi;
-        out[((size_t)NE + e) * C + c] = mid;
-        ss = fmaf(w, w, ss);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.0f;
-        for (int i = 0; i < 8; ++i) t += red[i];
-        // non-negative floats order like their bit patterns; a NaN (bits above +inf) stays the maximum, so a
-        // poisoned weight makes every token take the exact pass
-        atomicMax(reinterpret_cast<int*>(rstat), __float_as_int(sqrtf(t) * 1.001f));
-        atomicMax(reinterpret_cast<int*>(rstat) + 1, __float_as_int(fabsf(br[e])));
-    }
-}
-
 int router_ne(int E) { return E <= 16 ? 16 : E <= 32 ? 32 : E <= 64 ? 64 : 128; }
 
 template <int NE>
@@ -353,17 +321,6 @@ int launch_rt(const CUtensorMap& mx, const CUtensorMap& mw, const RtP& p, int gr
 }
 
 }  // namespace
-
-// Rebuilds the router's transposed BF16 pieces and the norms of the error bound (after the masters changed).
-int launch_router_pieces(mgpt_moe_layer* L, cudaStream_t st)
-{
-    const Dims& d = L->d;
-    if (!L->sWrT2 || !L->router_bound) return 0;
-    MGPT_CUDA(cudaMemsetAsync(L->d_rstat, 0, 2 * sizeof(float), st));
-    MGPT_CUDA(launch_pdl(router_pieces_kernel, d.E, 256, 0, st, L->p_data[0], L->p_data[1], d.C, d.E, L->router_ne, L->sWrT2, L->d_rstat));
-    MGPT_LAUNCHED("router_pieces_kernel");
-    return 0;
-}
 
 // The two-pass router pays off once the exact kernel's 2*N*C*E multiply-adds take longer than two launches and a
 // first pass over x: below ~4e8 of them (config 2: 6.7e7; decode batches) the exact kernel alone is faster.
