@@ -60,6 +60,9 @@ Workspace make_workspace(const Dims& d, int n_tokens, int kind)
     w.tile_expert = take((size_t)w.max_tiles * 4);
     w.n_tiles = take(4);
     w.status = take(4);
+    w.decode = (kind == 0 || kind == 3) && decode_usable(d, n_tokens);
+    w.groups = take(w.decode ? (size_t)decode_max_groups(d, n_tokens) * 16 : 0);
+    w.n_groups = take(4);
     w.map = take(N * k * 4);
     w.pos = take(N * k * 4);
     w.row_src = take(rc * 4);
@@ -456,7 +459,8 @@ int mgpt_moe_selftest_bounded_wait(mgpt_moe_layer* L, mgpt_stream_t stream)
 }
 
 // Routing results and plan of one forward: the workspace bytes from probs up to (not including) the plan's
-// scratch -- probs, top_idx, top_p, counts, offsets, padded_offsets, tile_expert, n_tiles, status, map, pos, row_src.
+// scratch -- probs, top_idx, top_p, counts, offsets, padded_offsets, tile_expert, n_tiles, status, groups, n_groups,
+// map, pos, row_src.
 static size_t routing_begin(const Workspace& w) { return w.probs; }
 static size_t routing_end(const Workspace& w) { return w.blk_cnt; }
 
@@ -551,10 +555,17 @@ static int forward_impl(mgpt_moe_layer* L, const void* x, void* y, int n_tokens,
         L->stage_end(ST_PLAN, st);
     }
     if (n_tokens > 0) {
-        L->stage_begin(ST_DISPATCH, st);
-        MGPT_TRY(launch_dispatch(d, w, ws, x, io, st));
-        L->stage_end(ST_DISPATCH, st);
-        if (use_tc(L)) MGPT_TRY(tc_experts_forward(L, w, ws, st));
+        // (the decode kernels fetch the tokens' rows themselves; training keeps the permuted rows for backward)
+        const bool gathered = w.decode && inference;
+        if (!gathered) {
+            L->stage_begin(ST_DISPATCH, st);
+            MGPT_TRY(launch_dispatch(d, w, ws, x, io, st));
+            // padding rows of what backward reads: finite (the other product kernels compute them)
+            if (w.decode) MGPT_CUDA(cudaMemsetAsync(ws + w.G, 0, w.Yg - w.G, st));
+            L->stage_end(ST_DISPATCH, st);
+        }
+        if (w.decode) MGPT_TRY(launch_decode_forward(L, w, ws, x, io, !gathered, st));
+        else if (use_tc(L)) MGPT_TRY(tc_experts_forward(L, w, ws, st));
         else MGPT_TRY(simt_experts_forward(L, w, ws, st));
         L->stage_begin(ST_COMBINE, st);
         MGPT_TRY(launch_combine_fwd(d, w, ws, y, io, st, residual));

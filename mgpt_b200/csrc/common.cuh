@@ -97,6 +97,8 @@ struct Workspace {
     size_t logits, probs, top_idx, top_p;
     // plan
     size_t counts, offsets, padded_offsets, tile_expert, n_tiles, status;
+    size_t groups, n_groups;    // decode kernels: {expert, first padded row, rows, 0} per row group
+    bool decode;                // few rows per expert: the products are decode.cu's
     size_t map, pos, row_src, blk_cnt, slot, seg, tile_order;
     // forward activations (kept for backward)
     size_t Xg, G, U, Hh, Yg;
@@ -120,6 +122,11 @@ struct Dims {
 // kind 0: whole layer; kind 1: routing side only (no activation buffers; rows are exchanged by the caller);
 // kind 2: expert side (the four [rows, C] buffers belong to the caller); kind 3: whole layer, forward only (inference)
 Workspace make_workspace(const Dims& d, int n_tokens, int kind = 0);
+
+// decode.cu: rows of one expert are worked on in groups of at most this many
+constexpr int DECODE_GROUP = 16;
+bool decode_usable(const Dims& d, int n_tokens);
+int decode_max_groups(const Dims& d, int n_tokens);
 
 // Device-side tables of per-expert pointers (index = expert).
 // The transposed BF16 weight copies (the B operands of the forward products) are stored tile-major: per expert the
@@ -243,6 +250,7 @@ int launch_router_bwd(mgpt_moe_layer* L, const Workspace& w, char* ws, const voi
                       void* dx, cudaStream_t st, const void* dXg_rows = nullptr, const int32_t* pos_rows = nullptr);
 
 // plan.cu
+struct PlanArgs plan_args(const Dims& d, const Workspace& w, char* ws, int32_t* sticky);      // plan_block.cuh
 int launch_plan(const Dims& d, const Workspace& w, char* ws, cudaStream_t st, int32_t* sticky);
 int launch_dispatch(const Dims& d, const Workspace& w, char* ws, const void* x, int io, cudaStream_t st);
 int launch_combine_fwd(const Dims& d, const Workspace& w, char* ws, void* y, int io, cudaStream_t st,
@@ -258,10 +266,9 @@ int combine_rows(const void* rows, const int32_t* pos, const float* top_p, int N
 int combine_rows_backward(const void* dy, int io, const void* rows, const int32_t* row_src, const float* top_p,
                           const int32_t* n_tiles, int n_rows, int grid_rows, int C, int k, void* d_rows, float* d_top_p,
                           size_t act_bytes, cudaStream_t st);
-int run_plan(const int32_t* top_idx, int R, int E, int32_t* counts, int32_t* offsets, int32_t* padded_offsets,
-             int32_t* tile_expert, int32_t* n_tiles, int max_tiles, int32_t* map, int32_t* pos,
-             int32_t* row_src, int row_cap, int32_t* status, int32_t* blk, cudaStream_t st, int32_t* slot_of,
-             int32_t* sticky);
+
+// decode.cu
+int launch_decode_forward(mgpt_moe_layer* L, const Workspace& w, char* ws, const void* x, int io, bool from_rows, cudaStream_t st);
 
 // gemm_simt.cu
 int simt_experts_forward(mgpt_moe_layer* L, const Workspace& w, char* ws, cudaStream_t st);

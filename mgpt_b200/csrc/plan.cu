@@ -18,13 +18,11 @@
 // weight gradients.
 #include <mutex>
 
-#include "common.cuh"
+#include "plan_block.cuh"
 
 namespace mgpt {
 
 namespace {
-
-constexpr int PLAN_BLOCK = 1024;   // flat indices per block
 
 __device__ __forceinline__ float to_f32(float v) { return v; }
 __device__ __forceinline__ float to_f32(bf16 v) { return __bfloat162float(v); }
@@ -34,11 +32,12 @@ template <> __device__ __forceinline__ bf16 from_f32<bf16>(float v) { return __f
 
 // (1) per-block expert histogram
 __global__ void __launch_bounds__(PLAN_BLOCK)
-plan_count_kernel(const int32_t* __restrict__ top_idx, int R, int E, int32_t* __restrict__ blk_cnt)
+plan_count_kernel(const int32_t* __restrict__ top_idx, int R, int E, int32_t* __restrict__ blk_cnt, int32_t* __restrict__ status)
 {
     pdl_wait();
     __shared__ int cnt[MAX_EXPERTS];
     if (threadIdx.x < E) cnt[threadIdx.x] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
     __syncthreads();
     const int i = blockIdx.x * PLAN_BLOCK + threadIdx.x;
     if (i < R) {
@@ -49,71 +48,49 @@ plan_count_kernel(const int32_t* __restrict__ top_idx, int R, int E, int32_t* __
     if (threadIdx.x < E) blk_cnt[(size_t)blockIdx.x * E + threadIdx.x] = cnt[threadIdx.x];
 }
 
-// (2) scan: per expert over blocks, then over experts (compact and padded), tile list
-__global__ void __launch_bounds__(MAX_EXPERTS)
-plan_scan_kernel(int32_t* __restrict__ blk_cnt, int n_blocks, int E,
-                 int32_t* __restrict__ counts, int32_t* __restrict__ offsets,
-                 int32_t* __restrict__ padded_offsets, int32_t* __restrict__ tile_expert,
-                 int32_t* __restrict__ n_tiles, int max_tiles, int32_t* __restrict__ status,
-                 int32_t* __restrict__ sticky)
+// (2) everything else.  Each block sums the histograms of all blocks and of those before it (8 slices of blocks x 128
+// experts; n_blocks * E integers out of L2), scans the experts, and gives its own rows their stable rank -> map / pos /
+// row_src; block 0 also writes what is not per row.  (A scan kernel of one block between the two took 11-17 us at 64
+// blocks: a serial walk over the blocks per expert, then over the experts in one thread.)
+__global__ void __launch_bounds__(PLAN_BLOCK) plan_assign_kernel(const PlanArgs p, int n_blocks, const int32_t* __restrict__ blk_cnt)
 {
     pdl_wait();
-    __shared__ int tot[MAX_EXPERTS];
-    __shared__ int poff[MAX_EXPERTS + 1];
-    const int e = threadIdx.x;
-    if (e < E) {
-        int run = 0;
-        for (int b = 0; b < n_blocks; ++b) {
-            const int c = blk_cnt[(size_t)b * E + e];
-            blk_cnt[(size_t)b * E + e] = run;      // becomes the block's base within the expert
-            run += c;
+    __shared__ int warp_cnt[PLAN_SEGS][MAX_EXPERTS];
+    __shared__ int part[2][8][MAX_EXPERTS];
+    __shared__ int tot[MAX_EXPERTS], base[MAX_EXPERTS], off[MAX_EXPERTS], tile0[MAX_EXPERTS + 1], goff[MAX_EXPERTS];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int i = blockIdx.x * PLAN_BLOCK + tid;
+    bool valid = i < p.R;
+    int e = valid ? p.top_idx[i] : 0;
+    {
+        const int x = tid & (MAX_EXPERTS - 1), slice = tid / MAX_EXPERTS;
+        int before = 0, all = 0;
+        if (x < p.E) {
+#pragma unroll 8
+            for (int b = slice; b < n_blocks; b += 8) {
+                const int c = __ldcg(blk_cnt + (size_t)b * p.E + x);
+                all += c;
+                if (b < (int)blockIdx.x) before += c;
+            }
         }
-        tot[e] = run;
-        counts[e] = run;
+        part[0][slice][x] = before;
+        part[1][slice][x] = all;
     }
+    for (int j = tid; j < PLAN_SEGS * MAX_EXPERTS; j += PLAN_BLOCK) (&warp_cnt[0][0])[j] = 0;
     __syncthreads();
-    if (e == 0) {
-        int off = 0, p = 0;
-        for (int i = 0; i < E; ++i) {
-            offsets[i] = off;
-            poff[i] = p;
-            padded_offsets[i] = p;
-            off += tot[i];
-            p += (tot[i] + ROW_TILE - 1) / ROW_TILE * ROW_TILE;
+    if (tid < MAX_EXPERTS) {
+        int before = 0, all = 0;
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            before += part[0][s][tid];
+            all += part[1][s][tid];
         }
-        poff[E] = p;
-        padded_offsets[E] = p;
-        const int nt = p / ROW_TILE;
-        *n_tiles = nt;
-        *status = nt > max_tiles ? ST_PLAN_OVERFLOW : 0;      // cannot happen: max_tiles bounds sum(ceil); also clears the word
-        if (sticky && nt > max_tiles) atomicOr(sticky, ST_PLAN_OVERFLOW);
+        base[tid] = before;
+        tot[tid] = all;
     }
-    __syncthreads();
-    if (e < E) {
-        const int t0 = poff[e] / ROW_TILE, t1 = poff[e + 1] / ROW_TILE;
-        for (int t = t0; t < t1 && t < max_tiles; ++t) tile_expert[t] = e;
-    }
-}
-
-// (3) stable rank of every flat index within its expert -> map / pos / row_src
-__global__ void __launch_bounds__(PLAN_BLOCK)
-plan_assign_kernel(const int32_t* __restrict__ top_idx, int R, int E,
-                   const int32_t* __restrict__ blk_base, const int32_t* __restrict__ counts,
-                   const int32_t* __restrict__ offsets, const int32_t* __restrict__ padded_offsets,
-                   int32_t* __restrict__ map, int32_t* __restrict__ pos, int32_t* __restrict__ row_src,
-                   int32_t* __restrict__ slot_of, int32_t* __restrict__ status, int32_t* __restrict__ sticky)
-{
-    pdl_wait();
-    __shared__ int warp_cnt[PLAN_BLOCK / 32][MAX_EXPERTS];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < (PLAN_BLOCK / 32) * MAX_EXPERTS; i += PLAN_BLOCK) (&warp_cnt[0][0])[i] = 0;
-    __syncthreads();
-    const int i = blockIdx.x * PLAN_BLOCK + threadIdx.x;
-    bool valid = i < R;
-    int e = valid ? top_idx[i] : 0;
-    if (valid && (unsigned)e >= (unsigned)E) {                    // an id no expert has: no slot, and the caller is told
-        atomicOr(status, ST_BAD_EXPERT);
-        if (sticky) atomicOr(sticky, ST_BAD_EXPERT);
+    if (valid && (unsigned)e >= (unsigned)p.E) {                  // an id no expert has: no slot, and the caller is told
+        atomicOr(p.status, ST_BAD_EXPERT);
+        if (p.sticky) atomicOr(p.sticky, ST_BAD_EXPERT);
         valid = false;
     }
     if (!valid) e = -1 - lane;                                    // distinct keys for idle lanes
@@ -121,92 +98,55 @@ plan_assign_kernel(const int32_t* __restrict__ top_idx, int R, int E,
     const int rank_in_warp = __popc(peers & ((1u << lane) - 1u));
     if (valid && rank_in_warp == 0) warp_cnt[warp][e] = __popc(peers);
     __syncthreads();
-    if (valid) {
-        int base = 0;
-        for (int w = 0; w < warp; ++w) base += warp_cnt[w][e];
-        const int r = blk_base[(size_t)blockIdx.x * E + e] + base + rank_in_warp;
-        const int slot = offsets[e] + r;
-        const int p = padded_offsets[e] + r;
-        map[slot] = i;
-        pos[i] = p;
-        row_src[p] = i;
-        if (slot_of) slot_of[i] = slot;
+    if (warp == 0) {
+        int nt, ng;
+        plan_scan_experts(tot, p.E, lane, off, tile0, goff, nt, ng);
+        if (lane == 0) {
+            tile0[p.E] = nt;
+            if (blockIdx.x == 0) {
+                *p.n_tiles = nt;
+                p.padded_offsets[p.E] = nt * ROW_TILE;
+                if (p.groups) *p.n_groups = ng;
+                if (nt > p.max_tiles) {                           // cannot happen: max_tiles bounds sum(ceil)
+                    atomicOr(p.status, ST_PLAN_OVERFLOW);
+                    if (p.sticky) atomicOr(p.sticky, ST_PLAN_OVERFLOW);
+                }
+            }
+        }
     }
-    // padding rows of every expert's segment carry no source (block 0, one thread per expert)
-    if (blockIdx.x == 0 && threadIdx.x < E) {
-        const int e2 = threadIdx.x;
-        for (int q = padded_offsets[e2] + counts[e2]; q < padded_offsets[e2 + 1]; ++q) row_src[q] = -1;
+    __syncthreads();
+    if (valid) {
+        int r = base[e] + rank_in_warp;
+        for (int w = 0; w < warp; ++w) r += warp_cnt[w][e];
+        const int slot = off[e] + r, q = tile0[e] * ROW_TILE + r;
+        p.map[slot] = i;
+        p.pos[i] = q;
+        p.row_src[q] = i;
+        if (p.slot_of) p.slot_of[i] = slot;
+    }
+    if (blockIdx.x != 0) return;
+    for (int x = warp; x < p.E; x += PLAN_SEGS) {
+        const int t0 = tile0[x], t1 = tile0[x + 1], n = tot[x];
+        if (lane == 0) {
+            p.counts[x] = n;
+            p.offsets[x] = off[x];
+            p.padded_offsets[x] = t0 * ROW_TILE;
+        }
+        for (int t = t0 + lane; t < t1 && t < p.max_tiles; t += 32) p.tile_expert[t] = x;
+        // padding rows of the expert's segment carry no source
+        for (int q = t0 * ROW_TILE + n + lane; q < t1 * ROW_TILE; q += 32) p.row_src[q] = -1;
+        if (p.groups)
+            for (int g = lane; g * DECODE_GROUP < n; g += 32)
+                p.groups[goff[x] + g] = make_int4(x, t0 * ROW_TILE + g * DECODE_GROUP, min(DECODE_GROUP, n - g * DECODE_GROUP), 0);
     }
 }
 
-// The whole plan in one block, for up to PLAN_BLOCK routed rows (decode-sized batches): histogram, prefix sums, tile
-// list and the stable slot assignment without leaving the SM -- one launch instead of three.
-__global__ void __launch_bounds__(PLAN_BLOCK)
-plan_small_kernel(const int32_t* __restrict__ top_idx, int R, int E, int32_t* __restrict__ counts,
-                  int32_t* __restrict__ offsets, int32_t* __restrict__ padded_offsets, int32_t* __restrict__ tile_expert,
-                  int32_t* __restrict__ n_tiles, int max_tiles, int32_t* __restrict__ map, int32_t* __restrict__ pos,
-                  int32_t* __restrict__ row_src, int32_t* __restrict__ slot_of, int32_t* __restrict__ status,
-                  int32_t* __restrict__ sticky)
+// The whole plan in one block, for up to PLAN_BLOCK routed rows: one launch instead of two.
+__global__ void __launch_bounds__(512) plan_small_kernel(const PlanArgs p)
 {
     pdl_wait();
-    __shared__ int warp_cnt[PLAN_BLOCK / 32][MAX_EXPERTS];
-    __shared__ int tot[MAX_EXPERTS], off[MAX_EXPERTS + 1], poff[MAX_EXPERTS + 1];
-    __shared__ int bad;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < (PLAN_BLOCK / 32) * MAX_EXPERTS; i += PLAN_BLOCK) (&warp_cnt[0][0])[i] = 0;
-    if (threadIdx.x == 0) bad = 0;
-    __syncthreads();
-    const int i = threadIdx.x;
-    bool valid = i < R;
-    int e = valid ? top_idx[i] : 0;
-    if (valid && (unsigned)e >= (unsigned)E) {
-        bad = 1;
-        valid = false;
-    }
-    if (!valid) e = -1 - lane;
-    const unsigned peers = __match_any_sync(0xffffffffu, e);
-    const int rank_in_warp = __popc(peers & ((1u << lane) - 1u));
-    if (valid && rank_in_warp == 0) warp_cnt[warp][e] = __popc(peers);
-    __syncthreads();
-    if (threadIdx.x < E) {
-        int t = 0;
-        for (int w = 0; w < PLAN_BLOCK / 32; ++w) t += warp_cnt[w][threadIdx.x];
-        tot[threadIdx.x] = t;
-        counts[threadIdx.x] = t;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int o = 0, p = 0;
-        for (int x = 0; x < E; ++x) {
-            off[x] = o; poff[x] = p;
-            offsets[x] = o; padded_offsets[x] = p;
-            const int tiles = (tot[x] + ROW_TILE - 1) / ROW_TILE;
-            o += tot[x]; p += tiles * ROW_TILE;
-        }
-        off[E] = o; poff[E] = p;
-        padded_offsets[E] = p;
-        *n_tiles = p / ROW_TILE;
-        const int st = (p / ROW_TILE > max_tiles ? ST_PLAN_OVERFLOW : 0) | (bad ? ST_BAD_EXPERT : 0);
-        *status = st;
-        if (sticky && st) atomicOr(sticky, st);
-    }
-    __syncthreads();
-    if (threadIdx.x < E) {
-        const int x = threadIdx.x;
-        const int t0 = poff[x] / ROW_TILE, t1 = poff[x + 1] / ROW_TILE;
-        for (int t = t0; t < t1 && t < max_tiles; ++t) tile_expert[t] = x;
-        for (int q = poff[x] + tot[x]; q < poff[x + 1]; ++q) row_src[q] = -1;
-    }
-    if (valid) {
-        int base = 0;
-        for (int w = 0; w < warp; ++w) base += warp_cnt[w][e];
-        const int r = base + rank_in_warp;
-        const int slot = off[e] + r, p = poff[e] + r;
-        map[slot] = i;
-        pos[i] = p;
-        row_src[p] = i;
-        if (slot_of) slot_of[i] = slot;
-    }
+    __shared__ PlanShared sh;
+    plan_block<16>(p, sh);
 }
 
 // Xg[p,:] = x[row_src[p]/k,:]  (zero for padding rows).  One warp per row, 16-byte accesses.
@@ -411,38 +351,34 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(BiasGradArgs a)
 
 }  // namespace
 
-// The three plan kernels on explicit buffers.  `blk` is scratch of plan_blocks*E ints:
-// every element is written by plan_count_kernel before it is read, so it needs no clearing.
-int run_plan(const int32_t* top_idx, int R, int E, int32_t* counts, int32_t* offsets, int32_t* padded_offsets,
-             int32_t* tile_expert, int32_t* n_tiles, int max_tiles, int32_t* map, int32_t* pos,
-             int32_t* row_src, int row_cap, int32_t* status, int32_t* blk, cudaStream_t st, int32_t* slot_of,
-             int32_t* sticky)
+// The plan on explicit buffers.  `blk` is scratch of plan_blocks*E ints: every element is written by plan_count_kernel
+// before it is read, so it needs no clearing.  (Rows beyond the plan's tiles are never read.)
+static int run_plan_args(const PlanArgs& p, int32_t* blk, cudaStream_t st)
 {
-    const int plan_blocks = R > 0 ? (R + PLAN_BLOCK - 1) / PLAN_BLOCK : 1;
-    if (R <= PLAN_BLOCK) {
-        MGPT_CUDA(launch_pdl(plan_small_kernel, 1, PLAN_BLOCK, 0, st, top_idx, R, E, counts, offsets, padded_offsets, tile_expert, n_tiles,
-                                                    max_tiles, map, pos, row_src, slot_of, status, sticky));
+    if (p.R <= PLAN_BLOCK) {
+        MGPT_CUDA(launch_pdl(plan_small_kernel, 1, 512, 0, st, p));
         MGPT_LAUNCHED("plan_small_kernel");
         return 0;
     }
-    (void)row_cap;      // rows beyond the plan's tiles are never read; padding rows are marked by plan_assign_kernel
-    MGPT_CUDA(launch_pdl(plan_count_kernel, plan_blocks, PLAN_BLOCK, 0, st, top_idx, R, E, blk));
+    const int plan_blocks = (p.R + PLAN_BLOCK - 1) / PLAN_BLOCK;
+    MGPT_CUDA(launch_pdl(plan_count_kernel, plan_blocks, PLAN_BLOCK, 0, st, p.top_idx, p.R, p.E, blk, p.status));
     MGPT_LAUNCHED("plan_count_kernel");
-    MGPT_CUDA(launch_pdl(plan_scan_kernel, 1, MAX_EXPERTS, 0, st, blk, plan_blocks, E, counts, offsets, padded_offsets, tile_expert,
-                                                n_tiles, max_tiles, status, sticky));
-    MGPT_LAUNCHED("plan_scan_kernel");
-    MGPT_CUDA(launch_pdl(plan_assign_kernel, plan_blocks, PLAN_BLOCK, 0, st, top_idx, R, E, blk, counts, offsets, padded_offsets, map, pos,
-                                                           row_src, slot_of, status, sticky));
+    MGPT_CUDA(launch_pdl(plan_assign_kernel, plan_blocks, PLAN_BLOCK, 0, st, p, plan_blocks, blk));
     MGPT_LAUNCHED("plan_assign_kernel");
     return 0;
 }
 
+PlanArgs plan_args(const Dims& d, const Workspace& w, char* ws, int32_t* sticky)
+{
+    auto I = [&](size_t o) { return (int32_t*)(ws + o); };
+    return PlanArgs{I(w.top_idx), w.R, d.E, I(w.counts), I(w.offsets), I(w.padded_offsets), I(w.tile_expert), I(w.n_tiles), w.max_tiles,
+                    I(w.map), I(w.pos), I(w.row_src), I(w.slot), I(w.status), sticky, w.decode ? (int4*)(ws + w.groups) : nullptr,
+                    I(w.n_groups)};
+}
+
 int launch_plan(const Dims& d, const Workspace& w, char* ws, cudaStream_t st, int32_t* sticky)
 {
-    return run_plan((const int32_t*)(ws + w.top_idx), w.R, d.E, (int32_t*)(ws + w.counts), (int32_t*)(ws + w.offsets),
-                    (int32_t*)(ws + w.padded_offsets), (int32_t*)(ws + w.tile_expert), (int32_t*)(ws + w.n_tiles),
-                    w.max_tiles, (int32_t*)(ws + w.map), (int32_t*)(ws + w.pos), (int32_t*)(ws + w.row_src),
-                    w.row_cap, (int32_t*)(ws + w.status), (int32_t*)(ws + w.blk_cnt), st, (int32_t*)(ws + w.slot), sticky);
+    return run_plan_args(plan_args(d, w, ws, sticky), (int32_t*)(ws + w.blk_cnt), st);
 }
 
 // dst[p,:] = src[row_src[p]/k,:] for p < rows (zero where row_src[p] < 0).  rows < 0: every tile of the plan.
@@ -637,8 +573,8 @@ extern "C" int mgpt_moe_op_plan(const int32_t* top_idx, int n_rows, int E, int32
     MGPT_TRY(check_plan_args(top_idx, n_rows, E, outs, 10, row_cap));
     if (scratch_bytes < mgpt_moe_op_plan_scratch_bytes(n_rows, E))
         return fail(MGPT_MOE_ENOMEM, "scratch smaller than mgpt_moe_op_plan_scratch_bytes()");
-    return run_plan(top_idx, n_rows, E, counts, offsets, padded_offsets, tile_expert, n_tiles, row_cap / ROW_TILE, map,
-                    pos, row_src, row_cap, status, (int32_t*)scratch, (cudaStream_t)stream, nullptr, nullptr);
+    return run_plan_args(PlanArgs{top_idx, n_rows, E, counts, offsets, padded_offsets, tile_expert, n_tiles, row_cap / ROW_TILE, map, pos,
+                                  row_src, nullptr, status, nullptr, nullptr, nullptr}, (int32_t*)scratch, (cudaStream_t)stream);
 }
 
 // ---- dispatch plan without any allocation ------------------------------------------
@@ -690,6 +626,6 @@ extern "C" int mgpt_moe_op_plan_noalloc(const int32_t* top_idx, int n_rows, int 
     MGPT_TRY(plan_static_scratch(&scratch));
     // The array still holds the previous call's block bases.  Nothing has to be cleared:
     // plan_count_kernel writes all plan_blocks*E entries this call reads before they are read.
-    return run_plan(top_idx, n_rows, E, counts, offsets, padded_offsets, tile_expert, n_tiles, row_cap / ROW_TILE, map,
-                    pos, row_src, row_cap, status, scratch, (cudaStream_t)stream, nullptr, nullptr);
+    return run_plan_args(PlanArgs{top_idx, n_rows, E, counts, offsets, padded_offsets, tile_expert, n_tiles, row_cap / ROW_TILE, map, pos,
+                                  row_src, nullptr, status, nullptr, nullptr, nullptr}, scratch, (cudaStream_t)stream);
 }
