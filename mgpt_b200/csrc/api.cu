@@ -5,7 +5,7 @@
 #include <cstdlib>
 #include <cstring>
 
-#include "common.cuh"
+#include "plan_block.cuh"
 
 namespace mgpt {
 
@@ -540,18 +540,21 @@ static int forward_impl(mgpt_moe_layer* L, const void* x, void* y, int n_tokens,
                                   cudaMemcpyDeviceToDevice, st));
         L->stage_end(ST_PLAN, st);
     } else {
+        bool planned = false;
         if (n_tokens > 0) {
             L->stage_begin(ST_ROUTER, st);
+            const PlanArgs plan = plan_args(d, w, ws, L->d_status);
             if (tc_router_usable(L, x, io, n_tokens))
                 MGPT_TRY(tc_router_fwd(L, w, ws, x, st));
             else
                 MGPT_TRY(launch_router_fwd(x, io, L->p_data[0], L->p_data[1], n_tokens, d.C, d.E, d.k,
                                            (float*)(ws + w.logits), (float*)(ws + w.probs),
-                                           (int32_t*)(ws + w.top_idx), (float*)(ws + w.top_p), st));
+                                           (int32_t*)(ws + w.top_idx), (float*)(ws + w.top_p), st, nullptr, nullptr,
+                                           L->d_status, use_tc(L) ? &plan : nullptr, L->d_status + 4, &planned));
             L->stage_end(ST_ROUTER, st);
         }
         L->stage_begin(ST_PLAN, st);
-        MGPT_TRY(launch_plan(d, w, ws, st, L->d_status));
+        if (!planned) MGPT_TRY(launch_plan(d, w, ws, st, L->d_status));
         L->stage_end(ST_PLAN, st);
     }
     if (n_tokens > 0) {

@@ -163,7 +163,7 @@ struct mgpt_moe_layer {
 
     // Error bits of every kernel of this layer since the last mgpt_moe_check_status (device word, zero at create)
     // and the pinned host word they are read into.
-    int32_t* d_status = nullptr;
+    int32_t* d_status = nullptr;             // [0] the error bits, [4] blocks of the router that have finished (with a plan)
     int32_t* h_status = nullptr;
     bool router_dx_attr[2] = {};             // shared-memory opt-in of router_dx_kernel (1 / 4 tokens per thread) done on this layer's device
     bool router_tc_attr = false;             // the same for tc_router_fwd_kernel
@@ -240,7 +240,8 @@ inline char* buf_dXg(const mgpt_moe_layer* L, const Workspace& w, char* ws) { re
 // router.cu
 int launch_router_fwd(const void* x, int io, const float* Wr, const float* br, int N, int C, int E, int k,
                       float* logits, float* probs, int32_t* top_idx, float* top_p, cudaStream_t st,
-                      const int32_t* list = nullptr, const int32_t* list_count = nullptr);
+                      const int32_t* list = nullptr, const int32_t* list_count = nullptr, int32_t* status = nullptr,
+                      const struct PlanArgs* plan = nullptr, int32_t* done = nullptr, bool* planned = nullptr);
 // router_tc.cu: the router for BF16 tokens -- tensor-core first pass plus exact recompute of the tokens whose
 // routing the first pass cannot prove
 bool tc_router_usable(const mgpt_moe_layer* L, const void* x, int io, int n_tokens);

@@ -11,13 +11,15 @@
 // Routing must equal the CPU reference bit for bit, so the gating product is
 // accumulated per (token, expert) sequentially over channels with a separate
 // FP32 multiply and add, exactly the order of the reference's i-k-j loop.
-#include "common.cuh"
+#include <atomic>
+
+#include "plan_block.cuh"
 
 namespace mgpt {
 
 namespace {
 
-constexpr int R_WARPS = 4;     // warps per CTA
+constexpr int R_WARPS = 4;     // warps per CTA of the kernel for any shape
 constexpr int R_CK = 32;       // channels staged per step
 constexpr int R_XPAD = 36;     // padded row of the staged x tile (floats): rows land in distinct banks
 
@@ -110,13 +112,332 @@ __device__ __forceinline__ void router_finish(const float (&acc)[TPW][EPL], cons
     }
 }
 
+// The exact router.  What bounds it at scale is FP32 issue (one multiply and one add per token, expert and channel) and
+// for small batches the addition chain of one (token, expert) pair, C additions of four cycles.  A thread owns TM tokens x
+// TE experts, so that operands read from shared memory are used several times, and reads the next eight channels' operands
+// while it works on these eight; Wr and the tokens' rows stream through a ring that two warps fill with cp.async (one
+// bulk copy per stage cost its issuing thread ~500 cycles, more than a small batch spends on the stage), and the four
+// compute warps never wait for each other while they add.  The softmax is spread the same way: exponentials by the
+// threads that hold the logits, sums and top-k -- sequential in the reference -- by one thread per token.  With
+// plan.top_idx set, the last block to finish also builds the dispatch plan (one launch less for small batches).
+// WV: a thread's experts are neighbours read with one 16-byte load (E a multiple of 4), else E/TE apart.
+//
+// Before (lane = expert, chunks of 32 channels through registers or cp.async with a block barrier per chunk) -> now, us:
+// 64 tokens, C=1024, E=32, with the plan 22 -> 19; 1777 tokens 33 -> 20; 4096 tokens 33 -> 26; 8192 tokens, C=512, E=16
+// 19 -> 18; ~3900 listed tokens, C=2048, E=64 132 -> 99.
+struct RouterArgs {
+    const void* x;
+    const float *Wr, *br;
+    int N, C, E, k;
+    int ck, stages, tok;    // channels (a power of two) and stages of the ring, tokens per CTA
+    float *logits, *probs;
+    int32_t* top_idx;
+    float* top_p;
+    const int32_t *list, *list_count;
+    int32_t* status;        // error word (null: none)
+    int32_t* done;          // blocks finished, zero between launches (with a plan)
+    PlanArgs plan;
+};
+
+constexpr int RX_COMPUTE = 128, RX_PRODUCE = 64, RX_THREADS = RX_COMPUTE + RX_PRODUCE, RX_MAX_STAGES = 16;
+__host__ __device__ inline uint32_t rx_x_row(int ck, int elt) { return (uint32_t)(ck * elt + 16); }      // padded: rows in distinct banks
+__host__ __device__ inline uint32_t rx_stage(int ck, int E, int tok, int elt)
+{
+    return ((uint32_t)ck * E * 4 + tok * rx_x_row(ck, elt) + 127u) & ~127u;
+}
+// logits, exponentials [tok][E+1]; maximum and scale [tok]
+__host__ __device__ inline uint32_t rx_tail(int tok, int E) { return (uint32_t)tok * (2 * (E + 1) + 2) * 4; }
+
+// 8 consecutive channels of a staged row
+template <typename TIn> struct Row8;
+template <> struct Row8<bf16> {
+    uint4 u;
+    __device__ __forceinline__ void load(const uint8_t* p) { u = *reinterpret_cast<const uint4*>(p); }
+    __device__ __forceinline__ float get(int i) const
+    {
+        const uint32_t w = i < 2 ? u.x : i < 4 ? u.y : i < 6 ? u.z : u.w;
+        return __uint_as_float((i & 1) ? w & 0xffff0000u : w << 16);
+    }
+};
+template <> struct Row8<float> {
+    float4 a, b;
+    __device__ __forceinline__ void load(const uint8_t* p)
+    {
+        a = *reinterpret_cast<const float4*>(p);
+        b = *reinterpret_cast<const float4*>(p + 16);
+    }
+    __device__ __forceinline__ float get(int i) const
+    {
+        const float4& f = i < 4 ? a : b;
+        return (i & 3) == 0 ? f.x : (i & 3) == 1 ? f.y : (i & 3) == 2 ? f.z : f.w;
+    }
+};
+
+// One token's sum, scale and top-k from its exponentials: the reference's order and its strict '>' insertion
+// (utils/Tensor.cpp:850-883, 1296-1334).  K: k rounded up.
+template <int K>
+__device__ __forceinline__ float rx_top(const float* ex, int E, int k, int32_t* top_idx, float* top_p)
+{
+    float sum = 0.0f;
+#pragma unroll 8
+    for (int e = 0; e < E; ++e) sum = __fadd_rn(sum, ex[e]);
+    const float inv = __fdiv_rn(1.0f, fmaxf(sum, 1e-15f));
+    float val[K];
+    int idx[K];
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+        val[j] = -INFINITY;
+        idx[j] = -1;
+    }
+#pragma unroll 4
+    for (int e = 0; e < E; ++e) {
+        float v = fminf(fmaxf(__fmul_rn(ex[e], inv), 1e-7f), 1.0f);
+        int i = e;
+        // (an entry displaced from place j is larger than, or equal to and earlier than, everything after it)
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+            const bool up = v > val[j] || (v == val[j] && i < idx[j]);
+            const float tv = up ? val[j] : v;
+            const int ti = up ? idx[j] : i;
+            val[j] = up ? v : val[j];
+            idx[j] = up ? i : idx[j];
+            v = tv;
+            i = ti;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < K; ++j)
+        if (j < k) {
+            top_idx[j] = idx[j];
+            top_p[j] = val[j];
+        }
+    return inv;
+}
+
+template <typename TIn, int TM, int TE, bool WV>
+__global__ void __launch_bounds__(RX_THREADS) router_exact_kernel(const RouterArgs p)
+{
+    extern __shared__ __align__(128) uint8_t rx_smem[];
+    __shared__ __align__(8) uint64_t bars[2 * RX_MAX_STAGES];
+    __shared__ int last;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int C = p.C, E = p.E, CK = p.ck, ST = p.stages, TOK = p.tok;
+    const uint32_t x_row = rx_x_row(CK, sizeof(TIn)), x_off = (uint32_t)CK * E * 4, stage = rx_stage(CK, E, TOK, sizeof(TIn));
+    uint8_t* const ring = rx_smem;
+    const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(bars);
+    auto full = [&](int s) { return bar0 + 8u * s; };
+    auto empty = [&](int s) { return bar0 + 8u * (RX_MAX_STAGES + s); };
+    if (tid == 0) {
+        for (int s = 0; s < ST; ++s) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(full(s)), "r"(RX_PRODUCE));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(empty(s)), "r"(RX_COMPUTE / 32));
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    pdl_wait();
+    const int n_active = p.list ? *p.list_count : p.N;
+    const int n_tiles = (n_active + TOK - 1) / TOK;
+    auto wait = [&](uint32_t bar, uint32_t parity) {
+        for (uint32_t i = 0; i < (1u << 20); ++i) {
+            uint32_t ok;
+            asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+            if (ok) return;
+        }
+        if (p.status) atomicOr(p.status, ST_FULL_WAIT);
+    };
+
+    if (tid >= RX_COMPUTE) {
+        // fills the ring
+        constexpr int XV = 16 / sizeof(TIn);
+        const int per_log = __ffs(CK / XV) - 1, pt = tid - RX_COMPUTE;        // 16-byte pieces per row and chunk
+        int s = 0;
+        uint32_t round = 0;
+        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+            const int n = min(TOK, n_active - tile * TOK);
+            for (int c0 = 0; c0 < C; c0 += CK) {
+                if (round > 0) wait(empty(s), (round - 1) & 1);
+                const int len = min(CK, C - c0), pieces = len / XV, wp = len * E / 4;
+                const uint32_t dst = (uint32_t)__cvta_generic_to_shared(ring + s * stage);
+                const float* src = p.Wr + (size_t)c0 * E;
+#pragma unroll 4
+                for (int v = pt; v < wp; v += RX_PRODUCE)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + v * 16), "l"(src + v * 4) : "memory");
+                for (int v = pt; v < n << per_log; v += RX_PRODUCE) {
+                    const int i = v >> per_log, q = v & ((1 << per_log) - 1);
+                    if (q < pieces) {
+                        const int tok = p.list ? __ldg(p.list + tile * TOK + i) : tile * TOK + i;
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+                                     ::"r"(dst + x_off + i * x_row + q * 16), "l"((const TIn*)p.x + (size_t)tok * C + c0 + q * XV) : "memory");
+                    }
+                }
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full(s)) : "memory");
+                if (++s == ST) {
+                    s = 0;
+                    ++round;
+                }
+            }
+        }
+    } else {
+        float* const lg = reinterpret_cast<float*>(rx_smem + ST * stage);
+        float* const ex = lg + TOK * (E + 1);
+        float* const smax = ex + TOK * (E + 1);
+        float* const sinv = smax + TOK;
+        const int ET = (E + TE - 1) / TE, te = tid % ET, tt = tid / ET, TT = TOK / TM;
+        const bool works = tt < TT;
+        int eo[TE];                                     // this thread's experts (past the last: the last again, not stored)
+        float bias[TE];
+#pragma unroll
+        for (int j = 0; j < TE; ++j) {
+            eo[j] = WV ? te * TE + j : min(te + j * ET, E - 1);
+            bias[j] = p.br[eo[j]];
+        }
+        auto compute_sync = [] {
+            __syncwarp();
+            asm volatile("bar.sync 1, %0;" ::"n"(RX_COMPUTE) : "memory");
+        };
+        int s = 0;
+        uint32_t round = 0;
+        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+            const int n = min(TOK, n_active - tile * TOK);
+            float acc[TM][TE];
+#pragma unroll
+            for (int t = 0; t < TM; ++t)
+#pragma unroll
+                for (int j = 0; j < TE; ++j) acc[t][j] = 0.0f;
+            for (int c0 = 0; c0 < C; c0 += CK) {
+                const int len = min(CK, C - c0);
+                wait(full(s), round & 1);
+                if (works) {
+                    const float* ws = reinterpret_cast<const float*>(ring + s * stage);
+                    const uint8_t* xs = ring + s * stage + x_off + tt * x_row;
+                    struct Ops {
+                        float w[8][TE];
+                        Row8<TIn> x[TM];
+                    };
+                    auto load = [&](Ops& o, int c) {
+#pragma unroll
+                        for (int t = 0; t < TM; ++t) o.x[t].load(xs + t * TT * x_row + c * sizeof(TIn));
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            if constexpr (WV) {
+                                const float4 f = *reinterpret_cast<const float4*>(ws + (c + u) * E + eo[0]);
+                                o.w[u][0] = f.x; o.w[u][1] = f.y; o.w[u][2] = f.z; o.w[u][3] = f.w;
+                            } else {
+#pragma unroll
+                                for (int j = 0; j < TE; ++j) o.w[u][j] = ws[(c + u) * E + eo[j]];
+                            }
+                        }
+                    };
+                    // acc = fadd(acc, fmul(x, w)) in channel order, the reference's order; four channels' products first, so
+                    // that no addition waits for its product
+                    auto work = [&](const Ops& o) {
+#pragma unroll
+                        for (int h = 0; h < 8; h += 4) {
+                            float pr[4][TM][TE];
+#pragma unroll
+                            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                                for (int t = 0; t < TM; ++t) {
+                                    const float xv = o.x[t].get(h + u);
+#pragma unroll
+                                    for (int j = 0; j < TE; ++j) pr[u][t][j] = __fmul_rn(xv, o.w[h + u][j]);
+                                }
+#pragma unroll
+                            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                                for (int t = 0; t < TM; ++t)
+#pragma unroll
+                                    for (int j = 0; j < TE; ++j) acc[t][j] = __fadd_rn(acc[t][j], pr[u][t][j]);
+                        }
+                    };
+                    Ops a, b;
+                    load(a, 0);
+                    for (int c = 0; c + 16 <= len; c += 16) {
+                        load(b, c + 8);
+                        work(a);
+                        load(a, min(c + 16, len - 8));              // (the last one again: no branch)
+                        work(b);
+                    }
+                    if (len & 8) work(a);
+                }
+                __syncwarp();
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty(s)) : "memory");
+                if (++s == ST) {
+                    s = 0;
+                    ++round;
+                }
+            }
+            if (works)
+#pragma unroll
+                for (int t = 0; t < TM; ++t)
+#pragma unroll
+                    for (int j = 0; j < TE; ++j) {
+                        acc[t][j] = __fadd_rn(acc[t][j], bias[j]);
+                        if (WV || te + j * ET < E) lg[(tt + t * TT) * (E + 1) + eo[j]] = acc[t][j];
+                    }
+            compute_sync();
+            for (int i = tid; i < n; i += RX_COMPUTE) {
+                float mx = -INFINITY;
+#pragma unroll 8
+                for (int e = 0; e < E; ++e) mx = fmaxf(mx, lg[i * (E + 1) + e]);
+                smax[i] = mx;
+            }
+            compute_sync();
+            // exp through double and one rounding: agrees with a correctly rounded expf
+            if (works)
+#pragma unroll
+                for (int t = 0; t < TM; ++t)
+#pragma unroll
+                    for (int j = 0; j < TE; ++j) {
+                        const int i = tt + t * TT;
+                        if (i < n && (WV || te + j * ET < E)) ex[i * (E + 1) + eo[j]] = (float)exp((double)__fsub_rn(acc[t][j], smax[i]));
+                    }
+            compute_sync();
+            for (int i = tid; i < n; i += RX_COMPUTE) {
+                const size_t tok = p.list ? p.list[tile * TOK + i] : tile * TOK + i;
+                const float* ei = ex + i * (E + 1);
+                int32_t* ti = p.top_idx + tok * p.k;
+                float* tp = p.top_p + tok * p.k;
+                sinv[i] = p.k <= 1 ? rx_top<1>(ei, E, p.k, ti, tp) : p.k <= 2 ? rx_top<2>(ei, E, p.k, ti, tp)
+                        : p.k <= 4 ? rx_top<4>(ei, E, p.k, ti, tp) : rx_top<8>(ei, E, p.k, ti, tp);
+            }
+            compute_sync();
+            {
+                int i = tid / E, e = tid % E;
+                const int di = RX_COMPUTE / E, de = RX_COMPUTE % E;
+                while (i < n) {
+                    const size_t tok = p.list ? p.list[tile * TOK + i] : tile * TOK + i;
+                    p.probs[tok * E + e] = fminf(fmaxf(__fmul_rn(ex[i * (E + 1) + e], sinv[i]), 1e-7f), 1.0f);
+                    if (p.logits) p.logits[tok * E + e] = lg[i * (E + 1) + e];
+                    i += di;
+                    e += de;
+                    if (e >= E) {
+                        e -= E;
+                        ++i;
+                    }
+                }
+            }
+            compute_sync();                             // the tail may be overwritten
+        }
+    }
+    if (!p.plan.top_idx) return;
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) last = atomicAdd(p.done, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (tid == 0) *p.done = 0;
+    plan_block<RX_THREADS / 32>(p.plan, *reinterpret_cast<PlanShared*>(rx_smem));
+}
+
 // EL lanes share one token (lane % EL owns experts el, el+32, ...: EPL of them, EPL > 1 only
 // with EL = 32); a warp therefore works on 32/EL tokens at once and on TPW such groups in
 // sequence, which gives every lane TPW*EPL independent accumulation chains.
-// FAST: C is a multiple of 32 and E fills the staged columns exactly, so both tiles are copied
-// with 16-byte loads into registers one chunk ahead of the arithmetic (double-buffered tiles,
-// one barrier per chunk); otherwise a plain staged loop handles ragged shapes.
-template <typename TIn, int EL, int EPL, int TPW, bool FAST>
+// For shapes and addresses the kernel above cannot take (C not a multiple of 8, x or Wr not 16-byte aligned).
+template <typename TIn, int EL, int EPL, int TPW>
 __global__ void __launch_bounds__(R_WARPS * 32)
 router_fwd_kernel(const TIn* __restrict__ x, const float* __restrict__ Wr, const float* __restrict__ br,
                   int N, int C, int E, int k,
@@ -129,10 +450,9 @@ router_fwd_kernel(const TIn* __restrict__ x, const float* __restrict__ Wr, const
     constexpr int TOK_W = TPW * SUB;                // tokens per warp
     constexpr int TOK = R_WARPS * TOK_W;            // tokens per CTA
     constexpr int WCOLS = EPL * EL;                 // staged expert columns
-    constexpr int NBUF = FAST ? 2 : 1;
     constexpr int THREADS = R_WARPS * 32;
-    __shared__ __align__(16) float xs[NBUF][TOK][R_XPAD];
-    __shared__ __align__(16) float wsm[NBUF][R_CK][WCOLS];
+    __shared__ __align__(16) float xs[TOK][R_XPAD];
+    __shared__ __align__(16) float wsm[R_CK][WCOLS];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int sub = lane / EL, el = lane % EL;
@@ -148,17 +468,6 @@ router_fwd_kernel(const TIn* __restrict__ x, const float* __restrict__ Wr, const
         stok[i] = idx < n_active ? (list ? list[idx] : idx) : -1;
     }
     __syncthreads();
-    if (list) {
-        // Listed tokens are scattered rows the first pass read a while ago: ask for all of each row now, so that the
-        // per-chunk loads below find it in L2 instead of paying a DRAM round trip per 32 channels.
-        const int lines = (C * (int)sizeof(TIn) + 127) / 128;
-        for (int i = tid; i < TOK * lines; i += THREADS) {
-            const int tok = stok[i / lines];
-            if (tok >= 0)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)(x + (size_t)tok * C) + (size_t)(i % lines) * 128));
-        }
-    }
-
     float acc[TPW][EPL];
 #pragma unroll
     for (int t = 0; t < TPW; ++t)
@@ -166,18 +475,18 @@ router_fwd_kernel(const TIn* __restrict__ x, const float* __restrict__ Wr, const
         for (int i = 0; i < EPL; ++i) acc[t][i] = 0.0f;
 
     // sequential over the 32 staged channels: acc = fadd(acc, fmul(x, w)), the reference's order
-    auto compute = [&](int buf) {
+    auto compute = [&]() {
 #pragma unroll 2
         for (int j = 0; j < R_CK; j += 4) {
             float4 xv[TPW];
 #pragma unroll
             for (int t = 0; t < TPW; ++t)
-                xv[t] = *reinterpret_cast<const float4*>(&xs[buf][warp * TOK_W + t * SUB + sub][j]);
+                xv[t] = *reinterpret_cast<const float4*>(&xs[warp * TOK_W + t * SUB + sub][j]);
 #pragma unroll
             for (int jj = 0; jj < 4; ++jj) {
                 float w[EPL];
 #pragma unroll
-                for (int i = 0; i < EPL; ++i) w[i] = wsm[buf][j + jj][el + 32 * i];
+                for (int i = 0; i < EPL; ++i) w[i] = wsm[j + jj][el + 32 * i];
 #pragma unroll
                 for (int t = 0; t < TPW; ++t) {
                     const float xe = jj == 0 ? xv[t].x : jj == 1 ? xv[t].y : jj == 2 ? xv[t].z : xv[t].w;
@@ -188,188 +497,26 @@ router_fwd_kernel(const TIn* __restrict__ x, const float* __restrict__ Wr, const
         }
     };
 
-    if constexpr (FAST) {
-        constexpr int XV = 16 / sizeof(TIn);            // elements per 16-byte piece
-        constexpr int XPT = R_CK / XV;                  // pieces per token per chunk
-        constexpr int X_VECS = TOK * XPT, X_PER = (X_VECS + THREADS - 1) / THREADS;
-        constexpr int W_VECS = R_CK * WCOLS / 4, W_PER = (W_VECS + THREADS - 1) / THREADS;
-        uint4 xr[X_PER];
-        float4 wr[W_PER];
-        auto gload = [&](int c0) {
-#pragma unroll
-            for (int u = 0; u < X_PER; ++u) {
-                const int v = tid + u * THREADS;
-                xr[u] = make_uint4(0, 0, 0, 0);
-                if (v < X_VECS) {
-                    const int tok = stok[v / XPT];
-                    if (tok >= 0) xr[u] = *reinterpret_cast<const uint4*>(x + (size_t)tok * C + c0 + (v % XPT) * XV);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < W_PER; ++u) {
-                const int v = tid + u * THREADS;
-                if (v < W_VECS) wr[u] = *reinterpret_cast<const float4*>(Wr + (size_t)c0 * E + v * 4);
-            }
-        };
-        auto sstore = [&](int buf) {
-#pragma unroll
-            for (int u = 0; u < X_PER; ++u) {
-                const int v = tid + u * THREADS;
-                if (v < X_VECS) {
-                    float* dst = &xs[buf][v / XPT][(v % XPT) * XV];
-                    if constexpr (sizeof(TIn) == 2) {
-                        const uint32_t w4[4] = {xr[u].x, xr[u].y, xr[u].z, xr[u].w};
-                        *reinterpret_cast<float4*>(dst) = make_float4(
-                            __uint_as_float(w4[0] << 16), __uint_as_float(w4[0] & 0xffff0000u),
-                            __uint_as_float(w4[1] << 16), __uint_as_float(w4[1] & 0xffff0000u));
-                        *reinterpret_cast<float4*>(dst + 4) = make_float4(
-                            __uint_as_float(w4[2] << 16), __uint_as_float(w4[2] & 0xffff0000u),
-                            __uint_as_float(w4[3] << 16), __uint_as_float(w4[3] & 0xffff0000u));
-                    } else {
-                        *reinterpret_cast<uint4*>(dst) = xr[u];
-                    }
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < W_PER; ++u) {
-                const int v = tid + u * THREADS;
-                if (v < W_VECS) *reinterpret_cast<float4*>(&wsm[buf][0][0] + v * 4) = wr[u];
-            }
-        };
-        const int nchunks = C / R_CK;
-        gload(0);
-        sstore(0);
+    for (int c0 = 0; c0 < C; c0 += R_CK) {
+        // stage x[tok0.., c0..c0+31] and Wr[c0..c0+31, :] (zero padded: adding 0*w is exact)
+#pragma unroll 4
+        for (int i = tid; i < TOK * R_CK; i += THREADS) {
+            const int t = i / R_CK, j = i % R_CK;
+            const int tok = stok[t], c = c0 + j;
+            xs[t][j] = (tok >= 0 && c < C) ? to_f32(x[(size_t)tok * C + c]) : 0.0f;
+        }
+#pragma unroll 4
+        for (int i = tid; i < R_CK * WCOLS; i += THREADS) {
+            const int j = i / WCOLS, e = i % WCOLS;
+            const int c = c0 + j;
+            wsm[j][e] = (c < C && e < E) ? Wr[(size_t)c * E + e] : 0.0f;
+        }
         __syncthreads();
-        for (int ci = 0; ci < nchunks; ++ci) {
-            const bool more = ci + 1 < nchunks;
-            if (more) gload((ci + 1) * R_CK);          // next chunk's loads fly during this chunk's arithmetic
-            compute(ci & 1);
-            if (more) sstore((ci + 1) & 1);
-            __syncthreads();
-        }
-    } else {
-        for (int c0 = 0; c0 < C; c0 += R_CK) {
-            // stage x[tok0.., c0..c0+31] and Wr[c0..c0+31, :] (zero padded: adding 0*w is exact)
-#pragma unroll 4
-            for (int i = tid; i < TOK * R_CK; i += THREADS) {
-                const int t = i / R_CK, j = i % R_CK;
-                const int tok = stok[t], c = c0 + j;
-                xs[0][t][j] = (tok >= 0 && c < C) ? to_f32(x[(size_t)tok * C + c]) : 0.0f;
-            }
-#pragma unroll 4
-            for (int i = tid; i < R_CK * WCOLS; i += THREADS) {
-                const int j = i / WCOLS, e = i % WCOLS;
-                const int c = c0 + j;
-                wsm[0][j][e] = (c < C && e < E) ? Wr[(size_t)c * E + e] : 0.0f;
-            }
-            __syncthreads();
-            compute(0);
-            __syncthreads();
-        }
+        compute();
+        __syncthreads();
     }
 
     router_finish<EL, EPL, TPW>(acc, stok, warp, sub, el, E, k, br, logits, probs, top_idx, top_p);
-}
-
-// The exact pass over a LIST of tokens (second pass of the screened router): a few thousand tokens, so only a CTA or
-// two per SM, and what decides the time is the latency of one CTA's 64 chunk steps.  The chunks therefore come
-// through a ring of shared-memory stages filled by cp.async three chunks ahead (the kernel above loads one chunk
-// ahead through registers, which is enough only when a dozen CTAs per SM hide each other's waits).  Same arithmetic:
-// one warp pass per token, lane el owns experts el, el+32, ..., acc = fadd(acc, fmul(x, w)) in channel order.
-// Needs C % 32 == 0, E == 32*EPL and 16-byte aligned x and Wr.
-// TPW tokens per warp: 4 for the list pass (fewer instructions per token), 1 for decode batches without a list
-// (tokens 0..N-1; the shortest chains per lane, so that a handful of CTAs finish soonest).
-template <typename TIn, int EPL, int TPW>
-__global__ void __launch_bounds__(R_WARPS * 32)
-router_list_kernel(const TIn* __restrict__ x, const float* __restrict__ Wr, const float* __restrict__ br,
-                   int N, int C, int E, int k, float* __restrict__ logits, float* __restrict__ probs,
-                   int32_t* __restrict__ top_idx, float* __restrict__ top_p,
-                   const int32_t* __restrict__ list, const int32_t* __restrict__ list_count)
-{
-    pdl_wait();
-    constexpr int TOK = R_WARPS * TPW, WCOLS = 32 * EPL, THREADS = R_WARPS * 32;
-    constexpr int ST = EPL <= 2 ? 4 : 2;            // stages: 36 KiB of static shared memory at most
-    constexpr int XV = 16 / sizeof(TIn);            // elements per 16-byte piece
-    constexpr int XPT = R_CK / XV;                  // pieces per token per chunk
-    constexpr int W_VECS = R_CK * WCOLS / 4;
-    __shared__ __align__(16) TIn xs[ST][TOK][R_CK];
-    __shared__ __align__(16) float wsm[ST][R_CK][WCOLS];
-    __shared__ int stok[TOK];
-
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n_active = list ? *list_count : N;
-    const int tok0 = blockIdx.x * TOK;
-    if (tok0 >= n_active) return;
-    for (int i = tid; i < TOK; i += THREADS) stok[i] = tok0 + i < n_active ? (list ? list[tok0 + i] : tok0 + i) : -1;
-    __syncthreads();
-
-    auto issue = [&](int ci, int buf) {
-        const int c0 = ci * R_CK;
-        for (int v = tid; v < W_VECS; v += THREADS) {
-            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&wsm[buf][0][0] + v * 4);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(Wr + (size_t)c0 * E + v * 4) : "memory");
-        }
-        for (int v = tid; v < TOK * XPT; v += THREADS) {
-            const int tok = stok[v / XPT];
-            TIn* d = &xs[buf][v / XPT][(v % XPT) * XV];
-            if (tok >= 0) {
-                const uint32_t dst = (uint32_t)__cvta_generic_to_shared(d);
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(x + (size_t)tok * C + c0 + (v % XPT) * XV) : "memory");
-            } else {
-                *reinterpret_cast<uint4*>(d) = make_uint4(0, 0, 0, 0);      // adding 0*w is exact
-            }
-        }
-    };
-
-    float acc[TPW][EPL];
-#pragma unroll
-    for (int t = 0; t < TPW; ++t)
-#pragma unroll
-        for (int i = 0; i < EPL; ++i) acc[t][i] = 0.0f;
-
-    auto compute = [&](int buf) {
-#pragma unroll 2
-        for (int j = 0; j < R_CK; j += 4) {
-            float xv[TPW][4];
-#pragma unroll
-            for (int t = 0; t < TPW; ++t) {
-                if constexpr (sizeof(TIn) == 2) {
-                    const uint2 u = *reinterpret_cast<const uint2*>(&xs[buf][warp * TPW + t][j]);
-                    xv[t][0] = __uint_as_float(u.x << 16); xv[t][1] = __uint_as_float(u.x & 0xffff0000u);
-                    xv[t][2] = __uint_as_float(u.y << 16); xv[t][3] = __uint_as_float(u.y & 0xffff0000u);
-                } else {
-                    const float4 f = *reinterpret_cast<const float4*>(&xs[buf][warp * TPW + t][j]);
-                    xv[t][0] = f.x; xv[t][1] = f.y; xv[t][2] = f.z; xv[t][3] = f.w;
-                }
-            }
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj) {
-                float w[EPL];
-#pragma unroll
-                for (int i = 0; i < EPL; ++i) w[i] = wsm[buf][j + jj][lane + 32 * i];
-#pragma unroll
-                for (int t = 0; t < TPW; ++t)
-#pragma unroll
-                    for (int i = 0; i < EPL; ++i) acc[t][i] = __fadd_rn(acc[t][i], __fmul_rn(xv[t][jj], w[i]));
-            }
-        }
-    };
-
-    const int nchunks = C / R_CK;
-#pragma unroll
-    for (int s = 0; s < ST - 1; ++s) {
-        if (s < nchunks) issue(s, s);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    for (int ci = 0; ci < nchunks; ++ci) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
-        __syncthreads();                               // chunk ci has landed for everyone; chunk ci-1's stage is free
-        const int nxt = ci + ST - 1;
-        if (nxt < nchunks) issue(nxt, nxt % ST);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        compute(ci % ST);
-    }
-    router_finish<32, EPL, TPW>(acc, stok, warp, 0, lane, E, k, br, logits, probs, top_idx, top_p);
 }
 
 // dlogits = P * (dP - <dP,P>),  dP = scatter(d_top_p) + alpha*E*f_e/N
@@ -653,78 +800,89 @@ router_wgrad_reduce_kernel(const float* __restrict__ part, const float* __restri
     }
 }
 
+template <typename TIn, int TM, int TE, bool WV>
+int router_exact_launch(RouterArgs p, int device, cudaStream_t st)
+{
+    auto* kernel = router_exact_kernel<TIn, TM, TE, WV>;
+    p.tok = RX_COMPUTE / ((p.E + TE - 1) / TE) * TM;
+    // stages of about 16-40 KiB; one CTA per SM takes what fits, more of them share.  A list's length is only known on the
+    // device.
+    for (p.ck = 128; p.ck > 16 && ((uint32_t)p.ck * p.E * 4 > 16384u || rx_stage(p.ck, p.E, p.tok, sizeof(TIn)) > 40960u);) p.ck /= 2;
+    const int ctas = (p.N + p.tok - 1) / p.tok, grid = p.list ? (ctas < 296 ? ctas : 296) : ctas;
+    const uint32_t stage = rx_stage(p.ck, p.E, p.tok, sizeof(TIn)), tail = rx_tail(p.tok, p.E);
+    const uint32_t budget = (grid <= 148 ? 200 : 104) * 1024u;
+    int stages = (int)((budget - tail) / stage);
+    const int chunks = (p.C + p.ck - 1) / p.ck;
+    if (stages > RX_MAX_STAGES) stages = RX_MAX_STAGES;
+    if (grid <= 148 && stages > chunks) stages = chunks;
+    p.stages = stages < 2 ? 2 : stages;
+    size_t smem = (size_t)p.stages * stage + tail;
+    if (p.plan.top_idx && smem < sizeof(PlanShared)) smem = sizeof(PlanShared);
+    static std::atomic<uint64_t> opted{0};             // devices that have the shared-memory opt-in (bit per ordinal)
+    if (device >= 64 || !(opted.load(std::memory_order_relaxed) >> device & 1)) {
+        MGPT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024));
+        if (device < 64) opted.fetch_or(1ull << device);
+    }
+    MGPT_CUDA(launch_pdl(kernel, grid, RX_THREADS, smem, st, p));
+    MGPT_LAUNCHED("router_exact_kernel");
+    return 0;
+}
+
+// One (token, expert) pair per thread while that leaves no SM more than one CTA, then four, then eight.
+template <typename TIn>
+int router_exact_dispatch(const RouterArgs& p, int device, cudaStream_t st)
+{
+    const long long pairs = (long long)p.N * p.E, wave = 148 * RX_COMPUTE;
+    const bool wv = p.E % 4 == 0;
+    if (!p.list && pairs <= wave) return router_exact_launch<TIn, 1, 1, false>(p, device, st);
+    if (!p.list && pairs <= 4 * wave)
+        return wv ? router_exact_launch<TIn, 1, 4, true>(p, device, st) : router_exact_launch<TIn, 1, 4, false>(p, device, st);
+    return wv ? router_exact_launch<TIn, 2, 4, true>(p, device, st) : router_exact_launch<TIn, 2, 4, false>(p, device, st);
+}
+
 template <typename TIn, int EL, int EPL, int TPW>
-int router_fwd_launch(const TIn* x, const float* Wr, const float* br, int N, int C, int E, int k,
-                      float* logits, float* probs, int32_t* top_idx, float* top_p, cudaStream_t st,
-                      const int32_t* list, const int32_t* list_count)
+int router_any_launch(const RouterArgs& p, cudaStream_t st)
 {
     constexpr int TOK = R_WARPS * TPW * (32 / EL);
-    const int grid = (N + TOK - 1) / TOK;
-    const bool fast = C % R_CK == 0 && E == EPL * EL && ((uintptr_t)x & 15) == 0 && ((uintptr_t)Wr & 15) == 0;
-    if (fast)
-        MGPT_CUDA(launch_pdl(router_fwd_kernel<TIn, EL, EPL, TPW, true>, grid, R_WARPS * 32, 0, st, x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, list, list_count));
-    else
-        MGPT_CUDA(launch_pdl(router_fwd_kernel<TIn, EL, EPL, TPW, false>, grid, R_WARPS * 32, 0, st, x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, list, list_count));
+    MGPT_CUDA(launch_pdl(router_fwd_kernel<TIn, EL, EPL, TPW>, (p.N + TOK - 1) / TOK, R_WARPS * 32, 0, st, (const TIn*)p.x, p.Wr, p.br, p.N,
+                         p.C, p.E, p.k, p.logits, p.probs, p.top_idx, p.top_p, p.list, p.list_count));
     MGPT_LAUNCHED("router_fwd_kernel");
     return 0;
 }
 
 template <typename TIn>
-int router_fwd_dispatch(const TIn* x, const float* Wr, const float* br, int N, int C, int E, int k,
-                        float* logits, float* probs, int32_t* top_idx, float* top_p, cudaStream_t st,
-                        const int32_t* list, const int32_t* list_count)
+int router_fwd_dispatch(const RouterArgs& p, int device, bool fast, cudaStream_t st)
 {
-    // Decode-sized batches: too few tokens to fill the device, what is left is the latency of one CTA, which is the
-    // length of its dependent addition chains: one token per warp pass keeps it shortest.
-    if (!list && N <= 1024 && C % R_CK == 0 && E % 32 == 0 && E <= 128 && E != 96 && ((uintptr_t)x & 15) == 0 &&
-        ((uintptr_t)Wr & 15) == 0) {
-        // the chunks through the cp.async ring: with a handful of CTAs, nothing else hides the loads of a chunk
-        const int grid = (N + R_WARPS - 1) / R_WARPS;
-        if (E == 32) MGPT_CUDA(launch_pdl(router_list_kernel<TIn, 1, 1>, grid, R_WARPS * 32, 0, st, x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, nullptr, nullptr));
-        else if (E == 64) MGPT_CUDA(launch_pdl(router_list_kernel<TIn, 2, 1>, grid, R_WARPS * 32, 0, st, x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, nullptr, nullptr));
-        else MGPT_CUDA(launch_pdl(router_list_kernel<TIn, 4, 1>, grid, R_WARPS * 32, 0, st, x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, nullptr, nullptr));
-        MGPT_LAUNCHED("router_list_kernel<decode>");
-        return 0;
-    }
-    if (!list && N <= 1024) {
-        if (E <= 8) return router_fwd_launch<TIn, 8, 1, 1>(x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, st, list, list_count);
-        if (E <= 16) return router_fwd_launch<TIn, 16, 1, 1>(x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, st, list, list_count);
-        if (E <= 32) return router_fwd_launch<TIn, 32, 1, 1>(x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, st, list, list_count);
-        if (E <= 64) return router_fwd_launch<TIn, 32, 2, 1>(x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, st, list, list_count);
-        return router_fwd_launch<TIn, 32, 4, 1>(x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, st, list, list_count);
-    }
-    // Second pass of the screened router: a fraction of the tokens, how many is only known on the device.  Small
-    // CTAs (16 tokens) so that the few thousand listed tokens still spread over every SM.
-    if (list && C % R_CK == 0 && E % 32 == 0 && E <= 128 && E != 96 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)Wr & 15) == 0) {
-        const int grid = (N + 15) / 16;
-        if (E == 32) MGPT_CUDA(launch_pdl(router_list_kernel<TIn, 1, 4>, grid, R_WARPS * 32, 0, st, x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, list, list_count));
-        else if (E == 64) MGPT_CUDA(launch_pdl(router_list_kernel<TIn, 2, 4>, grid, R_WARPS * 32, 0, st, x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, list, list_count));
-        else MGPT_CUDA(launch_pdl(router_list_kernel<TIn, 4, 4>, grid, R_WARPS * 32, 0, st, x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, list, list_count));
-        MGPT_LAUNCHED("router_list_kernel");
-        return 0;
-    }
-    if (list && E > 32 && E <= 64)
-        return router_fwd_launch<TIn, 32, 2, 4>(x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, st, list, list_count);
-    if (list && E > 16 && E <= 32)
-        return router_fwd_launch<TIn, 32, 1, 4>(x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, st, list, list_count);
-    if (E <= 8) return router_fwd_launch<TIn, 8, 1, 4>(x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, st, list, list_count);
-    if (E <= 16) return router_fwd_launch<TIn, 16, 1, 4>(x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, st, list, list_count);
-    if (E <= 32) return router_fwd_launch<TIn, 32, 1, 8>(x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, st, list, list_count);
-    if (E <= 64) return router_fwd_launch<TIn, 32, 2, 8>(x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, st, list, list_count);
-    return router_fwd_launch<TIn, 32, 4, 4>(x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, st, list, list_count);
+    if (fast) return router_exact_dispatch<TIn>(p, device, st);
+    if (p.E <= 32) return router_any_launch<TIn, 32, 1, 2>(p, st);
+    if (p.E <= 64) return router_any_launch<TIn, 32, 2, 2>(p, st);
+    return router_any_launch<TIn, 32, 4, 2>(p, st);
 }
 
 }  // namespace
 
-// list / list_count (device): run only on the tokens list[0 .. *list_count), at most N of them
+// list / list_count (device): run only on the tokens list[0 .. *list_count), at most N of them.  plan / done: the last
+// block builds the plan too; *planned says whether this launch does.
 int launch_router_fwd(const void* x, int io, const float* Wr, const float* br, int N, int C, int E, int k,
                       float* logits, float* probs, int32_t* top_idx, float* top_p, cudaStream_t st,
-                      const int32_t* list, const int32_t* list_count)
+                      const int32_t* list, const int32_t* list_count, int32_t* status, const PlanArgs* plan, int32_t* done, bool* planned)
 {
+    if (planned) *planned = false;
     if (N <= 0) return 0;
-    if (io == MGPT_MOE_IO_F32)
-        return router_fwd_dispatch((const float*)x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, st, list, list_count);
-    return router_fwd_dispatch((const bf16*)x, Wr, br, N, C, E, k, logits, probs, top_idx, top_p, st, list, list_count);
+    RouterArgs p = {};
+    p.x = x; p.Wr = Wr; p.br = br; p.N = N; p.C = C; p.E = E; p.k = k;
+    p.logits = logits; p.probs = probs; p.top_idx = top_idx; p.top_p = top_p;
+    p.list = list; p.list_count = list_count; p.status = status;
+    const bool fast = C % 8 == 0 && (((uintptr_t)x | (uintptr_t)Wr) & 15) == 0;
+    if (fast && plan && plan->R <= 256) {      // (more rows: six warps take longer than the plan's own kernel and its launch)
+        p.plan = *plan;
+        p.done = done;
+        *planned = true;
+    }
+    int device = 0;
+    MGPT_CUDA(cudaGetDevice(&device));
+    if (io == MGPT_MOE_IO_F32) return router_fwd_dispatch<float>(p, device, fast, st);
+    return router_fwd_dispatch<bf16>(p, device, fast, st);
 }
 
 template <int TPT>

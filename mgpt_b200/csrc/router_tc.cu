@@ -363,7 +363,7 @@ int tc_router_fwd(mgpt_moe_layer* L, const Workspace& w, char* ws, const void* x
     }
     // exact pass over the listed tokens (how many is known only on the device: CTAs beyond the list leave at once)
     return launch_router_fwd(x, MGPT_MOE_IO_BF16, L->p_data[0], L->p_data[1], N, d.C, d.E, d.k, p.logits, p.probs,
-                             p.top_idx, p.top_p, st, p.list, p.list_count);
+                             p.top_idx, p.top_p, st, p.list, p.list_count, L->d_status);
 }
 
 int router_tc_ne(int E) { return router_ne(E); }
