@@ -77,7 +77,16 @@ __device__ __forceinline__ void put(float* S, int t, const float4 (&r)[2])
         }
     }
 }
+// Two FP32 multiply-adds in one instruction: they take the FMA pipe as long as two would and leave every other issue slot to
+// the loads.  Worth it where an SM has 16 warps to issue from (KS > 1: dXg 38 -> 33 us, down 20 -> 19); with half of them
+// the pairs' register moves cost more (gate-up 24 -> 26).
+__device__ __forceinline__ void fma2(float& d0, float& d1, float a0, float a1, float b)
+{
+    asm("{\n .reg .b64 ra, rb, rd;\n mov.b64 ra, {%2, %3};\n mov.b64 rb, {%4, %4};\n mov.b64 rd, {%0, %1};\n"
+        " fma.rn.f32x2 rd, ra, rb, rd;\n mov.b64 {%0, %1}, rd;\n}" : "+f"(d0), "+f"(d1) : "f"(a0), "f"(a1), "f"(b));
+}
 // acc[8][4] += rows ty*8.. x columns tx*4.. over the TK staged k
+template <bool PACK>
 __device__ __forceinline__ void mac(const float* As, const float* Bs, int ty, int tx, float (&acc)[8][4])
 {
 #pragma unroll
@@ -87,9 +96,16 @@ __device__ __forceinline__ void mac(const float* As, const float* Bs, int ty, in
         const float4 b = *reinterpret_cast<const float4*>(Bs + k * SROW + tx * 4);
         const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < 8; i += 2)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+            for (int j = 0; j < 4; ++j) {
+                if (PACK) {
+                    fma2(acc[i][j], acc[i + 1][j], av[i], av[i + 1], bv[j]);
+                } else {
+                    acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+                    acc[i + 1][j] = fmaf(av[i + 1], bv[j], acc[i + 1][j]);
+                }
+            }
     }
 }
 // The groups' sums, added to group 0's in group order.  S: shared memory of 64*64 floats per group beyond the first.
@@ -179,8 +195,8 @@ __global__ void __launch_bounds__(GT * KS) simt_rows_kernel(RowsArgs a)
         const int buf = (s - s0) & 1;
         if (s + 1 < s1) gload(s + 1);
         const float* c = S + buf * NOP * OPER;
-        mac(c, c + OPER, ty, tx, acc);
-        if (NOP == 3) mac(c, c + 2 * OPER, ty, tx, acc2);
+        mac<(KS > 1)>(c, c + OPER, ty, tx, acc);
+        if (NOP == 3) mac<(KS > 1)>(c, c + 2 * OPER, ty, tx, acc2);
         if (s + 1 < s1) sstore(buf ^ 1);
         group_sync(group);
     }
@@ -295,7 +311,7 @@ __global__ void __launch_bounds__(GT * KS) simt_wgrad_kernel(WgradArgs a)
             const int buf = (s - s0) & 1;
             if (s + 1 < s1) gload(s + 1);
             const float* c = S + buf * 2 * OPER;
-            mac(c, c + OPER, ty, tx, acc);
+            mac<(KS > 1)>(c, c + OPER, ty, tx, acc);
             if (bias && ty == 0)
 #pragma unroll
                 for (int k = 0; k < TK; ++k) {
@@ -317,11 +333,11 @@ __global__ void __launch_bounds__(GT * KS) simt_wgrad_kernel(WgradArgs a)
         if (threadIdx.x < TN && n0 + (int)threadIdx.x < N) {
             float v = 0.0f;
             for (int g = 0; g < KS; ++g) v += sb[g * TN + threadIdx.x];
-            a.gb[which][e][n0 + threadIdx.x] += v;
+            (which == 0 ? a.gb[0] : which == 1 ? a.gb[1] : a.gb[2])[e][n0 + threadIdx.x] += v;
         }
     }
     if (group > 0 || n >= N) return;
-    float* g = a.grad[which][e];
+    float* g = (which == 0 ? a.grad[0] : which == 1 ? a.grad[1] : a.grad[2])[e];      // (a dynamic index would copy the arguments to local memory)
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int m = m0 + ty * 8 + i;
