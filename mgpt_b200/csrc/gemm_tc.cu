@@ -63,26 +63,6 @@ __device__ __forceinline__ void add_bias32(float (&v)[32], const float* __restri
     }
 }
 
-__device__ __forceinline__ void load_bf16x32(const bf16* src, float (&v)[32], int valid)
-{
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        if (q * 8 < valid) {
-            const uint4 u = reinterpret_cast<const uint4*>(src)[q];
-            const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(&w[i]);
-                v[q * 8 + 2 * i] = __low2float(h);
-                v[q * 8 + 2 * i + 1] = __high2float(h);
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[q * 8 + i] = 0.0f;
-        }
-    }
-}
-
 // Shared memory of one CTA: operand ring, one 4 KiB staging tile per epilogue warp, barriers.
 struct Pipe {
     uint32_t bars, tmem_slot;          // shared-space addresses
@@ -287,10 +267,13 @@ struct RowsP {
     const bf16* gather_src;     // dXg rows [*, n_out]
     const int32_t* gather_pos;  // [tokens, gather_k] row of dXg for (token, j)
     int gather_k;
+    bf16* dx;                   // MODE_DX: the output
 };
 
 // The epilogue of one work item for one of the 16 epilogue warps: TMEM lane quarter q (rows q*32..+31 of the row
 // tile), column group h.  False: a bounded wait ran out.
+//
+// MODE_DX has its own (dx_epilogue).
 template <int MODE>
 __device__ __forceinline__ bool rows_epilogue(const RowsP& p, uint32_t acc_full_bar, uint32_t acc_empty_bar,
                                               uint32_t tmem_base, uint32_t buf, uint32_t t, int row_tile, int n0, int e,
@@ -390,38 +373,112 @@ __device__ __forceinline__ bool rows_epilogue(const RowsP& p, uint32_t acc_full_
                 stage_row_bf16(stage, lane, gw);
                 flush_stage(stage, tmD0, n, row_w, lane);
                 continue;
-            } else if (MODE == MODE_DX) {
-                // dx = (sum of the token's expert rows, ascending row order) + dlogits * Wr^T
-                const int tok = row_w + lane;
-                if (tok < p.n_valid_rows) {
-                    int ps[MAX_TOPK];
-#pragma unroll
-                    for (int j = 0; j < MAX_TOPK; ++j)
-                        ps[j] = j < p.gather_k ? p.gather_pos[(size_t)tok * p.gather_k + j] : 0x7fffffff;
-#pragma unroll
-                    for (int a = 0; a < MAX_TOPK - 1; ++a)
-#pragma unroll
-                        for (int b = 0; b < MAX_TOPK - 1 - a; ++b)
-                            if (ps[b] > ps[b + 1]) {
-                                const int tmp = ps[b];
-                                ps[b] = ps[b + 1];
-                                ps[b + 1] = tmp;
-                            }
-                    const int valid = min(32, p.n_out - n);
-#pragma unroll
-                    for (int j = 0; j < MAX_TOPK; ++j) {
-                        if (j < p.gather_k) {
-                            float g[32];
-                            load_bf16x32(p.gather_src + (size_t)ps[j] * p.n_out + n, g, valid);
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) v[i] += g[i];
-                        }
-                    }
-                }
             }
             pack32(v, pk);
             stage_row_bf16(stage, lane, pk);
             flush_stage(stage, tmD0, n, row_w, lane);
+        }
+    }
+    return true;
+}
+
+// dx = dlogits * Wr^T (the accumulator) + the token's expert rows in ascending order.  Bound by the gather of those rows
+// (64 bytes of a row at a time): with a lane per token every 16-byte load touched 32 lines, one cycle of the L1 each (155 us
+// for 402 MB at 32768 tokens, C=2048, top-2).  So four lanes share a row, eight rows per load, and the accumulator crosses
+// to that order through `stage` (32 rows x 32 columns FP32, padded); the positions are looked up once per item and the
+// first rows requested before the wait for the accumulator.
+constexpr int DX_LD = 36;                            // floats per staged row
+constexpr uint32_t DX_STAGING = 32 * DX_LD * 4;      // per epilogue warp
+static_assert(EPI_WARPS * DX_STAGING <= (STAGES - 2) * STAGE_BYTES, "the staging of dx lies in the unused stages");
+__device__ __forceinline__ bool dx_epilogue(const RowsP& p, uint32_t acc_full_bar, uint32_t acc_empty_bar, uint32_t tmem_base,
+                                            uint32_t buf, uint32_t t, int row_tile, int n0, int q, int h, int lane, float* stage,
+                                            bf16* __restrict__ dx)
+{
+    const int row_w = row_tile * BM + q * 32, rsub = lane >> 2, c8 = (lane & 3) * 8;
+    const int k = p.gather_k;
+    int ps[MAX_TOPK];                                // this lane's token's rows, ascending
+#pragma unroll
+    for (int j = 0; j < MAX_TOPK; ++j)
+        ps[j] = j < k && row_w + lane < p.n_valid_rows ? __ldg(p.gather_pos + (size_t)(row_w + lane) * k + j) : 0x7fffffff;
+#pragma unroll
+    for (int a = 0; a < MAX_TOPK - 1; ++a)
+        if (a < k - 1)
+#pragma unroll
+            for (int b = 0; b < MAX_TOPK - 1 - a; ++b)
+                if (b < k - 1 - a && ps[b] > ps[b + 1]) {
+                    const int tmp = ps[b];
+                    ps[b] = ps[b + 1];
+                    ps[b + 1] = tmp;
+                }
+    // rows 8g + rsub, eight columns from n + c8, of the j-th expert row
+    auto fetch = [&](uint4 (&v)[4], int psj, int n) {
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            const int row = __shfl_sync(0xffffffffu, psj, 8 * g + rsub);
+            v[g] = make_uint4(0, 0, 0, 0);
+            if (row_w + 8 * g + rsub < p.n_valid_rows && n + c8 < p.n_out)
+                v[g] = __ldg(reinterpret_cast<const uint4*>(p.gather_src + (size_t)row * p.n_out + n + c8));
+        }
+    };
+#pragma unroll
+    for (int un = 0; un < 2; ++un) {
+        const int n = n0 + h * 64 + un * 32;
+        uint4 r0[4], r1[4];
+        fetch(r0, ps[0], n);
+        if (k > 1) fetch(r1, ps[1], n);
+        if (un == 0) {
+            if (!mbar_wait(acc_full_bar, (t >> 1) & 1, p.status, ERR_ACC_WAIT)) return false;
+            tc_fence_after();
+        }
+        float v[32];
+        __syncwarp();                                // the tile staged before has been read
+        tmem_ld32(tmem_base + buf * BN + ((uint32_t)(q * 32) << 16) + h * 64 + un * 32, v);
+        tmem_ld_wait();
+        if (un == 1) release_acc(acc_empty_bar, lane);
+#pragma unroll
+        for (int i = 0; i < 32; i += 4)
+            *reinterpret_cast<float4*>(stage + lane * DX_LD + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+        __syncwarp();
+        float s[4][8];
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            const float* src = stage + (8 * g + rsub) * DX_LD + c8;
+            const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
+            s[g][0] = a.x; s[g][1] = a.y; s[g][2] = a.z; s[g][3] = a.w; s[g][4] = b.x; s[g][5] = b.y; s[g][6] = b.z; s[g][7] = b.w;
+        }
+        auto add = [&](const uint4 (&r)[4]) {
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                const uint32_t w[4] = {r[g].x, r[g].y, r[g].z, r[g].w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    s[g][2 * i] += bf_lo(w[i]);
+                    s[g][2 * i + 1] += bf_hi(w[i]);
+                }
+            }
+        };
+        add(r0);
+        if (k > 1) add(r1);
+#pragma unroll
+        for (int j = 2; j < MAX_TOPK; j += 2)
+            if (j < k) {
+                fetch(r0, ps[j], n);
+                if (j + 1 < k) fetch(r1, ps[j + 1], n);
+                add(r0);
+                if (j + 1 < k) add(r1);
+            }
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            const int tok = row_w + 8 * g + rsub;
+            if (tok < p.n_valid_rows && n + c8 < p.n_out) {
+                uint32_t o[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    __nv_bfloat162 x = __floats2bfloat162_rn(s[g][2 * i], s[g][2 * i + 1]);
+                    o[i] = *reinterpret_cast<uint32_t*>(&x);
+                }
+                *reinterpret_cast<uint4*>(dx + (size_t)tok * p.n_out + n + c8) = make_uint4(o[0], o[1], o[2], o[3]);
+            }
         }
     }
     return true;
@@ -443,6 +500,8 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
     constexpr bool DATA_GRAD = MODE == MODE_DHH || MODE == MODE_DXG;
     const int kb_per_item = (MODE == MODE_DXG ? 2 : 1) * p.kblocks;
 
+    // (MODE_DX: an item is one or two k-blocks; two stages, and the epilogue's staging lies where the others would)
+    constexpr int ST = MODE == MODE_DX ? 2 : STAGES;
     const Pipe pipe = carve(smem_raw);
     const uint32_t tmem_base = cta_setup(pipe, warp);
     pdl_wait();                                         // the setup above overlaps the end of the kernel before
@@ -461,8 +520,8 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
                 const int row0 = row_tile * BM;
                 const int e_rows = MODE == MODE_DX ? 0 : p.tile_expert[row_tile] * p.b_row_blocks;      // row blocks before this expert's
                 for (int kb = 0; kb < kb_per_item; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (it >= STAGES && !mbar_wait(pipe.empty(s), ((it / STAGES) - 1) & 1, p.status, ERR_EMPTY_WAIT)) {
+                    const int s = it % ST;
+                    if (it >= ST && !mbar_wait(pipe.empty(s), ((it / ST) - 1) & 1, p.status, ERR_EMPTY_WAIT)) {
                         ok = false;
                         break;
                     }
@@ -509,8 +568,8 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
                 const int ncols = DATA_GRAD ? min(BN, 64 * p.b_col_blocks - (item % p.n_col_tiles) * BN) : BN;
                 const uint32_t idesc = make_idesc(BM, ncols, 0, DATA_GRAD ? 1 : 0);
                 for (int kb = 0; kb < kb_per_item; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (!mbar_wait(pipe.full(s), (it / STAGES) & 1, p.status, ERR_FULL_WAIT)) {
+                    const int s = it % ST;
+                    if (!mbar_wait(pipe.full(s), (it / ST) & 1, p.status, ERR_FULL_WAIT)) {
                         ok = false;
                         break;
                     }
@@ -541,7 +600,10 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
             const int row_i = item / p.n_col_tiles, n0 = (item % p.n_col_tiles) * COLS_PER_ITEM;
             const int row_tile = p.tile_order ? p.tile_order[row_i] : row_i;
             const int e = MODE == MODE_DX ? 0 : p.tile_expert[row_tile];
-            if (!rows_epilogue<MODE>(p, pipe.acc_full(buf), pipe.acc_empty(buf), tmem_base, buf, t, row_tile, n0, e, q, h,
+            if constexpr (MODE == MODE_DX) {
+                float* dstage = reinterpret_cast<float*>(pipe.tiles + ST * STAGE_BYTES + (warp - 2) * DX_STAGING);
+                if (!dx_epilogue(p, pipe.acc_full(buf), pipe.acc_empty(buf), tmem_base, buf, t, row_tile, n0, q, h, lane, dstage, p.dx)) break;
+            } else if (!rows_epilogue<MODE>(p, pipe.acc_full(buf), pipe.acc_empty(buf), tmem_base, buf, t, row_tile, n0, e, q, h,
                                      lane, stage, &tmD0, &tmD1, &tmD2))
                 break;
         }
@@ -1173,10 +1235,9 @@ int tc_router_dx(mgpt_moe_layer* L, const Workspace& w, char* ws, const void* dX
     TcState* s = (TcState*)L->tc_state;
     const Dims& d = L->d;
     const int E8 = (d.E + 7) / 8 * 8;
-    CUtensorMap mA, mB, mD;
+    CUtensorMap mA, mB;
     MGPT_TRY(make_map(&mA, ws + w.dl16, (uint64_t)w.n_tokens, (uint64_t)E8, 128));
     MGPT_TRY(make_map(&mB, L->sWr, (uint64_t)d.C, (uint64_t)E8, 128));
-    MGPT_TRY(make_map(&mD, dx, (uint64_t)w.n_tokens, (uint64_t)d.C, 32));
     RowsP p = {};
     p.n_tiles = (const int32_t*)(ws + w.n_tiles);
     p.tile_expert = (const int32_t*)(ws + w.tile_expert);
@@ -1184,8 +1245,9 @@ int tc_router_dx(mgpt_moe_layer* L, const Workspace& w, char* ws, const void* dX
     p.kblocks = cdiv(E8, BK); p.n_out = d.C; p.n_col_tiles = cdiv(d.C, BN);
     p.fixed_tiles = cdiv(w.n_tokens, BM); p.n_valid_rows = w.n_tokens;
     p.gather_src = (const bf16*)dXg; p.gather_pos = pos; p.gather_k = d.k;
+    p.dx = (bf16*)dx;
     p.sched = s->sched + 10;
-    MGPT_CUDA(launch_pdl(tc_rows_kernel<MODE_DX>, imin(grid_sms(L, s), p.fixed_tiles * p.n_col_tiles), TC_THREADS, SMEM_BYTES, st, mA, mA, mB, mB, mD, mD, mD, p));
+    MGPT_CUDA(launch_pdl(tc_rows_kernel<MODE_DX>, imin(grid_sms(L, s), p.fixed_tiles * p.n_col_tiles), TC_THREADS, SMEM_BYTES, st, mA, mA, mB, mB, mA, mA, mA, p));
     MGPT_LAUNCHED("tc_rows_kernel<dx>");
     return 0;
 }
