@@ -520,8 +520,9 @@ router_fwd_kernel(const TIn* __restrict__ x, const float* __restrict__ Wr, const
 }
 
 // dlogits = P * (dP - <dP,P>),  dP = scatter(d_top_p) + alpha*E*f_e/N
-// (layers/MoELayer.cpp:189-210).  One warp for four tokens at a time, grid-stride: the sum over the experts has the
-// reference's order, a chain of E additions, and four chains hide each other (one at a time: 28 us at 32768 tokens, E=64).
+// (layers/MoELayer.cpp:189-210).  One warp for four tokens at a time, grid-stride.  The sum over the experts has the
+// reference's order, a chain of E additions: the products cross through shared memory, and four lanes run the chains of
+// the four tokens (one shuffle per expert and token instead was the kernel: 27 -> 14 us at 32768 tokens, E=64).
 // Optionally also writes a bf16 copy with rows padded to E8 columns (for the tensor-core backward) and adds
 // the column sums to gbr (layers/LinearLayer.cpp:56-57).
 template <int EPL>
@@ -534,6 +535,7 @@ router_dlogits_kernel(const float* __restrict__ probs, const int32_t* __restrict
     pdl_wait();
     constexpr int T = 4;
     __shared__ float bred[8][EPL * 32];
+    __shared__ __align__(16) float prods[8][T][EPL * 32 + 4];     // (+ 4: the rows of a 16-byte read in different banks)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned full = 0xffffffffu;
     float lb[EPL], bsum[EPL];
@@ -572,26 +574,29 @@ router_dlogits_kernel(const float* __restrict__ probs, const int32_t* __restrict
 #pragma unroll
             for (int i = 0; i < EPL; ++i) dp[t][i] = lane + 32 * i < E ? __fadd_rn(dp[t][i], lb[i]) : 0.0f;
         }
-        float dot[T] = {};
+        __syncwarp();
 #pragma unroll
-        for (int i = 0; i < EPL; ++i) {
-            float prod[T];
+        for (int t = 0; t < T; ++t)
 #pragma unroll
-            for (int t = 0; t < T; ++t) prod[t] = __fmul_rn(dp[t][i], p[t][i]);
-            const int lim = min(32, E - 32 * i);
+            for (int i = 0; i < EPL; ++i) prods[warp][t][lane + 32 * i] = __fmul_rn(dp[t][i], p[t][i]);
+        __syncwarp();
+        float chain = 0.0f;                                       // (the products past E are zeros)
+        if (lane < T)
 #pragma unroll 8
-            for (int l = 0; l < lim; ++l)
-#pragma unroll
-                for (int t = 0; t < T; ++t) dot[t] = __fadd_rn(dot[t], __shfl_sync(full, prod[t], l));
-        }
+            for (int e = 0; e < E; e += 4) {
+                const float4 v = *reinterpret_cast<const float4*>(&prods[warp][lane][e]);
+                chain = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(chain, v.x), v.y), v.z), v.w);
+            }
+        __syncwarp();
 #pragma unroll
         for (int t = 0; t < T; ++t) {
             const int tok = tok0 + t;
-            if (tok >= N) break;
+            const float dot = __shfl_sync(full, chain, t);
+            if (tok >= N) continue;
 #pragma unroll
             for (int i = 0; i < EPL; ++i) {
                 const int e = lane + 32 * i;
-                const float v = e < E ? __fmul_rn(p[t][i], __fsub_rn(dp[t][i], dot[t])) : 0.0f;
+                const float v = e < E ? __fmul_rn(p[t][i], __fsub_rn(dp[t][i], dot)) : 0.0f;
                 if (e < E) dlogits[(size_t)tok * E + e] = v;
                 if (dl16 && e < E8) dl16[(size_t)tok * E8 + e] = __float2bfloat16(v);
                 bsum[i] += v;
@@ -948,7 +953,7 @@ int launch_router_bwd(mgpt_moe_layer* L, const Workspace& w, char* ws, const voi
     const bool tc_wgrad = tc && L->has_grad && E % 4 == 0;
     const int E8 = (E + 7) / 8 * 8;
     {
-        const int grid = min((N + 31) / 32, 1184);
+        const int grid = min((N + 31) / 32, 592);
         bf16* dl16 = tc ? (bf16*)(ws + w.dl16) : nullptr;
         float* gbr = tc_wgrad ? L->p_grad[1] : nullptr;
         if (E <= 32) MGPT_CUDA(launch_pdl(router_dlogits_kernel<1>, grid, 256, 0, st, probs, top_idx, dtp, counts, N, E, k, d.alpha, dl, dl16, E8, gbr));
