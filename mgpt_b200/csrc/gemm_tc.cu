@@ -382,106 +382,134 @@ __device__ __forceinline__ bool rows_epilogue(const RowsP& p, uint32_t acc_full_
     return true;
 }
 
-// dx = dlogits * Wr^T (the accumulator) + the token's expert rows in ascending order.  Bound by the gather of those rows
-// (64 bytes of a row at a time): with a lane per token every 16-byte load touched 32 lines, one cycle of the L1 each (155 us
-// for 402 MB at 32768 tokens, C=2048, top-2).  So four lanes share a row, eight rows per load, and the accumulator crosses
-// to that order through `stage` (32 rows x 32 columns FP32, padded); the positions are looked up once per item and the
-// first rows requested before the wait for the accumulator.
-constexpr int DX_LD = 36;                            // floats per staged row
-constexpr uint32_t DX_STAGING = 32 * DX_LD * 4;      // per epilogue warp
-static_assert(EPI_WARPS * DX_STAGING <= (STAGES - 2) * STAGE_BYTES, "the staging of dx lies in the unused stages");
-__device__ __forceinline__ bool dx_epilogue(const RowsP& p, uint32_t acc_full_bar, uint32_t acc_empty_bar, uint32_t tmem_base,
-                                            uint32_t buf, uint32_t t, int row_tile, int n0, int q, int h, int lane, float* stage,
-                                            bf16* __restrict__ dx)
+// dx = dlogits * Wr^T (the accumulator) + the token's expert rows in ascending order: the epilogue of all of a CTA's items.
+// Bound by the gather of those rows.  With a lane per token every 16-byte load touched 32 lines, one cycle of the L1 each
+// (155 us for 402 MB at 32768 tokens, C=2048, top-2), with four lanes per row half of a line (144 us); so eight lanes read
+// a line of 128 bytes, four rows per load (123-132 us; 50 us at E=64 and 16384 tokens, before 70).  The accumulator crosses
+// to that order through `stage` (32 rows x 64 columns FP32, padded).  Each load is requested right after the registers it
+// fills have been added, before the results are written, and the positions of an item while the one before it is worked on:
+// that is why this mode deals its items out by stride instead of the queue.
+constexpr int DX_LD = 68;                            // floats per staged row
+constexpr uint32_t DX_STAGING = 32 * DX_LD * 4 + MAX_TOPK * 32 * 4;     // per epilogue warp: that tile and the positions of 32 tokens
+static_assert(EPI_WARPS * DX_STAGING <= (STAGES - 1) * STAGE_BYTES + EPI_WARPS * STAGING_BYTES, "the staging of dx lies behind one stage");
+__device__ __forceinline__ void dx_epilogue(const RowsP& p, const Pipe& pipe, uint32_t tmem_base, int total_items, int q, int h,
+                                            int lane, float* stage)
 {
-    const int row_w = row_tile * BM + q * 32, rsub = lane >> 2, c8 = (lane & 3) * 8;
-    const int k = p.gather_k;
-    int ps[MAX_TOPK];                                // this lane's token's rows, ascending
+    const int rsub = lane >> 3, c8 = (lane & 7) * 8, k = p.gather_k;
+    bf16* __restrict__ dx = p.dx;
+    int* pos = reinterpret_cast<int*>(stage + 32 * DX_LD);       // [j][token]: the item's rows, ascending in j
+    int ps[MAX_TOPK];                                // rows of this lane's token
+    auto positions = [&](int item) {
+        const int tok = item / p.n_col_tiles * BM + q * 32 + lane;
 #pragma unroll
-    for (int j = 0; j < MAX_TOPK; ++j)
-        ps[j] = j < k && row_w + lane < p.n_valid_rows ? __ldg(p.gather_pos + (size_t)(row_w + lane) * k + j) : 0x7fffffff;
+        for (int j = 0; j < MAX_TOPK; ++j)
+            ps[j] = j < k && item < total_items && tok < p.n_valid_rows ? __ldg(p.gather_pos + (size_t)tok * k + j) : 0x7fffffff;
+    };
+    auto keep_positions = [&]() {
+        __syncwarp();                                // the ones before have been read
 #pragma unroll
-    for (int a = 0; a < MAX_TOPK - 1; ++a)
-        if (a < k - 1)
+        for (int a = 0; a < MAX_TOPK - 1; ++a)
+            if (a < k - 1)
 #pragma unroll
-            for (int b = 0; b < MAX_TOPK - 1 - a; ++b)
-                if (b < k - 1 - a && ps[b] > ps[b + 1]) {
-                    const int tmp = ps[b];
-                    ps[b] = ps[b + 1];
-                    ps[b + 1] = tmp;
-                }
-    // rows 8g + rsub, eight columns from n + c8, of the j-th expert row
-    auto fetch = [&](uint4 (&v)[4], int psj, int n) {
+                for (int b = 0; b < MAX_TOPK - 1 - a; ++b)
+                    if (b < k - 1 - a) {
+                        const int lo = min(ps[b], ps[b + 1]);
+                        ps[b + 1] = max(ps[b], ps[b + 1]);
+                        ps[b] = lo;
+                    }
+#pragma unroll
+        for (int j = 0; j < MAX_TOPK; ++j)
+            if (j < k) pos[j * 32 + lane] = ps[j];
+        __syncwarp();
+    };
+    // rows r16 + 4g + rsub, eight columns from n + c8, of the j-th expert row (0x7fffffff: no such token)
+    auto fetch = [&](uint4 (&v)[4], int j, int r16, int n) {
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
-            const int row = __shfl_sync(0xffffffffu, psj, 8 * g + rsub);
+            const int row = pos[j * 32 + r16 + 4 * g + rsub];
             v[g] = make_uint4(0, 0, 0, 0);
-            if (row_w + 8 * g + rsub < p.n_valid_rows && n + c8 < p.n_out)
+            if (row != 0x7fffffff && n + c8 < p.n_out)
                 v[g] = __ldg(reinterpret_cast<const uint4*>(p.gather_src + (size_t)row * p.n_out + n + c8));
         }
     };
-#pragma unroll
-    for (int un = 0; un < 2; ++un) {
-        const int n = n0 + h * 64 + un * 32;
-        uint4 r0[4], r1[4];
-        fetch(r0, ps[0], n);
-        if (k > 1) fetch(r1, ps[1], n);
-        if (un == 0) {
-            if (!mbar_wait(acc_full_bar, (t >> 1) & 1, p.status, ERR_ACC_WAIT)) return false;
-            tc_fence_after();
-        }
-        float v[32];
+    const int stride = gridDim.x;
+    int item = blockIdx.x;
+    positions(item);
+    keep_positions();
+    uint4 r0[4], r1[4];
+    fetch(r0, 0, 0, item % p.n_col_tiles * BN + h * 64);
+    if (k > 1) fetch(r1, 1, 0, item % p.n_col_tiles * BN + h * 64);
+    for (uint32_t t = 0; item < total_items; ++t, item += stride) {
+        const uint32_t buf = t & 1u;
+        const int row_w = item / p.n_col_tiles * BM + q * 32, n = item % p.n_col_tiles * BN + h * 64;
+        if (!mbar_wait(pipe.acc_full(buf), (t >> 1) & 1, p.status, ERR_ACC_WAIT)) return;
+        tc_fence_after();
         __syncwarp();                                // the tile staged before has been read
-        tmem_ld32(tmem_base + buf * BN + ((uint32_t)(q * 32) << 16) + h * 64 + un * 32, v);
-        tmem_ld_wait();
-        if (un == 1) release_acc(acc_empty_bar, lane);
 #pragma unroll
-        for (int i = 0; i < 32; i += 4)
-            *reinterpret_cast<float4*>(stage + lane * DX_LD + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-        __syncwarp();
-        float s[4][8];
+        for (int un = 0; un < 2; ++un) {
+            float v[32];
+            tmem_ld32(tmem_base + buf * BN + ((uint32_t)(q * 32) << 16) + h * 64 + un * 32, v);
+            tmem_ld_wait();
+            if (un == 1) release_acc(pipe.acc_empty(buf), lane);
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-            const float* src = stage + (8 * g + rsub) * DX_LD + c8;
-            const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
-            s[g][0] = a.x; s[g][1] = a.y; s[g][2] = a.z; s[g][3] = a.w; s[g][4] = b.x; s[g][5] = b.y; s[g][6] = b.z; s[g][7] = b.w;
+            for (int i = 0; i < 32; i += 4)
+                *reinterpret_cast<float4*>(stage + lane * DX_LD + un * 32 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
         }
-        auto add = [&](const uint4 (&r)[4]) {
+        __syncwarp();
+#pragma unroll
+        for (int r16 = 0; r16 < 32; r16 += 16) {
+            if (r16) positions(item + stride);
+            float s[4][8];
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
-                const uint32_t w[4] = {r[g].x, r[g].y, r[g].z, r[g].w};
+                const float* src = stage + (r16 + 4 * g + rsub) * DX_LD + c8;
+                const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
+                s[g][0] = a.x; s[g][1] = a.y; s[g][2] = a.z; s[g][3] = a.w; s[g][4] = b.x; s[g][5] = b.y; s[g][6] = b.z; s[g][7] = b.w;
+            }
+            auto add = [&](const uint4 (&r)[4]) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    s[g][2 * i] += bf_lo(w[i]);
-                    s[g][2 * i + 1] += bf_hi(w[i]);
+                for (int g = 0; g < 4; ++g) {
+                    const uint32_t w[4] = {r[g].x, r[g].y, r[g].z, r[g].w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        s[g][2 * i] += bf_lo(w[i]);
+                        s[g][2 * i + 1] += bf_hi(w[i]);
+                    }
                 }
-            }
-        };
-        add(r0);
-        if (k > 1) add(r1);
+            };
+            add(r0);
+            if (k > 1) add(r1);
 #pragma unroll
-        for (int j = 2; j < MAX_TOPK; j += 2)
-            if (j < k) {
-                fetch(r0, ps[j], n);
-                if (j + 1 < k) fetch(r1, ps[j + 1], n);
-                add(r0);
-                if (j + 1 < k) add(r1);
-            }
+            for (int j = 2; j < MAX_TOPK; j += 2)
+                if (j < k) {
+                    fetch(r0, j, r16, n);
+                    if (j + 1 < k) fetch(r1, j + 1, r16, n);
+                    add(r0);
+                    if (j + 1 < k) add(r1);
+                }
+            uint4 o[4];
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-            const int tok = row_w + 8 * g + rsub;
-            if (tok < p.n_valid_rows && n + c8 < p.n_out) {
-                uint32_t o[4];
+            for (int g = 0; g < 4; ++g) {
+                uint32_t w[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     __nv_bfloat162 x = __floats2bfloat162_rn(s[g][2 * i], s[g][2 * i + 1]);
-                    o[i] = *reinterpret_cast<uint32_t*>(&x);
+                    w[i] = *reinterpret_cast<uint32_t*>(&x);
                 }
-                *reinterpret_cast<uint4*>(dx + (size_t)tok * p.n_out + n + c8) = make_uint4(o[0], o[1], o[2], o[3]);
+                o[g] = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+            // what the next half or the next item adds first
+            if (r16) keep_positions();
+            const int n_next = r16 ? (item + stride) % p.n_col_tiles * BN + h * 64 : n;
+            fetch(r0, 0, r16 ^ 16, n_next);
+            if (k > 1) fetch(r1, 1, r16 ^ 16, n_next);
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                const int tok = row_w + r16 + 4 * g + rsub;
+                if (tok < p.n_valid_rows && n + c8 < p.n_out) *reinterpret_cast<uint4*>(dx + (size_t)tok * p.n_out + n + c8) = o[g];
             }
         }
     }
-    return true;
 }
 
 // Persistent: CTA b works on items b, b+grid, ... where item = row_tile * n_col_tiles + col_tile.
@@ -500,8 +528,9 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
     constexpr bool DATA_GRAD = MODE == MODE_DHH || MODE == MODE_DXG;
     const int kb_per_item = (MODE == MODE_DXG ? 2 : 1) * p.kblocks;
 
-    // (MODE_DX: an item is one or two k-blocks; two stages, and the epilogue's staging lies where the others would)
-    constexpr int ST = MODE == MODE_DX ? 2 : STAGES;
+    // (MODE_DX: an item is one or two k-blocks; one stage, and the epilogue's staging lies where the others would)
+    constexpr int ST = MODE == MODE_DX ? 1 : STAGES;
+    constexpr bool DEALT = MODE == MODE_DX;             // its items are all alike: by stride, no queue
     const Pipe pipe = carve(smem_raw);
     const uint32_t tmem_base = cta_setup(pipe, warp);
     pdl_wait();                                         // the setup above overlaps the end of the kernel before
@@ -513,8 +542,8 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
             uint32_t it = 0;
             bool ok = true;
             int item = blockIdx.x;
-            ok = sched_publish(pipe, 0, item, total_items, p.status);
-            for (uint32_t nf = 1; ok && item >= 0; ++nf) {
+            if (!DEALT) ok = sched_publish(pipe, 0, item, total_items, p.status);
+            for (uint32_t nf = 1; ok && (DEALT ? item < total_items : item >= 0); ++nf) {
                 const int row_i = item / p.n_col_tiles, n0 = (item % p.n_col_tiles) * COLS_PER_ITEM;
                 const int row_tile = p.tile_order ? p.tile_order[row_i] : row_i;
                 const int row0 = row_tile * BM;
@@ -544,22 +573,32 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
                         tma_load_2d(b_dst + HALF_B, &tmB0, kx, n0 + BN / 2, pipe.full(s));
                     }
                 }
+                if (DEALT) {
+                    item += gridDim.x;
+                    continue;
+                }
                 // the next item is claimed as late as possible (the ring is full by now, so the round trip to the
                 // counter does not starve the tensor core): early claims would sit behind this CTA's unfinished work
                 int next = sched_fetch(p.sched);
                 if (ok) ok = sched_publish(pipe, nf, next, total_items, p.status);
                 item = next;
             }
-            sched_finish(p.sched);                       // this CTA asks for no more items
+            if (!DEALT) sched_finish(p.sched);           // this CTA asks for no more items
         }
     } else if (warp == 1) {
         if (lane == 0) {
             uint32_t it = 0, t = 0;
             bool ok = true;
             for (; ok; ++t) {
-                const int item = sched_consume(pipe, t, p.status);
-                if (item >= 0) sched_release(pipe, t);
-                if (item < 0) break;
+                int item;
+                if constexpr (DEALT) {
+                    item = blockIdx.x + t * gridDim.x;
+                    if (item >= total_items) break;
+                } else {
+                    item = sched_consume(pipe, t, p.status);
+                    if (item >= 0) sched_release(pipe, t);
+                    if (item < 0) break;
+                }
                 const uint32_t buf = t & 1u;
                 if (t >= 2 && !mbar_wait(pipe.acc_empty(buf), ((t >> 1) - 1) & 1, p.status, ERR_ACC_WAIT)) break;
                 tc_fence_after();
@@ -591,23 +630,22 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
         // 16 epilogue warps: TMEM lane quarter q = warp % 4 (rows q*32..+31), column group h = 0..3
         const int q = warp & 3, h = (warp - 2) >> 2;
         uint8_t* stage = pipe.staging + (warp - 2) * STAGING_BYTES;
-        uint32_t t = 0;
-        for (;; ++t) {
-            const int item = __shfl_sync(0xffffffffu, sched_consume(pipe, t, p.status), 0);   // warp-uniform
-            if (item < 0) break;
-            if (lane == 0) sched_release(pipe, t);
-            const uint32_t buf = t & 1u;
-            const int row_i = item / p.n_col_tiles, n0 = (item % p.n_col_tiles) * COLS_PER_ITEM;
-            const int row_tile = p.tile_order ? p.tile_order[row_i] : row_i;
-            const int e = MODE == MODE_DX ? 0 : p.tile_expert[row_tile];
-            if constexpr (MODE == MODE_DX) {
-                float* dstage = reinterpret_cast<float*>(pipe.tiles + ST * STAGE_BYTES + (warp - 2) * DX_STAGING);
-                if (!dx_epilogue(p, pipe.acc_full(buf), pipe.acc_empty(buf), tmem_base, buf, t, row_tile, n0, q, h, lane, dstage, p.dx)) break;
-            } else if (!rows_epilogue<MODE>(p, pipe.acc_full(buf), pipe.acc_empty(buf), tmem_base, buf, t, row_tile, n0, e, q, h,
-                                     lane, stage, &tmD0, &tmD1, &tmD2))
-                break;
+        if constexpr (DEALT) {
+            dx_epilogue(p, pipe, tmem_base, total_items, q, h, lane, reinterpret_cast<float*>(pipe.tiles + ST * STAGE_BYTES + (warp - 2) * DX_STAGING));
+        } else {
+            for (uint32_t t = 0;; ++t) {
+                const int item = __shfl_sync(0xffffffffu, sched_consume(pipe, t, p.status), 0);   // warp-uniform
+                if (item < 0) break;
+                if (lane == 0) sched_release(pipe, t);
+                const uint32_t buf = t & 1u;
+                const int row_i = item / p.n_col_tiles, n0 = (item % p.n_col_tiles) * COLS_PER_ITEM;
+                const int row_tile = p.tile_order ? p.tile_order[row_i] : row_i;
+                if (!rows_epilogue<MODE>(p, pipe.acc_full(buf), pipe.acc_empty(buf), tmem_base, buf, t, row_tile, n0, p.tile_expert[row_tile], q, h,
+                                         lane, stage, &tmD0, &tmD1, &tmD2))
+                    break;
+            }
+            if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // stores landed before exit
         }
-        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // stores landed before exit
     }
     cta_teardown(tmem_base, warp);
 }
@@ -1246,7 +1284,6 @@ int tc_router_dx(mgpt_moe_layer* L, const Workspace& w, char* ws, const void* dX
     p.fixed_tiles = cdiv(w.n_tokens, BM); p.n_valid_rows = w.n_tokens;
     p.gather_src = (const bf16*)dXg; p.gather_pos = pos; p.gather_k = d.k;
     p.dx = (bf16*)dx;
-    p.sched = s->sched + 10;
     MGPT_CUDA(launch_pdl(tc_rows_kernel<MODE_DX>, imin(grid_sms(L, s), p.fixed_tiles * p.n_col_tiles), TC_THREADS, SMEM_BYTES, st, mA, mA, mB, mB, mA, mA, mA, p));
     MGPT_LAUNCHED("tc_rows_kernel<dx>");
     return 0;
@@ -1273,7 +1310,7 @@ int tc_router_wgrad(mgpt_moe_layer* L, const Workspace& w, char* ws, const void*
     chunks = cdiv(w.n_tokens, rows);
     q.n_groups = chunks; q.uniform_rows = rows; q.single_grad = L->p_grad[0]; q.item_begin = 0;
     g.total_items = chunks * per_chunk;
-    g.sched = s->sched + 12;
+    g.sched = s->sched + 10;
     MGPT_CUDA(launch_pdl(tc_wgrad_kernel, imin(grid_sms(L, s), g.total_items), WG_THREADS, SMEM_BYTES, st, mA, mB, mA, mB, mA, mB, g));
     MGPT_LAUNCHED("tc_wgrad_kernel<Wr>");
     return 0;
