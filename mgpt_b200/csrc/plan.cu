@@ -149,39 +149,6 @@ __global__ void __launch_bounds__(512) plan_small_kernel(const PlanArgs p)
     plan_block<16>(p, sh);
 }
 
-// Xg[p,:] = x[row_src[p]/k,:]  (zero for padding rows).  One warp per row, 16-byte accesses.
-template <typename TIn, typename TAct>
-__global__ void __launch_bounds__(256)
-dispatch_rows_kernel(const TIn* __restrict__ x, const int32_t* __restrict__ row_src,
-                     const int32_t* __restrict__ n_tiles, int fixed_rows, int C, int k, TAct* __restrict__ Xg)
-{
-    pdl_wait();
-    const int lane = threadIdx.x & 31;
-    const int p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    // rows in use: all tiles of the plan, or a count the host already knows
-    if (p >= (fixed_rows >= 0 ? fixed_rows : *n_tiles * ROW_TILE)) return;
-    const int src = row_src[p];
-    TAct* dst = Xg + (size_t)p * C;
-    constexpr int VIN = 16 / sizeof(TIn), VOUT = 16 / sizeof(TAct);
-    constexpr int V = VIN < VOUT ? VIN : VOUT;     // elements per lane per step
-    if (src < 0) {
-        for (int c = lane * V; c < C; c += 32 * V)
-#pragma unroll
-            for (int i = 0; i < V; ++i) dst[c + i] = from_f32<TAct>(0.0f);
-        return;
-    }
-    const TIn* s = x + (size_t)(src / k) * C;
-    if constexpr (sizeof(TIn) == sizeof(TAct)) {
-        const uint4* s4 = reinterpret_cast<const uint4*>(s);
-        uint4* d4 = reinterpret_cast<uint4*>(dst);
-        const int n4 = C / VIN;
-        for (int i = lane; i < n4; i += 32) d4[i] = s4[i];
-        for (int c = n4 * VIN + lane; c < C; c += 32) dst[c] = from_f32<TAct>(to_f32(s[c]));
-    } else {
-        for (int c = lane; c < C; c += 32) dst[c] = from_f32<TAct>(to_f32(s[c]));
-    }
-}
-
 // 8 consecutive elements <-> 8 floats (16 bytes of bf16, 32 bytes of float)
 template <typename T> __device__ __forceinline__ void load8(const T* p, float (&v)[8]);
 template <> __device__ __forceinline__ void load8<float>(const float* p, float (&v)[8])
@@ -213,6 +180,74 @@ template <> __device__ __forceinline__ void store8<bf16>(bf16* p, const float (&
     u.x = *reinterpret_cast<uint32_t*>(&h0); u.y = *reinterpret_cast<uint32_t*>(&h1);
     u.z = *reinterpret_cast<uint32_t*>(&h2); u.w = *reinterpret_cast<uint32_t*>(&h3);
     *reinterpret_cast<uint4*>(p) = u;
+}
+
+// The rows of a token: lane j < k gets the padded row of the token's j-th choice, or -1 (a choice without a slot: an id no
+// expert has, which the plan has reported).
+__device__ __forceinline__ int token_row(const int32_t* __restrict__ pos, const int32_t* __restrict__ row_src, int row_cap, int tok,
+                                         int k, int lane)
+{
+    if (lane >= k) return -1;
+    const int q = pos[(size_t)tok * k + lane];
+    return (unsigned)q < (unsigned)row_cap && row_src[q] == tok * k + lane ? q : -1;
+}
+
+// Zeros in those of the PAD_ROWS rows of group `g` that carry no token, eight rows to a warp.  (With 32 rows to a warp,
+// and these blocks behind the tokens', an expert's last tile was the end of the launch: 2-4 us more at 8192 tokens.)
+constexpr int PAD_ROWS = 64;
+template <typename TAct>
+__device__ __forceinline__ void zero_padding(const int32_t* __restrict__ row_src, int rows, int g, int C, TAct* __restrict__ dst)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q0 = g * PAD_ROWS + warp * 8;
+    unsigned m = __ballot_sync(0xffffffffu, lane < 8 && q0 + lane < rows && row_src[q0 + lane] < 0);
+    const float z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (; m; m &= m - 1) {
+        TAct* row = dst + (size_t)(q0 + __ffs(m) - 1) * C;
+        for (int c = lane * 8; c < C; c += 256) store8(row + c, z);
+    }
+}
+
+// Xg[pos(tok,j),:] = x[tok,:] for every choice j; the blocks before the tokens' write the padding rows' zeros (none are
+// launched where nothing reads those rows: the products of inference keep rows apart).  Bound by HBM: one warp per token
+// reads its row once, four 16-byte loads per lane in flight, and writes it k times.  (A warp per padded row read every
+// token k times and wrote padding by single elements: 104 -> 79-94 us at 32768 tokens, C=2048, top-2; 14.4 -> 3.2 us
+// at 256 tokens and 32 experts, where seven of eight rows are padding.)
+template <typename TIn, typename TAct, bool VEC>
+__global__ void __launch_bounds__(256)
+dispatch_kernel(const TIn* __restrict__ x, const int32_t* __restrict__ pos, const int32_t* __restrict__ row_src,
+                const int32_t* __restrict__ n_tiles, int row_cap, int N, int C, int k, int pad_blocks, TAct* __restrict__ Xg)
+{
+    pdl_wait();
+    const int lane = threadIdx.x & 31;
+    if ((int)blockIdx.x < pad_blocks) {
+        zero_padding(row_src, *n_tiles * ROW_TILE, blockIdx.x, C, Xg);
+        return;
+    }
+    const int tok = (blockIdx.x - pad_blocks) * 8 + (threadIdx.x >> 5);
+    if (tok >= N) return;
+    const int mine = token_row(pos, row_src, row_cap, tok, k, lane);
+    const TIn* s = x + (size_t)tok * C;
+    constexpr int U = sizeof(TIn) == sizeof(TAct) && sizeof(TIn) == 2 ? 4 : 2;
+    for (int c0 = lane * 8; c0 - lane * 8 < C; c0 += 256 * U) {
+        float v[U][8];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (c0 + 256 * u < C) {
+                if constexpr (VEC) {
+                    load8(s + c0 + 256 * u, v[u]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[u][i] = to_f32(s[c0 + 256 * u + i]);
+                }
+            }
+        for (int j = 0; j < k; ++j) {
+            const int q = __shfl_sync(0xffffffffu, mine, j);
+            if (q < 0) continue;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (c0 + 256 * u < C) store8(Xg + (size_t)q * C + c0 + 256 * u, v[u]);
+        }
+    }
 }
 
 // y[tok,:] = sum_j p[tok,j] * Yg[pos(tok,j),:], slots visited in ascending order
@@ -263,42 +298,61 @@ combine_fwd_kernel(const TAct* __restrict__ Yg, const int32_t* __restrict__ pos,
     }
 }
 
-// dYg[p,:] = p * dy[tok,:],  d_top_p[flat] = <Yg[p,:], dy[tok,:]>; padding rows -> 0.
-template <typename TAct, typename TIo>
+// dYg[q,:] = p * dy[tok,:],  d_top_p[flat] = <Yg[q,:], dy[tok,:]> for the rows q of every token; padding rows -> 0 (the
+// blocks before the tokens').  Bound by HBM: one warp per token, which reads dy once for all its K >= k rows (a warp per
+// padded row read it k times: 124 -> 110-115 us at 32768 tokens, C=2048, top-2; 56 -> 47 us at 16384, C=1024, top-4).
+template <typename TAct, typename TIo, int K>
 __global__ void __launch_bounds__(256)
-combine_bwd_kernel(const TIo* __restrict__ dy, const TAct* __restrict__ Yg, const int32_t* __restrict__ row_src,
-                   const float* __restrict__ top_p, const int32_t* __restrict__ n_tiles, int fixed_rows, int C, int k,
-                   TAct* __restrict__ dYg, float* __restrict__ d_top_p)
+combine_bwd_kernel(const TIo* __restrict__ dy, const TAct* __restrict__ Yg, const int32_t* __restrict__ pos,
+                   const int32_t* __restrict__ row_src, const float* __restrict__ top_p, const int32_t* __restrict__ n_tiles,
+                   int row_cap, int N, int C, int k, int pad_blocks, TAct* __restrict__ dYg, float* __restrict__ d_top_p)
 {
     pdl_wait();
     const int lane = threadIdx.x & 31;
-    const int p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (p >= (fixed_rows >= 0 ? fixed_rows : *n_tiles * ROW_TILE)) return;
-    const int src = row_src[p];
-    TAct* dst = dYg + (size_t)p * C;
-    if (src < 0) {
-        const float z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int c = lane * 8; c < C; c += 256) store8(dst + c, z);
+    if ((int)blockIdx.x < pad_blocks) {
+        zero_padding(row_src, *n_tiles * ROW_TILE, blockIdx.x, C, dYg);
         return;
     }
-    const float prob = top_p[src];
-    const TIo* g = dy + (size_t)(src / k) * C;
-    const TAct* yg = Yg + (size_t)p * C;
-    float dot = 0.0f;
-    for (int c = lane * 8; c < C; c += 256) {
-        float gv[8], yv[8], o[8];
-        load8(g + c, gv);
-        load8(yg + c, yv);
+    const int tok = (blockIdx.x - pad_blocks) * 8 + (threadIdx.x >> 5);
+    if (tok >= N) return;
+    const int mine = token_row(pos, row_src, row_cap, tok, k, lane);
+    const float prob = lane < k ? top_p[(size_t)tok * k + lane] : 0.0f;
+    int q[K];
+    float pr[K], dot[K];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            o[i] = __fmul_rn(gv[i], prob);
-            dot = fmaf(yv[i], gv[i], dot);
+    for (int j = 0; j < K; ++j) {
+        q[j] = __shfl_sync(0xffffffffu, mine, j);
+        pr[j] = __shfl_sync(0xffffffffu, prob, j);
+        dot[j] = 0.0f;
+    }
+    const TIo* g = dy + (size_t)tok * C;
+    constexpr int KB = K < 4 ? K : 4;                // rows in flight
+    for (int c = lane * 8; c < C; c += 256) {
+        float gv[8];
+        load8(g + c, gv);
+#pragma unroll
+        for (int j0 = 0; j0 < K; j0 += KB) {
+            float yv[KB][8];
+#pragma unroll
+            for (int j = 0; j < KB; ++j) load8(Yg + (size_t)max(q[j0 + j], 0) * C + c, yv[j]);
+#pragma unroll
+            for (int j = 0; j < KB; ++j) {
+                float o[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    o[i] = __fmul_rn(gv[i], pr[j0 + j]);
+                    dot[j0 + j] = fmaf(yv[j][i], gv[i], dot[j0 + j]);
+                }
+                if (q[j0 + j] >= 0) store8(dYg + (size_t)q[j0 + j] * C + c, o);
+            }
         }
-        store8(dst + c, o);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-    if (lane == 0) d_top_p[src] = dot;
+    for (int j = 0; j < K; ++j) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) dot[j] += __shfl_xor_sync(0xffffffffu, dot[j], o);
+        if (lane == 0 && q[j] >= 0) d_top_p[(size_t)tok * k + j] = dot[j];
+    }
 }
 
 // Column sums over each expert's rows, for the three bias gradients in one launch:
@@ -381,28 +435,36 @@ int launch_plan(const Dims& d, const Workspace& w, char* ws, cudaStream_t st, in
     return run_plan_args(plan_args(d, w, ws, sticky), (int32_t*)(ws + w.blk_cnt), st);
 }
 
-// dst[p,:] = src[row_src[p]/k,:] for p < rows (zero where row_src[p] < 0).  rows < 0: every tile of the plan.
-int gather_rows(const void* src, int src_io, const int32_t* row_src, const int32_t* n_tiles, int rows, int grid_rows,
-                int C, int k, void* dst, size_t act_bytes, cudaStream_t st)
+// dst[pos(tok,j),:] = src[tok,:]; with `zero_pad`, zeros in every other row of the plan's tiles
+int dispatch_rows(const Workspace& w, char* ws, const void* src, int src_io, int C, int k, void* dst, bool zero_pad, cudaStream_t st)
 {
-    if (grid_rows <= 0) return 0;
-    const int grid = (grid_rows + 7) / 8;
-    if (act_bytes == 4) {
+    if (w.n_tokens <= 0) return 0;
+    const int32_t* pos = (const int32_t*)(ws + w.pos);
+    const int32_t* row_src = (const int32_t*)(ws + w.row_src);
+    const int32_t* n_tiles = (const int32_t*)(ws + w.n_tiles);
+    const int N = w.n_tokens, pad_blocks = zero_pad ? (w.row_cap + PAD_ROWS - 1) / PAD_ROWS : 0, grid = pad_blocks + (N + 7) / 8;
+    const bool vec = ((uintptr_t)src & 15) == 0;
+#define MGPT_DISPATCH(TIN, TACT)                                                                                          \
+    do {                                                                                                                  \
+        auto* kernel = vec ? dispatch_kernel<TIN, TACT, true> : dispatch_kernel<TIN, TACT, false>;                        \
+        MGPT_CUDA(launch_pdl(kernel, grid, 256, 0, st, (const TIN*)src, pos, row_src, n_tiles, w.row_cap, N, C, k, pad_blocks, (TACT*)dst)); \
+    } while (0)
+    if (w.act_bytes == 4) {
         if (src_io != MGPT_MOE_IO_F32) return fail(MGPT_MOE_EINVAL, "FP32 mode takes FP32 rows");
-        MGPT_CUDA(launch_pdl(dispatch_rows_kernel<float, float>, grid, 256, 0, st, (const float*)src, row_src, n_tiles, rows, C, k, (float*)dst));
+        MGPT_DISPATCH(float, float);
     } else if (src_io == MGPT_MOE_IO_F32) {
-        MGPT_CUDA(launch_pdl(dispatch_rows_kernel<float, bf16>, grid, 256, 0, st, (const float*)src, row_src, n_tiles, rows, C, k, (bf16*)dst));
+        MGPT_DISPATCH(float, bf16);
     } else {
-        MGPT_CUDA(launch_pdl(dispatch_rows_kernel<bf16, bf16>, grid, 256, 0, st, (const bf16*)src, row_src, n_tiles, rows, C, k, (bf16*)dst));
+        MGPT_DISPATCH(bf16, bf16);
     }
-    MGPT_LAUNCHED("dispatch_rows_kernel");
+#undef MGPT_DISPATCH
+    MGPT_LAUNCHED("dispatch_kernel");
     return 0;
 }
 
-int launch_dispatch(const Dims& d, const Workspace& w, char* ws, const void* x, int io, cudaStream_t st)
+int launch_dispatch(const Dims& d, const Workspace& w, char* ws, const void* x, int io, bool zero_pad, cudaStream_t st)
 {
-    return gather_rows(x, io, (const int32_t*)(ws + w.row_src), (const int32_t*)(ws + w.n_tiles), -1, w.row_cap, d.C, d.k,
-                       ws + w.Xg, w.act_bytes, st);
+    return dispatch_rows(w, ws, x, io, d.C, d.k, ws + w.Xg, zero_pad, st);
 }
 
 // y = weighted gather-sum of rows[pos[tok,j]]
@@ -435,31 +497,34 @@ int launch_combine_fwd(const Dims& d, const Workspace& w, char* ws, void* y, int
                         io, w.act_bytes, st, residual);
 }
 
-// d_rows[p] = top_p * dy[tok], d_top_p[flat] = <rows[p], dy[tok]> for p < rows (rows < 0: every tile of the plan)
-int combine_rows_backward(const void* dy, int io, const void* rows, const int32_t* row_src, const float* top_p,
-                          const int32_t* n_tiles, int n_rows, int grid_rows, int C, int k, void* d_rows, float* d_top_p,
-                          size_t act_bytes, cudaStream_t st)
+// d_rows[pos(tok,j)] = top_p * dy[tok] (other rows of the plan's tiles: 0), d_top_p[flat] = <rows[pos(tok,j)], dy[tok]>
+int combine_rows_backward(const Workspace& w, char* ws, const void* dy, int io, const void* rows, int C, int k, void* d_rows, cudaStream_t st)
 {
-    if (grid_rows <= 0) return 0;
-    const int grid = (grid_rows + 7) / 8;
-    if (act_bytes == 4)
-        MGPT_CUDA(launch_pdl(combine_bwd_kernel<float, float>, grid, 256, 0, st, (const float*)dy, (const float*)rows, row_src, top_p,
-                                                               n_tiles, n_rows, C, k, (float*)d_rows, d_top_p));
-    else if (io == MGPT_MOE_IO_F32)
-        MGPT_CUDA(launch_pdl(combine_bwd_kernel<bf16, float>, grid, 256, 0, st, (const float*)dy, (const bf16*)rows, row_src, top_p,
-                                                              n_tiles, n_rows, C, k, (bf16*)d_rows, d_top_p));
-    else
-        MGPT_CUDA(launch_pdl(combine_bwd_kernel<bf16, bf16>, grid, 256, 0, st, (const bf16*)dy, (const bf16*)rows, row_src, top_p,
-                                                             n_tiles, n_rows, C, k, (bf16*)d_rows, d_top_p));
+    if (w.n_tokens <= 0) return 0;
+    const int N = w.n_tokens, pad_blocks = (w.row_cap + PAD_ROWS - 1) / PAD_ROWS, grid = pad_blocks + (N + 7) / 8;
+#define MGPT_COMBINE(TACT, TIO, KK)                                                                                       \
+    MGPT_CUDA(launch_pdl(combine_bwd_kernel<TACT, TIO, KK>, grid, 256, 0, st, (const TIO*)dy, (const TACT*)rows,          \
+                         (const int32_t*)(ws + w.pos), (const int32_t*)(ws + w.row_src), (const float*)(ws + w.top_p),    \
+                         (const int32_t*)(ws + w.n_tiles), w.row_cap, N, C, k, pad_blocks, (TACT*)d_rows, (float*)(ws + w.d_top_p)))
+#define MGPT_COMBINE_K(KK)                                                                                                \
+    do {                                                                                                                  \
+        if (w.act_bytes == 4) MGPT_COMBINE(float, float, KK);                                                             \
+        else if (io == MGPT_MOE_IO_F32) MGPT_COMBINE(bf16, float, KK);                                                    \
+        else MGPT_COMBINE(bf16, bf16, KK);                                                                                \
+    } while (0)
+    if (k <= 1) MGPT_COMBINE_K(1);
+    else if (k <= 2) MGPT_COMBINE_K(2);
+    else if (k <= 4) MGPT_COMBINE_K(4);
+    else MGPT_COMBINE_K(8);
+#undef MGPT_COMBINE_K
+#undef MGPT_COMBINE
     MGPT_LAUNCHED("combine_bwd_kernel");
     return 0;
 }
 
 int launch_combine_bwd(const Dims& d, const Workspace& w, char* ws, const void* dy, int io, cudaStream_t st)
 {
-    return combine_rows_backward(dy, io, ws + w.Yg, (const int32_t*)(ws + w.row_src), (const float*)(ws + w.top_p),
-                                 (const int32_t*)(ws + w.n_tiles), -1, w.row_cap, d.C, d.k, ws + w.dYg,
-                                 (float*)(ws + w.d_top_p), w.act_bytes, st);
+    return combine_rows_backward(w, ws, dy, io, ws + w.Yg, d.C, d.k, ws + w.dYg, st);
 }
 
 int launch_bias_grads(const mgpt_moe_layer* L, const Workspace& w, char* ws, cudaStream_t st)

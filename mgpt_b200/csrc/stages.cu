@@ -99,8 +99,7 @@ int mgpt_moe_route_rows(mgpt_moe_layer* L, const void* x, int io, void* workspac
     MGPT_CUDA(cudaSetDevice(L->device));
     char* ws = (char*)workspace;
     // expert-major rows, each expert padded to whole tiles with zero rows; stable within an expert
-    MGPT_TRY(gather_rows(x, io, (const int32_t*)(ws + w.row_src), (const int32_t*)(ws + w.n_tiles), -1, w.row_cap, L->d.C,
-                         L->d.k, send_rows, w.act_bytes, (cudaStream_t)stream));
+    MGPT_TRY(dispatch_rows(w, ws, x, io, L->d.C, L->d.k, send_rows, true, (cudaStream_t)stream));
     L->fwd_done = true;
     return 0;
 }
@@ -137,9 +136,7 @@ int mgpt_moe_combine_backward(mgpt_moe_layer* L, const void* rows_back, const vo
     if (L->last_n > 0 && (!rows_back || !dy || !d_rows)) return fail(MGPT_MOE_EINVAL, "null buffer");
     MGPT_CUDA(cudaSetDevice(L->device));
     char* ws = (char*)workspace;
-    return combine_rows_backward(dy, io, rows_back, (const int32_t*)(ws + w.row_src), (const float*)(ws + w.top_p),
-                                 (const int32_t*)(ws + w.n_tiles), -1, w.row_cap, L->d.C, L->d.k, d_rows,
-                                 (float*)(ws + w.d_top_p), w.act_bytes, (cudaStream_t)stream);
+    return combine_rows_backward(w, ws, dy, io, rows_back, L->d.C, L->d.k, d_rows, (cudaStream_t)stream);
 }
 
 int mgpt_moe_route_backward(mgpt_moe_layer* L, const void* x, const void* d_rows_in, void* dx, int io,
