@@ -671,6 +671,7 @@ struct WgradP {
     int n_probs, total_items;
     int overwrite;          // grad = product (zeros for experts without rows) instead of grad += product
     int block_loads;        // the tensor maps are the column-block form: one load per operand tile and stage
+    int b_boxes;            // > 0: B has no more than this many 64-column boxes, loaded one by one (block_loads: A's form only)
     // bias gradients from the same operand tiles (null: none): gb[pr][e][col] += column sums, over the expert's
     // rows, of the operand of problem pr whose columns are that bias's (the A operand when the problem is
     // computed transposed, else the B operand)
@@ -739,8 +740,16 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant_
                             break;
                         }
                         const uint32_t a_dst = smem_u32(pipe.tiles + s * STAGE_BYTES), b_dst = a_dst + A_BYTES;
-                        mbar_expect_tx(pipe.full(s), STAGE_BYTES);
                         const int row = seg_r0 + kb * BK;
+                        if (p.b_boxes > 0) {
+                            mbar_expect_tx(pipe.full(s), A_BYTES + p.b_boxes * BOX);
+                            if (p.block_loads) tma_load_3d(a_dst, mA, 0, row, w.m0 / 64, pipe.full(s));
+                            else
+                                for (int i = 0; i < BM / 64; ++i) tma_load_2d(a_dst + i * BOX, mA, w.m0 + 64 * i, row, pipe.full(s));
+                            for (int i = 0; i < p.b_boxes; ++i) tma_load_2d(b_dst + i * BOX, mB, 64 * i, row, pipe.full(s));
+                            continue;
+                        }
+                        mbar_expect_tx(pipe.full(s), STAGE_BYTES);
                         if (p.block_loads) {
                             // two loads per stage instead of six: with 64-row stages this kernel waits for the
                             // producer thread's issue rate as much as for the bytes (measured: 1.44 -> 1.39 ms)
@@ -764,7 +773,6 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant_
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc(BM, BN, 1, 1);
             uint32_t it = 0, t = 0;
             bool ok = true;
             for (uint32_t nf = 0; ok; ++nf) {
@@ -773,6 +781,8 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant_
                 sched_release(pipe, nf);
                 const WgradItem w = wgrad_item(p, item);
                 if (w.nkb <= 0) continue;
+                // no more 64-column boxes than the product has
+                const uint32_t idesc = make_idesc(BM, min(BN, (p.prob[w.pr].N - w.n0 + 63) / 64 * 64), 1, 1);
                 const uint32_t buf = t & 1u;
                 if (t >= 2 && !mbar_wait(pipe.acc_empty(buf), ((t >> 1) - 1) & 1, p.status, ERR_ACC_WAIT)) break;
                 tc_fence_after();
@@ -1289,7 +1299,10 @@ int tc_router_dx(mgpt_moe_layer* L, const Workspace& w, char* ws, const void* dX
     return 0;
 }
 
-// gWr[C,E] += x^T * dlogits on the tensor cores, split over uniform token chunks (RED accumulation).
+// gWr[C,E] += x^T * dlogits on the tensor cores, split over uniform token chunks (RED accumulation).  Bound by the stream of
+// x; but a producer thread spends 250-500 cycles on a TMA load, and with six per 64 tokens (all of a 256-column tile, mostly
+// zero fill) that was the kernel: two now where the channels come in whole blocks of 64 and E <= 64.  As many chunks as
+// make one wave: 51-57 -> 39 us at 32768 tokens, C=2048, E=64 (8.8 and 15 us at 8192 x 512 and 16384 x 1024: unchanged).
 int tc_router_wgrad(mgpt_moe_layer* L, const Workspace& w, char* ws, const void* x, cudaStream_t st)
 {
     MGPT_TRY(prepare_attrs(L));
@@ -1297,15 +1310,17 @@ int tc_router_wgrad(mgpt_moe_layer* L, const Workspace& w, char* ws, const void*
     const Dims& d = L->d;
     const int E8 = (d.E + 7) / 8 * 8;
     CUtensorMap mA, mB;
-    MGPT_TRY(make_map(&mA, x, (uint64_t)w.n_tokens, (uint64_t)d.C, 64));
-    MGPT_TRY(make_map(&mB, ws + w.dl16, (uint64_t)w.n_tokens, (uint64_t)E8, 64));
     WgradP g = {};
+    g.block_loads = make_map_blocks(&mA, x, (uint64_t)w.n_tokens, (uint64_t)d.C, 64, BM / 64) ? 1 : 0;
+    if (!g.block_loads) MGPT_TRY(make_map(&mA, x, (uint64_t)w.n_tokens, (uint64_t)d.C, 64));
+    MGPT_TRY(make_map(&mB, ws + w.dl16, (uint64_t)w.n_tokens, (uint64_t)E8, 64));
+    g.b_boxes = cdiv(E8, 64);
     g.status = L->d_status;
     g.n_probs = 1;
     WgradProb& q = g.prob[0];
     q.M = d.C; q.N = d.E; q.n_tiles_m = cdiv(d.C, BM); q.n_tiles_n = cdiv(d.E, BN);
     const int per_chunk = q.n_tiles_m * q.n_tiles_n;
-    int chunks = imin(64, (2 * s->sms + per_chunk - 1) / per_chunk);
+    int chunks = imin(64, per_chunk < s->sms ? s->sms / per_chunk : 1);
     int rows = cdiv(cdiv(w.n_tokens, chunks), BK) * BK;           // tokens per chunk, whole k-blocks
     chunks = cdiv(w.n_tokens, rows);
     q.n_groups = chunks; q.uniform_rows = rows; q.single_grad = L->p_grad[0]; q.item_begin = 0;
