@@ -558,8 +558,8 @@ static int forward_impl(mgpt_moe_layer* L, const void* x, void* y, int n_tokens,
         L->stage_end(ST_PLAN, st);
     }
     if (n_tokens > 0) {
-        // (the decode kernels fetch the tokens' rows themselves; training keeps the permuted rows for backward)
-        const bool gathered = w.decode && inference;
+        // (the decode kernels fetch the tokens' rows themselves, by 16 bytes; training keeps the permuted rows for backward)
+        const bool gathered = w.decode && inference && ((uintptr_t)x & 15) == 0;
         if (!gathered) {
             L->stage_begin(ST_DISPATCH, st);
             MGPT_TRY(launch_dispatch(d, w, ws, x, io, !inference, st));      // (only backward reads padding rows)
