@@ -253,6 +253,8 @@ dispatch_kernel(const TIn* __restrict__ x, const int32_t* __restrict__ pos, cons
 // y[tok,:] = sum_j p[tok,j] * Yg[pos(tok,j),:], slots visited in ascending order
 // like the reference's scatter-add.  One warp per token, 8 channels per lane per step; K = top-k rounded up
 // to a power of two, so the sort is a fixed network and the kernel fits 32 registers (all 64 warps resident).
+// Few tokens: the 256-channel pieces of a token go to blocks of their own (grid.y) while those fit the chip at once; in one
+// warp they follow each other, each a trip to L2 (C=1024: 4.7 -> 2.5 us for one token, 5.4 -> 2.9 for 256, 5.7 -> 3.7 for 1777).
 template <typename TAct, typename TIo, int K>
 __global__ void __launch_bounds__(256, 8)
 combine_fwd_kernel(const TAct* __restrict__ Yg, const int32_t* __restrict__ pos, const float* __restrict__ top_p,
@@ -277,7 +279,7 @@ combine_fwd_kernel(const TAct* __restrict__ Yg, const int32_t* __restrict__ pos,
                 int ti = ps[b]; ps[b] = ps[b + 1]; ps[b + 1] = ti;
                 float tf = pr[b]; pr[b] = pr[b + 1]; pr[b + 1] = tf;
             }
-    for (int c = lane * 8; c < C; c += 256) {
+    for (int c = (blockIdx.y * 32 + lane) * 8; c < C; c += gridDim.y * 256) {
         float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
         for (int j = 0; j < K; ++j) {
@@ -472,7 +474,8 @@ int combine_rows(const void* rows, const int32_t* pos, const float* top_p, int N
                  size_t act_bytes, cudaStream_t st, const void* residual)
 {
     if (N <= 0) return 0;
-    const int grid = (N + 7) / 8;
+    const int blocks = (N + 7) / 8, pieces = (C + 255) / 256, room = 148 * 8 / blocks;
+    const dim3 grid(blocks, room < 1 ? 1 : room < pieces ? room : pieces);
 #define MGPT_COMBINE(KK)                                                                                                  \
     do {                                                                                                                  \
         if (act_bytes == 4)                                                                                               \
