@@ -475,7 +475,7 @@ def time_optimizer(layer, w):
     except torch.OutOfMemoryError:
         return None
     n_w = sum(p.numel() for p in layer.get_parameters())
-    byts = n_w * (28 + (4 if w.dtype == "bf16" else 0))      # read w,g,m,v; write w,m,v (+ two BF16 copies)
+    byts = n_w * (28 + (2 if w.dtype == "bf16" else 0))      # read w,g,m,v; write w,m,v (+ the BF16 copy)
     return {"adamw_fused_ms": round(adamw_ms, 4), "adamw_fused_gbs": round(byts / (adamw_ms * 1e-3) / 1e9, 1),
             "bytes": byts, "sync_weights_alone_ms": round(sync_ms, 4),
             "note": "not part of the timed step; one optimiser step over all 2+6E tensors, copies refreshed in the same pass"}
