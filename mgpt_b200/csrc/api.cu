@@ -477,9 +477,7 @@ int mgpt_moe_save_routing(mgpt_moe_layer* L, void* dst, mgpt_stream_t stream)
     if (!L->fwd_done) return fail(MGPT_MOE_ESTATE, "save_routing without a forward");
     const Workspace w = make_workspace(L->d, L->last_n);
     MGPT_CUDA(cudaSetDevice(L->device));
-    MGPT_CUDA(cudaMemcpyAsync(dst, (const char*)L->last_ws + routing_begin(w), routing_end(w) - routing_begin(w),
-                              cudaMemcpyDeviceToDevice, (cudaStream_t)stream));
-    return 0;
+    return copy_on_device(dst, (const char*)L->last_ws + routing_begin(w), routing_end(w) - routing_begin(w), (cudaStream_t)stream);
 }
 
 static int forward_impl(mgpt_moe_layer* L, const void* x, void* y, int n_tokens, int io, void* workspace,
@@ -536,8 +534,7 @@ static int forward_impl(mgpt_moe_layer* L, const void* x, void* y, int n_tokens,
         // recompute of a forward whose routing was saved: the same tokens route the same way, so router and plan
         // are replaced by one copy (the logits are not part of the saved state and stay undefined)
         L->stage_begin(ST_PLAN, st);
-        MGPT_CUDA(cudaMemcpyAsync(ws + routing_begin(w), routing, routing_end(w) - routing_begin(w),
-                                  cudaMemcpyDeviceToDevice, st));
+        MGPT_TRY(copy_on_device(ws + routing_begin(w), routing, routing_end(w) - routing_begin(w), st));
         L->stage_end(ST_PLAN, st);
     } else {
         bool planned = false;

@@ -252,6 +252,7 @@ int launch_router_bwd(mgpt_moe_layer* L, const Workspace& w, char* ws, const voi
 
 // plan.cu
 struct PlanArgs plan_args(const Dims& d, const Workspace& w, char* ws, int32_t* sticky);      // plan_block.cuh
+int copy_on_device(void* dst, const void* src, size_t bytes, cudaStream_t st);
 int launch_plan(const Dims& d, const Workspace& w, char* ws, cudaStream_t st, int32_t* sticky);
 int launch_dispatch(const Dims& d, const Workspace& w, char* ws, const void* x, int io, bool zero_pad, cudaStream_t st);
 int launch_combine_fwd(const Dims& d, const Workspace& w, char* ws, void* y, int io, cudaStream_t st,

@@ -407,6 +407,26 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(BiasGradArgs a)
 
 }  // namespace
 
+// A copy within the device as one of the step's kernels: cudaMemcpyAsync, a copy of its own, breaks the chain of launches
+// that overlap each other's start and end (0.6 MB of routing: 1.7-2.4 us and 1.5-2.2 us before it, now 1.9-2.2 us and none; 2 us of a checkpointed step of 718).
+static __global__ void __launch_bounds__(256) copy_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, size_t n)
+{
+    pdl_wait();
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) dst[i] = src[i];
+}
+
+int copy_on_device(void* dst, const void* src, size_t bytes, cudaStream_t st)
+{
+    if ((((uintptr_t)dst | (uintptr_t)src | bytes) & 15) || bytes == 0) {
+        MGPT_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, st));
+        return 0;
+    }
+    const size_t n = bytes / 16, blocks = (n + 255) / 256;
+    MGPT_CUDA(launch_pdl(copy_kernel, (int)(blocks < 1184 ? blocks : 1184), 256, 0, st, (const uint4*)src, (uint4*)dst, n));
+    MGPT_LAUNCHED("copy_kernel");
+    return 0;
+}
+
 // The plan on explicit buffers.  `blk` is scratch of plan_blocks*E ints: every element is written by plan_count_kernel
 // before it is read, so it needs no clearing.  (Rows beyond the plan's tiles are never read.)
 static int run_plan_args(const PlanArgs& p, int32_t* blk, cudaStream_t st)
