@@ -60,12 +60,13 @@ Workspace make_workspace(const Dims& d, int n_tokens, int kind)
     w.tile_expert = take((size_t)w.max_tiles * 4);
     w.n_tiles = take(4);
     w.status = take(4);
-    w.decode = (kind == 0 || kind == 3) && decode_usable(d, n_tokens);
-    w.groups = take(w.decode ? (size_t)decode_max_groups(d, n_tokens) * 16 : 0);
-    w.n_groups = take(4);
     w.map = take(N * k * 4);
     w.pos = take(N * k * 4);
     w.row_src = take(rc * 4);
+    // (sized alike for every kind, like all before Xg: mgpt_moe_workspace_view and the saved routing know one layout)
+    w.decode = decode_usable(d, n_tokens);
+    w.groups = take(w.decode ? (size_t)decode_max_groups(d, n_tokens) * 16 : 0);
+    w.n_groups = take(4);
     w.blk_cnt = take((size_t)w.plan_blocks * E * 4);
     w.slot = take(N * k * 4);
     w.seg = take(E * MAX_SOURCES * 2 * 4);
@@ -459,8 +460,8 @@ int mgpt_moe_selftest_bounded_wait(mgpt_moe_layer* L, mgpt_stream_t stream)
 }
 
 // Routing results and plan of one forward: the workspace bytes from probs up to (not including) the plan's
-// scratch -- probs, top_idx, top_p, counts, offsets, padded_offsets, tile_expert, n_tiles, status, groups, n_groups,
-// map, pos, row_src.
+// scratch -- probs, top_idx, top_p, counts, offsets, padded_offsets, tile_expert, n_tiles, status, map, pos, row_src,
+// groups, n_groups.
 static size_t routing_begin(const Workspace& w) { return w.probs; }
 static size_t routing_end(const Workspace& w) { return w.blk_cnt; }
 

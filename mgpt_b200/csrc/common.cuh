@@ -97,9 +97,10 @@ struct Workspace {
     size_t logits, probs, top_idx, top_p;
     // plan
     size_t counts, offsets, padded_offsets, tile_expert, n_tiles, status;
+    size_t map, pos, row_src;
     size_t groups, n_groups;    // decode kernels: {expert, first padded row, rows, 0} per row group
-    bool decode;                // few rows per expert: the products are decode.cu's
-    size_t map, pos, row_src, blk_cnt, slot, seg, tile_order;
+    bool decode;                // few rows per expert: the plan lists row groups, a whole layer's products are decode.cu's
+    size_t blk_cnt, slot, seg, tile_order;
     // forward activations (kept for backward)
     size_t Xg, G, U, Hh, Yg;
     // backward temporaries
