@@ -170,7 +170,11 @@ int  mgpt_moe_forward_residual(mgpt_moe_layer* layer, const void* x, const void*
  * layer sees forward-only calls of a few to a few hundred tokens.  This entry point is mgpt_moe_forward without
  * anything kept for a backward pass: a workspace of mgpt_moe_inference_workspace_bytes(n_tokens) (no saved
  * activation factors, no backward buffers), the same routing and the same y.  Token batches too small to fill the
- * device take the low-latency form of the exact router.  mgpt_moe_backward cannot follow it (MGPT_MOE_ESTATE);
+ * device take the low-latency form of the exact router.
+ * A token's y keeps its bits as a context grows, with two exceptions (of both forward calls; the order of the sums in the
+ * products, and the kernel that computes the top-k weights, change with the number of tokens): calls of few rows per
+ * expert -- n_tokens * top_k <= 8 * num_experts, BF16 mode, gemm_impl 0 -- against larger ones, and BF16 tokens from
+ * n_tokens * embed_dim * num_experts = 4e8 on.  mgpt_moe_backward cannot follow it (MGPT_MOE_ESTATE);
  * mgpt_moe_expert_counts can. */
 size_t mgpt_moe_inference_workspace_bytes(const mgpt_moe_layer* layer, int n_tokens);
 int  mgpt_moe_forward_inference(mgpt_moe_layer* layer, const void* x, void* y, int n_tokens, int io_dtype,

@@ -12,10 +12,12 @@
 //
 // A k-block's order of k within the fragments is chosen so that one 16-byte load feeds two MMAs (A and B agree on it, so
 // the sum is the same set of products).  A row group is up to 16 rows of one expert (the plan lists them); more rows
-// read the weights again, mostly from L2.  KS = 4: four warps share a task's k-blocks and add up, in order, through
-// shared memory -- for launches with too few tasks to give every warp some.  Which KS is taken depends on the number of
-// tokens only through min(rows, experts), never on the routing, and every sum has a fixed order: a row's result does not
-// depend on which other rows are in the call.
+// read the weights again, mostly from L2.  A product is the sum of the sums over four equal parts of its k-blocks, added
+// in order (one part where it has fewer than eight k-blocks).  KS = 4: a warp for each part, which add up through shared
+// memory -- for launches with too few tasks to give every warp some; KS = 1: one warp runs through all parts.  Either way
+// the additions are the same: a row's bits depend neither on the other rows of the call, nor on how many there are, nor on
+// the number of SMs.  (The second accumulator costs KS = 1 3 % at 64 tokens, C=1024, H=2816, E=32: 123.3 -> 127.1 us for the
+// call; the sums kept in shared memory instead 128.2.)
 //
 // tcgen05 is no help here: its M side is 128 rows whatever the number of tokens, and with the weights on the M side
 // instead an MMA of N = 16 still took ~120 cycles for 4 KiB of weights (1000 cycles per 32 KiB stage, 135 us for the
@@ -42,6 +44,7 @@ struct DecP {
     const bf16* A;                     // down: Hh
     bf16 *out, *G, *U;
     int C, H, k, hb, cb, kb1, kb2;
+    int parts;                         // of this phase's reduction
 };
 
 __device__ __forceinline__ uint4 ld_weights(const bf16* p)
@@ -81,9 +84,10 @@ __device__ __forceinline__ void ld_frag(Frag& f, const bf16* ra, const bf16* rb,
 
 // acc[nn] += the task's weights x rows nn*8.. over the k-blocks [k0, k1).  `w` holds the first DEPTH of them, already
 // requested.
-template <int NN, typename TRow>
+// `after(kb)` follows every k-block.
+template <int NN, typename TRow, typename After>
 __device__ __forceinline__ void run_task(Frag (&w)[DEPTH], const bf16* ra, const bf16* rb, const TRow* const (&src)[NN], int k0, int k1,
-                                         int K, int t4, float (&acc)[NN][4])
+                                         int K, int t4, float (&acc)[NN][4], After after)
 {
     for (int kb = k0; kb < k1; kb += DEPTH) {
 #pragma unroll
@@ -106,6 +110,7 @@ __device__ __forceinline__ void run_task(Frag (&w)[DEPTH], const bf16* ra, const
                         mma16816(acc[n], f.v[s].x, f.v[2 + s].x, f.v[s].y, f.v[2 + s].y, b[n][s].x, b[n][s].y);
                         mma16816(acc[n], f.v[s].z, f.v[2 + s].z, f.v[s].w, f.v[2 + s].w, b[n][s].z, b[n][s].w);
                     }
+                after(kb + u);
             }
         }
     }
@@ -166,7 +171,29 @@ __global__ void __launch_bounds__(32 * DW, 1) decode_kernel(const DecP p)
             for (int n = 0; n < NN; ++n)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) acc[n][i] = 0.0f;
-            run_task<NN, TRow>(w, ra, rb, src, k0, k1, K, t4, acc);
+            float sum[NN][4];                               // KS = 1: of the parts that have ended
+#pragma unroll
+            for (int n = 0; n < NN; ++n)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) sum[n][i] = -0.0f;      // (-0 + v is v, whatever v is)
+            int part = 0, part_end = kbs / p.parts;
+            run_task<NN, TRow>(w, ra, rb, src, k0, k1, K, t4, acc, [&](int kb) {
+                if (KS > 1) return;
+                const bool ends = kb + 1 == part_end;
+#pragma unroll
+                for (int n = 0; n < NN; ++n)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        sum[n][i] = ends ? sum[n][i] + acc[n][i] : sum[n][i];
+                        acc[n][i] = ends ? 0.0f : acc[n][i];
+                    }
+                if (ends) part_end = kbs * (++part + 1) / p.parts;
+            });
+            if (KS == 1)
+#pragma unroll
+                for (int n = 0; n < NN; ++n)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) acc[n][i] = sum[n][i];
             if constexpr (KS > 1) {
                 if (ks > 0)
 #pragma unroll
@@ -227,10 +254,14 @@ __global__ void __launch_bounds__(32 * DW, 1) decode_kernel(const DecP p)
     if (!waited) pdl_wait();
 }
 
+// A product is the sum, in order, of this many sums over equal parts of its k-blocks.
+int decode_parts(int kblocks) { return kblocks >= 8 ? 4 : 1; }
+
 template <int PHASE, bool F32>
-int launch_phase(const DecP& p, int ks, int sms, cudaStream_t st)
+int launch_phase(DecP p, bool spread, int sms, cudaStream_t st)
 {
-    if (ks == 4) MGPT_CUDA(launch_pdl(decode_kernel<PHASE, 4, F32>, sms, 32 * DW, 0, st, p));
+    p.parts = decode_parts(PHASE == 1 ? p.kb1 : p.kb2);
+    if (spread && p.parts == 4) MGPT_CUDA(launch_pdl(decode_kernel<PHASE, 4, F32>, sms, 32 * DW, 0, st, p));
     else MGPT_CUDA(launch_pdl(decode_kernel<PHASE, 1, F32>, sms, 32 * DW, 0, st, p));
     MGPT_LAUNCHED(PHASE == 1 ? "decode_kernel<gateup>" : "decode_kernel<down>");
     return 0;
@@ -264,8 +295,7 @@ int launch_decode_forward(mgpt_moe_layer* L, const Workspace& w, char* ws, const
     // units / 16 columns)
     const long long T = w.R < d.E ? w.R : d.E;
     const long long warps = (long long)sms * DW;
-    const int ks1 = T * ((d.H + 7) / 8) < 2 * warps && p.kb1 >= 8 ? 4 : 1;
-    const int ks2 = T * ((d.C + 15) / 16) < 2 * warps && p.kb2 >= 8 ? 4 : 1;
+    const bool spread1 = T * ((d.H + 7) / 8) < 2 * warps, spread2 = T * ((d.C + 15) / 16) < 2 * warps;
     p.x = from_rows ? (const void*)(ws + w.Xg) : x;
     p.row_src = from_rows ? nullptr : (const int32_t*)(ws + w.row_src);
     p.out = (bf16*)(ws + w.Hh);
@@ -273,14 +303,14 @@ int launch_decode_forward(mgpt_moe_layer* L, const Workspace& w, char* ws, const
     p.U = w.inference ? nullptr : (bf16*)(ws + w.U);
     p.b0 = L->master.bg; p.b1 = L->master.bu;
     L->stage_begin(ST_GATEUP, st);
-    if (from_rows || io == MGPT_MOE_IO_BF16) MGPT_TRY((launch_phase<1, false>(p, ks1, sms, st)));
-    else MGPT_TRY((launch_phase<1, true>(p, ks1, sms, st)));
+    if (from_rows || io == MGPT_MOE_IO_BF16) MGPT_TRY((launch_phase<1, false>(p, spread1, sms, st)));
+    else MGPT_TRY((launch_phase<1, true>(p, spread1, sms, st)));
     L->stage_end(ST_GATEUP, st);
     p.A = (const bf16*)(ws + w.Hh);
     p.out = (bf16*)(ws + w.Yg);
     p.b0 = L->master.bd;
     L->stage_begin(ST_DOWN, st);
-    MGPT_TRY((launch_phase<2, false>(p, ks2, sms, st)));
+    MGPT_TRY((launch_phase<2, false>(p, spread2, sms, st)));
     L->stage_end(ST_DOWN, st);
     return 0;
 }

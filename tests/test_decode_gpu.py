@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import torch
 
-from mgpt_b200 import synth
+from mgpt_b200 import MoELayer, synth
 from oracle import oracle
 from tests.util import assert_routing_exact, assert_values, dims_of, run_layer
 
@@ -33,3 +33,27 @@ def test_few_rows_per_expert(n, C, H, E, k, crowd, io):
     xt = torch.from_numpy(x).cuda().to(io)
     assert torch.equal(layer.forward_inference(xt), layer.forward(xt))
     layer.check_status()
+
+
+@pytest.mark.parametrize("C,H,E,k,steps", [
+    (1024, 2816, 32, 2, [1, 2, 6, 7, 8, 64, 128]),     # gate/up goes from four warps per task to one between 6 and 7 tokens
+    (1024, 1032, 128, 2, [1, 18, 36, 37, 300, 512]),   # both products do between 36 and 37; 17 k-blocks in uneven parts
+    (256, 520, 16, 2, [1, 16, 63, 64]),                # four k-blocks: one part; nine: parts of 2, 2, 2 and 3
+])
+@pytest.mark.parametrize("io", [torch.float32, torch.bfloat16])
+def test_a_tokens_bits_do_not_depend_on_the_call(C, H, E, k, steps, io):
+    """Up to 8 rows per expert: the rows of a growing context keep their bits, whichever split of the reduction the number
+    of tokens and the SM budget lead to."""
+    w = synth.Workload("grow", steps[-1], C, H, E, k, "bf16")
+    x, params, _ = synth.make_inputs(w, seed=29, bias_std=0.02)
+    layer = MoELayer(C, H, E, k, mode="bf16")
+    layer.load_parameters(params)
+    xt = torch.from_numpy(x).cuda().to(io)
+    full = layer.forward_inference(xt).clone()
+    for n in steps:
+        assert torch.equal(layer.forward_inference(xt[:n].contiguous()), full[:n]), n
+    for sms in (1, 40):
+        layer.lib.mgpt_moe_set_sm_budget(layer._h, sms)
+        assert torch.equal(layer.forward_inference(xt[:8].contiguous()), full[:8]), sms
+    layer.check_status()
+    layer.close()
