@@ -197,9 +197,9 @@ WeightsArgs weights_args(const mgpt_moe_layer* L)
 
 // Router tensors alone (a layer whose experts live elsewhere).
 __global__ void __launch_bounds__(256)
-adamw_router_kernel(float* const* __restrict__ w_ptrs, const float* const* __restrict__ g_ptrs,
-                    float* const* __restrict__ m_ptrs, float* const* __restrict__ v_ptrs, int len0, int len1,
-                    float* __restrict__ rstat, const AdamwScalars a)
+adamw_router_kernel(float* const* w_ptrs, const float* const* g_ptrs,
+                    float* const* m_ptrs, float* const* v_ptrs, int len0, int len1,
+                    float* rstat, const AdamwScalars a)
 {
     pdl_wait();
     if (rstat && blockIdx.x == 0 && threadIdx.x < 2) rstat[threadIdx.x] = 0.0f;

@@ -87,6 +87,10 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
+// What an earlier kernel on the stream may have written is read with plain loads: a `const __restrict__` parameter and __ldg
+// promise memory that nobody writes while the kernel lives, and it lives from before pdl_wait().  Left to __ldg are weights,
+// biases, the saved SwiGLU factors and the rows of dXg, in kernels that another kernel of the same call separates from their
+// writer: that one has waited for the writer's end.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ---- workspace ------------------------------------------------------------

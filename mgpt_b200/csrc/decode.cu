@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(32 * DW, 1) decode_kernel(const DecP p)
         auto source = [&](int j) -> const TRow* {           // this lane's row j of the group (past the end: the last one)
             const int pr = gr.y + min(j, rows - 1);
             if (PHASE == 2) return (const TRow*)(const void*)p.A + (size_t)pr * K;
-            return (const TRow*)p.x + (size_t)(p.row_src ? __ldg(p.row_src + pr) / p.k : pr) * K;
+            return (const TRow*)p.x + (size_t)(p.row_src ? p.row_src[pr] / p.k : pr) * K;
         };
         const int wa = w0 + g, wb = wa + 8;                 // hidden unit, or output columns
         auto task = [&](auto nn) {

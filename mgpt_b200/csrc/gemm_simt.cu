@@ -54,7 +54,7 @@ __device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %
 // A staged operand is [TK][SROW]: element (k, m) at k*SROW + m.  Thread t of a group fetches two pieces of four
 // elements: along k for a matrix whose k is contiguous (KMAJOR), along m otherwise; out of range reads as zero.
 template <typename T, bool KMAJOR, bool VEC>
-__device__ __forceinline__ void fetch(const T* __restrict__ P, long ld, int m0, int M, int k0, int K, int t, float4 (&r)[2])
+__device__ __forceinline__ void fetch(const T* P, long ld, int m0, int M, int k0, int K, int t, float4 (&r)[2])
 {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {

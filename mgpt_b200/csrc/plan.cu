@@ -32,7 +32,7 @@ template <> __device__ __forceinline__ bf16 from_f32<bf16>(float v) { return __f
 
 // (1) per-block expert histogram
 __global__ void __launch_bounds__(PLAN_BLOCK)
-plan_count_kernel(const int32_t* __restrict__ top_idx, int R, int E, int32_t* __restrict__ blk_cnt, int32_t* __restrict__ status)
+plan_count_kernel(const int32_t* top_idx, int R, int E, int32_t* blk_cnt, int32_t* status)
 {
     pdl_wait();
     __shared__ int cnt[MAX_EXPERTS];
@@ -52,7 +52,7 @@ plan_count_kernel(const int32_t* __restrict__ top_idx, int R, int E, int32_t* __
 // experts; n_blocks * E integers out of L2), scans the experts, and gives its own rows their stable rank -> map / pos /
 // row_src; block 0 also writes what is not per row.  (A scan kernel of one block between the two took 11-17 us at 64
 // blocks: a serial walk over the blocks per expert, then over the experts in one thread.)
-__global__ void __launch_bounds__(PLAN_BLOCK) plan_assign_kernel(const PlanArgs p, int n_blocks, const int32_t* __restrict__ blk_cnt)
+__global__ void __launch_bounds__(PLAN_BLOCK) plan_assign_kernel(const PlanArgs p, int n_blocks, const int32_t* blk_cnt)
 {
     pdl_wait();
     __shared__ int warp_cnt[PLAN_SEGS][MAX_EXPERTS];
@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(PLAN_BLOCK) plan_assign_kernel(const PlanArgs 
         if (x < p.E) {
 #pragma unroll 8
             for (int b = slice; b < n_blocks; b += 8) {
-                const int c = __ldcg(blk_cnt + (size_t)b * p.E + x);
+                const int c = blk_cnt[(size_t)b * p.E + x];
                 all += c;
                 if (b < (int)blockIdx.x) before += c;
             }
@@ -184,7 +184,7 @@ template <> __device__ __forceinline__ void store8<bf16>(bf16* p, const float (&
 
 // The rows of a token: lane j < k gets the padded row of the token's j-th choice, or -1 (a choice without a slot: an id no
 // expert has, which the plan has reported).
-__device__ __forceinline__ int token_row(const int32_t* __restrict__ pos, const int32_t* __restrict__ row_src, int row_cap, int tok,
+__device__ __forceinline__ int token_row(const int32_t* pos, const int32_t* row_src, int row_cap, int tok,
                                          int k, int lane)
 {
     if (lane >= k) return -1;
@@ -196,7 +196,7 @@ __device__ __forceinline__ int token_row(const int32_t* __restrict__ pos, const 
 // and these blocks behind the tokens', an expert's last tile was the end of the launch: 2-4 us more at 8192 tokens.)
 constexpr int PAD_ROWS = 64;
 template <typename TAct>
-__device__ __forceinline__ void zero_padding(const int32_t* __restrict__ row_src, int rows, int g, int C, TAct* __restrict__ dst)
+__device__ __forceinline__ void zero_padding(const int32_t* row_src, int rows, int g, int C, TAct* dst)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q0 = g * PAD_ROWS + warp * 8;
     unsigned m = __ballot_sync(0xffffffffu, lane < 8 && q0 + lane < rows && row_src[q0 + lane] < 0);
@@ -214,8 +214,8 @@ __device__ __forceinline__ void zero_padding(const int32_t* __restrict__ row_src
 // at 256 tokens and 32 experts, where seven of eight rows are padding.)
 template <typename TIn, typename TAct, bool VEC>
 __global__ void __launch_bounds__(256)
-dispatch_kernel(const TIn* __restrict__ x, const int32_t* __restrict__ pos, const int32_t* __restrict__ row_src,
-                const int32_t* __restrict__ n_tiles, int row_cap, int N, int C, int k, int pad_blocks, TAct* __restrict__ Xg)
+dispatch_kernel(const TIn* x, const int32_t* pos, const int32_t* row_src,
+                const int32_t* n_tiles, int row_cap, int N, int C, int k, int pad_blocks, TAct* Xg)
 {
     pdl_wait();
     const int lane = threadIdx.x & 31;
@@ -257,8 +257,8 @@ dispatch_kernel(const TIn* __restrict__ x, const int32_t* __restrict__ pos, cons
 // warp they follow each other, each a trip to L2 (C=1024: 4.7 -> 2.5 us for one token, 5.4 -> 2.9 for 256, 5.7 -> 3.7 for 1777).
 template <typename TAct, typename TIo, int K>
 __global__ void __launch_bounds__(256, 8)
-combine_fwd_kernel(const TAct* __restrict__ Yg, const int32_t* __restrict__ pos, const float* __restrict__ top_p,
-                   int N, int C, int k, const TIo* __restrict__ residual, TIo* __restrict__ y)
+combine_fwd_kernel(const TAct* Yg, const int32_t* pos, const float* top_p,
+                   int N, int C, int k, const TIo* residual, TIo* y)
 {
     pdl_wait();
     const int lane = threadIdx.x & 31;
@@ -305,9 +305,9 @@ combine_fwd_kernel(const TAct* __restrict__ Yg, const int32_t* __restrict__ pos,
 // padded row read it k times: 124 -> 110-115 us at 32768 tokens, C=2048, top-2; 56 -> 47 us at 16384, C=1024, top-4).
 template <typename TAct, typename TIo, int K>
 __global__ void __launch_bounds__(256)
-combine_bwd_kernel(const TIo* __restrict__ dy, const TAct* __restrict__ Yg, const int32_t* __restrict__ pos,
-                   const int32_t* __restrict__ row_src, const float* __restrict__ top_p, const int32_t* __restrict__ n_tiles,
-                   int row_cap, int N, int C, int k, int pad_blocks, TAct* __restrict__ dYg, float* __restrict__ d_top_p)
+combine_bwd_kernel(const TIo* dy, const TAct* Yg, const int32_t* pos,
+                   const int32_t* row_src, const float* top_p, const int32_t* n_tiles,
+                   int row_cap, int N, int C, int k, int pad_blocks, TAct* dYg, float* d_top_p)
 {
     pdl_wait();
     const int lane = threadIdx.x & 31;
@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(BiasGradArgs a)
 
 // A copy within the device as one of the step's kernels: cudaMemcpyAsync, a copy of its own, breaks the chain of launches
 // that overlap each other's start and end (0.6 MB of routing: 1.7-2.4 us and 1.5-2.2 us before it, now 1.9-2.2 us and none; 2 us of a checkpointed step of 718).
-static __global__ void __launch_bounds__(256) copy_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, size_t n)
+static __global__ void __launch_bounds__(256) copy_kernel(const uint4* src, uint4* dst, size_t n)
 {
     pdl_wait();
     for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) dst[i] = src[i];
@@ -570,10 +570,10 @@ int launch_bias_grads(const mgpt_moe_layer* L, const Workspace& w, char* ws, cud
 // 128-row-padded segment per local expert.  From the [n_src][E] real row counts this builds the tile ->
 // expert table in arrival order, the per-expert segment list {first row, padded rows} and the totals.
 __global__ void __launch_bounds__(256)
-segment_tiles_kernel(const int32_t* __restrict__ seg_counts, int n_src, int E, int32_t* __restrict__ counts,
-                     int32_t* __restrict__ tile_expert, int32_t* __restrict__ tile_order,
-                     int32_t* __restrict__ n_tiles, int max_tiles, int32_t* __restrict__ seg,
-                     int32_t* __restrict__ status, int32_t* __restrict__ sticky)
+segment_tiles_kernel(const int32_t* seg_counts, int n_src, int E, int32_t* counts,
+                     int32_t* tile_expert, int32_t* tile_order,
+                     int32_t* n_tiles, int max_tiles, int32_t* seg,
+                     int32_t* status, int32_t* sticky)
 {
     pdl_wait();
     __shared__ int first_tile[MAX_SEGMENTS + 1];     // in arrival order (s, e)

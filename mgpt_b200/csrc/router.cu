@@ -30,9 +30,9 @@ __device__ __forceinline__ float to_f32(bf16 v) { return __bfloat162float(v); }
 // logit sums are in acc (layers/MoELayer.cpp:96-131).
 template <int EL, int EPL, int TPW>
 __device__ __forceinline__ void router_finish(const float (&acc)[TPW][EPL], const int* stok, int warp, int sub, int el,
-                                              int E, int k, const float* __restrict__ br, float* __restrict__ logits,
-                                              float* __restrict__ probs, int32_t* __restrict__ top_idx,
-                                              float* __restrict__ top_p)
+                                              int E, int k, const float* br, float* logits,
+                                              float* probs, int32_t* top_idx,
+                                              float* top_p)
 {
     constexpr int SUB = 32 / EL;
     constexpr int TOK_W = TPW * SUB;
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(RX_THREADS) router_exact_kernel(const RouterAr
                 for (int v = pt; v < n << per_log; v += RX_PRODUCE) {
                     const int i = v >> per_log, q = v & ((1 << per_log) - 1);
                     if (q < pieces) {
-                        const int tok = p.list ? __ldg(p.list + tile * TOK + i) : tile * TOK + i;
+                        const int tok = p.list ? p.list[tile * TOK + i] : tile * TOK + i;
                         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
                                      ::"r"(dst + x_off + i * x_row + q * 16), "l"((const TIn*)p.x + (size_t)tok * C + c0 + q * XV) : "memory");
                     }
@@ -439,11 +439,11 @@ __global__ void __launch_bounds__(RX_THREADS) router_exact_kernel(const RouterAr
 // For shapes and addresses the kernel above cannot take (C not a multiple of 8, x or Wr not 16-byte aligned).
 template <typename TIn, int EL, int EPL, int TPW>
 __global__ void __launch_bounds__(R_WARPS * 32)
-router_fwd_kernel(const TIn* __restrict__ x, const float* __restrict__ Wr, const float* __restrict__ br,
+router_fwd_kernel(const TIn* x, const float* Wr, const float* br,
                   int N, int C, int E, int k,
-                  float* __restrict__ logits, float* __restrict__ probs,
-                  int32_t* __restrict__ top_idx, float* __restrict__ top_p,
-                  const int32_t* __restrict__ list, const int32_t* __restrict__ list_count)
+                  float* logits, float* probs,
+                  int32_t* top_idx, float* top_p,
+                  const int32_t* list, const int32_t* list_count)
 {
     pdl_wait();
     constexpr int SUB = 32 / EL;                    // tokens per warp pass
@@ -527,10 +527,10 @@ router_fwd_kernel(const TIn* __restrict__ x, const float* __restrict__ Wr, const
 // the column sums to gbr (layers/LinearLayer.cpp:56-57).
 template <int EPL>
 __global__ void __launch_bounds__(256)
-router_dlogits_kernel(const float* __restrict__ probs, const int32_t* __restrict__ top_idx,
-                      const float* __restrict__ d_top_p, const int32_t* __restrict__ counts,
-                      int N, int E, int k, float alpha, float* __restrict__ dlogits,
-                      bf16* __restrict__ dl16, int E8, float* __restrict__ gbr)
+router_dlogits_kernel(const float* probs, const int32_t* top_idx,
+                      const float* d_top_p, const int32_t* counts,
+                      int N, int E, int k, float alpha, float* dlogits,
+                      bf16* dl16, int E8, float* gbr)
 {
     pdl_wait();
     constexpr int T = 4;
@@ -644,8 +644,8 @@ template <int TPT> constexpr size_t dx_smem(int E) { return (size_t)E * (DX_CH +
 
 template <typename TAct, typename TIo, int TPT>
 __global__ void __launch_bounds__(256)
-router_dx_kernel(const TAct* __restrict__ dXg, const int32_t* __restrict__ pos, const float* __restrict__ dlogits,
-                 const float* __restrict__ Wr, int N, int C, int E, int k, TIo* __restrict__ dx)
+router_dx_kernel(const TAct* dXg, const int32_t* pos, const float* dlogits,
+                 const float* Wr, int N, int C, int E, int k, TIo* dx)
 {
     pdl_wait();
     constexpr int TOK = 32 * TPT, WS = DX_CH + 4;       // padded row: transposed staging without 32-way conflicts
@@ -734,8 +734,8 @@ router_dx_kernel(const TAct* __restrict__ dXg, const int32_t* __restrict__ pos, 
 // A thread keeps a 4 channel x 4 expert block of accumulators.
 template <typename TIo>
 __global__ void __launch_bounds__(256)
-router_wgrad_partial_kernel(const TIo* __restrict__ x, const float* __restrict__ dlogits, int N, int C, int E,
-                            int tok_per_chunk, float* __restrict__ part, float* __restrict__ partb)
+router_wgrad_partial_kernel(const TIo* x, const float* dlogits, int N, int C, int E,
+                            int tok_per_chunk, float* part, float* partb)
 {
     pdl_wait();
     const int E4 = (E + 3) / 4;                         // expert groups of 4
@@ -802,8 +802,8 @@ router_wgrad_partial_kernel(const TIo* __restrict__ x, const float* __restrict__
 // 32 elements per CTA, the chunks shared out over 8 threads per element (one thread per element walked up to 64 chunks
 // one after another: 6 us for 1024 elements)
 __global__ void __launch_bounds__(256)
-router_wgrad_reduce_kernel(const float* __restrict__ part, const float* __restrict__ partb, int n_chunks, int CE, int E,
-                           float* __restrict__ gWr, float* __restrict__ gbr)
+router_wgrad_reduce_kernel(const float* part, const float* partb, int n_chunks, int CE, int E,
+                           float* gWr, float* gbr)
 {
     pdl_wait();
     __shared__ float red[8][32];

@@ -14,8 +14,8 @@ namespace {
 // in the padding columns; backward) and, where pieces is set, the transposed BF16 pieces [2][NE][C] (hi = bf16(w),
 // mid = bf16(w - hi)) with the largest column norm / bias magnitude for the error bound of the screened router.
 __global__ void __launch_bounds__(256)
-router_copies_kernel(const float* __restrict__ Wr, const float* __restrict__ br, int C, int E, int E8, int NE,
-                     bf16* __restrict__ out, bf16* __restrict__ pieces, float* __restrict__ rstat)
+router_copies_kernel(const float* Wr, const float* br, int C, int E, int E8, int NE,
+                     bf16* out, bf16* pieces, float* rstat)
 {
     pdl_wait();
     __shared__ float red[8];
