@@ -48,10 +48,41 @@ plan_count_kernel(const int32_t* top_idx, int R, int E, int32_t* blk_cnt, int32_
     if (threadIdx.x < E) blk_cnt[(size_t)blockIdx.x * E + threadIdx.x] = cnt[threadIdx.x];
 }
 
-// (2) everything else.  Each block sums the histograms of all blocks and of those before it (8 slices of blocks x 128
-// experts; n_blocks * E integers out of L2), scans the experts, and gives its own rows their stable rank -> map / pos /
-// row_src; block 0 also writes what is not per row.  (A scan kernel of one block between the two took 11-17 us at 64
-// blocks: a serial walk over the blocks per expert, then over the experts in one thread.)
+// (2) for many blocks only: the histograms become, in place, the rows of an expert in the blocks before; totals -> counts.
+// One block per 32 experts (lane = expert), each warp a contiguous share of the blocks, walked twice.
+__global__ void __launch_bounds__(1024) plan_scan_kernel(int32_t* blk_cnt, int n_blocks, int E, int32_t* counts)
+{
+    pdl_wait();
+    __shared__ int part[32][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, x = blockIdx.x * 32 + lane;
+    const int b0 = (int)((long long)n_blocks * warp / 32), b1 = (int)((long long)n_blocks * (warp + 1) / 32);
+    int sum = 0;
+    if (x < E)
+#pragma unroll 8
+        for (int b = b0; b < b1; ++b) sum += blk_cnt[(size_t)b * E + x];
+    part[warp][lane] = sum;
+    __syncthreads();
+    int run = 0;
+    for (int w = 0; w < warp; ++w) run += part[w][lane];
+    if (x >= E) return;
+    if (warp == 31) counts[x] = run + sum;
+    for (int b = b0; b < b1; b += 8) {
+        int c[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) c[u] = b + u < b1 ? blk_cnt[(size_t)(b + u) * E + x] : 0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            if (b + u < b1) blk_cnt[(size_t)(b + u) * E + x] = run;
+            run += c[u];
+        }
+    }
+}
+
+// (3) everything else: the sums of the histograms over all blocks and over those before this one, a scan of the experts, and
+// the stable rank of the block's own rows -> map / pos / row_src; block 0 also writes what is not per row.  SCANNED: the
+// sums are plan_scan_kernel's; else each block makes them itself (8 slices of blocks x 128 experts; n_blocks * E integers
+// out of L2), which saves the launch but grows with the square of the rows.
+template <bool SCANNED>
 __global__ void __launch_bounds__(PLAN_BLOCK) plan_assign_kernel(const PlanArgs p, int n_blocks, const int32_t* blk_cnt)
 {
     pdl_wait();
@@ -62,7 +93,7 @@ __global__ void __launch_bounds__(PLAN_BLOCK) plan_assign_kernel(const PlanArgs 
     const int i = blockIdx.x * PLAN_BLOCK + tid;
     bool valid = i < p.R;
     int e = valid ? p.top_idx[i] : 0;
-    {
+    if (!SCANNED) {
         const int x = tid & (MAX_EXPERTS - 1), slice = tid / MAX_EXPERTS;
         int before = 0, all = 0;
         if (x < p.E) {
@@ -80,10 +111,17 @@ __global__ void __launch_bounds__(PLAN_BLOCK) plan_assign_kernel(const PlanArgs 
     __syncthreads();
     if (tid < MAX_EXPERTS) {
         int before = 0, all = 0;
+        if (SCANNED) {
+            if (tid < p.E) {
+                before = blk_cnt[(size_t)blockIdx.x * p.E + tid];
+                all = p.counts[tid];
+            }
+        } else {
 #pragma unroll
-        for (int s = 0; s < 8; ++s) {
-            before += part[0][s][tid];
-            all += part[1][s][tid];
+            for (int s = 0; s < 8; ++s) {
+                before += part[0][s][tid];
+                all += part[1][s][tid];
+            }
         }
         base[tid] = before;
         tot[tid] = all;
@@ -128,7 +166,7 @@ __global__ void __launch_bounds__(PLAN_BLOCK) plan_assign_kernel(const PlanArgs 
     for (int x = warp; x < p.E; x += PLAN_SEGS) {
         const int t0 = tile0[x], t1 = tile0[x + 1], n = tot[x];
         if (lane == 0) {
-            p.counts[x] = n;
+            if (!SCANNED) p.counts[x] = n;
             p.offsets[x] = off[x];
             p.padded_offsets[x] = t0 * ROW_TILE;
         }
@@ -427,6 +465,10 @@ int copy_on_device(void* dst, const void* src, size_t bytes, cudaStream_t st)
     return 0;
 }
 
+// Blocks from which the histograms are scanned by a kernel of their own.  Call us without / with it (E = 64): 128 blocks
+// 13 / 14, 256 16 / 13, 512 25 / 18, 1024 59 / 29, 16384 8846 / 404; E = 8 meets at 512 (17 / 17), E = 128 at 128 (16 / 15).
+constexpr int PLAN_SCAN_FROM = 256;
+
 // The plan on explicit buffers.  `blk` is scratch of plan_blocks*E ints: every element is written by plan_count_kernel
 // before it is read, so it needs no clearing.  (Rows beyond the plan's tiles are never read.)
 static int run_plan_args(const PlanArgs& p, int32_t* blk, cudaStream_t st)
@@ -439,7 +481,13 @@ static int run_plan_args(const PlanArgs& p, int32_t* blk, cudaStream_t st)
     const int plan_blocks = (p.R + PLAN_BLOCK - 1) / PLAN_BLOCK;
     MGPT_CUDA(launch_pdl(plan_count_kernel, plan_blocks, PLAN_BLOCK, 0, st, p.top_idx, p.R, p.E, blk, p.status));
     MGPT_LAUNCHED("plan_count_kernel");
-    MGPT_CUDA(launch_pdl(plan_assign_kernel, plan_blocks, PLAN_BLOCK, 0, st, p, plan_blocks, blk));
+    if (plan_blocks >= PLAN_SCAN_FROM) {
+        MGPT_CUDA(launch_pdl(plan_scan_kernel, (p.E + 31) / 32, 1024, 0, st, blk, plan_blocks, p.E, p.counts));
+        MGPT_LAUNCHED("plan_scan_kernel");
+        MGPT_CUDA(launch_pdl(plan_assign_kernel<true>, plan_blocks, PLAN_BLOCK, 0, st, p, plan_blocks, blk));
+    } else {
+        MGPT_CUDA(launch_pdl(plan_assign_kernel<false>, plan_blocks, PLAN_BLOCK, 0, st, p, plan_blocks, blk));
+    }
     MGPT_LAUNCHED("plan_assign_kernel");
     return 0;
 }
