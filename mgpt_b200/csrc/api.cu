@@ -65,7 +65,7 @@ Workspace make_workspace(const Dims& d, int n_tokens, int kind)
     w.row_src = take(rc * 4);
     // (sized alike for every kind, like all before Xg: mgpt_moe_workspace_view and the saved routing know one layout)
     w.decode = decode_usable(d, n_tokens);
-    w.groups = take(w.decode ? (size_t)decode_max_groups(d, n_tokens) * 16 : 0);
+    w.groups = take((size_t)decode_max_groups(d, n_tokens) * 16);
     w.n_groups = take(4);
     w.blk_cnt = take((size_t)w.plan_blocks * E * 4);
     w.slot = take(N * k * 4);

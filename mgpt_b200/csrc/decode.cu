@@ -276,7 +276,13 @@ bool decode_usable(const Dims& d, int n_tokens)
 {
     return d.mode == MGPT_MOE_BF16 && d.gemm_impl == 0 && (long long)n_tokens * d.k <= 8ll * d.E;
 }
-int decode_max_groups(const Dims& d, int n_tokens) { return d.E + (int)((long long)n_tokens * d.k / DECODE_GROUP); }
+// Room in the workspace, also where these kernels are not taken: a workspace never shrinks as the tokens grow.
+int decode_max_groups(const Dims& d, int n_tokens)
+{
+    if (d.mode != MGPT_MOE_BF16 || d.gemm_impl != 0) return 0;
+    const long long rows = (long long)n_tokens * d.k, most = 8ll * d.E;
+    return d.E + (int)((rows < most ? rows : most) / DECODE_GROUP);
+}
 
 // gate/up and down; x: the tokens, or (from_rows) the permuted rows in the workspace.
 int launch_decode_forward(mgpt_moe_layer* L, const Workspace& w, char* ws, const void* x, int io, bool from_rows, cudaStream_t st)

@@ -48,6 +48,20 @@ def test_views_of_a_routing_side_workspace(n, E):
     layer.close()
 
 
+@pytest.mark.parametrize("E,k", [(8, 2), (128, 1), (128, 8)])
+def test_sizes_never_shrink_as_the_tokens_grow(E, k):
+    """A workspace for the largest call serves every smaller one."""
+    layer = MoELayer(64, 64, E, k, mode="bf16")
+    lib, h = layer.lib, layer._h
+    sizes = {"layer": lambda n: lib.mgpt_moe_workspace_bytes(h, n), "inference": lambda n: lib.mgpt_moe_inference_workspace_bytes(h, n),
+             "routing side": lambda n: lib.mgpt_moe_stage_workspace_bytes(h, n, 1),
+             "expert side": lambda n: lib.mgpt_moe_stage_workspace_bytes(h, n, 0), "routing": lambda n: lib.mgpt_moe_routing_bytes(h, n)}
+    for what, size in sizes.items():
+        s = [int(size(n)) for n in range(8 * E // k + 40)]
+        assert all(a <= b for a, b in zip(s, s[1:])), what
+    layer.close()
+
+
 @pytest.mark.parametrize("n,E", [(8, 32), (300, 64)])
 def test_saved_routing_of_a_routing_side_call(n, E):
     """Routing saved after mgpt_moe_route feeds the whole layer's recompute: the outputs of its own forward."""
