@@ -269,12 +269,25 @@ int launch_phase(DecP p, bool spread, int sms, cudaStream_t st)
 
 }  // namespace
 
-// Which forward calls take these kernels: up to 8 rows per expert on average.  From 16 on the B fragments and the MMAs
-// take longer than the weights (256 tokens, E=32: 180 us against 103 + dispatch 14 of the 128-row tcgen05 tiles).
-// Training forwards follow the same rule, so that both give the same bits.
+// Which forward calls take these kernels, training forwards like inference, so that both give the same bits: few rows, and
+// either so few column tiles that the 128-row tcgen05 tiles' down product leaves half of the 148 SMs without one, or few
+// weight bytes times rows.  These kernels save about 15 us of a call (no dispatch where nothing is kept, no first tile to
+// wait for) and lose the more, the more weights stream by and the more rows meet each of them (B fragments and MMAs per
+// weight, and a crowded expert's weights again for every 16 rows).  Inference calls, us with tiles / with these kernels, L2
+// flushed (training steps at the same sizes: 3-9 % faster where few tiles decide, within 2 % of each other elsewhere):
+//   tokens                           1        8       16        32        64       128
+//   C=1024 H=2816 E=32 top-2     68/46    92/79  123/116   137/138   141/142   148/161
+//     a few experts take most    68/46    70/52    70/56     70/56     72/73   76/108
+//   C=2048 H=1408 E=64 top-2     82/60  121/107  158/159   201/206   234/237   250/271
+//   C=1024 H= 512 E=64 top-4     66/46    76/65    92/78     98/87    102/95     96/92
+//   C=2048 H=2816 E= 8 top-2     84/58   115/95   115/95    115/99         .         .
+//   C= 768 H=2048 E=16 top-2     57/38    74/52    78/67     78/69     78/71         .
 bool decode_usable(const Dims& d, int n_tokens)
 {
-    return d.mode == MGPT_MOE_BF16 && d.gemm_impl == 0 && (long long)n_tokens * d.k <= 8ll * d.E;
+    const double rows = (double)n_tokens * d.k, experts = rows < d.E ? rows : d.E;
+    if (d.mode != MGPT_MOE_BF16 || d.gemm_impl != 0 || rows > 8.0 * d.E) return false;
+    if (experts * ((d.C + 255) / 256) <= 74.0) return true;
+    return experts * 6.0 * d.C * d.H * (1.0 + rows / d.E) <= 1.25e9;
 }
 // Room in the workspace, also where these kernels are not taken: a workspace never shrinks as the tokens grow.
 int decode_max_groups(const Dims& d, int n_tokens)
