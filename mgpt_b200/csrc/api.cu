@@ -561,8 +561,6 @@ static int forward_impl(mgpt_moe_layer* L, const void* x, void* y, int n_tokens,
         if (!gathered) {
             L->stage_begin(ST_DISPATCH, st);
             MGPT_TRY(launch_dispatch(d, w, ws, x, io, !inference, st));      // (only backward reads padding rows)
-            // padding rows of what backward reads: finite (the other product kernels compute them)
-            if (w.decode) MGPT_CUDA(cudaMemsetAsync(ws + w.G, 0, w.Yg - w.G, st));
             L->stage_end(ST_DISPATCH, st);
         }
         if (w.decode) MGPT_TRY(launch_decode_forward(L, w, ws, x, io, !gathered, st));

@@ -266,7 +266,9 @@ int launch_combine_bwd(const Dims& d, const Workspace& w, char* ws, const void* 
 int launch_bias_grads(const mgpt_moe_layer* L, const Workspace& w, char* ws, cudaStream_t st);
 int launch_segment_tiles(const Dims& d, const Workspace& w, char* ws, const int32_t* seg_counts, int n_src, cudaStream_t st,
                          int32_t* sticky);
-int dispatch_rows(const Workspace& w, char* ws, const void* src, int src_io, int C, int k, void* dst, bool zero_pad, cudaStream_t st);
+struct PaddingZeros { bf16 *Hh, *G, *U; int H; };      // what backward reads beside Xg; null: its padding rows are not dispatch's
+int dispatch_rows(const Workspace& w, char* ws, const void* src, int src_io, int C, int k, void* dst, bool zero_pad, cudaStream_t st,
+                  PaddingZeros kept = {});
 int combine_rows(const void* rows, const int32_t* pos, const float* top_p, int N, int C, int k, void* y, int io,
                  size_t act_bytes, cudaStream_t st, const void* residual = nullptr);
 int combine_rows_backward(const Workspace& w, char* ws, const void* dy, int io, const void* rows, int C, int k, void* d_rows, cudaStream_t st);

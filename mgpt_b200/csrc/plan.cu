@@ -245,6 +245,23 @@ __device__ __forceinline__ void zero_padding(const int32_t* row_src, int rows, i
     }
 }
 
+// The same in one of the buffers that backward reads beside Xg where the decode kernels, which leave padding rows alone,
+// make the forward: 0: Hh, 1 and 2: the saved SwiGLU factors ([row tile][8-column chunk][128 rows][8], gemm_tc.cu).  Four
+// times the blocks of Xg's instead of a memset of the three whole buffers, which broke the chain of launches and cleared
+// what the worst routing would need (a training step of 1 token, C=1024, H=2816, E=32: 222 -> 214 us; 16 tokens, C=2048,
+// H=1408, E=64: 747 -> 739).
+__device__ __forceinline__ void zero_padding_kept(const int32_t* row_src, int rows, int g, const PaddingZeros& z, int which)
+{
+    if (which == 0) {
+        zero_padding(row_src, rows, g, z.H, z.Hh);
+        return;
+    }
+    const int lane = threadIdx.x & 31, q0 = g * PAD_ROWS + (threadIdx.x >> 5) * 8, row = q0 + (lane & 7);
+    if (row >= rows || row_src[row] >= 0) return;
+    uint4* chunk = reinterpret_cast<uint4*>(which == 1 ? z.G : z.U) + (size_t)(q0 / ROW_TILE) * (z.H >> 3) * ROW_TILE + row % ROW_TILE;
+    for (int c = lane >> 3; c < z.H >> 3; c += 4) chunk[(size_t)c * ROW_TILE] = make_uint4(0, 0, 0, 0);
+}
+
 // Xg[pos(tok,j),:] = x[tok,:] for every choice j; the blocks before the tokens' write the padding rows' zeros (none are
 // launched where nothing reads those rows: the products of inference keep rows apart).  Bound by HBM: one warp per token
 // reads its row once, four 16-byte loads per lane in flight, and writes it k times.  (A warp per padded row read every
@@ -253,15 +270,17 @@ __device__ __forceinline__ void zero_padding(const int32_t* row_src, int rows, i
 template <typename TIn, typename TAct, bool VEC>
 __global__ void __launch_bounds__(256)
 dispatch_kernel(const TIn* x, const int32_t* pos, const int32_t* row_src,
-                const int32_t* n_tiles, int row_cap, int N, int C, int k, int pad_blocks, TAct* Xg)
+                const int32_t* n_tiles, int row_cap, int N, int C, int k, int pad_blocks, TAct* Xg, PaddingZeros kept)
 {
     pdl_wait();
-    const int lane = threadIdx.x & 31;
-    if ((int)blockIdx.x < pad_blocks) {
-        zero_padding(row_src, *n_tiles * ROW_TILE, blockIdx.x, C, Xg);
+    const int lane = threadIdx.x & 31, all_pads = kept.Hh ? 4 * pad_blocks : pad_blocks;
+    if ((int)blockIdx.x < all_pads) {
+        const int rows = *n_tiles * ROW_TILE;
+        if ((int)blockIdx.x < pad_blocks) zero_padding(row_src, rows, blockIdx.x, C, Xg);
+        else zero_padding_kept(row_src, rows, blockIdx.x % pad_blocks, kept, blockIdx.x / pad_blocks - 1);
         return;
     }
-    const int tok = (blockIdx.x - pad_blocks) * 8 + (threadIdx.x >> 5);
+    const int tok = (blockIdx.x - all_pads) * 8 + (threadIdx.x >> 5);
     if (tok >= N) return;
     const int mine = token_row(pos, row_src, row_cap, tok, k, lane);
     const TIn* s = x + (size_t)tok * C;
@@ -506,18 +525,21 @@ int launch_plan(const Dims& d, const Workspace& w, char* ws, cudaStream_t st, in
 }
 
 // dst[pos(tok,j),:] = src[tok,:]; with `zero_pad`, zeros in every other row of the plan's tiles
-int dispatch_rows(const Workspace& w, char* ws, const void* src, int src_io, int C, int k, void* dst, bool zero_pad, cudaStream_t st)
+// (there, and in the buffers of `kept` if given)
+int dispatch_rows(const Workspace& w, char* ws, const void* src, int src_io, int C, int k, void* dst, bool zero_pad, cudaStream_t st,
+                  PaddingZeros kept)
 {
     if (w.n_tokens <= 0) return 0;
     const int32_t* pos = (const int32_t*)(ws + w.pos);
     const int32_t* row_src = (const int32_t*)(ws + w.row_src);
     const int32_t* n_tiles = (const int32_t*)(ws + w.n_tiles);
-    const int N = w.n_tokens, pad_blocks = zero_pad ? (w.row_cap + PAD_ROWS - 1) / PAD_ROWS : 0, grid = pad_blocks + (N + 7) / 8;
+    const int N = w.n_tokens, pad_blocks = zero_pad ? (w.row_cap + PAD_ROWS - 1) / PAD_ROWS : 0;
+    const int grid = (kept.Hh ? 4 * pad_blocks : pad_blocks) + (N + 7) / 8;
     const bool vec = ((uintptr_t)src & 15) == 0;
 #define MGPT_DISPATCH(TIN, TACT)                                                                                          \
     do {                                                                                                                  \
         auto* kernel = vec ? dispatch_kernel<TIN, TACT, true> : dispatch_kernel<TIN, TACT, false>;                        \
-        MGPT_CUDA(launch_pdl(kernel, grid, 256, 0, st, (const TIN*)src, pos, row_src, n_tiles, w.row_cap, N, C, k, pad_blocks, (TACT*)dst)); \
+        MGPT_CUDA(launch_pdl(kernel, grid, 256, 0, st, (const TIN*)src, pos, row_src, n_tiles, w.row_cap, N, C, k, pad_blocks, (TACT*)dst, kept)); \
     } while (0)
     if (w.act_bytes == 4) {
         if (src_io != MGPT_MOE_IO_F32) return fail(MGPT_MOE_EINVAL, "FP32 mode takes FP32 rows");
@@ -534,7 +556,9 @@ int dispatch_rows(const Workspace& w, char* ws, const void* src, int src_io, int
 
 int launch_dispatch(const Dims& d, const Workspace& w, char* ws, const void* x, int io, bool zero_pad, cudaStream_t st)
 {
-    return dispatch_rows(w, ws, x, io, d.C, d.k, ws + w.Xg, zero_pad, st);
+    PaddingZeros kept = {};
+    if (zero_pad && w.decode) kept = PaddingZeros{(bf16*)(ws + w.Hh), (bf16*)(ws + w.G), (bf16*)(ws + w.U), d.H};
+    return dispatch_rows(w, ws, x, io, d.C, d.k, ws + w.Xg, zero_pad, st, kept);
 }
 
 // y = weighted gather-sum of rows[pos[tok,j]]

@@ -61,3 +61,31 @@ def test_a_tokens_bits_do_not_depend_on_the_call(C, H, E, k, ranges, io):
         assert torch.equal(layer.forward_inference(xt[:8].contiguous()), few), sms
     layer.check_status()
     layer.close()
+
+
+@pytest.mark.parametrize("n,C,H,E,k", [(1, 64, 64, 4, 2), (40, 264, 200, 16, 2), (130, 72, 1032, 17, 1)])
+def test_padding_rows_of_a_workspace_full_of_nans(n, C, H, E, k):
+    """Backward multiplies the padding rows of what forward keeps by zeros: they have to be finite whatever was there."""
+    w = synth.Workload("pads", n, C, H, E, k, "bf16")
+    x, params, dy = synth.make_inputs(w, seed=n, bias_std=0.02)
+    layer = MoELayer(C, H, E, k, mode="bf16")
+    layer.load_parameters(params)
+    xt, dyt = torch.from_numpy(x).cuda().bfloat16(), torch.from_numpy(dy).cuda().bfloat16()
+    runs = []
+    for fill in (0, 255):
+        layer.zero_grad()
+        layer._workspace(n).fill_(fill)
+        y = layer.forward(xt).clone()
+        runs.append([y, layer.backward(dyt).clone()] + [p.grad.clone() for p in layer.get_parameters()])
+    rows = int(layer.workspace_view("n_tiles", torch.int32)[0]) * 128
+    pads = layer.workspace_view("row_src", torch.int32)[:rows] < 0
+    for name in ("Xg", "Hh"):
+        assert not layer.workspace_view(name, torch.bfloat16).view(-1, C if name == "Xg" else H)[:rows][pads].any(), name
+    for name in ("G", "U"):
+        t = layer.workspace_view(name, torch.bfloat16)[:rows * H].view(-1, H // 8, 128, 8).permute(0, 2, 1, 3).reshape(-1, H)
+        assert not t[pads].any(), name
+    for a, b in zip(*runs):
+        assert torch.isfinite(b).all()
+        torch.testing.assert_close(b.float(), a.float(), rtol=1e-5, atol=1e-6)      # (only the order of FP32 atomics differs)
+    layer.check_status()
+    layer.close()
