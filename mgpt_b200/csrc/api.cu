@@ -523,6 +523,10 @@ static int forward_impl(mgpt_moe_layer* L, const void* x, void* y, int n_tokens,
     Workspace w;
     MGPT_TRY(check_call(L, n_tokens, io, workspace, ws_bytes, &w, inference ? 3 : 0));
     if (n_tokens > 0 && (!x || !y)) return fail(MGPT_MOE_EINVAL, "null token buffer");
+    if (n_tokens > 0) {
+        MGPT_TRY(check_aligned(y, "y"));
+        MGPT_TRY(check_aligned(residual, "residual"));
+    }
     MGPT_CUDA(cudaSetDevice(L->device));
     cudaStream_t st = (cudaStream_t)stream;
     char* ws = (char*)workspace;
@@ -590,6 +594,9 @@ int mgpt_moe_backward(mgpt_moe_layer* L, const void* x, const void* dy, void* dx
     MGPT_TRY(check_call(L, L->last_n, io, workspace, ws_bytes, &w));
     if (L->last_n == 0) return 0;
     if (!x || !dy || !dx) return fail(MGPT_MOE_EINVAL, "null token buffer");
+    MGPT_TRY(check_aligned(dy, "dy"));
+    MGPT_TRY(check_aligned(dx, "dx"));
+    if (L->has_grad) MGPT_TRY(check_aligned(x, "x", io == MGPT_MOE_IO_F32 ? 16 : 8));      // (the router's weight gradient reads four channels at once)
     MGPT_CUDA(cudaSetDevice(L->device));
     cudaStream_t st = (cudaStream_t)stream;
     char* ws = (char*)workspace;

@@ -63,6 +63,13 @@ void count_launch(int n = 1);
         if (rc__ != 0) return rc__;    \
     } while (0)
 
+// Buffers that kernels touch in pieces of `bytes`: refused here, where a misaligned access would fault on the device.
+inline int check_aligned(const void* p, const char* what, uintptr_t bytes = 16)
+{
+    if ((uintptr_t)p & (bytes - 1)) return fail(MGPT_MOE_EINVAL, std::string(what) + " must be " + std::to_string(bytes) + "-byte aligned");
+    return 0;
+}
+
 // ---- launches -------------------------------------------------------------
 // The kernels of the library are launched with programmatic stream serialization: a kernel's blocks may become resident as
 // soon as the blocks of the kernel before it on the stream have left, do what touches no global memory (barriers, TMEM,

@@ -94,6 +94,7 @@ int mgpt_moe_route_rows(mgpt_moe_layer* L, const void* x, int io, void* workspac
     if (workspace != L->last_ws || io != L->last_io) return fail(MGPT_MOE_ESTATE, "route_rows follows route_plan on the same workspace");
     const int n_tokens = L->last_n;
     if (n_tokens > 0 && (!x || !send_rows)) return fail(MGPT_MOE_EINVAL, "bad token buffer");
+    if (n_tokens > 0) MGPT_TRY(check_aligned(send_rows, "send_rows"));
     const Workspace w = make_workspace(L->d, n_tokens, 1);
     MGPT_TRY(check_ws(L, workspace, ws_bytes, w));
     MGPT_CUDA(cudaSetDevice(L->device));
@@ -120,6 +121,10 @@ int mgpt_moe_combine(mgpt_moe_layer* L, const void* rows_back, void* y, int io, 
     const Workspace w = make_workspace(L->d, L->last_n, 1);
     MGPT_TRY(check_ws(L, workspace, ws_bytes, w));
     if (L->last_n > 0 && (!rows_back || !y)) return fail(MGPT_MOE_EINVAL, "null buffer");
+    if (L->last_n > 0) {
+        MGPT_TRY(check_aligned(rows_back, "rows_back"));
+        MGPT_TRY(check_aligned(y, "y"));
+    }
     MGPT_CUDA(cudaSetDevice(L->device));
     char* ws = (char*)workspace;
     return combine_rows(rows_back, (const int32_t*)(ws + w.pos), (const float*)(ws + w.top_p), w.n_tokens, L->d.C,
@@ -134,6 +139,11 @@ int mgpt_moe_combine_backward(mgpt_moe_layer* L, const void* rows_back, const vo
     const Workspace w = make_workspace(L->d, L->last_n, 1);
     MGPT_TRY(check_ws(L, workspace, ws_bytes, w));
     if (L->last_n > 0 && (!rows_back || !dy || !d_rows)) return fail(MGPT_MOE_EINVAL, "null buffer");
+    if (L->last_n > 0) {
+        MGPT_TRY(check_aligned(rows_back, "rows_back"));
+        MGPT_TRY(check_aligned(dy, "dy"));
+        MGPT_TRY(check_aligned(d_rows, "d_rows"));
+    }
     MGPT_CUDA(cudaSetDevice(L->device));
     char* ws = (char*)workspace;
     return combine_rows_backward(w, ws, dy, io, rows_back, L->d.C, L->d.k, d_rows, (cudaStream_t)stream);
@@ -148,6 +158,9 @@ int mgpt_moe_route_backward(mgpt_moe_layer* L, const void* x, const void* d_rows
     MGPT_TRY(check_ws(L, workspace, ws_bytes, w));
     if (L->last_n == 0) return 0;
     if (!x || !d_rows_in || !dx) return fail(MGPT_MOE_EINVAL, "null buffer");
+    MGPT_TRY(check_aligned(d_rows_in, "d_rows_in"));
+    MGPT_TRY(check_aligned(dx, "dx"));
+    if (L->has_grad) MGPT_TRY(check_aligned(x, "x", io == MGPT_MOE_IO_F32 ? 16 : 8));
     MGPT_CUDA(cudaSetDevice(L->device));
     char* ws = (char*)workspace;
     return launch_router_bwd(L, w, ws, x, io, dx, (cudaStream_t)stream, d_rows_in, (const int32_t*)(ws + w.pos));
