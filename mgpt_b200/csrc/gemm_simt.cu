@@ -37,15 +37,24 @@ template <bool VEC> __device__ __forceinline__ float4 load4(const float* p)
 }
 template <bool VEC> __device__ __forceinline__ float4 load4(const bf16* p)
 {
-    const uint2 u = *reinterpret_cast<const uint2*>(p);       // the library's own buffers: always aligned
+    if constexpr (!VEC) return make_float4(__bfloat162float(p[0]), __bfloat162float(p[1]), __bfloat162float(p[2]), __bfloat162float(p[3]));
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
     return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
                        __uint_as_float(u.y & 0xffff0000u));
 }
 __device__ __forceinline__ float round_to(float v, float) { return v; }
 __device__ __forceinline__ float round_to(float v, bf16) { return __bfloat162float(__float2bfloat16(v)); }
-__device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-__device__ __forceinline__ void store4(bf16* p, float4 v)
+template <bool VEC> __device__ __forceinline__ void store4(float* p, float4 v)
 {
+    if constexpr (VEC) *reinterpret_cast<float4*>(p) = v;
+    else { p[0] = v.x; p[1] = v.y; p[2] = v.z; p[3] = v.w; }
+}
+template <bool VEC> __device__ __forceinline__ void store4(bf16* p, float4 v)
+{
+    if constexpr (!VEC) {
+        p[0] = __float2bfloat16(v.x); p[1] = __float2bfloat16(v.y); p[2] = __float2bfloat16(v.z); p[3] = __float2bfloat16(v.w);
+        return;
+    }
     __nv_bfloat162 h0 = __floats2bfloat162_rn(v.x, v.y), h1 = __floats2bfloat162_rn(v.z, v.w);
     *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t*>(&h0), *reinterpret_cast<uint32_t*>(&h1));
 }
@@ -151,7 +160,8 @@ template <int EPI, int KS> constexpr size_t rows_smem()
     return ops > red ? ops : red;
 }
 
-template <typename TAct, typename TW, int EPI, int KS, bool VEC>
+// VEC: weights and their gradients, AVEC: rows, start on boundaries of four elements.
+template <typename TAct, typename TW, int EPI, int KS, bool VEC, bool AVEC>
 __global__ void __launch_bounds__(GT * KS) simt_rows_kernel(RowsArgs a)
 {
     extern __shared__ __align__(16) float sm[];
@@ -176,7 +186,7 @@ __global__ void __launch_bounds__(GT * KS) simt_rows_kernel(RowsArgs a)
     auto gload = [&](int s) {
         const bool second = EPI == EPI_DXG && s >= per;
         const int k0 = (second ? s - per : s) * TK;
-        fetch<TAct, true, true>((const TAct*)(second ? a.A2 : a.A), K, m0, rows, k0, K, t, ra);
+        fetch<TAct, true, AVEC>((const TAct*)(second ? a.A2 : a.A), K, m0, rows, k0, K, t, ra);
         fetch<TW, BK_MAJOR, VEC>(second ? B2 : B1, BK_MAJOR ? K : N, n0, N, k0, K, t, rb);
         if (NOP == 3) fetch<TW, BK_MAJOR, VEC>(B2, N, n0, N, k0, K, t, rc);
     };
@@ -241,9 +251,9 @@ __global__ void __launch_bounds__(GT * KS) simt_rows_kernel(RowsArgs a)
                 d[j] = acc[i][j];
             }
         }
-        store4((TAct*)a.D + o, make_float4(d[0], d[1], d[2], d[3]));
-        if (EPI == EPI_GATEUP || EPI == EPI_DHH) store4((TAct*)a.D2 + o, make_float4(d2[0], d2[1], d2[2], d2[3]));
-        if (EPI == EPI_GATEUP) store4((TAct*)a.D3 + o, make_float4(d3[0], d3[1], d3[2], d3[3]));
+        store4<AVEC>((TAct*)a.D + o, make_float4(d[0], d[1], d[2], d[3]));
+        if (EPI == EPI_GATEUP || EPI == EPI_DHH) store4<true>((TAct*)a.D2 + o, make_float4(d2[0], d2[1], d2[2], d2[3]));
+        if (EPI == EPI_GATEUP) store4<true>((TAct*)a.D3 + o, make_float4(d3[0], d3[1], d3[2], d3[3]));
     }
 }
 
@@ -268,7 +278,7 @@ template <int KS> constexpr size_t wgrad_smem()
     return ops > red ? ops : red;
 }
 
-template <typename TAct, int KS, bool VEC>
+template <typename TAct, int KS, bool VEC, bool AVEC>
 __global__ void __launch_bounds__(GT * KS) simt_wgrad_kernel(WgradArgs a)
 {
     extern __shared__ __align__(16) float sm[];
@@ -295,8 +305,8 @@ __global__ void __launch_bounds__(GT * KS) simt_wgrad_kernel(WgradArgs a)
         const TAct *As = A + (size_t)r0 * M, *Bs = B + (size_t)r0 * N;
         float4 ra[2], rb[2];
         auto gload = [&](int s) {
-            fetch<TAct, false, true>(As, M, m0, M, s * TK, len, t, ra);
-            fetch<TAct, false, true>(Bs, N, n0, N, s * TK, len, t, rb);
+            fetch<TAct, false, AVEC>(As, M, m0, M, s * TK, len, t, ra);
+            fetch<TAct, false, AVEC>(Bs, N, n0, N, s * TK, len, t, rb);
         };
         auto sstore = [&](int buf) {
             put<false>(S + buf * 2 * OPER, t, ra);
@@ -363,11 +373,20 @@ int split_k(int tiles, int k)
     return ks;
 }
 
+// The row buffers of an expert side are the caller's, at any address; those in the workspace are aligned.
+template <typename TAct> bool rows_aligned(const mgpt_moe_layer* L)
+{
+    const uintptr_t any = (uintptr_t)L->ext_Xg | (uintptr_t)L->ext_Yg | (uintptr_t)L->ext_dYg | (uintptr_t)L->ext_dXg;
+    return (any & (4 * sizeof(TAct) - 1)) == 0;
+}
+
 template <typename TAct, typename TW, int EPI, int KS>
 int launch_rows_ks(const mgpt_moe_layer* L, const RowsArgs& a, dim3 grid, cudaStream_t st)
 {
     constexpr size_t smem = rows_smem<EPI, KS>();
-    auto* kernel = L->masters_aligned ? simt_rows_kernel<TAct, TW, EPI, KS, true> : simt_rows_kernel<TAct, TW, EPI, KS, false>;
+    auto* kernel = !rows_aligned<TAct>(L) ? simt_rows_kernel<TAct, TW, EPI, KS, false, false>
+                   : L->masters_aligned   ? simt_rows_kernel<TAct, TW, EPI, KS, true, true>
+                                          : simt_rows_kernel<TAct, TW, EPI, KS, false, true>;
     if (smem > 48 * 1024) MGPT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     MGPT_CUDA(launch_pdl(kernel, grid, GT * KS, smem, st, a));
     return 0;
@@ -389,7 +408,9 @@ template <typename TAct, int KS>
 int launch_wgrad_ks(const mgpt_moe_layer* L, const WgradArgs& a, dim3 grid, cudaStream_t st)
 {
     constexpr size_t smem = wgrad_smem<KS>();
-    auto* kernel = L->masters_aligned ? simt_wgrad_kernel<TAct, KS, true> : simt_wgrad_kernel<TAct, KS, false>;
+    auto* kernel = !rows_aligned<TAct>(L) ? simt_wgrad_kernel<TAct, KS, false, false>
+                   : L->masters_aligned   ? simt_wgrad_kernel<TAct, KS, true, true>
+                                          : simt_wgrad_kernel<TAct, KS, false, true>;
     if (smem > 48 * 1024) MGPT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     MGPT_CUDA(launch_pdl(kernel, grid, GT * KS, smem, st, a));
     return 0;

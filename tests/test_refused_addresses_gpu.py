@@ -1,4 +1,4 @@
-"""Token buffers that the kernels touch 16 bytes at a time: another address is an error before anything is launched, and
+"""Token buffers that the kernels touch 16 bytes at a time: another address is an error before those are launched, and
 buffers on such boundaries work as before afterwards."""
 import ctypes as ct
 
@@ -70,5 +70,35 @@ def test_stage_calls():
     _refused(lambda: check(lib.mgpt_moe_route_backward(h, p(xt), p(bad_rows), p(dx), layer._io(xt), *tail)))
     _refused(lambda: check(lib.mgpt_moe_route_backward(h, p(xt), p(rows), p(bad_x), layer._io(xt), *tail)))
     check(lib.mgpt_moe_combine(h, p(rows), p(y), layer._io(xt), *tail))
+    layer.check_status()
+    layer.close()
+
+
+@pytest.mark.parametrize("mode,io", [("fp32", torch.float32), ("bf16", torch.bfloat16)])
+def test_expert_side_rows_of_the_cuda_core_products_at_any_address(mode, io):
+    """The row buffers of mgpt_moe_experts_* belong to the caller: the CUDA-core products take them wherever they start."""
+    C, H, E = 72, 136, 3
+    counts = torch.tensor([130, 0, 5], dtype=torch.int32, device="cuda")
+    layer = MoELayer(C, H, E, 1, mode=mode, gemm_impl=1)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    for p in layer.get_parameters():
+        p.normal_(0.0, 0.05, generator=gen)
+    layer.sync_weights()
+    lib, h, st, n = layer.lib, layer._h, layer._stream(), 384
+    ws = torch.empty(int(lib.mgpt_moe_stage_workspace_bytes(h, n, 0)), dtype=torch.uint8, device="cuda")
+    rows, d_out = torch.zeros(n, C, dtype=io, device="cuda"), torch.zeros(n, C, dtype=io, device="cuda")
+    for t in (rows, d_out):
+        for r0, r1 in ((0, 130), (256, 261)):
+            t[r0:r1] = torch.randn(r1 - r0, C, generator=gen, device="cuda").to(io)
+    runs = []
+    for place in (lambda t: t.clone(), off_by_one):
+        layer.zero_grad()
+        x, y, dy, dx = place(rows), place(torch.zeros_like(rows)), place(d_out), place(torch.zeros_like(rows))
+        _lib.check(lib.mgpt_moe_experts_forward(h, x.data_ptr(), counts.data_ptr(), 1, n, y.data_ptr(), ws.data_ptr(), ws.numel(), st))
+        _lib.check(lib.mgpt_moe_experts_backward(h, dy.data_ptr(), dx.data_ptr(), ws.data_ptr(), ws.numel(), st))
+        torch.cuda.synchronize()
+        assert y[:130].any() and dx[256:261].any()
+        runs.append([y, dx] + [p.grad.clone() for p in layer.get_parameters()])
+    assert all(torch.equal(a, b) for a, b in zip(*runs))
     layer.check_status()
     layer.close()
