@@ -7,7 +7,7 @@ import torch
 
 from mgpt_b200 import MoELayer, synth
 from oracle import oracle
-from tests.util import assert_routing_exact, assert_values, dims_of, run_layer
+from tests.util import assert_routing_exact, assert_values, dims_of, rel_l2, run_layer
 
 pytestmark = pytest.mark.gpu
 
@@ -89,3 +89,46 @@ def test_padding_rows_of_a_workspace_full_of_nans(n, C, H, E, k):
         torch.testing.assert_close(b.float(), a.float(), rtol=1e-5, atol=1e-6)      # (only the order of FP32 atomics differs)
     layer.check_status()
     layer.close()
+
+
+@pytest.mark.parametrize("n,C,H,E,k,crowd", [
+    (1, 64, 64, 4, 2, False),
+    (7, 72, 200, 8, 3, False),
+    (32, 1032, 136, 16, 4, False),
+    (33, 520, 520, 17, 1, True),
+    (6, 1024, 2816, 32, 2, False),        # four warps per task
+    (20, 1024, 2816, 32, 2, False),       # one
+])
+@pytest.mark.parametrize("io", [torch.float32, torch.bfloat16])
+def test_buffers_against_the_cuda_core_products(n, C, H, E, k, crowd, io):
+    """What these kernels write, buffer by buffer, against the CUDA-core products on the same BF16 data, at the bar of the
+    tensor-core ones: each side's stored value is within 2^-9 of its FP32 sum, and the cross-check makes Hh and the factors
+    from gate and up as it has stored them, so three such roundings lie between the two at most."""
+    w = synth.Workload("cross", n, C, H, E, k, "bf16")
+    x, params, _ = synth.make_inputs(w, seed=5 + n, bias_std=0.02)
+    if crowd:
+        params[1][0, 5] = np.float32(64.0)
+    xt = torch.from_numpy(x).cuda().to(io)
+    got = {}
+    for impl in (0, 1):
+        layer = MoELayer(C, H, E, k, mode="bf16", gemm_impl=impl)
+        layer.load_parameters(params)
+        y = layer.forward(xt)
+        real = layer.workspace_view("row_src", torch.int32) >= 0
+        real[int(layer.workspace_view("n_tiles", torch.int32)[0]) * 128:] = False
+        bufs = {"y": y.float()}
+        for name, width in (("G", H), ("U", H), ("Hh", H), ("Yg", C)):
+            t = layer.workspace_view(name, torch.bfloat16)
+            if impl == 0 and name in "GU":          # [row tile][8-column chunk][128 rows][8]
+                t = t.view(-1, width // 8, 128, 8).permute(0, 2, 1, 3).reshape(-1, width)
+            bufs[name] = t.view(-1, width)[real].double()
+        if impl == 1:
+            g, u = bufs["G"], bufs["U"]
+            sig = torch.sigmoid(g)
+            bufs["G"], bufs["U"] = u * sig * (1.0 + g * (1.0 - sig)), g * sig
+        got[impl] = bufs
+        layer.check_status()
+        layer.close()
+    for name, want in got[1].items():
+        err = rel_l2(got[0][name].cpu().numpy(), want.cpu().numpy())
+        assert err < 6e-3, (name, err)
