@@ -76,9 +76,10 @@ inline int check_aligned(const void* p, const char* what, uintptr_t bytes = 16)
 // addresses) while that kernel's writes are still being flushed, and wait in pdl_wait() until all of it has finished
 // and is visible.  EVERY block of EVERY kernel launched this way goes through pdl_wait(), also one that has nothing to do: "the kernel
 // before has finished" then implies the same for all kernels before that one.  Takes the ~2 us between two kernels of
-// a step to ~1 us.  No kernel releases its successor early (griddepcontrol.launch_dependents): the waiting blocks then
-// pile up several kernels deep and spread the next kernel's blocks unevenly over the SMs (a 256-token decode call:
-// 155 us without any of this, 144 us with the wait alone, 194 us with the early release).
+// a step to ~1 us.  Only decode_kernel's gate/up releases its successor early (griddepcontrol.launch_dependents), after its
+// own wait, for a kernel that can request weights meanwhile.  With an early release at the top of every kernel the waiting
+// blocks pile up several kernels deep and spread the next kernel's blocks unevenly over the SMs (a 256-token decode call:
+// 155 us without any of this, 144 us with the wait alone, 194 us with that).
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args)
 {

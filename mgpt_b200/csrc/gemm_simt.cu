@@ -25,10 +25,6 @@ constexpr int GT = 128;                       // threads per K group
 constexpr int SROW = TM + 4;                  // padded row of a staged operand (floats)
 constexpr int OPER = TK * SROW;               // one staged operand
 
-template <typename T> __device__ __forceinline__ T from_f32(float v);
-template <> __device__ __forceinline__ float from_f32<float>(float v) { return v; }
-template <> __device__ __forceinline__ bf16 from_f32<bf16>(float v) { return __float2bfloat16(v); }
-
 // four consecutive elements (VEC: the address is aligned to four elements)
 template <bool VEC> __device__ __forceinline__ float4 load4(const float* p)
 {
