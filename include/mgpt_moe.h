@@ -174,7 +174,7 @@ int  mgpt_moe_forward_residual(mgpt_moe_layer* layer, const void* x, const void*
  * A token's y keeps its bits as a context grows, with two exceptions (of both forward calls; the order of the sums in the
  * products, and the kernel that computes the top-k weights, change with the number of tokens).  In BF16 mode, gemm_impl
  * 0: calls of few rows -- with R = n_tokens * top_k, T = min(R, num_experts): R <= 8 * num_experts, and either
- * T * ceil(embed_dim / 256) <= 74 or T * 6 * embed_dim * hidden_dim * (1 + R / num_experts) <= 1.25e9 -- against larger
+ * T * ceil(embed_dim / 256) <= 74 or T * 6 * embed_dim * hidden_dim * (1 + R / num_experts) <= 1.7e9 -- against larger
  * ones; and BF16 tokens from n_tokens * embed_dim * num_experts = 4e8 on.  mgpt_moe_backward cannot follow it (MGPT_MOE_ESTATE);
  * mgpt_moe_expert_counts can. */
 size_t mgpt_moe_inference_workspace_bytes(const mgpt_moe_layer* layer, int n_tokens);

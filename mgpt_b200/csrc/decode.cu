@@ -12,12 +12,12 @@
 //
 // A k-block's order of k within the fragments is chosen so that one 16-byte load feeds two MMAs (A and B agree on it, so
 // the sum is the same set of products).  A row group is up to 16 rows of one expert (the plan lists them); more rows
-// read the weights again, mostly from L2.  A product is the sum of the sums over four equal parts of its k-blocks, added
-// in order (one part where it has fewer than eight k-blocks).  KS = 4: a warp for each part, which add up through shared
-// memory -- for launches with too few tasks to give every warp some; KS = 1: one warp runs through all parts.  Either way
-// the additions are the same: a row's bits depend neither on the other rows of the call, nor on how many there are, nor on
-// the number of SMs.  (The second accumulator costs KS = 1 3 % at 64 tokens, C=1024, H=2816, E=32: 123.3 -> 127.1 us for the
-// call; the sums kept in shared memory instead 128.2.)
+// read the weights again, mostly from L2.  KS = 4 warps share a task's k-blocks and add up, in order, through shared
+// memory; where a product has fewer than eight k-blocks one warp does it alone.  The widths alone decide that: a row's bits
+// depend neither on the other rows of the call, nor on how many there are, nor on the number of SMs.  (One warp per task
+// from two tasks per warp on, which adds up in another order, was as fast at 20 and 32 tokens, C=1024, H=2816, E=32, 124
+// and 134 us for the call, slower at 16 with C=2048, H=1408, E=64, 155 against 142, and ahead only at 64, 138 against 144,
+// which tiles do in 141.  One warp that keeps the four parts' sums apart: 130, 138, 155 and 142.)
 //
 // tcgen05 is no help here: its M side is 128 rows whatever the number of tokens, and with the weights on the M side
 // instead an MMA of N = 16 still took ~120 cycles for 4 KiB of weights (1000 cycles per 32 KiB stage, 135 us for the
@@ -44,7 +44,6 @@ struct DecP {
     const bf16* A;                     // down: Hh
     bf16 *out, *G, *U;
     int C, H, k, hb, cb, kb1, kb2;
-    int parts;                         // of this phase's reduction
 };
 
 __device__ __forceinline__ uint4 ld_weights(const bf16* p)
@@ -84,10 +83,9 @@ __device__ __forceinline__ void ld_frag(Frag& f, const bf16* ra, const bf16* rb,
 
 // acc[nn] += the task's weights x rows nn*8.. over the k-blocks [k0, k1).  `w` holds the first DEPTH of them, already
 // requested.
-// `after(kb)` follows every k-block.
-template <int NN, typename TRow, typename After>
+template <int NN, typename TRow>
 __device__ __forceinline__ void run_task(Frag (&w)[DEPTH], const bf16* ra, const bf16* rb, const TRow* const (&src)[NN], int k0, int k1,
-                                         int K, int t4, float (&acc)[NN][4], After after)
+                                         int K, int t4, float (&acc)[NN][4])
 {
     for (int kb = k0; kb < k1; kb += DEPTH) {
 #pragma unroll
@@ -110,7 +108,6 @@ __device__ __forceinline__ void run_task(Frag (&w)[DEPTH], const bf16* ra, const
                         mma16816(acc[n], f.v[s].x, f.v[2 + s].x, f.v[s].y, f.v[2 + s].y, b[n][s].x, b[n][s].y);
                         mma16816(acc[n], f.v[s].z, f.v[2 + s].z, f.v[s].w, f.v[2 + s].w, b[n][s].z, b[n][s].w);
                     }
-                after(kb + u);
             }
         }
     }
@@ -171,29 +168,7 @@ __global__ void __launch_bounds__(32 * DW, 1) decode_kernel(const DecP p)
             for (int n = 0; n < NN; ++n)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) acc[n][i] = 0.0f;
-            float sum[NN][4];                               // KS = 1: of the parts that have ended
-#pragma unroll
-            for (int n = 0; n < NN; ++n)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) sum[n][i] = -0.0f;      // (-0 + v is v, whatever v is)
-            int part = 0, part_end = kbs / p.parts;
-            run_task<NN, TRow>(w, ra, rb, src, k0, k1, K, t4, acc, [&](int kb) {
-                if (KS > 1) return;
-                const bool ends = kb + 1 == part_end;
-#pragma unroll
-                for (int n = 0; n < NN; ++n)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        sum[n][i] = ends ? sum[n][i] + acc[n][i] : sum[n][i];
-                        acc[n][i] = ends ? 0.0f : acc[n][i];
-                    }
-                if (ends) part_end = kbs * (++part + 1) / p.parts;
-            });
-            if (KS == 1)
-#pragma unroll
-                for (int n = 0; n < NN; ++n)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) acc[n][i] = sum[n][i];
+            run_task<NN, TRow>(w, ra, rb, src, k0, k1, K, t4, acc);
             if constexpr (KS > 1) {
                 if (ks > 0)
 #pragma unroll
@@ -254,14 +229,10 @@ __global__ void __launch_bounds__(32 * DW, 1) decode_kernel(const DecP p)
     if (!waited) pdl_wait();
 }
 
-// A product is the sum, in order, of this many sums over equal parts of its k-blocks.
-int decode_parts(int kblocks) { return kblocks >= 8 ? 4 : 1; }
-
 template <int PHASE, bool F32>
-int launch_phase(DecP p, bool spread, int sms, cudaStream_t st)
+int launch_phase(const DecP& p, int sms, cudaStream_t st)
 {
-    p.parts = decode_parts(PHASE == 1 ? p.kb1 : p.kb2);
-    if (spread && p.parts == 4) MGPT_CUDA(launch_pdl(decode_kernel<PHASE, 4, F32>, sms, 32 * DW, 0, st, p));
+    if ((PHASE == 1 ? p.kb1 : p.kb2) >= 8) MGPT_CUDA(launch_pdl(decode_kernel<PHASE, 4, F32>, sms, 32 * DW, 0, st, p));
     else MGPT_CUDA(launch_pdl(decode_kernel<PHASE, 1, F32>, sms, 32 * DW, 0, st, p));
     MGPT_LAUNCHED(PHASE == 1 ? "decode_kernel<gateup>" : "decode_kernel<down>");
     return 0;
@@ -274,20 +245,21 @@ int launch_phase(DecP p, bool spread, int sms, cudaStream_t st)
 // weight bytes times rows.  These kernels save about 15 us of a call (no dispatch where nothing is kept, no first tile to
 // wait for) and lose the more, the more weights stream by and the more rows meet each of them (B fragments and MMAs per
 // weight, and a crowded expert's weights again for every 16 rows).  Inference calls, us with tiles / with these kernels, L2
-// flushed (training steps at the same sizes: 3-9 % faster where few tiles decide, within 2 % of each other elsewhere):
+// flushed (training steps at the same sizes: up to 11 % faster where few tiles decide, within 3 % of each other elsewhere):
 //   tokens                           1        8       16        32        64       128
-//   C=1024 H=2816 E=32 top-2     68/46    92/79  123/116   137/138   141/142   148/161
-//     a few experts take most    68/46    70/52    70/56     70/56     72/73   76/108
-//   C=2048 H=1408 E=64 top-2     82/60  121/107  158/159   201/206   234/237   250/271
-//   C=1024 H= 512 E=64 top-4     66/46    76/65    92/78     98/87    102/95     96/92
-//   C=2048 H=2816 E= 8 top-2     84/58   115/95   115/95    115/99         .         .
-//   C= 768 H=2048 E=16 top-2     57/38    74/52    78/67     78/69     78/71         .
+//   C=1024 H=2816 E=32 top-2     66/46    90/77  121/116   137/136   141/144   145/159
+//     a few experts take most    66/46    68/48    68/50     68/56     72/69    74/108
+//   C=2048 H=1408 E=64 top-2     80/60  121/106  157/147   199/194   232/241   250/271
+//     a few experts take most    82/59    84/61    88/75     88/81     92/95    96/130
+//   C=1024 H= 512 E=64 top-4     64/46    76/65    92/78     98/87    102/95     95/92
+//   C=2048 H=2816 E= 8 top-2     82/58   113/95   113/95    113/99         .         .
+//   C= 768 H=2048 E=16 top-2     57/38    72/54    78/65     78/67     78/71         .
 bool decode_usable(const Dims& d, int n_tokens)
 {
     const double rows = (double)n_tokens * d.k, experts = rows < d.E ? rows : d.E;
     if (d.mode != MGPT_MOE_BF16 || d.gemm_impl != 0 || rows > 8.0 * d.E) return false;
     if (experts * ((d.C + 255) / 256) <= 74.0) return true;
-    return experts * 6.0 * d.C * d.H * (1.0 + rows / d.E) <= 1.25e9;
+    return experts * 6.0 * d.C * d.H * (1.0 + rows / d.E) <= 1.7e9;
 }
 // Room in the workspace, also where these kernels are not taken: a workspace never shrinks as the tokens grow.
 int decode_max_groups(const Dims& d, int n_tokens)
@@ -310,11 +282,6 @@ int launch_decode_forward(mgpt_moe_layer* L, const Workspace& w, char* ws, const
     int sms = 0;
     MGPT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, L->device));
     if (L->sm_budget > 0 && L->sm_budget < sms) sms = L->sm_budget;
-    // four warps per task while there are fewer than two tasks per warp (tasks: one per touched expert and 8 hidden
-    // units / 16 columns)
-    const long long T = w.R < d.E ? w.R : d.E;
-    const long long warps = (long long)sms * DW;
-    const bool spread1 = T * ((d.H + 7) / 8) < 2 * warps, spread2 = T * ((d.C + 15) / 16) < 2 * warps;
     p.x = from_rows ? (const void*)(ws + w.Xg) : x;
     p.row_src = from_rows ? nullptr : (const int32_t*)(ws + w.row_src);
     p.out = (bf16*)(ws + w.Hh);
@@ -322,14 +289,14 @@ int launch_decode_forward(mgpt_moe_layer* L, const Workspace& w, char* ws, const
     p.U = w.inference ? nullptr : (bf16*)(ws + w.U);
     p.b0 = L->master.bg; p.b1 = L->master.bu;
     L->stage_begin(ST_GATEUP, st);
-    if (from_rows || io == MGPT_MOE_IO_BF16) MGPT_TRY((launch_phase<1, false>(p, spread1, sms, st)));
-    else MGPT_TRY((launch_phase<1, true>(p, spread1, sms, st)));
+    if (from_rows || io == MGPT_MOE_IO_BF16) MGPT_TRY((launch_phase<1, false>(p, sms, st)));
+    else MGPT_TRY((launch_phase<1, true>(p, sms, st)));
     L->stage_end(ST_GATEUP, st);
     p.A = (const bf16*)(ws + w.Hh);
     p.out = (bf16*)(ws + w.Yg);
     p.b0 = L->master.bd;
     L->stage_begin(ST_DOWN, st);
-    MGPT_TRY((launch_phase<2, false>(p, spread2, sms, st)));
+    MGPT_TRY((launch_phase<2, false>(p, sms, st)));
     L->stage_end(ST_DOWN, st);
     return 0;
 }

@@ -37,14 +37,14 @@ def test_few_rows_per_expert(n, C, H, E, k, crowd, io):
 
 @pytest.mark.parametrize("C,H,E,k,ranges", [
     # (a range: token counts that take the same kernels)
-    (1024, 2816, 32, 2, [[1, 2, 6, 7, 8, 20], [21, 64, 128]]),     # gate/up goes from four warps per task to one between 6 and 7
-    (1024, 1032, 128, 2, [[1, 18, 36, 37, 53], [54, 300]]),        # both products do between 36 and 37; 17 k-blocks, uneven parts
-    (256, 520, 16, 2, [[1, 16, 63, 64], [65, 90]]),                # four k-blocks: one part; nine: parts of 2, 2, 2 and 3
+    (1024, 2816, 32, 2, [[1, 2, 6, 7, 8, 33], [34, 64, 128]]),     # from 7 tokens on every warp could have two tasks of its own
+    (1024, 1032, 128, 2, [[1, 18, 36, 37, 70], [71, 300]]),        # from 37; 17 k-blocks in uneven parts
+    (256, 520, 16, 2, [[1, 16, 63, 64], [65, 90]]),                # four k-blocks: one warp; nine: parts of 2, 2, 2 and 3
 ])
 @pytest.mark.parametrize("io", [torch.float32, torch.bfloat16])
 def test_a_tokens_bits_do_not_depend_on_the_call(C, H, E, k, ranges, io):
-    """The rows of a growing context keep their bits, whichever split of the reduction the number of tokens and the SM
-    budget lead to, but for the one step between the kernels for few rows per expert and the others."""
+    """The rows of a growing context keep their bits, whatever the number of tokens and the SM budget, but for the one step
+    between the kernels for few rows per expert and the others."""
     n_all = ranges[-1][-1]
     w = synth.Workload("grow", n_all, C, H, E, k, "bf16")
     x, params, _ = synth.make_inputs(w, seed=29, bias_std=0.02)
@@ -96,8 +96,8 @@ def test_padding_rows_of_a_workspace_full_of_nans(n, C, H, E, k):
     (7, 72, 200, 8, 3, False),
     (32, 1032, 136, 16, 4, False),
     (33, 520, 520, 17, 1, True),
-    (6, 1024, 2816, 32, 2, False),        # four warps per task
-    (20, 1024, 2816, 32, 2, False),       # one
+    (6, 1024, 2816, 32, 2, False),
+    (33, 1024, 2816, 32, 2, False),       # the most tokens of this shape
 ])
 @pytest.mark.parametrize("io", [torch.float32, torch.bfloat16])
 def test_buffers_against_the_cuda_core_products(n, C, H, E, k, crowd, io):
