@@ -268,14 +268,18 @@ int mgpt_moe_bind_params(mgpt_moe_layer* L, float* const* data, float* const* gr
     const bool router = data[0] != nullptr && data[1] != nullptr;
     const bool experts = n == L->n_params;
     if (!router && !experts) return fail(MGPT_MOE_EINVAL, "null parameter pointer");
-    L->masters_aligned = true;
+    L->masters_aligned = L->biases_aligned = L->grad_wd_aligned = true;
     for (int i = 0; i < L->n_params; ++i) {
         const bool want = i < 2 ? router : experts;
         if (want && !data[i]) return fail(MGPT_MOE_EINVAL, "null parameter pointer");
         if (want && grad && !grad[i]) return fail(MGPT_MOE_EINVAL, "null gradient pointer");
         L->p_data[i] = want ? data[i] : nullptr;
         L->p_grad[i] = (want && grad) ? grad[i] : nullptr;
-        if (i >= 2 && (((uintptr_t)L->p_data[i] | (uintptr_t)L->p_grad[i]) & 15)) L->masters_aligned = false;
+        if (i < 2) continue;
+        if (((uintptr_t)L->p_data[i] | (uintptr_t)L->p_grad[i]) & 15) L->masters_aligned = false;
+        const int kind = (i - 2) % 6;
+        if (kind % 2 == 1 && (kind == 5 ? L->d.C : L->d.H) >= 32 && ((uintptr_t)L->p_data[i] & 15)) L->biases_aligned = false;
+        if (kind == 4 && ((uintptr_t)L->p_grad[i] & 15)) L->grad_wd_aligned = false;
     }
     L->has_grad = grad != nullptr;
     L->router_bound = router;

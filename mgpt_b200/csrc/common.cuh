@@ -173,6 +173,8 @@ struct mgpt_moe_layer {
     bool bound = false, has_grad = false, shadows_fresh = false;
     bool router_bound = false, experts_bound = false;
     bool masters_aligned = false;            // every bound expert tensor (data and gradient) starts on a 16-byte boundary
+    bool biases_aligned = false;             // the expert biases of 32 elements or more do
+    bool grad_wd_aligned = false;            // the gradients of Wd do
 
     // Error bits of every kernel of this layer since the last mgpt_moe_check_status (device word, zero at create)
     // and the pinned host word they are read into.

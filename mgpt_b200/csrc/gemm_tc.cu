@@ -1171,6 +1171,7 @@ int launch_rows(mgpt_moe_layer* L, TcState* s, const Workspace& w, const RowsP& 
 
 int tc_experts_forward(mgpt_moe_layer* L, const Workspace& w, char* ws, cudaStream_t st)
 {
+    if (!L->biases_aligned) return fail(MGPT_MOE_EINVAL, "the expert biases must be 16-byte aligned");
     MGPT_TRY(prepare(L, w, ws));
     TcState* s = (TcState*)L->tc_state;
     const Dims& d = L->d;
@@ -1203,6 +1204,7 @@ int tc_experts_forward(mgpt_moe_layer* L, const Workspace& w, char* ws, cudaStre
 // phase: 1 = gradients w.r.t. the rows (dHh, dXg), 2 = gradients w.r.t. the parameters, 3 = both
 int tc_experts_backward(mgpt_moe_layer* L, const Workspace& w, char* ws, cudaStream_t st, int phase)
 {
+    if (L->has_grad && !L->grad_wd_aligned) return fail(MGPT_MOE_EINVAL, "the gradients of Wd must be 16-byte aligned");
     MGPT_TRY(prepare(L, w, ws));
     TcState* s = (TcState*)L->tc_state;
     const Dims& d = L->d;
@@ -1305,6 +1307,7 @@ int tc_router_dx(mgpt_moe_layer* L, const Workspace& w, char* ws, const void* dX
 // make one wave: 51-57 -> 39 us at 32768 tokens, C=2048, E=64 (8.8 and 15 us at 8192 x 512 and 16384 x 1024: unchanged).
 int tc_router_wgrad(mgpt_moe_layer* L, const Workspace& w, char* ws, const void* x, cudaStream_t st)
 {
+    MGPT_TRY(check_aligned(L->p_grad[0], "the gradient of Wr"));
     MGPT_TRY(prepare_attrs(L));
     TcState* s = (TcState*)L->tc_state;
     const Dims& d = L->d;

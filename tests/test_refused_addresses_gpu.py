@@ -102,3 +102,27 @@ def test_expert_side_rows_of_the_cuda_core_products_at_any_address(mode, io):
     assert all(torch.equal(a, b) for a, b in zip(*runs))
     layer.check_status()
     layer.close()
+
+
+@pytest.mark.parametrize("what,first", [("bias", 3), ("bias", 7), ("gradient", 6), ("gradient", 0)])
+def test_parameters_of_the_tensor_core_products(what, first):
+    """Expert biases (of gate, of down) and the gradients of Wd and Wr, which those kernels touch 16 bytes at a time."""
+    n, C, H, E = 300, 64, 64, 4                                 # (too many rows for the decode kernels)
+    layer = MoELayer(C, H, E, 2, mode="bf16")
+    for i, p in enumerate(layer.params):
+        p.normal_(0.0, 0.05)
+        if what == "gradient" and (i == first or first > 0 and i >= 2 and (i - first) % 6 == 0):
+            p.grad = off_by_one(torch.zeros_like(p))
+        if what == "bias" and i >= 2 and (i - first) % 6 == 0:
+            grad, layer.params[i] = p.grad, off_by_one(p)
+            layer.params[i].grad = grad
+    layer._bind()
+    layer.sync_weights()
+    x = torch.randn(n, C, device="cuda").bfloat16()
+    if what == "bias":
+        _refused(lambda: layer.forward(x))
+    else:
+        layer.forward(x)
+        _refused(lambda: layer.backward(x))
+    layer.check_status()
+    layer.close()
