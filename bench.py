@@ -28,12 +28,12 @@ METRIC = "moe_layer_fwd_bwd_tokens_per_sec"
 # c4 is too large to capture with many passes: its figures are those of c4q (a quarter of the tokens and of the
 # experts, same rows per expert) times four -- every term of the traffic is proportional to the number of experts.
 TRAFFIC = {
-    ("c3", "wgrad_gemm"): 827.5e6, ("c3", "gateup_gemm"): 337.8e6, ("c3", "dhh_gemm"): 397.0e6,
-    ("c3", "down_gemm"): 177.2e6, ("c3", "dxg_gemm"): 282.2e6,
-    ("c4q", "wgrad_gemm"): 1413.9e6, ("c4q", "gateup_gemm"): 373.7e6, ("c4q", "dhh_gemm"): 344.1e6,
-    ("c4q", "down_gemm"): 188.5e6, ("c4q", "dxg_gemm"): 339.5e6,
-    ("c4", "wgrad_gemm"): 4 * 1413.9e6, ("c4", "gateup_gemm"): 4 * 373.7e6, ("c4", "dhh_gemm"): 4 * 344.1e6,
-    ("c4", "down_gemm"): 4 * 188.5e6, ("c4", "dxg_gemm"): 4 * 339.5e6,
+    ("c3", "wgrad_gemm"): 822.7e6, ("c3", "gateup_gemm"): 338.8e6, ("c3", "dhh_gemm"): 396.5e6,
+    ("c3", "down_gemm"): 176.1e6, ("c3", "dxg_gemm"): 281.1e6,
+    ("c4q", "wgrad_gemm"): 1410.0e6, ("c4q", "gateup_gemm"): 369.5e6, ("c4q", "dhh_gemm"): 343.0e6,
+    ("c4q", "down_gemm"): 184.7e6, ("c4q", "dxg_gemm"): 335.5e6,
+    ("c4", "wgrad_gemm"): 4 * 1410.0e6, ("c4", "gateup_gemm"): 4 * 369.5e6, ("c4", "dhh_gemm"): 4 * 343.0e6,
+    ("c4", "down_gemm"): 4 * 184.7e6, ("c4", "dxg_gemm"): 4 * 335.5e6,
 }
 UNIT = "tokens/s"
 
