@@ -16,7 +16,11 @@
  *     stream the reference uses everywhere) and nothing synchronises unless
  *     the comment says so;
  *   - token tensors are row-major [n_tokens, embed_dim] (the reference's
- *     [B,T,C] flattened, MoELayer.cpp:30);
+ *     [B,T,C] flattened, MoELayer.cpp:30); y, residual, dy, dx and exchanged
+ *     rows start on a 16-byte boundary, x too where a weight gradient is
+ *     formed from it (8 bytes for BF16), else MGPT_MOE_EINVAL; the same holds
+ *     for the expert biases and the gradients of Wd and Wr where the
+ *     tensor-core products use them;
  *   - parameter order is the reference's get_parameters() order
  *     (MoELayer.cpp:225-236): Wr[C,E], br[E], then per expert
  *     Wg[C,H], bg[H], Wu[C,H], bu[H], Wd[H,C], bd[C]  (2+6E tensors).
@@ -109,8 +113,10 @@ int  mgpt_moe_expert_counts(mgpt_moe_layer* layer, int32_t* host_counts);
 /* Offset and size of a named buffer inside the workspace for n_tokens, for
  * tests and for callers that read routing results in place. Names:
  * logits probs top_idx top_p counts offsets padded_offsets map pos row_src
- * tile_expert n_tiles Xg G U Hh Yg dYg dG dU dXg d_top_p dlogits status
+ * tile_expert n_tiles slot Xg G U Hh Yg dYg dG dU dXg d_top_p dlogits status
  * router_recompute (one int32: tokens the BF16-token router recomputed exactly).
+ * The views from logits to slot also fit the workspace of a routing-side call
+ * (mgpt_moe_route) and of an inference forward; the others the whole layer's.
  * Activation buffers are row-major [padded rows, width], except G and U on
  * the tensor-core path (mode BF16, gemm_impl 0), which only its own epilogues
  * read: there the buffer named G holds U*sigmoid(G)*(1 + G*(1 - sigmoid(G))) and
