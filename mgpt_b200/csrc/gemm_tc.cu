@@ -161,11 +161,11 @@ __device__ __forceinline__ int sched_consume(const Pipe& pipe, uint32_t n, int32
     return item;
 }
 __device__ __forceinline__ void sched_release(const Pipe& pipe, uint32_t n) { mbar_arrive(pipe.sched_empty(n % SCHED_Q)); }
-// Once per CTA of the grid, by the producer thread after its last fetch (also CTAs that leave without fetching).
-__device__ __forceinline__ void sched_finish(int32_t* counter)
+// Once per CTA of the grid (CTA pair: by the leader), by the producer thread after its last fetch.
+__device__ __forceinline__ void sched_finish(int32_t* counter, int callers)
 {
     __threadfence();
-    if (atomicAdd(counter + 1, 1) == (int)gridDim.x - 1) {
+    if (atomicAdd(counter + 1, 1) == callers - 1) {
         counter[0] = 0;
         counter[1] = 0;
         __threadfence();
@@ -538,7 +538,7 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
     const int total_items = (MODE == MODE_DX ? p.fixed_tiles : *p.n_tiles) * p.n_col_tiles;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t it = 0;
             bool ok = true;
             int item = blockIdx.x;
@@ -583,10 +583,10 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
                 if (ok) ok = sched_publish(pipe, nf, next, total_items, p.status);
                 item = next;
             }
-            if (!DEALT) sched_finish(p.sched);           // this CTA asks for no more items
+            if (!DEALT) sched_finish(p.sched, gridDim.x);           // this CTA asks for no more items
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t it = 0, t = 0;
             bool ok = true;
             for (; ok; ++t) {
@@ -719,7 +719,7 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant_
     constexpr uint32_t BOX = BOX_BYTES;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t it = 0;
             bool ok = true;
             int item = blockIdx.x;
@@ -769,10 +769,10 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant_
                 if (ok) ok = sched_publish(pipe, nf, next, total_items, p.status);
                 item = next;
             }
-            sched_finish(p.sched);                       // this CTA asks for no more items
+            sched_finish(p.sched, gridDim.x);            // this CTA asks for no more items
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t it = 0, t = 0;
             bool ok = true;
             for (uint32_t nf = 0; ok; ++nf) {
@@ -940,7 +940,7 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant_
                         const int n = n_w + j;
                         if (n < N) {
                             if (p.overwrite) gm[(size_t)n * M] = v[j >> 5][j & 31];
-                            else atomicAdd(gm + (size_t)n * M, v[j >> 5][j & 31]);
+                            else red_add(gm + (size_t)n * M, v[j >> 5][j & 31]);
                         }
                     }
                 }
@@ -979,6 +979,396 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant_
         }
     }
     cta_teardown(tmem_base, warp);
+}
+
+// ---- the three weight gradients on CTA pairs ---------------------------------------
+// A cluster of two CTAs computes 256 x 256 of a gradient: each CTA loads 128 of the 256 columns of both operands (32 KiB
+// per 64 rows instead of the 48 KiB of a 128 x 256 tile alone), the leader issues tcgen05.mma.cta_group::2, and each
+// CTA writes back the 128 rows whose sums lie in its TMEM.
+//
+// All three are computed transposed, with the gradient's contiguous dimension on the M side, so that the 32 lanes of a
+// TMEM row group are one line of the gradient:
+//   gWg, gWu [C,H]: M = H, N = C.  They share B (Xg), so their 128-column tiles are paired across the two: 2 ceil(H/128)
+//                   tiles, never an odd one.
+//   gWd [H,C]     : M = C, N = H.
+// A last column tile of 128 or less is an MMA of N = 128.
+//
+// Items are numbered expert by expert, most rows first: the longest items start first (a skewed routing's crowded expert
+// used to be the tail of every problem), and an expert's rows are read for all three at about the same time.  Experts
+// without rows have items only where gradients are stored instead of added to (zeros).
+//
+// The leader's producer takes an item and passes it to the peer's; each decodes it once and hands its own CTA's
+// roles what they need, pointers from tables in shared memory.  (Decoded by every warp, with loads from global memory that
+// queue behind the reductions, an item cost 6.7 us however few rows it had: 793 us where gradients of 64 experts, C=2048,
+// H=1408, are stored, now 498.)
+//
+// Bound by the sums: 128 KiB of `+=` per CTA and item, which the memory takes at 2.6 TB/s whatever sends them (reductions
+// of 4 or 16 bytes, bulk reductions; read-add-write is faster alone, 3.0, and slower here), so 0.85 ms for 64 experts,
+// C=2048, H=1408, whose MMAs take 0.7 ms at 1.9 GHz.  Against the kernel above, us, gradients added / stored:
+//   rows per expert          256          512          768          1024         2048
+//   C=2048 H=1408 E=64   828/600      988/793      1262/1062    1498/1263      .          tc_wgrad_kernel
+//                        873/609      953/770      1087/911     1322/1126      .          this one
+//   C=1024 H=1408 E=32   218/150      247/195      297/250      340/304      547/512
+//                        226/158      242/191      275/232      308/275      492/457
+//   C= 512 H=1376 E=16    64/52        72/62        84/76        97/91       148/140
+//                         68/52        74/64        84/74        95/84       136/127
+//   C=1024 H= 512 E=64   166/121      189/162      228/201      263/240        .
+//                        172/125      191/152      211/181      236/207        .
+// Few rows leave nothing for a pair to save, and its CTAs wait for one another; hence the line at 512 (pair_wgrad_usable).
+//
+// The bias gradients are column sums of the A tiles.  Two warps of the LEADER add them up (the peer has no barrier that
+// says when its tiles are there: all bytes are counted on the leader's); the pair swaps its two A tiles from one column
+// tile to the next, so that the leader has each of them in turn.
+struct PairWgradP {
+    const int32_t* padded_offsets;
+    const int32_t* seg;     // as in WgradP
+    int n_seg;
+    int32_t *status, *sched;
+    int C, H, E;
+    float* const* grad[3];  // gWg, gWu, gWd per expert
+    float* const* gb[3];
+    int overwrite;
+    int c_blocks;           // the maps of Xg and dYg are the column-block form (C a multiple of 64)
+};
+constexpr int WP_STAGES = 6;
+constexpr uint32_t WP_STAGE = 2 * A_BYTES;
+constexpr int WP_CLAIM = 6;                     // the next item is claimed this many stages before the last one's loads end
+struct PairWgradItem {      // one CTA's share of an item
+    float* g;               // its first element of the gradient
+    float* gb;              // bias gradient of its first column
+    int M, rows, cols;      // leading dimension of the gradient; rows and columns from g to its end
+    int nkb, half;          // 64-row blocks of the reduction; columns of B per CTA
+    int sum;                // leader: which of the A tile's two 64-column boxes to add up (bits)
+};
+static_assert(sizeof(PairWgradItem) == 40, "read in 8-byte pieces");
+struct PairWgradShared {
+    PairWgradItem item[SCHED_Q];
+    float* grad[3][MAX_EXPERTS];
+    float* gb[3][MAX_EXPERTS];
+    int rows[MAX_EXPERTS], row0[MAX_EXPERTS];
+    int order[MAX_EXPERTS];                     // experts, most rows first
+    int passed[SCHED_Q];                        // peer: items from the leader
+    uint64_t full[WP_STAGES], empty[WP_STAGES], acc_full[2], acc_empty[2];
+    uint64_t item_full[SCHED_Q], item_empty[SCHED_Q], passed_full[SCHED_Q], passed_empty[SCHED_Q];
+    uint32_t tmem;
+};
+constexpr uint32_t WP_SMEM = WP_STAGES * WP_STAGE + 1024 + sizeof(PairWgradShared);
+static_assert(WP_SMEM <= 232448, "shared memory of one CTA");
+// Rows per expert on average from which pairs are the faster form (table above); both widths need two column tiles, over
+// which a bias gradient is summed.
+inline bool pair_wgrad_usable(const Dims& d, int R) { return d.C > BN && d.H > BN && R >= 512 * d.E; }
+__host__ __device__ inline int pair_wgrad_items(int C, int H)       // of one expert
+{
+    const int mh = (H + BM - 1) / BM, mc = (C + BM - 1) / BM;
+    return mh * ((C + BN - 1) / BN) + (mc + 1) / 2 * ((H + BN - 1) / BN);
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(WG_THREADS, 1)
+tc_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmXg, const __grid_constant__ CUtensorMap tmdYg,
+                     const __grid_constant__ CUtensorMap tmdG, const __grid_constant__ CUtensorMap tmdU,
+                     const __grid_constant__ CUtensorMap tmHh, const PairWgradP p)
+{
+    extern __shared__ uint8_t smem_raw[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = (int)cluster_ctarank();
+    uint8_t* const tiles = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    PairWgradShared& sh = *reinterpret_cast<PairWgradShared*>(tiles + WP_STAGES * WP_STAGE);
+    const uint32_t full = smem_u32(sh.full), empty = smem_u32(sh.empty), acc_full = smem_u32(sh.acc_full), acc_empty = smem_u32(sh.acc_empty);
+    const uint32_t item_full = smem_u32(sh.item_full), item_empty = smem_u32(sh.item_empty);
+    const uint32_t passed_full = smem_u32(sh.passed_full), passed_empty = smem_u32(sh.passed_empty);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < WP_STAGES; ++s) {
+            mbar_init(full + 8 * s, 1);                     // (the leader's; the peer's loads count on it too)
+            mbar_init(empty + 8 * s, rank == 0 ? 1 + CS_WARPS : 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(acc_full + 8 * b, 1);
+            mbar_init(acc_empty + 8 * b, 2 * EPI_WARPS);
+        }
+        for (int i = 0; i < SCHED_Q; ++i) {
+            mbar_init(item_full + 8 * i, 1);
+            mbar_init(item_empty + 8 * i, rank == 0 ? EPI_WARPS + 1 + CS_WARPS : EPI_WARPS);
+            mbar_init(passed_full + 8 * i, 1);
+            mbar_init(passed_empty + 8 * i, 1);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) tmem_alloc_pair(smem_u32(&sh.tmem), TMEM_COLS);
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();                                         // the peer's barriers exist before anything is sent to them
+    tc_fence_after();
+    const uint32_t tmem_base = sh.tmem;
+    pdl_wait();
+    int mine = 0;
+    if (threadIdx.x < p.E) {
+        const int e = threadIdx.x;
+        sh.row0[e] = p.n_seg > 0 ? 0 : p.padded_offsets[e];
+        if (p.n_seg > 0)
+            for (int i = 0; i < p.n_seg; ++i) mine += p.seg[(e * p.n_seg + i) * 2 + 1];
+        else
+            mine = p.padded_offsets[e + 1] - sh.row0[e];
+        sh.rows[e] = mine;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            sh.grad[i][e] = p.grad[i][e];
+            sh.gb[i][e] = p.gb[i][e];
+        }
+    }
+    const int busy = __syncthreads_count(mine > 0);
+    if (threadIdx.x < p.E) {
+        int before = 0;
+        for (int e = 0; e < p.E; ++e) before += sh.rows[e] > mine || (sh.rows[e] == mine && e < (int)threadIdx.x);
+        sh.order[before] = threadIdx.x;
+    }
+    __syncthreads();
+
+    // the CTA's n-th item; false: no more
+    auto consume = [&](uint32_t n, PairWgradItem& w) -> bool {
+        const int slot = n % SCHED_Q;
+        if (!mbar_wait(item_full + 8 * slot, (n / SCHED_Q) & 1, p.status, ERR_SCHED_WAIT)) return false;
+        w = sh.item[slot];
+        return w.nkb >= 0;
+    };
+    auto release = [&](uint32_t n) { mbar_arrive(item_empty + 8 * (n % SCHED_Q)); };
+
+    if (warp == 0) {
+        if (elect_one()) {
+            const int mh = (p.H + BM - 1) / BM, nc = (p.C + BN - 1) / BN, nh = (p.H + BN - 1) / BN, per = pair_wgrad_items(p.C, p.H);
+            const int total_items = (p.overwrite ? p.E : busy) * per, grid = gridDim.x >> 1;
+            int s = 0, item = blockIdx.x >> 1, next = 0;
+            uint32_t free_phase = 1;                        // (the first round finds every stage free)
+            const uint32_t lead_full = mapa(full, 0), tile0 = smem_u32(tiles);
+            const uint32_t peer_passed = mapa(smem_u32(sh.passed), 1), peer_passed_full = mapa(passed_full, 1), lead_passed_empty = mapa(passed_empty, 0);
+            for (uint32_t n = 0;; ++n) {
+                const int slot = n % SCHED_Q;
+                const uint32_t round = (n / SCHED_Q) & 1;
+                if (rank == 0) {
+                    if (item >= total_items) item = -1;
+                    if (!mbar_wait_cluster(passed_empty + 8 * slot, round ^ 1, p.status, ERR_SCHED_WAIT)) break;
+                    st_cluster_u32(peer_passed + 4 * slot, (uint32_t)item);
+                    mbar_arrive_cluster(peer_passed_full + 8 * slot);       // (release at cluster scope: the item is visible)
+                } else {
+                    if (!mbar_wait_cluster(passed_full + 8 * slot, round, p.status, ERR_SCHED_WAIT)) break;
+                    item = sh.passed[slot];
+                    mbar_arrive_cluster(lead_passed_empty + 8 * slot);
+                }
+                if (!mbar_wait(item_empty + 8 * slot, round ^ 1, p.status, ERR_SCHED_WAIT)) break;
+                PairWgradItem& w = sh.item[slot];
+                if (item < 0) {
+                    w.nkb = -1;
+                    mbar_arrive(item_full + 8 * slot);
+                    break;
+                }
+                const int e = sh.order[item / per];
+                int r = item % per;
+                const bool down = r >= mh * nc;
+                if (down) r -= mh * nc;
+                const int others = down ? nh : nc, other = r % others, M = down ? p.C : p.H, N = down ? p.H : p.C;
+                int tile = r / others * 2 + ((other & 1) ^ rank);
+                const int mat = down ? 2 : tile >= mh ? 1 : 0;
+                if (mat == 1) tile -= mh;
+                const int m0 = tile * BM, n0 = other * BN, half = N - n0 <= BN / 2 ? BN / 4 : BN / 2, nkb = sh.rows[e] / BK;
+                // the leader has this A tile in every second column tile: of these visits the first sums the tile's first 64
+                // columns and the second the other 64, or one visit both
+                const int visit = other >> 1, visits = (others - (other & 1) + 1) >> 1;
+                w.g = sh.grad[mat][e] + (size_t)n0 * M + m0;
+                w.gb = sh.gb[mat][e] + m0;
+                w.M = M; w.rows = N - n0; w.cols = M - m0; w.nkb = nkb; w.half = half;
+                w.sum = visits > 1 ? (visit == 0 ? 1 : visit == 1 ? 2 : 0) : 3;
+                mbar_arrive(item_full + 8 * slot);
+                // this CTA's loads; the leader arms its barrier with both CTAs' bytes
+                const CUtensorMap *mA = down ? &tmdYg : mat ? &tmdU : &tmdG, *mB = down ? &tmHh : &tmXg;
+                const int colB = n0 + rank * half;
+                const bool a_blocks = !down || p.c_blocks, b_blocks = down || p.c_blocks;
+                int left = nkb;
+                if (rank == 0 && left <= WP_CLAIM) next = atomicAdd(p.sched, 1);
+                bool ok = true;
+                for (int sg = 0; ok && sg < (p.n_seg > 0 ? p.n_seg : 1); ++sg) {
+                    int row = sh.row0[e], end = row + sh.rows[e];
+                    if (p.n_seg > 0) {
+                        row = p.seg[(e * p.n_seg + sg) * 2];
+                        end = row + p.seg[(e * p.n_seg + sg) * 2 + 1];
+                    }
+                    for (; row < end; row += BK, --left) {
+                        if (rank == 0 && left == WP_CLAIM + 1) next = atomicAdd(p.sched, 1);
+                        if (!mbar_wait_cluster(empty + 8 * s, free_phase, p.status, ERR_EMPTY_WAIT)) {
+                            ok = false;
+                            break;
+                        }
+                        const uint32_t a_dst = tile0 + s * WP_STAGE, b_dst = a_dst + A_BYTES, bar = lead_full + 8 * s;
+                        if (rank == 0) mbar_expect_tx(full + 8 * s, 2 * WP_STAGE);
+                        if (a_blocks) {
+                            tma_load_3d_pair(a_dst, mA, 0, row, m0 / 64, bar);
+                        } else {
+                            tma_load_2d_pair(a_dst, mA, m0, row, bar);
+                            tma_load_2d_pair(a_dst + BOX_BYTES, mA, m0 + 64, row, bar);
+                        }
+                        if (b_blocks) {
+                            tma_load_3d_pair(b_dst, mB, 0, row, colB / 64, bar);
+                        } else {
+                            tma_load_2d_pair(b_dst, mB, colB, row, bar);
+                            tma_load_2d_pair(b_dst + BOX_BYTES, mB, colB + 64, row, bar);
+                        }
+                        if (++s == WP_STAGES) {
+                            s = 0;
+                            free_phase ^= 1;
+                        }
+                    }
+                }
+                if (!ok) break;
+                item = grid + next;
+            }
+            if (rank == 0) sched_finish(p.sched, grid);
+        }
+    } else if (warp == 1) {
+        if (rank == 0 && elect_one()) {
+            uint32_t t = 0, phase = 0;
+            int s = 0;
+            bool ok = true;
+            const uint32_t peer_empty = mapa(empty, 1), peer_acc_full = mapa(acc_full, 1);
+            const uint64_t desc0 = make_desc(smem_u32(tiles), BOX_BYTES, 1024);
+            PairWgradItem w;
+            for (uint32_t n = 0; ok && consume(n, w); ++n) {
+                release(n);
+                if (w.nkb == 0) continue;
+                const uint32_t idesc = make_idesc(2 * BM, 2 * w.half, 1, 1), buf = t & 1u;
+                if (!mbar_wait_cluster(acc_empty + 8 * buf, ((t >> 1) & 1) ^ 1, p.status, ERR_ACC_WAIT)) break;
+                tc_fence_after();
+                const uint32_t d_tmem = tmem_base + buf * BN;
+                for (int kb = 0; kb < w.nkb; ++kb) {
+                    if (!mbar_wait_cluster(full + 8 * s, phase, p.status, ERR_FULL_WAIT)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint64_t ad = desc0 + s * (WP_STAGE >> 4), bd = ad + (A_BYTES >> 4);      // (the address field: 16-byte units)
+#pragma unroll
+                    for (int k = 0; k < BK / 16; ++k)
+                        umma_bf16_pair(d_tmem, ad + k * (2048 >> 4), bd + k * (2048 >> 4), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                    umma_commit_pair(empty + 8 * s);
+                    umma_commit_pair(peer_empty + 8 * s);
+                    if (++s == WP_STAGES) {
+                        s = 0;
+                        phase ^= 1;
+                    }
+                }
+                if (ok) {
+                    umma_commit_pair(acc_full + 8 * buf);
+                    umma_commit_pair(peer_acc_full + 8 * buf);
+                }
+                ++t;
+            }
+        }
+    } else if (warp >= 2 + EPI_WARPS) {
+        if (rank == 0) {                                   // column sums of the leader's A tile
+            const int cw = warp - (2 + EPI_WARPS);
+            const int c8 = lane & 7, rg = lane >> 3;       // 16-byte piece of a 128-byte row; rows rg + 4i
+            int s = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            PairWgradItem w;
+            for (uint32_t n = 0; ok && __any_sync(0xffffffffu, consume(n, w)); ++n) {
+                __syncwarp();
+                if (lane == 0) release(n);
+                float acc[2][8] = {};
+                for (int kb = 0; kb < w.nkb; ++kb) {
+                    if (!mbar_wait(full + 8 * s, phase, p.status, ERR_FULL_WAIT)) {
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t tile = smem_u32(tiles + s * WP_STAGE);
+#pragma unroll
+                    for (int b = 0; b < 2; ++b)
+                        if (w.sum >> b & 1) {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) {
+                                const uint32_t r = (uint32_t)(rg + 32 * cw + 4 * i);
+                                uint32_t w0, w1, w2, w3;
+                                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                                             : "=r"(w0), "=r"(w1), "=r"(w2), "=r"(w3)
+                                             : "r"(tile + b * BOX_BYTES + r * 128u + ((((uint32_t)c8) ^ (r & 7u)) << 4)));
+                                acc[b][0] += bf_lo(w0); acc[b][1] += bf_hi(w0); acc[b][2] += bf_lo(w1); acc[b][3] += bf_hi(w1);
+                                acc[b][4] += bf_lo(w2); acc[b][5] += bf_hi(w2); acc[b][6] += bf_lo(w3); acc[b][7] += bf_hi(w3);
+                            }
+                        }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(empty + 8 * s);
+                    if (++s == WP_STAGES) {
+                        s = 0;
+                        phase ^= 1;
+                    }
+                }
+                if (!ok) break;
+                if (w.nkb > 0)
+#pragma unroll
+                    for (int b = 0; b < 2; ++b)
+                        if (w.sum >> b & 1) {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) {
+                                float v = acc[b][i];
+                                v += __shfl_xor_sync(0xffffffffu, v, 8);
+                                v += __shfl_xor_sync(0xffffffffu, v, 16);
+                                const int col = b * 64 + c8 * 8 + i;
+                                if (rg == 0 && col < w.cols) red_add(w.gb + col, v);      // two partial sums per column: one per warp
+                            }
+                        }
+            }
+        }
+    } else {
+        // 16 epilogue warps: TMEM lane quarter q (columns of the gradient), 64 of the product's columns (its rows) each
+        const int q = warp & 3, h = (warp - 2) >> 2;
+        const uint32_t acc_free = rank == 0 ? acc_empty : mapa(acc_empty, 0);
+        uint32_t t = 0;
+        PairWgradItem w;
+        for (uint32_t n = 0; __any_sync(0xffffffffu, consume(n, w)); ++n) {
+            __syncwarp();
+            if (lane == 0) release(n);
+            const int cols = min(32, w.cols - q * 32), rows = cols > 0 ? min(64, w.rows - h * 64) : 0;
+            float* const g = w.g + (size_t)(h * 64) * w.M + q * 32;
+            if (w.nkb == 0) {                              // an expert without rows
+                if (lane < cols)
+                    for (int j = 0; j < rows; ++j) g[(size_t)j * w.M + lane] = 0.0f;
+                continue;
+            }
+            const uint32_t buf = t & 1u;
+            if (!mbar_wait_cluster(acc_full + 8 * buf, (t >> 1) & 1, p.status, ERR_ACC_WAIT)) break;
+            tc_fence_after();
+            const uint32_t t_lane = tmem_base + buf * BN + ((uint32_t)(q * 32) << 16) + h * 64;
+            float* d = g + lane;                           // one line of the gradient per instruction
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                float v[16];
+                tmem_ld16(t_lane + c * 16, v);
+                tmem_ld_wait();
+                if (c == 3) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (rank == 0) mbar_arrive(acc_free + 8 * buf);
+                        else mbar_arrive_cluster(acc_free + 8 * buf);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    if (16 * c + j < rows && lane < cols) {
+                        if (p.overwrite) *d = v[j];
+                        else red_add(d, v[j]);
+                    }
+                    d += w.M;
+                }
+            }
+            ++t;
+        }
+    }
+    // neither CTA may leave (or give its TMEM back) while the other can still read its shared memory or signal it
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    }
 }
 
 }  // namespace
@@ -1024,18 +1414,19 @@ int make_map_kind(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols
     return 0;
 }
 
-bool make_map_blocks(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t n_blocks)
+int make_map_blocks(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t n_blocks)
 {
     EncodeTiledFn fn = encode_fn();
-    if (!fn || cols % 64 != 0) return false;
-    cuuint64_t dims[3] = {64, rows, cols / 64};
+    if (!fn) return fail(MGPT_MOE_ECUDA, "cuTensorMapEncodeTiled is not available from this driver");
+    cuuint64_t dims[3] = {64, rows, (cols + 63) / 64};
     cuuint64_t strides[2] = {cols * sizeof(bf16), 64 * sizeof(bf16)};
     cuuint32_t box[3] = {64, box_rows, n_blocks};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS;
+    if (r != CUDA_SUCCESS) return fail(MGPT_MOE_ECUDA, "cuTensorMapEncodeTiled failed (code " + std::to_string((int)r) + ")");
+    return 0;
 }
 
 // A tile-major weight copy as {64 columns, 128 rows, n2 blocks at stride2 elements, n3 at stride3}, box {64, rows, b2, b3}.
@@ -1075,7 +1466,8 @@ struct TcState {
     CUtensorMap Xg_t, Hh_t, dYg_t, dG_t, dU_t;
     // the same operands by column blocks (one load per operand tile): A side {64, 64 rows, 2}, B side {64, 64 rows, 4}
     CUtensorMap Xg_b4, dYg_b4, dG_b2, dU_b2, Hh_b2;
-    bool blocks_ok = false;      // the driver took the block maps (else six 2-D loads per stage)
+    CUtensorMap Xg_b2, dYg_b2;
+    bool c_blocks = false;       // the maps of Xg and dYg are there (C a multiple of 64); those of dG, dU, Hh always are
     // epilogue stores (box 32 x 32 rows, 64-byte swizzle)
     CUtensorMap Hh_s, Yg_s, dG_s, dU_s, dXg_s;
 };
@@ -1108,9 +1500,17 @@ int prepare(mgpt_moe_layer* L, const Workspace& w, char* ws)
     MGPT_TRY(make_map(&s->dYg_t, dyg, rc, C, 64));
     MGPT_TRY(make_map(&s->dG_t, ws + w.dG, rc, H, 64));
     MGPT_TRY(make_map(&s->dU_t, ws + w.dU, rc, H, 64));
-    s->blocks_ok = make_map_blocks(&s->Xg_b4, xg, rc, C, 64, BN / 64) && make_map_blocks(&s->dYg_b4, dyg, rc, C, 64, BN / 64) &&
-                   make_map_blocks(&s->dG_b2, ws + w.dG, rc, H, 64, BM / 64) && make_map_blocks(&s->dU_b2, ws + w.dU, rc, H, 64, BM / 64) &&
-                   make_map_blocks(&s->Hh_b2, ws + w.Hh, rc, H, 64, BM / 64);
+    s->c_blocks = C % 64 == 0;
+    if (s->c_blocks) {
+        MGPT_TRY(make_map_blocks(&s->Xg_b4, xg, rc, C, 64, BN / 64));
+        MGPT_TRY(make_map_blocks(&s->dYg_b4, dyg, rc, C, 64, BN / 64));
+        MGPT_TRY(make_map_blocks(&s->Xg_b2, xg, rc, C, 64, BM / 64));
+        MGPT_TRY(make_map_blocks(&s->dYg_b2, dyg, rc, C, 64, BM / 64));
+    }
+    // (the last block may reach up to 112 bytes past the buffer: other buffers of the workspace follow all three)
+    MGPT_TRY(make_map_blocks(&s->dG_b2, ws + w.dG, rc, H, 64, BM / 64));
+    MGPT_TRY(make_map_blocks(&s->dU_b2, ws + w.dU, rc, H, 64, BM / 64));
+    MGPT_TRY(make_map_blocks(&s->Hh_b2, ws + w.Hh, rc, H, 64, BM / 64));
     MGPT_TRY(make_map(&s->Hh_s, ws + w.Hh, rc, H, 32));
     MGPT_TRY(make_map(&s->Yg_s, yg, rc, C, 32));
     MGPT_TRY(make_map(&s->dG_s, ws + w.dG, rc, H, 32));
@@ -1133,6 +1533,7 @@ int prepare_attrs(mgpt_moe_layer* L)
         MGPT_CUDA(cudaFuncSetAttribute(tc_rows_kernel<MODE_DXG>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
         MGPT_CUDA(cudaFuncSetAttribute(tc_rows_kernel<MODE_DX>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
         MGPT_CUDA(cudaFuncSetAttribute(tc_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        MGPT_CUDA(cudaFuncSetAttribute(tc_wgrad_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WP_SMEM));
         MGPT_CUDA(cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, L->device));
         // the work-item counters must read zero before the first launch on any stream: allocate and clear them
         // here, at layer creation, and wait for the clear (nothing orders the legacy stream with a caller's
@@ -1232,6 +1633,27 @@ int tc_experts_backward(mgpt_moe_layer* L, const Workspace& w, char* ws, cudaStr
     }
     if (!L->has_grad || !(phase & 2)) return 0;
 
+    if (pair_wgrad_usable(d, w.R) && grid_sms(L, s) >= 2) {
+        PairWgradP g = {};
+        g.padded_offsets = (const int32_t*)(ws + w.padded_offsets);
+        g.seg = (const int32_t*)(ws + w.seg);
+        g.n_seg = L->n_seg;
+        g.status = L->d_status;
+        g.sched = s->sched + 8;
+        g.C = d.C; g.H = d.H; g.E = d.E;
+        g.grad[0] = L->master.gWg; g.grad[1] = L->master.gWu; g.grad[2] = L->master.gWd;
+        g.gb[0] = L->master.gbg; g.gb[1] = L->master.gbu; g.gb[2] = L->master.gbd;
+        g.overwrite = L->bwd_overwrite ? 1 : 0;
+        g.c_blocks = s->c_blocks ? 1 : 0;
+        const int pairs = imin(grid_sms(L, s) / 2, d.E * pair_wgrad_items(d.C, d.H));
+        L->stage_begin(ST_WGRAD, st);
+        MGPT_CUDA(launch_pdl(tc_wgrad_pair_kernel, 2 * pairs, WG_THREADS, WP_SMEM, st, g.c_blocks ? s->Xg_b2 : s->Xg_t,
+                             g.c_blocks ? s->dYg_b2 : s->dYg_t, s->dG_b2, s->dU_b2, s->Hh_b2, g));
+        MGPT_LAUNCHED("tc_wgrad_pair_kernel");
+        L->stage_end(ST_WGRAD, st);
+        return 0;
+    }
+
     // all three weight gradients in one launch:
     //   gWg += Xg^T dG, gWu += Xg^T dU   [C,H];   gWd += Hh^T dYg   [H,C]
     // The first two are computed transposed, (dG^T Xg) [H,C]: H = 1408 splits into eleven 128-row tiles and C into
@@ -1264,7 +1686,7 @@ int tc_experts_backward(mgpt_moe_layer* L, const Workspace& w, char* ws, cudaStr
     if (tc_fused_bias_grads(d)) {
         g.gb[0] = L->master.gbg; g.gb[1] = L->master.gbu; g.gb[2] = L->master.gbd;
     }
-    g.block_loads = s->blocks_ok ? 1 : 0;
+    g.block_loads = s->c_blocks ? 1 : 0;
     if (g.block_loads)
         MGPT_CUDA(launch_pdl(tc_wgrad_kernel, imin(grid_sms(L, s), items), WG_THREADS, SMEM_BYTES, st, s->dG_b2, s->Xg_b4, s->dU_b2, s->Xg_b4,
                                                                            s->Hh_b2, s->dYg_b4, g));
@@ -1314,8 +1736,9 @@ int tc_router_wgrad(mgpt_moe_layer* L, const Workspace& w, char* ws, const void*
     const int E8 = (d.E + 7) / 8 * 8;
     CUtensorMap mA, mB;
     WgradP g = {};
-    g.block_loads = make_map_blocks(&mA, x, (uint64_t)w.n_tokens, (uint64_t)d.C, 64, BM / 64) ? 1 : 0;
-    if (!g.block_loads) MGPT_TRY(make_map(&mA, x, (uint64_t)w.n_tokens, (uint64_t)d.C, 64));
+    g.block_loads = d.C % 64 == 0 ? 1 : 0;
+    if (g.block_loads) MGPT_TRY(make_map_blocks(&mA, x, (uint64_t)w.n_tokens, (uint64_t)d.C, 64, BM / 64));
+    else MGPT_TRY(make_map(&mA, x, (uint64_t)w.n_tokens, (uint64_t)d.C, 64));
     MGPT_TRY(make_map(&mB, ws + w.dl16, (uint64_t)w.n_tokens, (uint64_t)E8, 64));
     g.b_boxes = cdiv(E8, 64);
     g.status = L->d_status;
