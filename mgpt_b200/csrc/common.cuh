@@ -76,8 +76,9 @@ inline int check_aligned(const void* p, const char* what, uintptr_t bytes = 16)
 // addresses) while that kernel's writes are still being flushed, and wait in pdl_wait() until all of it has finished
 // and is visible.  EVERY block of EVERY kernel launched this way goes through pdl_wait(), also one that has nothing to do: "the kernel
 // before has finished" then implies the same for all kernels before that one.  Takes the ~2 us between two kernels of
-// a step to ~1 us.  Only decode_kernel's gate/up releases its successor early (griddepcontrol.launch_dependents), after its
-// own wait, for a kernel that can request weights meanwhile.  With an early release at the top of every kernel the waiting
+// a step to ~1 us.  A kernel whose successor can request weights meanwhile (dispatch and gate/up: the next product's first)
+// releases it early (pdl_release), after its own wait: what an earlier kernel wrote -- the plan, the weights -- is complete by
+// then, so that the successor may read it before it waits.  With an early release at the top of every kernel the waiting
 // blocks pile up several kernels deep and spread the next kernel's blocks unevenly over the SMs (a 256-token decode call:
 // 155 us without any of this, 144 us with the wait alone, 194 us with that).
 template <typename... KArgs, typename... Args>
@@ -100,6 +101,8 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 // biases, the saved SwiGLU factors and the rows of dXg, in kernels that another kernel of the same call separates from their
 // writer: that one has waited for the writer's end.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next kernel's blocks in as this one's leave; after pdl_wait().
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- workspace ------------------------------------------------------------
 // One arena per forward/backward pair, carved deterministically from

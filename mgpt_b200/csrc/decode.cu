@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(32 * DW, 1) decode_kernel(const DecP p)
     // read the plan before they wait: it was complete before phase 1 came this far.)
     if (PHASE == 1) {
         pdl_wait();
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        pdl_release();
     }
     const int total = __ldcg(p.n_groups) * per;
     bool waited = PHASE == 1;

@@ -39,6 +39,7 @@ constexpr uint32_t STAGING_BYTES = 2048;             // per epilogue warp: 32 ro
 constexpr uint32_t TMEM_COLS = 2 * BN;               // two accumulators
 constexpr uint32_t SMEM_BYTES = STAGES * STAGE_BYTES + EPI_WARPS * STAGING_BYTES + 1024 /*align slack*/ + 512 /*barriers, work queue*/;
 constexpr int TC_THREADS = 64 + 32 * EPI_WARPS;      // warp0 TMA, warp1 MMA, warps2-17 epilogue
+constexpr int ROWS_THREADS = TC_THREADS + 32;        // expert products: warp 18 brings the biases
 constexpr int CS_WARPS = 2;                          // weight-gradient kernel only: warps 18-19 sum operand columns (bias gradients)
 constexpr int WG_THREADS = TC_THREADS + 32 * CS_WARPS;
 
@@ -46,24 +47,53 @@ constexpr int SCHED_Q = 8;                           // queue entries: the produ
 
 using namespace tcx;
 
-// v[j] += bias[n + j] for 32 consecutive columns; 16-byte loads when the whole piece is inside the row
-__device__ __forceinline__ void add_bias32(float (&v)[32], const float* __restrict__ bias, int n, int n_out)
+// Two FP32 operations per instruction, on registers that lie side by side.
+__device__ __forceinline__ uint64_t pk2(float a, float b)
 {
-    if (n + 32 <= n_out) {
-        const float4* b4 = reinterpret_cast<const float4*>(bias + n);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const float4 b = __ldg(b4 + q);
-            v[4 * q] += b.x; v[4 * q + 1] += b.y; v[4 * q + 2] += b.z; v[4 * q + 3] += b.w;
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-            if (n + j < n_out) v[j] += bias[n + j];
-    }
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpk2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint32_t bf2(uint64_t v)
+{
+    float a, b;
+    unpk2(v, a, b);
+    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<uint32_t*>(&h);
+}
+__device__ __forceinline__ float ex2(float x)
+{
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rcp(float x)
+{
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
 }
 
-// Shared memory of one CTA: operand ring, one 4 KiB staging tile per epilogue warp, barriers.
+// Shared memory of one CTA: operand ring, one 2 KiB staging tile per epilogue warp, barriers.
 struct Pipe {
     uint32_t bars, tmem_slot;          // shared-space addresses
     uint8_t* tiles;
@@ -206,14 +236,6 @@ __device__ __forceinline__ void flush_stage(uint8_t* stage, const CUtensorMap* m
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
     }
 }
-__device__ __forceinline__ void pack32(const float (&a)[32], uint32_t (&out)[16])
-{
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        __nv_bfloat162 h = __floats2bfloat162_rn(a[2 * i], a[2 * i + 1]);
-        out[i] = *reinterpret_cast<uint32_t*>(&h);
-    }
-}
 // The two saved activation-derivative arrays (buffers "G" and "U") are private to the gate/up and dHh epilogues, so they are kept in the layout
 // both epilogues touch with full-width accesses: [row tile][8-column chunk][128 rows][8 bf16].  A thread owns one
 // row (its TMEM lane); the 32 lanes of a warp then read or write 512 contiguous bytes per instruction.
@@ -223,15 +245,10 @@ __device__ __forceinline__ void load_blocked32(const uint4* chunk0, uint32_t (&w
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         uint4 u = make_uint4(0, 0, 0, 0);
-        if (q * 8 < valid) u = __ldg(chunk0 + q * BM);
+        if (q * 8 < valid)
+            asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w) : "l"(chunk0 + q * BM));
         w[4 * q] = u.x; w[4 * q + 1] = u.y; w[4 * q + 2] = u.z; w[4 * q + 3] = u.w;
     }
-}
-__device__ __forceinline__ void store_blocked32(uint4* chunk0, const uint32_t (&w)[16], int valid)
-{
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-        if (q * 8 < valid) chunk0[q * BM] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
 }
 // this thread's row in chunk n/8 of row tile `row_tile` (n_out columns, a multiple of 8)
 __device__ __forceinline__ size_t blocked_index(int row_tile, int n_out, int n, int row_in_tile)
@@ -242,8 +259,9 @@ __device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w <<
 __device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 
 // ---- token-major products ------------------------------------------------------
-enum { MODE_GATEUP = 0, MODE_DOWN = 1, MODE_DHH = 2, MODE_DXG = 3, MODE_DX = 4 };
+enum { MODE_GATEUP = 0, MODE_DOWN = 1, MODE_DHH = 2, MODE_DXG = 3 };
 
+__host__ __device__ constexpr int rows_groups(int mode) { return mode == MODE_DHH ? 1 : 2; }
 struct RowsP {
     const int32_t* tile_expert;
     const int32_t* tile_order;  // optional: i-th row tile to work on (expert-major order over scattered tiles)
@@ -253,6 +271,7 @@ struct RowsP {
     int kblocks;            // k-blocks (of 64) per operand pair
     int n_out;              // output columns (H or C)
     int n_col_tiles;        // column tiles per row tile
+    int early;              // plan and weights were complete before the kernel before this one on the stream went past its pdl_wait
     bf16 *G, *U;            // P and Q (see the gate/up epilogue) in the blocked layout (written by MODE_GATEUP, read by MODE_DHH)
     const float* const* bias0;
     const float* const* bias1;
@@ -270,116 +289,168 @@ struct RowsP {
     bf16* dx;                   // MODE_DX: the output
 };
 
-// The epilogue of one work item for one of the 16 epilogue warps: TMEM lane quarter q (rows q*32..+31 of the row
-// tile), column group h.  False: a bounded wait ran out.
-//
-// MODE_DX has its own (dx_epilogue).
-template <int MODE>
-__device__ __forceinline__ bool rows_epilogue(const RowsP& p, uint32_t acc_full_bar, uint32_t acc_empty_bar,
-                                              uint32_t tmem_base, uint32_t buf, uint32_t t, int row_tile, int n0, int e,
-                                              int q, int h, int lane, uint8_t* stage, const CUtensorMap* tmD0,
-                                              const CUtensorMap* tmD1, const CUtensorMap* tmD2)
+// What follows the operand ring and the staging tiles of the four expert products.
+struct RowsItem {
+    int row_tile, n0, e, pad;       // row_tile < 0: no work left
+};
+struct RowsShared {
+    float bias[2][BN];              // per accumulator: the biases of its columns
+    RowsItem item[SCHED_Q];
+    uint64_t full[STAGES], empty[STAGES], acc_full[2], acc_empty[2], bias_full[2], item_full[SCHED_Q], item_empty[SCHED_Q];
+    uint32_t tmem;
+};
+constexpr int ROWS_CLAIM = 4;       // the next item is claimed this many k-blocks before the last one's loads end
+constexpr uint32_t ROWS_SMEM = STAGES * STAGE_BYTES + EPI_WARPS * STAGING_BYTES + sizeof(RowsShared);
+static_assert(ROWS_SMEM <= 232448, "shared memory of one CTA");
+
+// The epilogue of every second item of a CTA for one of the eight warps of its group: TMEM lane quarter q (rows q*32..+31 of
+// the row tile), column half h.  `next(n, w)`: the CTA's n-th item, false: no more.
+template <int MODE, class Next>
+__device__ __forceinline__ void rows_epilogue(const RowsP& p, RowsShared& sh, uint32_t tmem_base, int group, int q, int h, int lane,
+                                              uint8_t* stage, const CUtensorMap* tmD0, const CUtensorMap* tmD1, Next next)
 {
-    const int row_w = row_tile * BM + q * 32;           // first row of this warp
-    // MODE_DHH: the saved G and U of this item come from HBM.  Unit 0's pieces are requested before the wait
-    // for the accumulator, unit 1's while unit 0 is worked on, so their latency hides behind other work.
-    uint32_t gq[2][16], uq[2][16];
-    if (MODE == MODE_DHH) {
-        const int n = n0 + h * 64;
-        const size_t o = blocked_index(row_tile, p.n_out, n, q * 32 + lane);
-        load_blocked32(reinterpret_cast<const uint4*>(p.G) + o, gq[0], p.n_out - n);
-        load_blocked32(reinterpret_cast<const uint4*>(p.U) + o, uq[0], p.n_out - n);
-    }
-    if (!mbar_wait(acc_full_bar, (t >> 1) & 1, p.status, ERR_ACC_WAIT)) return false;
-    tc_fence_after();
-    const uint32_t t_lane = tmem_base + buf * BN + ((uint32_t)(q * 32) << 16);
+    const uint32_t acc_full = smem_u32(&sh.acc_full[group]), acc_empty = smem_u32(&sh.acc_empty[group]), bias_full = smem_u32(&sh.bias_full[group]);
+    const uint32_t t_lane = tmem_base + group * BN + ((uint32_t)(q * 32) << 16);
+    const float* bias = sh.bias[group];
+    const int ld = p.n_out;
+    uint32_t phase = 0;
+    RowsItem w = {};
+    auto store = [&](const uint32_t (&pk)[16], const CUtensorMap* tm, int n) {
+        stage_row_bf16(stage, lane, pk);
+        flush_stage(stage, tm, n, w.row_tile * BM + q * 32, lane);
+    };
     if (MODE == MODE_GATEUP) {
-        // this warp: hidden units n0 + h*32 .. +31  (gate columns h*32.., up columns 128 + h*32..)
-        const int n = n0 + h * 32;
-        float a[32], b[32];
-        tmem_ld32(t_lane + h * 32, a);
-        tmem_ld32(t_lane + BN / 2 + h * 32, b);
-        tmem_ld_wait();
-        release_acc(acc_empty_bar, lane);
-        if (n < p.n_out) {
-            // What backward needs of G and U is not the values themselves but
-            //   Q = silu(G)                       (dU = dHh * Q)
-            //   P = U * sigmoid(G) * (1 + G * (1 - sigmoid(G)))      (dG = dHh * P)
-            // (utils/Tensor.cpp:2020-2027), so those are what is kept: the sigmoid is evaluated once, here,
-            // in FP32 on the unrounded sums, and the dHh epilogue is left with two multiplies per element.
-            uint32_t pp[16], qp[16], hp[16];
-            add_bias32(a, p.bias0[e], n, p.n_out);
-            add_bias32(b, p.bias1[e], n, p.n_out);
+        for (uint32_t t = group; next(t, w); t += 2, phase ^= 1) {
+            if (!mbar_wait(acc_full, phase, p.status, ERR_ACC_WAIT)) return;
+            if (!mbar_wait(bias_full, phase, p.status, ERR_ACC_WAIT)) return;
+            tc_fence_after();
+#pragma unroll 1
+            for (int un = 0; un < 2; ++un) {
+                // hidden units n0 + col .. +31: gate columns col.., up columns 128 + col..
+                const int col = h * 64 + un * 32, n = w.n0 + col, valid = ld - n;
+                float a[32], b[32];
+                tmem_ld32(t_lane + col, a);
+                tmem_ld32(t_lane + BN / 2 + col, b);
+                tmem_ld_wait();
+                uint64_t g2[16], u2[16];
+                const float4 *b0 = reinterpret_cast<const float4*>(bias + col), *b1 = b0 + BN / 8;
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                float pv[2], qv[2], hv[2];
-#pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {
-                    const float g = a[2 * i + hh], u = b[2 * i + hh];
-                    const float sig = __fdividef(1.0f, 1.0f + __expf(-g));
-                    const float q = g * sig;
-                    qv[hh] = q;
-                    hv[hh] = q * u;
-                    pv[hh] = (u * sig) * (1.0f + (g - q));
+                for (int i = 0; i < 8; ++i) {
+                    const float4 x = b0[i], y = b1[i];
+                    g2[2 * i] = add2(pk2(a[4 * i], a[4 * i + 1]), pk2(x.x, x.y));
+                    g2[2 * i + 1] = add2(pk2(a[4 * i + 2], a[4 * i + 3]), pk2(x.z, x.w));
+                    u2[2 * i] = add2(pk2(b[4 * i], b[4 * i + 1]), pk2(y.x, y.y));
+                    u2[2 * i + 1] = add2(pk2(b[4 * i + 2], b[4 * i + 3]), pk2(y.z, y.w));
                 }
-                __nv_bfloat162 p2 = __floats2bfloat162_rn(pv[0], pv[1]);
-                __nv_bfloat162 q2 = __floats2bfloat162_rn(qv[0], qv[1]);
-                __nv_bfloat162 h2 = __floats2bfloat162_rn(hv[0], hv[1]);
-                pp[i] = *reinterpret_cast<uint32_t*>(&p2);
-                qp[i] = *reinterpret_cast<uint32_t*>(&q2);
-                hp[i] = *reinterpret_cast<uint32_t*>(&h2);
+                if (un == 1) release_acc(acc_empty, lane);
+                if (valid <= 0) continue;
+                // What backward needs of G and U is not the values themselves but
+                //   Q = silu(G)                       (dU = dHh * Q)
+                //   P = U * sigmoid(G) * (1 + G * (1 - sigmoid(G)))      (dG = dHh * P)
+                // (utils/Tensor.cpp:2020-2027), so those are what is kept: the sigmoid is evaluated once, here,
+                // in FP32 on the unrounded sums, and the dHh epilogue is left with two multiplies per element.
+                uint32_t hp[16];
+                const size_t o = blocked_index(w.row_tile, ld, n, q * 32 + lane);
+                uint4 *gp = reinterpret_cast<uint4*>(p.G) + o, *up = reinterpret_cast<uint4*>(p.U) + o;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {              // 8 hidden units at a time
+                    uint32_t pp[4], qp[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const uint64_t g = g2[4 * c + j], u = u2[4 * c + j], one = pk2(1.0f, 1.0f);
+                        float e0, e1;
+                        unpk2(mul2(g, pk2(-1.4426950408889634f, -1.4426950408889634f)), e0, e1);
+                        float d0, d1;
+                        unpk2(add2(pk2(ex2(e0), ex2(e1)), one), d0, d1);
+                        const uint64_t sig = pk2(rcp(d0), rcp(d1)), qv = mul2(g, sig), us = mul2(u, sig);
+                        hp[4 * c + j] = bf2(mul2(qv, u));
+                        qp[j] = bf2(qv);
+                        pp[j] = bf2(fma2(us, fma2(qv, pk2(-1.0f, -1.0f), g), us));
+                    }
+                    if (p.G && c * 8 < valid) {            // inference keeps nothing for a backward pass
+                        gp[c * BM] = make_uint4(pp[0], pp[1], pp[2], pp[3]);
+                        up[c * BM] = make_uint4(qp[0], qp[1], qp[2], qp[3]);
+                    }
+                }
+                store(hp, tmD0, n);
             }
-            if (p.G) {                                  // inference keeps nothing for a backward pass
-                const size_t o = blocked_index(row_tile, p.n_out, n, q * 32 + lane);
-                store_blocked32(reinterpret_cast<uint4*>(p.G) + o, pp, p.n_out - n);
-                store_blocked32(reinterpret_cast<uint4*>(p.U) + o, qp, p.n_out - n);
+        }
+    } else if (MODE == MODE_DHH) {
+        // The saved factors of a 32-column unit are requested while the unit before it is worked on, an item's first ones
+        // when the group is done with its item before.  (Not before a TMEM load: its wait would cover them.)
+        constexpr int GROUPS = rows_groups(MODE), UNITS = 2 * GROUPS;
+        const int c0 = h * 32 * UNITS;
+        uint32_t P[2][16], Q[2][16];
+        auto fetch = [&](int un, uint32_t (&pv)[16], uint32_t (&qv)[16]) {
+            const int n = w.n0 + c0 + un * 32;
+            const size_t o = blocked_index(w.row_tile, ld, n, q * 32 + lane);
+            load_blocked32(reinterpret_cast<const uint4*>(p.G) + o, pv, ld - n);
+            load_blocked32(reinterpret_cast<const uint4*>(p.U) + o, qv, ld - n);
+        };
+        bool more = next(group, w);
+        if (more) fetch(0, P[0], Q[0]);
+        for (uint32_t t = group; more; t += GROUPS) {
+            const uint32_t buf = GROUPS == 2 ? 0 : t & 1u;
+            if (!mbar_wait(acc_full + 8 * buf, (t >> 1) & 1, p.status, ERR_ACC_WAIT)) return;
+            tc_fence_after();
+#pragma unroll
+            for (int un = 0; un < UNITS; ++un) {
+                const int n = w.n0 + c0 + un * 32;
+                uint32_t (&pv)[16] = P[un & 1];
+                uint32_t (&qv)[16] = Q[un & 1];
+#pragma unroll
+                for (int hf = 0; hf < 2; ++hf) {
+                    float v[16];
+                    tmem_ld16(t_lane + buf * BN + c0 + un * 32 + hf * 16, v);
+                    tmem_ld_wait();
+                    if (hf == 1 && un == UNITS - 1) release_acc(acc_empty + 8 * buf, lane);
+                    if (hf == 1 && un < UNITS - 1) fetch(un + 1, P[(un + 1) & 1], Q[(un + 1) & 1]);
+                    // utils/Tensor.cpp:2020-2027 with dd = dHh: dG = dd * P, dU = dd * Q (P, Q saved by the forward epilogue)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const uint64_t d = pk2(v[2 * i], v[2 * i + 1]);
+                        uint32_t &pw = pv[hf * 8 + i], &qw = qv[hf * 8 + i];
+                        pw = bf2(mul2(d, pk2(bf_lo(pw), bf_hi(pw))));      // dG, packed in place
+                        qw = bf2(mul2(d, pk2(bf_lo(qw), bf_hi(qw))));      // dU
+                    }
+                }
+                if (n < ld) {
+                    store(pv, tmD0, n);
+                    store(qv, tmD1, n);
+                }
             }
-            stage_row_bf16(stage, lane, hp);
-            flush_stage(stage, tmD2, n, row_w, lane);
+            more = next(t + GROUPS, w);
+            if (more) fetch(0, P[0], Q[0]);
         }
     } else {
-        // this warp: columns n0 + h*64 .. +63, two units of 32
+        for (uint32_t t = group; next(t, w); t += 2, phase ^= 1) {
+            if (!mbar_wait(acc_full, phase, p.status, ERR_ACC_WAIT)) return;
+            if (MODE == MODE_DOWN && !mbar_wait(bias_full, phase, p.status, ERR_ACC_WAIT)) return;
+            tc_fence_after();
+#pragma unroll 1
+            for (int un = 0; un < 4; ++un) {               // columns n0 + h*128 .. +127, four units of 32
+                const int col = h * 128 + un * 32, n = w.n0 + col;
+                float v[32];
+                tmem_ld32(t_lane + col, v);
+                tmem_ld_wait();
+                uint32_t pk[16];
 #pragma unroll
-        for (int un = 0; un < 2; ++un) {
-            const int n = n0 + h * 64 + un * 32;
-            float v[32];
-            tmem_ld32(t_lane + h * 64 + un * 32, v);
-            tmem_ld_wait();
-            if (un == 1) release_acc(acc_empty_bar, lane);
-            if (n >= p.n_out) continue;                      // warp-uniform
-            uint32_t pk[16];
-            if (MODE == MODE_DOWN) {
-                add_bias32(v, p.bias0[e], n, p.n_out);
-            } else if (MODE == MODE_DHH) {
-                // utils/Tensor.cpp:2020-2027 with dd = dHh: dG = dd * P, dU = dd * Q (P, Q saved by the forward epilogue)
-                if (un == 0) {
-                    const int n1 = n + 32;
-                    const size_t o1 = blocked_index(row_tile, p.n_out, n1, q * 32 + lane);
-                    load_blocked32(reinterpret_cast<const uint4*>(p.G) + o1, gq[1], p.n_out - n1);
-                    load_blocked32(reinterpret_cast<const uint4*>(p.U) + o1, uq[1], p.n_out - n1);
+                for (int i = 0; i < 8; ++i) {
+                    uint64_t x = pk2(v[4 * i], v[4 * i + 1]), y = pk2(v[4 * i + 2], v[4 * i + 3]);
+                    if (MODE == MODE_DOWN) {
+                        const float4 b = *reinterpret_cast<const float4*>(bias + col + 4 * i);
+                        x = add2(x, pk2(b.x, b.y));
+                        y = add2(y, pk2(b.z, b.w));
+                    }
+                    pk[2 * i] = bf2(x);
+                    pk[2 * i + 1] = bf2(y);
                 }
-                uint32_t (&gw)[16] = gq[un];
-                uint32_t (&uw)[16] = uq[un];
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const float d0 = v[2 * i], d1 = v[2 * i + 1];
-                    __nv_bfloat162 a2 = __floats2bfloat162_rn(d0 * bf_lo(gw[i]), d1 * bf_hi(gw[i]));
-                    __nv_bfloat162 b2 = __floats2bfloat162_rn(d0 * bf_lo(uw[i]), d1 * bf_hi(uw[i]));
-                    gw[i] = *reinterpret_cast<uint32_t*>(&a2);      // dG, packed in place
-                    uw[i] = *reinterpret_cast<uint32_t*>(&b2);      // dU, packed in place
-                }
-                stage_row_bf16(stage, lane, uw);
-                flush_stage(stage, tmD1, n, row_w, lane);
-                stage_row_bf16(stage, lane, gw);
-                flush_stage(stage, tmD0, n, row_w, lane);
-                continue;
+                if (un == 3) release_acc(acc_empty, lane);
+                if (n < ld) store(pk, tmD0, n);
             }
-            pack32(v, pk);
-            stage_row_bf16(stage, lane, pk);
-            flush_stage(stage, tmD0, n, row_w, lane);
         }
     }
-    return true;
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // stores landed before exit
 }
 
 // dx = dlogits * Wr^T (the accumulator) + the token's expert rows in ascending order: the epilogue of all of a CTA's items.
@@ -512,140 +583,283 @@ __device__ __forceinline__ void dx_epilogue(const RowsP& p, const Pipe& pipe, ui
     }
 }
 
-// Persistent: CTA b works on items b, b+grid, ... where item = row_tile * n_col_tiles + col_tile.
-// Two 256-column accumulators in TMEM alternate, so the epilogue of one item runs while the
-// tensor core works on the next.
+// Persistent over items = row_tile * n_col_tiles + col_tile.  Two 256-column accumulators in TMEM alternate, so the epilogue
+// of one item runs while the tensor core works on the next.
+//
+// The producer decodes an item once, while the loads of the one before are still going out, and hands it on through a queue; a
+// warp of its own brings the biases of the item's columns into shared memory.  (Every epilogue warp used to look up the
+// tile's expert, its bias pointers and then the biases, one load after another: 3000 of the 9800 cycles that an item of 8 k-blocks
+// took in gate/up.)  Us for 8192 tokens, C=512, H=1376, E=16, before -> now: gate/up 73 -> 66, dHh 60 -> 54.
+//
+// What bounds it with few k-blocks: operands, factors and results share the way between L2 and the SM, 512 KiB an item in dHh
+// against 4096 cycles of MMAs.  Ring depth counts (three stages instead of four: dXg 54 -> 62 us, gate/up of 1777 tokens 74 ->
+// 78), so it is not given up for a second staging tile per epilogue warp; all results by TMA store, the factors too, from such
+// tiles: no gain.  dHh's results through 16-byte stores from registers instead of TMA: 54 -> 70 us.  Its factors sent to L2
+// an item ahead: 54 -> 56.  More weights sent to L2 before pdl_wait (8 or 16 k-blocks behind the ring): 120.0 -> 120.7 and
+// 121.2 us for 256 tokens, C=1024, H=2816, E=32.
 template <int MODE>
-__global__ void __launch_bounds__(TC_THREADS, 1)
+__global__ void __launch_bounds__(ROWS_THREADS, 1)
 tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                const __grid_constant__ CUtensorMap tmB0, const __grid_constant__ CUtensorMap tmB1,
-               const __grid_constant__ CUtensorMap tmD0, const __grid_constant__ CUtensorMap tmD1,
-               const __grid_constant__ CUtensorMap tmD2, const RowsP p)
+               const __grid_constant__ CUtensorMap tmD0, const __grid_constant__ CUtensorMap tmD1, const RowsP p)
 {
-    extern __shared__ uint8_t smem_raw[];
+    extern __shared__ __align__(1024) uint8_t smem_raw[];       // (the swizzled tiles start on 1024-byte boundaries)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int COLS_PER_ITEM = MODE == MODE_GATEUP ? BN / 2 : BN;
-    constexpr bool DATA_GRAD = MODE == MODE_DHH || MODE == MODE_DXG;
+    constexpr int ST = STAGES;
+    constexpr bool DATA_GRAD = MODE == MODE_DHH || MODE == MODE_DXG, BIAS = MODE == MODE_GATEUP || MODE == MODE_DOWN;
     const int kb_per_item = (MODE == MODE_DXG ? 2 : 1) * p.kblocks;
+    RowsShared& sh = *reinterpret_cast<RowsShared*>(smem_raw + STAGES * STAGE_BYTES + EPI_WARPS * STAGING_BYTES);
+    const uint32_t full = smem_u32(sh.full), empty = smem_u32(sh.empty), acc_full = smem_u32(sh.acc_full), acc_empty = smem_u32(sh.acc_empty);
+    const uint32_t item_full = smem_u32(sh.item_full), item_empty = smem_u32(sh.item_empty);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(full + 8 * s, 1);
+            mbar_init(empty + 8 * s, 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(acc_full + 8 * b, 1);
+            mbar_init(acc_empty + 8 * b, (EPI_WARPS / rows_groups(MODE)));
+            mbar_init(smem_u32(sh.bias_full) + 8 * b, 1);
+        }
+        for (int i = 0; i < SCHED_Q; ++i) {
+            mbar_init(item_full + 8 * i, 1);
+            mbar_init(item_empty + 8 * i, 1 + (BIAS ? 1 : 0) + (EPI_WARPS / rows_groups(MODE)));
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) tmem_alloc(smem_u32(&sh.tmem), TMEM_COLS);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = sh.tmem;
+    // The setup above overlaps the end of the kernel before, and so do the producer's first loads of weights.
+    if (warp > 0) {
+        pdl_wait();
+        if (MODE == MODE_GATEUP) pdl_release();
+    }
 
-    // (MODE_DX: an item is one or two k-blocks; one stage, and the epilogue's staging lies where the others would)
-    constexpr int ST = MODE == MODE_DX ? 1 : STAGES;
-    constexpr bool DEALT = MODE == MODE_DX;             // its items are all alike: by stride, no queue
+    auto consume = [&](uint32_t n, RowsItem& w) -> bool {
+        const int slot = n % SCHED_Q;
+        if (!mbar_wait(item_full + 8 * slot, (n / SCHED_Q) & 1, p.status, ERR_SCHED_WAIT)) return false;
+        w = sh.item[slot];
+        return w.row_tile >= 0;
+    };
+    auto release = [&](uint32_t n) { mbar_arrive(item_empty + 8 * (n % SCHED_Q)); };
+
+    if (warp == 0) {
+        if (elect_one()) {
+            int s = 0, claimed = 0;
+            uint32_t free_phase = 1;                    // (the first round finds every stage free)
+            bool ok = true;
+            const uint32_t tile0 = smem_u32(smem_raw);
+            RowsItem w = {}, next = {};
+            int total_items = 0;
+            auto decode = [&](int item) {               // (a CTA beyond the last item hands on "no work" and leaves through the teardown)
+                next.row_tile = -1;
+                if (item >= total_items) return;
+                const int row_i = item / p.n_col_tiles;
+                next.n0 = (item - row_i * p.n_col_tiles) * COLS_PER_ITEM;
+                next.row_tile = p.tile_order ? p.tile_order[row_i] : row_i;
+                next.e = p.tile_expert[next.row_tile];
+            };
+            auto load_b = [&](int kb, uint32_t b_dst, uint32_t bar) {
+                const bool second = MODE == MODE_DXG && kb >= p.kblocks;
+                const int kx = (second ? kb - p.kblocks : kb) * BK, e_rows = w.e * p.b_row_blocks;       // row blocks before this expert's
+                // One load for the whole 32 KiB of B: a k-block of two loads costs the producer ~230 cycles, one of five
+                // (B in 8 KiB pieces) made dXg 14 % slower
+                if (MODE == MODE_GATEUP)                // gate block and up block of the same hidden units
+                    tma_load_4d(b_dst, &tmB0, 0, 0, (e_rows + (w.n0 >> 7)) * p.b_col_blocks + kb, 0, bar);
+                else if (MODE == MODE_DOWN)             // two row blocks
+                    tma_load_4d(b_dst, &tmB0, 0, 0, kb, e_rows + (w.n0 >> 7), bar);
+                else                                    // four half blocks side by side (past the last column block: columns that are not computed)
+                    tma_load_3d(b_dst, second ? &tmB1 : &tmB0, 0, kx & 64, (e_rows + (kx >> 7)) * p.b_col_blocks + (w.n0 >> 6), bar);
+            };
+            int ahead = 0;                              // k-blocks of the first item whose B is on its way
+            if (p.early) {
+                total_items = *p.n_tiles * p.n_col_tiles;
+                decode(blockIdx.x);
+                w = next;
+                if (w.row_tile >= 0)
+                    for (; ahead < min(ST, kb_per_item); ++ahead) {
+                        mbar_expect_tx(full + 8 * ahead, STAGE_BYTES);
+                        load_b(ahead, tile0 + ahead * STAGE_BYTES + A_BYTES, full + 8 * ahead);
+                    }
+            }
+            pdl_wait();
+            if (MODE == MODE_GATEUP) pdl_release();
+            if (!p.early) {
+                total_items = *p.n_tiles * p.n_col_tiles;
+                decode(blockIdx.x);
+            }
+            // the next item is claimed, then decoded, some k-blocks before this one's loads end: not earlier, or the claim would
+            // sit behind this CTA's unfinished work while others run dry
+            const int claim = max(0, kb_per_item - ROWS_CLAIM), look = max(0, kb_per_item - 2);
+            for (uint32_t n = 0; ok; ++n) {
+                const int slot = n % SCHED_Q;
+                w = next;
+                if (!mbar_wait(item_empty + 8 * slot, ((n / SCHED_Q) & 1) ^ 1, p.status, ERR_SCHED_WAIT)) break;
+                sh.item[slot] = w;
+                mbar_arrive(item_full + 8 * slot);
+                if (w.row_tile < 0) {                   // one end for each group of the epilogue
+                    const int after = (n + 1) % SCHED_Q;
+                    if (!mbar_wait(item_empty + 8 * after, (((n + 1) / SCHED_Q) & 1) ^ 1, p.status, ERR_SCHED_WAIT)) break;
+                    sh.item[after].row_tile = -1;
+                    mbar_arrive(item_full + 8 * after);
+                    break;
+                }
+                const int row0 = w.row_tile * BM;
+                for (int kb = 0; kb < kb_per_item; ++kb) {
+                    if (kb == claim) claimed = atomicAdd(p.sched, 1);
+                    if (!mbar_wait(empty + 8 * s, free_phase, p.status, ERR_EMPTY_WAIT)) {
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t a_dst = tile0 + s * STAGE_BYTES, bar = full + 8 * s;
+                    const bool second = MODE == MODE_DXG && kb >= p.kblocks, loaded = n == 0 && kb < ahead;
+                    if (!loaded) mbar_expect_tx(bar, STAGE_BYTES);
+                    tma_load_2d(a_dst, second ? &tmA1 : &tmA0, (second ? kb - p.kblocks : kb) * BK, row0, bar);
+                    if (!loaded) load_b(kb, a_dst + A_BYTES, bar);
+                    if (++s == ST) {
+                        s = 0;
+                        free_phase ^= 1;
+                    }
+                    if (kb == look) decode(gridDim.x + claimed);
+                }
+            }
+            sched_finish(p.sched, gridDim.x);           // this CTA asks for no more items
+        }
+    } else if (warp == 1) {
+        if (elect_one()) {
+            int s = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            const uint64_t a0 = make_desc(smem_u32(smem_raw), 16, 1024);
+            // MN-major: 16 reduction rows = two 8-row groups (1 KiB each), 64-column blocks BOX_BYTES apart
+            const uint64_t b0 = DATA_GRAD ? make_desc(smem_u32(smem_raw) + A_BYTES, BOX_BYTES, 1024) : make_desc(smem_u32(smem_raw) + A_BYTES, 16, 1024);
+            constexpr uint32_t B_STEP = (DATA_GRAD ? 2048 : 32) >> 4;       // (the address field: 16-byte units)
+            RowsItem w;
+            for (uint32_t t = 0; ok && consume(t, w); ++t) {
+                release(t);
+                const uint32_t buf = t & 1u;
+                if (!mbar_wait(acc_empty + 8 * buf, ((t >> 1) & 1) ^ 1, p.status, ERR_ACC_WAIT)) break;
+                tc_fence_after();
+                const uint32_t d_tmem = tmem_base + buf * BN;
+                // a narrower product where the last item of a row tile has fewer columns
+                const uint32_t idesc = make_idesc(BM, DATA_GRAD ? min(BN, 64 * p.b_col_blocks - w.n0) : BN, 0, DATA_GRAD ? 1 : 0);
+                for (int kb = 0; kb < kb_per_item; ++kb) {
+                    if (!mbar_wait(full + 8 * s, phase, p.status, ERR_FULL_WAIT)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint64_t ad = a0 + s * (STAGE_BYTES >> 4), bd = b0 + s * (STAGE_BYTES >> 4);
+#pragma unroll
+                    for (int k = 0; k < BK / 16; ++k) umma_bf16(d_tmem, ad + k * (32 >> 4), bd + k * B_STEP, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                    umma_commit(empty + 8 * s);         // frees the stage once these MMAs have read it
+                    if (++s == STAGES) {
+                        s = 0;
+                        phase ^= 1;
+                    }
+                }
+                umma_commit(acc_full + 8 * buf);        // accumulator of this item complete
+            }
+        }
+    } else if (warp == 2 + EPI_WARPS) {
+        if (BIAS && elect_one()) {
+            RowsItem w;
+            for (uint32_t t = 0; consume(t, w); ++t) {
+                release(t);
+                const uint32_t buf = t & 1u, bar = smem_u32(&sh.bias_full[buf]);
+                const int cols = min(COLS_PER_ITEM, p.n_out - w.n0);
+                const float *g0 = p.bias0[w.e] + w.n0, *g1 = MODE == MODE_GATEUP ? p.bias1[w.e] + w.n0 : nullptr;
+                // (the epilogue has read this buffer's biases of two items ago: it arrives on acc_empty after that)
+                if (!mbar_wait(acc_empty + 8 * buf, ((t >> 1) & 1) ^ 1, p.status, ERR_ACC_WAIT)) break;
+                if (p.n_out >= 32) {
+                    mbar_expect_tx(bar, (MODE == MODE_GATEUP ? 2 : 1) * cols * 4);
+                    bulk_load(smem_u32(sh.bias[buf]), g0, cols * 4, bar);
+                    if (MODE == MODE_GATEUP) bulk_load(smem_u32(sh.bias[buf] + BN / 2), g1, cols * 4, bar);
+                } else {                                // (fewer may start anywhere)
+                    for (int i = 0; i < cols; ++i) {
+                        sh.bias[buf][i] = g0[i];
+                        if (MODE == MODE_GATEUP) sh.bias[buf][BN / 2 + i] = g1[i];
+                    }
+                    mbar_arrive(bar);
+                }
+            }
+        }
+    } else {
+        // 16 epilogue warps in two groups, one per accumulator, so that one group computes while the other one's stores drain:
+        // TMEM lane quarter q = warp % 4, column half h
+        constexpr int PER = EPI_WARPS / rows_groups(MODE);
+        const int i = warp - 2;
+        rows_epilogue<MODE>(p, sh, tmem_base, i / PER, warp & 3, i % PER / 4, lane, smem_raw + STAGES * STAGE_BYTES + i * STAGING_BYTES, &tmD0, &tmD1,
+                            [&](uint32_t n, RowsItem& w) -> bool {
+                                const bool more = __any_sync(0xffffffffu, consume(n, w));       // (warp-uniform)
+                                if (more && lane == 0) release(n);
+                                return more;
+                            });
+    }
+    cta_teardown(tmem_base, warp);
+}
+
+// MODE_DX: dlogits * Wr^T, an item of one or two k-blocks; one stage, and the epilogue's staging lies where the others would.
+// Its items are all alike: by stride, no queue.
+__global__ void __launch_bounds__(TC_THREADS, 1)
+tc_dx_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const RowsP p)
+{
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const Pipe pipe = carve(smem_raw);
     const uint32_t tmem_base = cta_setup(pipe, warp);
-    pdl_wait();                                         // the setup above overlaps the end of the kernel before
-    // a CTA beyond the last item publishes "no work" to its own queue and leaves through the teardown
-    const int total_items = (MODE == MODE_DX ? p.fixed_tiles : *p.n_tiles) * p.n_col_tiles;
-
+    pdl_wait();
+    const int total_items = p.fixed_tiles * p.n_col_tiles;
     if (warp == 0) {
         if (elect_one()) {
             uint32_t it = 0;
             bool ok = true;
-            int item = blockIdx.x;
-            if (!DEALT) ok = sched_publish(pipe, 0, item, total_items, p.status);
-            for (uint32_t nf = 1; ok && (DEALT ? item < total_items : item >= 0); ++nf) {
-                const int row_i = item / p.n_col_tiles, n0 = (item % p.n_col_tiles) * COLS_PER_ITEM;
-                const int row_tile = p.tile_order ? p.tile_order[row_i] : row_i;
-                const int row0 = row_tile * BM;
-                const int e_rows = MODE == MODE_DX ? 0 : p.tile_expert[row_tile] * p.b_row_blocks;      // row blocks before this expert's
-                for (int kb = 0; kb < kb_per_item; ++kb, ++it) {
-                    const int s = it % ST;
-                    if (it >= ST && !mbar_wait(pipe.empty(s), ((it / ST) - 1) & 1, p.status, ERR_EMPTY_WAIT)) {
+            for (int item = blockIdx.x; ok && item < total_items; item += gridDim.x) {
+                const int row0 = item / p.n_col_tiles * BM, n0 = item % p.n_col_tiles * BN;
+                for (int kb = 0; kb < p.kblocks; ++kb, ++it) {
+                    if (it >= 1 && !mbar_wait(pipe.empty(0), (it - 1) & 1, p.status, ERR_EMPTY_WAIT)) {
                         ok = false;
                         break;
                     }
-                    const uint32_t a_dst = smem_u32(pipe.tiles + s * STAGE_BYTES), b_dst = a_dst + A_BYTES;
-                    mbar_expect_tx(pipe.full(s), STAGE_BYTES);
-                    const bool second = MODE == MODE_DXG && kb >= p.kblocks;
-                    const int kx = (second ? kb - p.kblocks : kb) * BK;
-                    tma_load_2d(a_dst, second ? &tmA1 : &tmA0, kx, row0, pipe.full(s));
-                    // One load for the whole 32 KiB of B: a k-block of two loads costs the producer ~500 cycles, one of five
-                    // (B in 8 KiB pieces) made dXg 14 % slower
-                    if (MODE == MODE_GATEUP) {             // gate block and up block of the same hidden units
-                        tma_load_4d(b_dst, &tmB0, 0, 0, (e_rows + (n0 >> 7)) * p.b_col_blocks + kb, 0, pipe.full(s));
-                    } else if (MODE == MODE_DOWN) {        // two row blocks
-                        tma_load_4d(b_dst, &tmB0, 0, 0, kb, e_rows + (n0 >> 7), pipe.full(s));
-                    } else if (DATA_GRAD) {
-                        // four half blocks side by side (past the last column block: columns that are not computed)
-                        tma_load_3d(b_dst, second ? &tmB1 : &tmB0, 0, kx & 64, (e_rows + (kx >> 7)) * p.b_col_blocks + (n0 >> 6), pipe.full(s));
-                    } else {
-                        tma_load_2d(b_dst, &tmB0, kx, n0, pipe.full(s));
-                        tma_load_2d(b_dst + HALF_B, &tmB0, kx, n0 + BN / 2, pipe.full(s));
-                    }
+                    const uint32_t a_dst = smem_u32(pipe.tiles), b_dst = a_dst + A_BYTES;
+                    mbar_expect_tx(pipe.full(0), STAGE_BYTES);
+                    tma_load_2d(a_dst, &tmA, kb * BK, row0, pipe.full(0));
+                    tma_load_2d(b_dst, &tmB, kb * BK, n0, pipe.full(0));
+                    tma_load_2d(b_dst + HALF_B, &tmB, kb * BK, n0 + BN / 2, pipe.full(0));
                 }
-                if (DEALT) {
-                    item += gridDim.x;
-                    continue;
-                }
-                // the next item is claimed as late as possible (the ring is full by now, so the round trip to the
-                // counter does not starve the tensor core): early claims would sit behind this CTA's unfinished work
-                int next = sched_fetch(p.sched);
-                if (ok) ok = sched_publish(pipe, nf, next, total_items, p.status);
-                item = next;
             }
-            if (!DEALT) sched_finish(p.sched, gridDim.x);           // this CTA asks for no more items
         }
     } else if (warp == 1) {
         if (elect_one()) {
             uint32_t it = 0, t = 0;
             bool ok = true;
-            for (; ok; ++t) {
-                int item;
-                if constexpr (DEALT) {
-                    item = blockIdx.x + t * gridDim.x;
-                    if (item >= total_items) break;
-                } else {
-                    item = sched_consume(pipe, t, p.status);
-                    if (item >= 0) sched_release(pipe, t);
-                    if (item < 0) break;
-                }
+            for (int item = blockIdx.x; ok && item < total_items; item += gridDim.x, ++t) {
                 const uint32_t buf = t & 1u;
                 if (t >= 2 && !mbar_wait(pipe.acc_empty(buf), ((t >> 1) - 1) & 1, p.status, ERR_ACC_WAIT)) break;
                 tc_fence_after();
-                const uint32_t d_tmem = tmem_base + buf * BN;
-                // a narrower product where the last item of a row tile has fewer columns
-                const int ncols = DATA_GRAD ? min(BN, 64 * p.b_col_blocks - (item % p.n_col_tiles) * BN) : BN;
-                const uint32_t idesc = make_idesc(BM, ncols, 0, DATA_GRAD ? 1 : 0);
-                for (int kb = 0; kb < kb_per_item; ++kb, ++it) {
-                    const int s = it % ST;
-                    if (!mbar_wait(pipe.full(s), (it / ST) & 1, p.status, ERR_FULL_WAIT)) {
+                for (int kb = 0; kb < p.kblocks; ++kb, ++it) {
+                    if (!mbar_wait(pipe.full(0), it & 1, p.status, ERR_FULL_WAIT)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t a_addr = smem_u32(pipe.tiles + s * STAGE_BYTES), b_addr = a_addr + A_BYTES;
+                    const uint32_t a_addr = smem_u32(pipe.tiles), b_addr = a_addr + A_BYTES;
 #pragma unroll
-                    for (int k = 0; k < BK / 16; ++k) {
-                        const uint64_t ad = make_desc(a_addr + k * 32, 16, 1024);
-                        // MN-major: 16 reduction rows = two 8-row groups (1 KiB each), 64-column blocks BOX_BYTES apart
-                        const uint64_t bd = DATA_GRAD ? make_desc(b_addr + k * 2048, BOX_BYTES, 1024) : make_desc(b_addr + k * 32, 16, 1024);
-                        umma_bf16(d_tmem, ad, bd, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                    }
-                    umma_commit(pipe.empty(s));           // frees the stage once these MMAs have read it
+                    for (int k = 0; k < BK / 16; ++k)
+                        umma_bf16(tmem_base + buf * BN, make_desc(a_addr + k * 32, 16, 1024), make_desc(b_addr + k * 32, 16, 1024),
+                                  make_idesc(BM, BN, 0, 0), (kb > 0 || k > 0) ? 1u : 0u);
+                    umma_commit(pipe.empty(0));
                 }
-                umma_commit(pipe.acc_full(buf));          // accumulator of this item complete
+                umma_commit(pipe.acc_full(buf));
             }
         }
     } else {
-        // 16 epilogue warps: TMEM lane quarter q = warp % 4 (rows q*32..+31), column group h = 0..3
-        const int q = warp & 3, h = (warp - 2) >> 2;
-        uint8_t* stage = pipe.staging + (warp - 2) * STAGING_BYTES;
-        if constexpr (DEALT) {
-            dx_epilogue(p, pipe, tmem_base, total_items, q, h, lane, reinterpret_cast<float*>(pipe.tiles + ST * STAGE_BYTES + (warp - 2) * DX_STAGING));
-        } else {
-            for (uint32_t t = 0;; ++t) {
-                const int item = __shfl_sync(0xffffffffu, sched_consume(pipe, t, p.status), 0);   // warp-uniform
-                if (item < 0) break;
-                if (lane == 0) sched_release(pipe, t);
-                const uint32_t buf = t & 1u;
-                const int row_i = item / p.n_col_tiles, n0 = (item % p.n_col_tiles) * COLS_PER_ITEM;
-                const int row_tile = p.tile_order ? p.tile_order[row_i] : row_i;
-                if (!rows_epilogue<MODE>(p, pipe.acc_full(buf), pipe.acc_empty(buf), tmem_base, buf, t, row_tile, n0, p.tile_expert[row_tile], q, h,
-                                         lane, stage, &tmD0, &tmD1, &tmD2))
-                    break;
-            }
-            if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // stores landed before exit
-        }
+        dx_epilogue(p, pipe, tmem_base, total_items, warp & 3, (warp - 2) >> 2, lane,
+                    reinterpret_cast<float*>(pipe.tiles + STAGE_BYTES + (warp - 2) * DX_STAGING));
     }
     cta_teardown(tmem_base, warp);
 }
@@ -710,7 +924,7 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant_
                 const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUtensorMap tmB1,
                 const __grid_constant__ CUtensorMap tmA2, const __grid_constant__ CUtensorMap tmB2, const WgradP p)
 {
-    extern __shared__ uint8_t smem_raw[];
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int total_items = p.total_items;
     const Pipe pipe = carve(smem_raw);
@@ -1068,7 +1282,7 @@ tc_wgrad_pair_kernel(const __grid_constant__ CUtensorMap tmXg, const __grid_cons
                      const __grid_constant__ CUtensorMap tmdG, const __grid_constant__ CUtensorMap tmdU,
                      const __grid_constant__ CUtensorMap tmHh, const PairWgradP p)
 {
-    extern __shared__ uint8_t smem_raw[];
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = (int)cluster_ctarank();
     uint8_t* const tiles = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -1467,9 +1681,9 @@ struct TcState {
     // the same operands by column blocks (one load per operand tile): A side {64, 64 rows, 2}, B side {64, 64 rows, 4}
     CUtensorMap Xg_b4, dYg_b4, dG_b2, dU_b2, Hh_b2;
     CUtensorMap Xg_b2, dYg_b2;
-    bool c_blocks = false;       // the maps of Xg and dYg are there (C a multiple of 64); those of dG, dU, Hh always are
     // epilogue stores (box 32 x 32 rows, 64-byte swizzle)
     CUtensorMap Hh_s, Yg_s, dG_s, dU_s, dXg_s;
+    bool c_blocks = false;       // the maps of Xg and dYg are there (C a multiple of 64); those of dG, dU, Hh always are
 };
 
 int prepare_attrs(mgpt_moe_layer* L);
@@ -1527,11 +1741,11 @@ int prepare_attrs(mgpt_moe_layer* L)
     if (!L->tc_state) L->tc_state = new TcState();
     TcState* s = (TcState*)L->tc_state;
     if (!s->attr_set) {
-        MGPT_CUDA(cudaFuncSetAttribute(tc_rows_kernel<MODE_GATEUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        MGPT_CUDA(cudaFuncSetAttribute(tc_rows_kernel<MODE_DOWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        MGPT_CUDA(cudaFuncSetAttribute(tc_rows_kernel<MODE_DHH>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        MGPT_CUDA(cudaFuncSetAttribute(tc_rows_kernel<MODE_DXG>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        MGPT_CUDA(cudaFuncSetAttribute(tc_rows_kernel<MODE_DX>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        MGPT_CUDA(cudaFuncSetAttribute(tc_rows_kernel<MODE_GATEUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROWS_SMEM));
+        MGPT_CUDA(cudaFuncSetAttribute(tc_rows_kernel<MODE_DOWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROWS_SMEM));
+        MGPT_CUDA(cudaFuncSetAttribute(tc_rows_kernel<MODE_DHH>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROWS_SMEM));
+        MGPT_CUDA(cudaFuncSetAttribute(tc_rows_kernel<MODE_DXG>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROWS_SMEM));
+        MGPT_CUDA(cudaFuncSetAttribute(tc_dx_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
         MGPT_CUDA(cudaFuncSetAttribute(tc_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
         MGPT_CUDA(cudaFuncSetAttribute(tc_wgrad_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WP_SMEM));
         MGPT_CUDA(cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, L->device));
@@ -1560,11 +1774,9 @@ namespace {
 // One of the four token-major products.
 template <int MODE>
 int launch_rows(mgpt_moe_layer* L, TcState* s, const Workspace& w, const RowsP& p, const CUtensorMap& a0, const CUtensorMap& a1,
-                const CUtensorMap& b0, const CUtensorMap& b1, const CUtensorMap& d0, const CUtensorMap& d1,
-                const CUtensorMap& d2, cudaStream_t st, const char* what)
+                const CUtensorMap& b0, const CUtensorMap& b1, const CUtensorMap& d0, const CUtensorMap& d1, cudaStream_t st, const char* what)
 {
-    MGPT_CUDA(launch_pdl(tc_rows_kernel<MODE>, imin(grid_sms(L, s), w.max_tiles * p.n_col_tiles), TC_THREADS, SMEM_BYTES, st, a0, a1,
-                         b0, b1, d0, d1, d2, p));
+    MGPT_CUDA(launch_pdl(tc_rows_kernel<MODE>, imin(grid_sms(L, s), w.max_tiles * p.n_col_tiles), ROWS_THREADS, ROWS_SMEM, st, a0, a1, b0, b1, d0, d1, p));
     MGPT_LAUNCHED(what);
     return 0;
 }
@@ -1585,19 +1797,21 @@ int tc_experts_forward(mgpt_moe_layer* L, const Workspace& w, char* ws, cudaStre
     p.kblocks = cdiv(d.C, BK); p.n_out = d.H; p.n_col_tiles = cdiv(d.H, BN / 2);
     p.b_row_blocks = cdiv(d.H, 128); p.b_col_blocks = cdiv(d.C, BK);
     p.bias0 = L->master.bg; p.bias1 = L->master.bu;
+    p.early = L->ext_Xg == nullptr;                     // behind dispatch (an expert side's tiles are the kernel's before)
     p.G = w.inference ? nullptr : (bf16*)(ws + w.G);
     p.U = w.inference ? nullptr : (bf16*)(ws + w.U);
     L->stage_begin(ST_GATEUP, st);
     p.sched = s->sched + 0;
-    MGPT_TRY(launch_rows<MODE_GATEUP>(L, s, w, p, s->Xg, s->Xg, s->WguT, s->WguT, s->Hh_s, s->Hh_s, s->Hh_s, st, "tc_rows<gateup>"));
+    MGPT_TRY(launch_rows<MODE_GATEUP>(L, s, w, p, s->Xg, s->Xg, s->WguT, s->WguT, s->Hh_s, s->Hh_s, st, "tc_rows<gateup>"));
     L->stage_end(ST_GATEUP, st);
     // down: K = H
     p.kblocks = cdiv(d.H, BK); p.n_out = d.C; p.n_col_tiles = cdiv(d.C, BN);
     p.b_row_blocks = cdiv(d.C, 128); p.b_col_blocks = cdiv(d.H, BK);
     p.bias0 = L->master.bd; p.bias1 = nullptr;
+    p.early = 1;
     L->stage_begin(ST_DOWN, st);
     p.sched = s->sched + 2;
-    MGPT_TRY(launch_rows<MODE_DOWN>(L, s, w, p, s->Hh, s->Hh, s->WdT, s->WdT, s->Yg_s, s->Yg_s, s->Yg_s, st, "tc_rows<down>"));
+    MGPT_TRY(launch_rows<MODE_DOWN>(L, s, w, p, s->Hh, s->Hh, s->WdT, s->WdT, s->Yg_s, s->Yg_s, st, "tc_rows<down>"));
     L->stage_end(ST_DOWN, st);
     return 0;
 }
@@ -1621,14 +1835,14 @@ int tc_experts_backward(mgpt_moe_layer* L, const Workspace& w, char* ws, cudaStr
     p.G = (bf16*)(ws + w.G); p.U = (bf16*)(ws + w.U);
     L->stage_begin(ST_DHH, st);
     p.sched = s->sched + 4;
-    MGPT_TRY(launch_rows<MODE_DHH>(L, s, w, p, s->dYg, s->dYg, s->Wd_h, s->Wd_h, s->dG_s, s->dU_s, s->dU_s, st, "tc_rows<dhh>"));
+    MGPT_TRY(launch_rows<MODE_DHH>(L, s, w, p, s->dYg, s->dYg, s->Wd_h, s->Wd_h, s->dG_s, s->dU_s, st, "tc_rows<dhh>"));
     L->stage_end(ST_DHH, st);
     // dXg = dG * Wg^T + dU * Wu^T  (K = 2H)
     p.kblocks = cdiv(d.H, BK); p.n_out = d.C; p.n_col_tiles = cdiv(d.C, BN);
     p.b_row_blocks = cdiv(d.H, 128); p.b_col_blocks = cdiv(d.C, BK);
     L->stage_begin(ST_DXG, st);
     p.sched = s->sched + 6;
-    MGPT_TRY(launch_rows<MODE_DXG>(L, s, w, p, s->dG, s->dU, s->Wg_h, s->Wu_h, s->dXg_s, s->dXg_s, s->dXg_s, st, "tc_rows<dxg>"));
+    MGPT_TRY(launch_rows<MODE_DXG>(L, s, w, p, s->dG, s->dU, s->Wg_h, s->Wu_h, s->dXg_s, s->dXg_s, st, "tc_rows<dxg>"));
     L->stage_end(ST_DXG, st);
     }
     if (!L->has_grad || !(phase & 2)) return 0;
@@ -1718,8 +1932,8 @@ int tc_router_dx(mgpt_moe_layer* L, const Workspace& w, char* ws, const void* dX
     p.fixed_tiles = cdiv(w.n_tokens, BM); p.n_valid_rows = w.n_tokens;
     p.gather_src = (const bf16*)dXg; p.gather_pos = pos; p.gather_k = d.k;
     p.dx = (bf16*)dx;
-    MGPT_CUDA(launch_pdl(tc_rows_kernel<MODE_DX>, imin(grid_sms(L, s), p.fixed_tiles * p.n_col_tiles), TC_THREADS, SMEM_BYTES, st, mA, mA, mB, mB, mA, mA, mA, p));
-    MGPT_LAUNCHED("tc_rows_kernel<dx>");
+    MGPT_CUDA(launch_pdl(tc_dx_kernel, imin(grid_sms(L, s), p.fixed_tiles * p.n_col_tiles), TC_THREADS, SMEM_BYTES, st, mA, mB, p));
+    MGPT_LAUNCHED("tc_dx_kernel");
     return 0;
 }
 

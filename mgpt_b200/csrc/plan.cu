@@ -270,6 +270,7 @@ dispatch_kernel(const TIn* x, const int32_t* pos, const int32_t* row_src,
                 const int32_t* n_tiles, int row_cap, int N, int C, int k, int pad_blocks, TAct* Xg, PaddingZeros kept)
 {
     pdl_wait();
+    if constexpr (sizeof(TAct) == 2) pdl_release();  // the tensor-core product that follows requests its first weights
     const int lane = threadIdx.x & 31, all_pads = kept.Hh ? 4 * pad_blocks : pad_blocks;
     if ((int)blockIdx.x < all_pads) {
         const int rows = *n_tiles * ROW_TILE;
