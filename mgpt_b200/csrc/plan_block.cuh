@@ -131,13 +131,20 @@ __device__ __forceinline__ void plan_block(const PlanArgs& p, PlanShared& sh)
             if (p.slot_of) p.slot_of[i] = slot;
         }
     }
-    for (int x = warp; x < p.E; x += WARPS) {
-        const int t0 = sh.poff[x] / ROW_TILE, t1 = sh.poff[x + 1] / ROW_TILE;
-        for (int t = t0 + lane; t < t1 && t < p.max_tiles; t += 32) p.tile_expert[t] = x;
-        for (int q = sh.poff[x] + sh.tot[x] + lane; q < sh.poff[x + 1]; q += 32) p.row_src[q] = -1;
+    for (int x = tid; x < p.E; x += THREADS) {
+        for (int t = sh.poff[x] / ROW_TILE; t < sh.poff[x + 1] / ROW_TILE && t < p.max_tiles; ++t) p.tile_expert[t] = x;
         if (p.groups)
-            for (int g = lane; g * DECODE_GROUP < sh.tot[x]; g += 32)
+            for (int g = 0; g * DECODE_GROUP < sh.tot[x]; ++g)
                 p.groups[sh.goff[x] + g] = make_int4(x, sh.poff[x] + g * DECODE_GROUP, min(DECODE_GROUP, sh.tot[x] - g * DECODE_GROUP), 0);
+    }
+    // padding rows: the end of an expert's last tile
+    for (int x = warp; x < p.E; x += WARPS) {
+        const int end = sh.poff[x + 1];
+#pragma unroll
+        for (int i = 0; i < ROW_TILE / 32; ++i) {
+            const int q = end - ROW_TILE + 32 * i + lane;
+            if (q >= sh.poff[x] + sh.tot[x]) p.row_src[q] = -1;
+        }
     }
 }
 

@@ -113,23 +113,26 @@ __device__ __forceinline__ void router_finish(const float (&acc)[TPW][EPL], cons
 }
 
 // The exact router.  What bounds it at scale is FP32 issue (one multiply and one add per token, expert and channel) and
-// for small batches the addition chain of one (token, expert) pair, C additions of four cycles.  A thread owns TM tokens x
-// TE experts, so that operands read from shared memory are used several times, and reads the next eight channels' operands
-// while it works on these eight; Wr and the tokens' rows stream through a ring that two warps fill with cp.async (one
-// bulk copy per stage cost its issuing thread ~500 cycles, more than a small batch spends on the stage), and the four
-// compute warps never wait for each other while they add.  The softmax is spread the same way: exponentials by the
-// threads that hold the logits, sums and top-k -- sequential in the reference -- by one thread per token.  With
-// plan.top_idx set, the last block to finish also builds the dispatch plan (one launch less for small batches).
-// WV: a thread's experts are neighbours read with one 16-byte load (E a multiple of 4), else E/TE apart.
+// for small batches the addition chain of one (token, expert) pair, C additions of four cycles.
 //
-// Before (lane = expert, chunks of 32 channels through registers or cp.async with a block barrier per chunk) -> now, us:
-// 64 tokens, C=1024, E=32, with the plan 22 -> 19; 1777 tokens 33 -> 20; 4096 tokens 33 -> 26; 8192 tokens, C=512, E=16
-// 19 -> 18; ~3900 listed tokens, C=2048, E=64 132 -> 99.
+// RS: experts rounded up to 16, 32, 64 or 128, the row length of the staged Wr, so that a thread's operands lie at constant
+// offsets; ET = RS / TE lanes of one warp share a token, each with TE neighbouring experts of TM tokens, and read the next
+// operands while they work on these.  Wr and the tokens' rows stream through a ring that four warps fill with cp.async (one
+// bulk copy per stage cost its issuing thread ~500 cycles, more than a small batch spends on the stage); the eight
+// compute warps never wait for each other.  Softmax and top-k stay with the lanes that hold the logits: maximum and
+// arg-max by shuffles, the sum -- sequential in the reference -- by every lane of the token from shared memory.  With
+// plan.top_idx set, the last block to finish also builds the dispatch plan (one launch less for small batches).
+//
+// In a kernel of 128 compute threads with row lengths only known at run time, one thread per token for sum and top-k and stages of
+// 128 channels, a channel took 14 cycles with one pair per thread and 38 with eight, the top-k 4000 cycles and the plan 7000-
+// 17000.  Stage times before -> now, us: 1 token, C=1024, E=32, with the plan 22.4 -> 16.2; 64 tokens 28.7 -> 18.5; 256 tokens,
+// without, 18.6 -> 15; 1777 tokens 26.4 -> 22.6; 5003 FP32 tokens, C=512, E=16 28.5 -> 20.7; both passes of the screened
+// router, 16384 skewed tokens, C=1024, E=64, 91 -> 79.
 struct RouterArgs {
     const void* x;
     const float *Wr, *br;
     int N, C, E, k;
-    int ck, stages, tok;    // channels (a power of two) and stages of the ring, tokens per CTA
+    int ck, stages, tok;    // channels (a power of two) and stages of the ring, tokens per CTA and round
     float *logits, *probs;
     int32_t* top_idx;
     float* top_p;
@@ -139,20 +142,36 @@ struct RouterArgs {
     PlanArgs plan;
 };
 
-constexpr int RX_COMPUTE = 128, RX_PRODUCE = 64, RX_THREADS = RX_COMPUTE + RX_PRODUCE, RX_MAX_STAGES = 16;
+constexpr int RX_COMPUTE = 256, RX_PRODUCE = 128, RX_THREADS = RX_COMPUTE + RX_PRODUCE, RX_MAX_STAGES = 16;
 __host__ __device__ inline uint32_t rx_x_row(int ck, int elt) { return (uint32_t)(ck * elt + 16); }      // padded: rows in distinct banks
-__host__ __device__ inline uint32_t rx_stage(int ck, int E, int tok, int elt)
+__host__ __device__ inline uint32_t rx_stage(int ck, int rs, int tok, int elt)
 {
-    return ((uint32_t)ck * E * 4 + tok * rx_x_row(ck, elt) + 127u) & ~127u;
+    return ((uint32_t)ck * rs * 4 + tok * rx_x_row(ck, elt) + 127u) & ~127u;
 }
-// logits, exponentials [tok][E+1]; maximum and scale [tok]
-__host__ __device__ inline uint32_t rx_tail(int tok, int E) { return (uint32_t)tok * (2 * (E + 1) + 2) * 4; }
+constexpr uint32_t rx_tail(int te, int tm, int rs) { return (uint32_t)(RX_COMPUTE * te / rs) * tm * (rs + 4) * 4; }      // exponentials, a row per token
 
+// Loads with a 32-bit shared address: through pointers into the ring the compiler lost the address space, and a channel of one
+// pair took 13 cycles instead of 8.
+__device__ __forceinline__ uint4 lds128(uint32_t a)
+{
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+    return v;
+}
+template <int TE> __device__ __forceinline__ void lds_weights(float (&w)[TE], uint32_t a)
+{
+    if constexpr (TE == 4)
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(w[0]), "=f"(w[1]), "=f"(w[2]), "=f"(w[3]) : "r"(a));
+    else if constexpr (TE == 2)
+        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(w[0]), "=f"(w[1]) : "r"(a));
+    else
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(w[0]) : "r"(a));
+}
 // 8 consecutive channels of a staged row
 template <typename TIn> struct Row8;
 template <> struct Row8<bf16> {
     uint4 u;
-    __device__ __forceinline__ void load(const uint8_t* p) { u = *reinterpret_cast<const uint4*>(p); }
+    __device__ __forceinline__ void load(uint32_t a) { u = lds128(a); }
     __device__ __forceinline__ float get(int i) const
     {
         const uint32_t w = i < 2 ? u.x : i < 4 ? u.y : i < 6 ? u.z : u.w;
@@ -160,70 +179,31 @@ template <> struct Row8<bf16> {
     }
 };
 template <> struct Row8<float> {
-    float4 a, b;
-    __device__ __forceinline__ void load(const uint8_t* p)
+    uint4 u[2];
+    __device__ __forceinline__ void load(uint32_t a)
     {
-        a = *reinterpret_cast<const float4*>(p);
-        b = *reinterpret_cast<const float4*>(p + 16);
+        u[0] = lds128(a);
+        u[1] = lds128(a + 16);
     }
     __device__ __forceinline__ float get(int i) const
     {
-        const float4& f = i < 4 ? a : b;
-        return (i & 3) == 0 ? f.x : (i & 3) == 1 ? f.y : (i & 3) == 2 ? f.z : f.w;
+        const uint4& f = u[i >> 2];
+        return __uint_as_float((i & 3) == 0 ? f.x : (i & 3) == 1 ? f.y : (i & 3) == 2 ? f.z : f.w);
     }
 };
 
-// One token's sum, scale and top-k from its exponentials: the reference's order and its strict '>' insertion
-// (utils/Tensor.cpp:850-883, 1296-1334).  K: k rounded up.
-template <int K>
-__device__ __forceinline__ float rx_top(const float* ex, int E, int k, int32_t* top_idx, float* top_p)
-{
-    float sum = 0.0f;
-#pragma unroll 8
-    for (int e = 0; e < E; ++e) sum = __fadd_rn(sum, ex[e]);
-    const float inv = __fdiv_rn(1.0f, fmaxf(sum, 1e-15f));
-    float val[K];
-    int idx[K];
-#pragma unroll
-    for (int j = 0; j < K; ++j) {
-        val[j] = -INFINITY;
-        idx[j] = -1;
-    }
-#pragma unroll 4
-    for (int e = 0; e < E; ++e) {
-        float v = fminf(fmaxf(__fmul_rn(ex[e], inv), 1e-7f), 1.0f);
-        int i = e;
-        // (an entry displaced from place j is larger than, or equal to and earlier than, everything after it)
-#pragma unroll
-        for (int j = 0; j < K; ++j) {
-            const bool up = v > val[j] || (v == val[j] && i < idx[j]);
-            const float tv = up ? val[j] : v;
-            const int ti = up ? idx[j] : i;
-            val[j] = up ? v : val[j];
-            idx[j] = up ? i : idx[j];
-            v = tv;
-            i = ti;
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < K; ++j)
-        if (j < k) {
-            top_idx[j] = idx[j];
-            top_p[j] = val[j];
-        }
-    return inv;
-}
-
-template <typename TIn, int TM, int TE, bool WV>
-__global__ void __launch_bounds__(RX_THREADS) router_exact_kernel(const RouterArgs p)
+template <typename TIn, int RS, int TE, int TM>
+__global__ void __launch_bounds__(RX_THREADS, 1) router_exact_kernel(const RouterArgs p)
 {
     extern __shared__ __align__(128) uint8_t rx_smem[];
     __shared__ __align__(8) uint64_t bars[2 * RX_MAX_STAGES];
     __shared__ int last;
+    constexpr int ET = RS / TE, GROUPS = RX_COMPUTE / ET;
+    static_assert(ET <= 32, "a token's lanes lie in one warp");
     const int tid = threadIdx.x, lane = tid & 31;
-    const int C = p.C, E = p.E, CK = p.ck, ST = p.stages, TOK = p.tok;
-    const uint32_t x_row = rx_x_row(CK, sizeof(TIn)), x_off = (uint32_t)CK * E * 4, stage = rx_stage(CK, E, TOK, sizeof(TIn));
-    uint8_t* const ring = rx_smem;
+    const int C = p.C, E = p.E, CK = p.ck, ST = p.stages;
+    const uint32_t x_row = rx_x_row(CK, sizeof(TIn)), x_off = (uint32_t)CK * RS * 4, stage = rx_stage(CK, RS, p.tok, sizeof(TIn));
+    const uint32_t ring0 = (uint32_t)__cvta_generic_to_shared(rx_smem);
     const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(bars);
     auto full = [&](int s) { return bar0 + 8u * s; };
     auto empty = [&](int s) { return bar0 + 8u * (RX_MAX_STAGES + s); };
@@ -236,8 +216,9 @@ __global__ void __launch_bounds__(RX_THREADS) router_exact_kernel(const RouterAr
     }
     __syncthreads();
     pdl_wait();
-    const int n_active = p.list ? *p.list_count : p.N;
-    const int n_tiles = (n_active + TOK - 1) / TOK;
+    // as few rounds as the CTAs can do it in, all alike
+    const int n_active = p.list ? *p.list_count : p.N, rounds = max(1, (n_active + (int)gridDim.x * p.tok - 1) / ((int)gridDim.x * p.tok));
+    const int TOK = max(1, (n_active + (int)gridDim.x * rounds - 1) / ((int)gridDim.x * rounds)), n_tiles = (n_active + TOK - 1) / TOK;
     auto wait = [&](uint32_t bar, uint32_t parity) {
         for (uint32_t i = 0; i < (1u << 20); ++i) {
             uint32_t ok;
@@ -258,12 +239,21 @@ __global__ void __launch_bounds__(RX_THREADS) router_exact_kernel(const RouterAr
             const int n = min(TOK, n_active - tile * TOK);
             for (int c0 = 0; c0 < C; c0 += CK) {
                 if (round > 0) wait(empty(s), (round - 1) & 1);
-                const int len = min(CK, C - c0), pieces = len / XV, wp = len * E / 4;
-                const uint32_t dst = (uint32_t)__cvta_generic_to_shared(ring + s * stage);
+                const int len = min(CK, C - c0), pieces = len / XV;
+                const uint32_t dst = ring0 + s * stage;
                 const float* src = p.Wr + (size_t)c0 * E;
-#pragma unroll 4
-                for (int v = pt; v < wp; v += RX_PRODUCE)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + v * 16), "l"(src + v * 4) : "memory");
+                if (E == RS) {
+                    for (int v = pt; v < len * (RS / 4); v += RX_PRODUCE)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + v * 16), "l"(src + v * 4) : "memory");
+                } else if ((E & 3) == 0) {
+                    const int per = E / 4;
+                    for (int v = pt; v < len * per; v += RX_PRODUCE)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+                                     ::"r"(dst + v / per * (RS * 4) + v % per * 16), "l"(src + v * 4) : "memory");
+                } else {
+                    for (int v = pt; v < len * E; v += RX_PRODUCE)
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + v / E * (RS * 4) + v % E * 4), "l"(src + v) : "memory");
+                }
                 for (int v = pt; v < n << per_log; v += RX_PRODUCE) {
                     const int i = v >> per_log, q = v & ((1 << per_log) - 1);
                     if (q < pieces) {
@@ -280,27 +270,19 @@ __global__ void __launch_bounds__(RX_THREADS) router_exact_kernel(const RouterAr
             }
         }
     } else {
-        float* const lg = reinterpret_cast<float*>(rx_smem + ST * stage);
-        float* const ex = lg + TOK * (E + 1);
-        float* const smax = ex + TOK * (E + 1);
-        float* const sinv = smax + TOK;
-        const int ET = (E + TE - 1) / TE, te = tid % ET, tt = tid / ET, TT = TOK / TM;
-        const bool works = tt < TT;
-        int eo[TE];                                     // this thread's experts (past the last: the last again, not stored)
+        const int te = tid % ET, tt = tid / ET, e0 = te * TE;
+        float* const ex = reinterpret_cast<float*>(rx_smem + ST * stage) + (size_t)tt * TM * (RS + 4);
         float bias[TE];
 #pragma unroll
-        for (int j = 0; j < TE; ++j) {
-            eo[j] = WV ? te * TE + j : min(te + j * ET, E - 1);
-            bias[j] = p.br[eo[j]];
-        }
-        auto compute_sync = [] {
-            __syncwarp();
-            asm volatile("bar.sync 1, %0;" ::"n"(RX_COMPUTE) : "memory");
-        };
+        for (int j = 0; j < TE; ++j) bias[j] = e0 + j < E ? p.br[e0 + j] : 0.0f;
         int s = 0;
         uint32_t round = 0;
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
             const int n = min(TOK, n_active - tile * TOK);
+            const bool works = (tid & ~31) / ET < n;        // some lane of this warp has a token
+            uint32_t xr[TM];
+#pragma unroll
+            for (int t = 0; t < TM; ++t) xr[t] = x_off + min(tt + t * GROUPS, p.tok - 1) * x_row;      // (past the end: not stored)
             float acc[TM][TE];
 #pragma unroll
             for (int t = 0; t < TM; ++t)
@@ -310,37 +292,33 @@ __global__ void __launch_bounds__(RX_THREADS) router_exact_kernel(const RouterAr
                 const int len = min(CK, C - c0);
                 wait(full(s), round & 1);
                 if (works) {
-                    const float* ws = reinterpret_cast<const float*>(ring + s * stage);
-                    const uint8_t* xs = ring + s * stage + x_off + tt * x_row;
+                    const uint32_t base = ring0 + s * stage, ws = base + e0 * 4;
+                    // U channels' operands at a time; two sets, the next one on its way
+                    constexpr int U = TE * TM <= 2 ? 16 : 8;
                     struct Ops {
-                        float w[8][TE];
-                        Row8<TIn> x[TM];
+                        float w[U][TE];
+                        Row8<TIn> x[TM][U / 8];
                     };
                     auto load = [&](Ops& o, int c) {
+                        const uint32_t wc = ws + c * (RS * 4);
 #pragma unroll
-                        for (int t = 0; t < TM; ++t) o.x[t].load(xs + t * TT * x_row + c * sizeof(TIn));
+                        for (int t = 0; t < TM; ++t)
 #pragma unroll
-                        for (int u = 0; u < 8; ++u) {
-                            if constexpr (WV) {
-                                const float4 f = *reinterpret_cast<const float4*>(ws + (c + u) * E + eo[0]);
-                                o.w[u][0] = f.x; o.w[u][1] = f.y; o.w[u][2] = f.z; o.w[u][3] = f.w;
-                            } else {
+                            for (int i = 0; i < U / 8; ++i) o.x[t][i].load(base + xr[t] + (c + 8 * i) * sizeof(TIn));
 #pragma unroll
-                                for (int j = 0; j < TE; ++j) o.w[u][j] = ws[(c + u) * E + eo[j]];
-                            }
-                        }
+                        for (int u = 0; u < U; ++u) lds_weights<TE>(o.w[u], wc + u * (RS * 4));
                     };
                     // acc = fadd(acc, fmul(x, w)) in channel order, the reference's order; four channels' products first, so
                     // that no addition waits for its product
                     auto work = [&](const Ops& o) {
 #pragma unroll
-                        for (int h = 0; h < 8; h += 4) {
+                        for (int h = 0; h < U; h += 4) {
                             float pr[4][TM][TE];
 #pragma unroll
                             for (int u = 0; u < 4; ++u)
 #pragma unroll
                                 for (int t = 0; t < TM; ++t) {
-                                    const float xv = o.x[t].get(h + u);
+                                    const float xv = o.x[t][(h + u) / 8].get((h + u) & 7);
 #pragma unroll
                                     for (int j = 0; j < TE; ++j) pr[u][t][j] = __fmul_rn(xv, o.w[h + u][j]);
                                 }
@@ -353,14 +331,32 @@ __global__ void __launch_bounds__(RX_THREADS) router_exact_kernel(const RouterAr
                         }
                     };
                     Ops a, b;
-                    load(a, 0);
-                    for (int c = 0; c + 16 <= len; c += 16) {
-                        load(b, c + 8);
-                        work(a);
-                        load(a, min(c + 16, len - 8));              // (the last one again: no branch)
-                        work(b);
+                    int c = 0;
+                    if (len >= 2 * U) {
+                        load(a, 0);
+#pragma unroll 1
+                        for (; c + 2 * U <= len; c += 2 * U) {
+                            load(b, c + U);
+                            work(a);
+                            load(a, min(c + 2 * U, len - U));       // (the last one again: no branch)
+                            work(b);
+                        }
                     }
-                    if (len & 8) work(a);
+#pragma unroll 1
+                    for (; c < len; c += 8) {                       // the rest of a last chunk, eight channels at a time
+                        float w[8][TE];
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) lds_weights<TE>(w[u], ws + (c + u) * (RS * 4));
+#pragma unroll
+                        for (int t = 0; t < TM; ++t) {
+                            Row8<TIn> x;
+                            x.load(base + xr[t] + c * sizeof(TIn));
+#pragma unroll
+                            for (int u = 0; u < 8; ++u)
+#pragma unroll
+                                for (int j = 0; j < TE; ++j) acc[t][j] = __fadd_rn(acc[t][j], __fmul_rn(x.get(u), w[u][j]));
+                        }
+                    }
                 }
                 __syncwarp();
                 if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty(s)) : "memory");
@@ -369,67 +365,90 @@ __global__ void __launch_bounds__(RX_THREADS) router_exact_kernel(const RouterAr
                     ++round;
                 }
             }
-            if (works)
+            if (!works) continue;
+            // clamped softmax (utils/Tensor.cpp:850-883) and top-k, strict '>' (utils/Tensor.cpp:1296-1334)
+            const unsigned all = 0xffffffffu;
+            float lg[TM][TE], pr[TM][TE];
 #pragma unroll
-                for (int t = 0; t < TM; ++t)
-#pragma unroll
-                    for (int j = 0; j < TE; ++j) {
-                        acc[t][j] = __fadd_rn(acc[t][j], bias[j]);
-                        if (WV || te + j * ET < E) lg[(tt + t * TT) * (E + 1) + eo[j]] = acc[t][j];
-                    }
-            compute_sync();
-            for (int i = tid; i < n; i += RX_COMPUTE) {
+            for (int t = 0; t < TM; ++t) {
                 float mx = -INFINITY;
-#pragma unroll 8
-                for (int e = 0; e < E; ++e) mx = fmaxf(mx, lg[i * (E + 1) + e]);
-                smax[i] = mx;
+#pragma unroll
+                for (int j = 0; j < TE; ++j) {
+                    lg[t][j] = __fadd_rn(acc[t][j], bias[j]);
+                    if (e0 + j < E) mx = fmaxf(mx, lg[t][j]);
+                }
+#pragma unroll
+                for (int o = ET / 2; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(all, mx, o));
+                // exp through double and one rounding: agrees with a correctly rounded expf
+#pragma unroll
+                for (int j = 0; j < TE; ++j) pr[t][j] = e0 + j < E ? (float)exp((double)__fsub_rn(lg[t][j], mx)) : 0.0f;
+#pragma unroll
+                for (int j = 0; j < TE; ++j) ex[t * (RS + 4) + e0 + j] = pr[t][j];
             }
-            compute_sync();
-            // exp through double and one rounding: agrees with a correctly rounded expf
-            if (works)
+            __syncwarp();
+            float sum[TM] = {};
+            for (int e = 0; e < E; e += 4)                          // in index order (zeros past the last: they add nothing)
 #pragma unroll
-                for (int t = 0; t < TM; ++t)
+                for (int t = 0; t < TM; ++t) {
+                    const float4 v = *reinterpret_cast<const float4*>(ex + t * (RS + 4) + e);
+                    sum[t] = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum[t], v.x), v.y), v.z), v.w);
+                }
+            __syncwarp();
 #pragma unroll
-                    for (int j = 0; j < TE; ++j) {
-                        const int i = tt + t * TT;
-                        if (i < n && (WV || te + j * ET < E)) ex[i * (E + 1) + eo[j]] = (float)exp((double)__fsub_rn(acc[t][j], smax[i]));
+            for (int t = 0; t < TM; ++t) {
+                const int i = tt + t * GROUPS;
+                const bool live = i < n;
+                const size_t tok = live ? (p.list ? p.list[tile * TOK + i] : tile * TOK + i) : 0;
+                const float inv = __fdiv_rn(1.0f, fmaxf(sum[t], 1e-15f));
+#pragma unroll
+                for (int j = 0; j < TE; ++j) {
+                    pr[t][j] = fminf(fmaxf(__fmul_rn(pr[t][j], inv), 1e-7f), 1.0f);
+                    if (live && e0 + j < E) {
+                        p.probs[tok * E + e0 + j] = pr[t][j];
+                        if (p.logits) p.logits[tok * E + e0 + j] = lg[t][j];
                     }
-            compute_sync();
-            for (int i = tid; i < n; i += RX_COMPUTE) {
-                const size_t tok = p.list ? p.list[tile * TOK + i] : tile * TOK + i;
-                const float* ei = ex + i * (E + 1);
-                int32_t* ti = p.top_idx + tok * p.k;
-                float* tp = p.top_p + tok * p.k;
-                sinv[i] = p.k <= 1 ? rx_top<1>(ei, E, p.k, ti, tp) : p.k <= 2 ? rx_top<2>(ei, E, p.k, ti, tp)
-                        : p.k <= 4 ? rx_top<4>(ei, E, p.k, ti, tp) : rx_top<8>(ei, E, p.k, ti, tp);
-            }
-            compute_sync();
-            {
-                int i = tid / E, e = tid % E;
-                const int di = RX_COMPUTE / E, de = RX_COMPUTE % E;
-                while (i < n) {
-                    const size_t tok = p.list ? p.list[tile * TOK + i] : tile * TOK + i;
-                    p.probs[tok * E + e] = fminf(fmaxf(__fmul_rn(ex[i * (E + 1) + e], sinv[i]), 1e-7f), 1.0f);
-                    if (p.logits) p.logits[tok * E + e] = lg[i * (E + 1) + e];
-                    i += di;
-                    e += de;
-                    if (e >= E) {
-                        e -= E;
-                        ++i;
+                }
+                // k rounds of (value desc, index asc) arg-max == the reference's stable insertion
+                unsigned taken = 0;
+                for (int r = 0; r < p.k; ++r) {
+                    float bv = -INFINITY;
+                    int bi = 0x7fffffff;
+#pragma unroll
+                    for (int j = 0; j < TE; ++j)
+                        if (e0 + j < E && !(taken >> j & 1u) && pr[t][j] > bv) {
+                            bv = pr[t][j];
+                            bi = e0 + j;
+                        }
+#pragma unroll
+                    for (int o = ET / 2; o > 0; o >>= 1) {
+                        const float ov = __shfl_xor_sync(all, bv, o);
+                        const int oi = __shfl_xor_sync(all, bi, o);
+                        if (ov > bv || (ov == bv && oi < bi)) {
+                            bv = ov;
+                            bi = oi;
+                        }
+                    }
+                    if (bi / TE == te) taken |= 1u << (bi % TE);
+                    if (live && te == 0) {
+                        p.top_idx[tok * p.k + r] = bi;
+                        p.top_p[tok * p.k + r] = bv;
                     }
                 }
             }
-            compute_sync();                             // the tail may be overwritten
         }
     }
     if (!p.plan.top_idx) return;
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) last = atomicAdd(p.done, 1) == (int)gridDim.x - 1;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    if (tid == 0) *p.done = 0;
+    if (gridDim.x > 1) {
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) last = atomicAdd(p.done, 1) == (int)gridDim.x - 1;
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+        if (tid == 0) *p.done = 0;
+    } else {
+        __syncthreads();
+    }
     plan_block<RX_THREADS / 32>(p.plan, *reinterpret_cast<PlanShared*>(rx_smem));
 }
 
@@ -827,21 +846,23 @@ router_wgrad_reduce_kernel(const float* part, const float* partb, int n_chunks, 
     }
 }
 
-template <typename TIn, int TM, int TE, bool WV>
+template <typename TIn, int RS, int TE, int TM>
 int router_exact_launch(RouterArgs p, int device, cudaStream_t st)
 {
-    auto* kernel = router_exact_kernel<TIn, TM, TE, WV>;
-    p.tok = RX_COMPUTE / ((p.E + TE - 1) / TE) * TM;
-    // stages of about 16-40 KiB; one CTA per SM takes what fits, more of them share.  A list's length is only known on the
-    // device.
-    for (p.ck = 128; p.ck > 16 && ((uint32_t)p.ck * p.E * 4 > 16384u || rx_stage(p.ck, p.E, p.tok, sizeof(TIn)) > 40960u);) p.ck /= 2;
-    const int ctas = (p.N + p.tok - 1) / p.tok, grid = p.list ? (ctas < 296 ? ctas : 296) : ctas;
-    const uint32_t stage = rx_stage(p.ck, p.E, p.tok, sizeof(TIn)), tail = rx_tail(p.tok, p.E);
-    const uint32_t budget = (grid <= 148 ? 200 : 104) * 1024u;
-    int stages = (int)((budget - tail) / stage);
+    auto* kernel = router_exact_kernel<TIn, RS, TE, TM>;
+    // every SM its share of the tokens, up to what the compute threads hold at a time (a list's length is only known on the device)
+    constexpr int most = RX_COMPUTE * TE / RS * TM;
+    const int share = (p.N + 147) / 148;
+    p.tok = p.list || share > most ? most : share;
+    // A stage's beginning and end cost 650 cycles (one warp per scheduler hides no instruction fetch), so stages are long: 512
+    // channels with a few tokens, whose loads are all on their way at once, 256 with more; two of them fit.
+    for (p.ck = p.tok <= 4 ? 512 : 256; p.ck > 16 && rx_stage(p.ck, RS, p.tok, sizeof(TIn)) > 90u * 1024u;) p.ck /= 2;
+    const int ctas = (p.N + p.tok - 1) / p.tok, grid = ctas < 148 ? ctas : 148;
+    const uint32_t stage = rx_stage(p.ck, RS, p.tok, sizeof(TIn)), tail = rx_tail(TE, TM, RS);
+    int stages = (int)((200u * 1024u - tail) / stage);
     const int chunks = (p.C + p.ck - 1) / p.ck;
     if (stages > RX_MAX_STAGES) stages = RX_MAX_STAGES;
-    if (grid <= 148 && stages > chunks) stages = chunks;
+    if (ctas <= 148 && stages > chunks) stages = chunks;
     p.stages = stages < 2 ? 2 : stages;
     size_t smem = (size_t)p.stages * stage + tail;
     if (p.plan.top_idx && smem < sizeof(PlanShared)) smem = sizeof(PlanShared);
@@ -855,16 +876,31 @@ int router_exact_launch(RouterArgs p, int device, cudaStream_t st)
     return 0;
 }
 
-// One (token, expert) pair per thread while that leaves no SM more than one CTA, then four, then eight.
+// (Token, expert) pairs per thread: as few as hold an SM's share of the tokens in eight warps, for a channel's step is bound by
+// latency (one pair 7.5 cycles, two 15-18, four 22-30).  Not four experts of one token: shared memory then delivers a
+// step's weights no faster than 1.1 cycles per 32 pairs (two of two tokens 0.83, four of two 0.72, issue alone 0.5).
+template <typename TIn, int RS>
+int router_exact_pick(const RouterArgs& p, int device, cudaStream_t st)
+{
+    constexpr int one = RX_COMPUTE / RS;               // tokens held with one pair per thread
+    const int share = p.list ? 1 << 30 : (p.N + 147) / 148;
+    if constexpr (RS <= 32)
+        if (share <= one) return router_exact_launch<TIn, RS, 1, 1>(p, device, st);
+    if constexpr (RS <= 64) {
+        if (share <= 2 * one) return router_exact_launch<TIn, RS, 2, 1>(p, device, st);
+        if (share <= 4 * one) return router_exact_launch<TIn, RS, 2, 2>(p, device, st);
+    } else {
+        if (share <= 4 * one) return router_exact_launch<TIn, RS, 4, 1>(p, device, st);
+    }
+    return router_exact_launch<TIn, RS, 4, 2>(p, device, st);
+}
 template <typename TIn>
 int router_exact_dispatch(const RouterArgs& p, int device, cudaStream_t st)
 {
-    const long long pairs = (long long)p.N * p.E, wave = 148 * RX_COMPUTE;
-    const bool wv = p.E % 4 == 0;
-    if (!p.list && pairs <= wave) return router_exact_launch<TIn, 1, 1, false>(p, device, st);
-    if (!p.list && pairs <= 4 * wave)
-        return wv ? router_exact_launch<TIn, 1, 4, true>(p, device, st) : router_exact_launch<TIn, 1, 4, false>(p, device, st);
-    return wv ? router_exact_launch<TIn, 2, 4, true>(p, device, st) : router_exact_launch<TIn, 2, 4, false>(p, device, st);
+    if (p.E <= 16) return router_exact_pick<TIn, 16>(p, device, st);
+    if (p.E <= 32) return router_exact_pick<TIn, 32>(p, device, st);
+    if (p.E <= 64) return router_exact_pick<TIn, 64>(p, device, st);
+    return router_exact_pick<TIn, 128>(p, device, st);
 }
 
 template <typename TIn, int EL, int EPL, int TPW>
@@ -876,6 +912,10 @@ int router_any_launch(const RouterArgs& p, cudaStream_t st)
     MGPT_LAUNCHED("router_fwd_kernel");
     return 0;
 }
+
+// Routed rows up to which the router's last block builds the plan (with 512 or 1024 the plan's own kernel, which starts while the
+// router drains, is as fast: 256 tokens, top-2, 116.4 against 116.7 us for the call).
+constexpr int ROUTER_PLAN_ROWS = 256;
 
 template <typename TIn>
 int router_fwd_dispatch(const RouterArgs& p, int device, bool fast, cudaStream_t st)
@@ -901,7 +941,7 @@ int launch_router_fwd(const void* x, int io, const float* Wr, const float* br, i
     p.logits = logits; p.probs = probs; p.top_idx = top_idx; p.top_p = top_p;
     p.list = list; p.list_count = list_count; p.status = status;
     const bool fast = C % 8 == 0 && (((uintptr_t)x | (uintptr_t)Wr) & 15) == 0;
-    if (fast && plan && plan->R <= 256) {      // (more rows: six warps take longer than the plan's own kernel and its launch)
+    if (fast && plan && plan->R <= ROUTER_PLAN_ROWS) {
         p.plan = *plan;
         p.done = done;
         *planned = true;
