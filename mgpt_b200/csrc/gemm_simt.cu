@@ -6,7 +6,7 @@
 // (layers/MoELayer.cpp:94-118, 159-181; layers/SwiGLU.cpp:23-50, 57-96;
 // layers/LinearLayer.cpp:36-80) but grouped: one launch covers every expert,
 // reading the row tiles and the tile->expert table built by the plan.
-#include "common.cuh"
+#include "tc_common.cuh"
 
 namespace mgpt {
 
@@ -134,6 +134,30 @@ __device__ __forceinline__ void fold(float* S, int group, int t, float (&acc)[8]
     }
 }
 
+// The sums of the CTAs of a cluster that share a tile's k loop, added to the first CTA's in rank order through distributed shared
+// memory.  S: shared memory of 64*64 floats; `adds`: this thread holds sums (group 0).
+__device__ __forceinline__ void fold_cluster(float* S, int ctas, int rank, bool adds, int t, float (&acc)[8][4])
+{
+    float4* mine = reinterpret_cast<float4*>(S);
+    __syncthreads();                          // what S held has been read
+    if (rank > 0 && adds)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) mine[i * GT + t] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    tcx::cluster_sync();
+    if (rank == 0 && adds)
+        for (int r = 1; r < ctas; ++r) {
+            const uint32_t peer = tcx::mapa((uint32_t)__cvta_generic_to_shared(S), r);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                float4 v;
+                asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                             : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(peer + (i * GT + t) * 16) : "memory");
+                acc[i][0] += v.x; acc[i][1] += v.y; acc[i][2] += v.z; acc[i][3] += v.w;
+            }
+        }
+    tcx::cluster_sync();                      // nobody leaves, or writes S again, while it is being read
+}
+
 enum { EPI_GATEUP = 0, EPI_DOWN = 1, EPI_DHH = 2, EPI_DXG = 3 };
 
 struct RowsArgs {
@@ -147,6 +171,7 @@ struct RowsArgs {
     // reads them: the weight gradients below stop at the last real row).  Null where rows come in segments.
     const int32_t* counts; const int32_t* padded_offsets;
     int K, Nout;
+    int ctas;                                  // CTAs of a cluster that share a tile's k loop
 };
 
 template <int EPI, int KS> constexpr size_t rows_smem()
@@ -157,14 +182,16 @@ template <int EPI, int KS> constexpr size_t rows_smem()
 }
 
 // VEC: weights and their gradients, AVEC: rows, start on boundaries of four elements.
-template <typename TAct, typename TW, int EPI, int KS, bool VEC, bool AVEC>
+// CL: a cluster of a.ctas CTAs per tile.
+template <typename TAct, typename TW, int EPI, int KS, bool VEC, bool AVEC, bool CL>
 __global__ void __launch_bounds__(GT * KS) simt_rows_kernel(RowsArgs a)
 {
     extern __shared__ __align__(16) float sm[];
     pdl_wait();
     constexpr bool BK_MAJOR = EPI == EPI_DHH || EPI == EPI_DXG;      // B(k, n) at n*K + k
     constexpr int NOP = EPI == EPI_GATEUP ? 3 : 2;
-    const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
+    const int ctas = CL ? a.ctas : 1, rank = CL ? (int)tcx::cluster_ctarank() : 0;
+    const int m0 = (int)blockIdx.x / ctas * TM, n0 = blockIdx.y * TN;
     const int rows = *a.n_tiles * ROW_TILE;
     if (m0 >= rows) return;
     const int e = a.tile_expert[m0 / ROW_TILE];
@@ -176,7 +203,8 @@ __global__ void __launch_bounds__(GT * KS) simt_rows_kernel(RowsArgs a)
     float acc[8][4] = {}, acc2[8][4] = {};
     // this group's steps of TK; EPI_DXG runs through dG*Wg^T and then dU*Wu^T
     const int per = (K + TK - 1) / TK, steps = EPI == EPI_DXG ? 2 * per : per;
-    const int s0 = (int)((long)steps * group / KS), s1 = (int)((long)steps * (group + 1) / KS);
+    const int part = rank * KS + group, parts = KS * ctas;
+    const int s0 = (int)((long)steps * part / parts), s1 = (int)((long)steps * (part + 1) / parts);
     const TW *B1 = (const TW*)a.B[e], *B2 = NOP == 3 || EPI == EPI_DXG ? (const TW*)a.B2[e] : nullptr;
     float4 ra[2], rb[2], rc[2];
     auto gload = [&](int s) {
@@ -208,8 +236,12 @@ __global__ void __launch_bounds__(GT * KS) simt_rows_kernel(RowsArgs a)
     }
     fold<KS>(sm, group, t, acc);
     if (NOP == 3) fold<KS>(sm + (KS - 1) * TM * TN, group, t, acc2);
+    if constexpr (CL) {
+        fold_cluster(sm, ctas, rank, group == 0, t, acc);
+        if (NOP == 3) fold_cluster(sm, ctas, rank, group == 0, t, acc2);
+    }
     const int n = n0 + tx * 4;
-    if (group > 0 || n >= N) return;
+    if (rank > 0 || group > 0 || n >= N) return;
     float b1[4] = {}, b2[4] = {};
     if (EPI == EPI_GATEUP || EPI == EPI_DOWN)
 #pragma unroll
@@ -369,6 +401,17 @@ int split_k(int tiles, int k)
     return ks;
 }
 
+// CTAs per tile where four groups each leave SMs without one: a cluster of two, four or eight, no group with less than two steps.
+// Stage times without -> with, us: 1024 tokens, C=128, H=512, E=8, top-2 (two CTAs) down 23 -> 19, dXg 37 -> 27, the step 149 ->
+// 135; 64 tokens, C=256, H=1024 (four) 35 -> 20 and 66 -> 29, the step 172 -> 120; 256 tokens, C=256, H=1024, E=16, top-1 234
+// -> 203.
+int split_ctas(int tiles, int k)
+{
+    int ctas = 1;
+    while (ctas < 8 && tiles * ctas * 2 <= 148 && k >= ctas * 2 * 4 * 2 * TK) ctas *= 2;
+    return ctas;
+}
+
 // The row buffers of an expert side are the caller's, at any address; those in the workspace are aligned.
 template <typename TAct> bool rows_aligned(const mgpt_moe_layer* L)
 {
@@ -376,27 +419,31 @@ template <typename TAct> bool rows_aligned(const mgpt_moe_layer* L)
     return (any & (4 * sizeof(TAct) - 1)) == 0;
 }
 
-template <typename TAct, typename TW, int EPI, int KS>
+template <typename TAct, typename TW, int EPI, int KS, bool CL>
 int launch_rows_ks(const mgpt_moe_layer* L, const RowsArgs& a, dim3 grid, cudaStream_t st)
 {
     constexpr size_t smem = rows_smem<EPI, KS>();
-    auto* kernel = !rows_aligned<TAct>(L) ? simt_rows_kernel<TAct, TW, EPI, KS, false, false>
-                   : L->masters_aligned   ? simt_rows_kernel<TAct, TW, EPI, KS, true, true>
-                                          : simt_rows_kernel<TAct, TW, EPI, KS, false, true>;
+    auto* kernel = !rows_aligned<TAct>(L) ? simt_rows_kernel<TAct, TW, EPI, KS, false, false, CL>
+                   : L->masters_aligned   ? simt_rows_kernel<TAct, TW, EPI, KS, true, true, CL>
+                                          : simt_rows_kernel<TAct, TW, EPI, KS, false, true, CL>;
     if (smem > 48 * 1024) MGPT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    MGPT_CUDA(launch_pdl(kernel, grid, GT * KS, smem, st, a));
+    if (CL) MGPT_CUDA(launch_pdl_cluster(kernel, grid, a.ctas, GT * KS, smem, st, a));
+    else MGPT_CUDA(launch_pdl(kernel, grid, GT * KS, smem, st, a));
     return 0;
 }
 template <typename TAct, typename TW, int EPI>
-int launch_rows(const mgpt_moe_layer* L, const Workspace& w, const RowsArgs& a, cudaStream_t st, const char* what)
+int launch_rows(const mgpt_moe_layer* L, const Workspace& w, RowsArgs a, cudaStream_t st, const char* what)
 {
     const int cols = (a.Nout + TN - 1) / TN;
     // tiles with real rows: about R/64 and half a tile per expert
-    const int ks = split_k((w.R / TM + (L->d.E + 1) / 2) * cols, EPI == EPI_DXG ? 2 * a.K : a.K);
-    const dim3 grid(w.row_cap / TM, cols);
-    if (ks == 4) MGPT_TRY((launch_rows_ks<TAct, TW, EPI, 4>(L, a, grid, st)));
-    else if (ks == 2) MGPT_TRY((launch_rows_ks<TAct, TW, EPI, 2>(L, a, grid, st)));
-    else MGPT_TRY((launch_rows_ks<TAct, TW, EPI, 1>(L, a, grid, st)));
+    const int tiles = (w.R / TM + (L->d.E + 1) / 2) * cols, k = EPI == EPI_DXG ? 2 * a.K : a.K;
+    const int ks = split_k(tiles, k);
+    a.ctas = ks == 4 ? split_ctas(tiles, k) : 1;
+    const dim3 grid(w.row_cap / TM * a.ctas, cols);
+    if (a.ctas > 1) MGPT_TRY((launch_rows_ks<TAct, TW, EPI, 4, true>(L, a, grid, st)));
+    else if (ks == 4) MGPT_TRY((launch_rows_ks<TAct, TW, EPI, 4, false>(L, a, grid, st)));
+    else if (ks == 2) MGPT_TRY((launch_rows_ks<TAct, TW, EPI, 2, false>(L, a, grid, st)));
+    else MGPT_TRY((launch_rows_ks<TAct, TW, EPI, 1, false>(L, a, grid, st)));
     MGPT_LAUNCHED(what);
     return 0;
 }

@@ -1,0 +1,38 @@
+"""FP32 products whose k loop several CTAs of a cluster share: two, four and eight of them, ends of rows, columns and k inside a
+tile, parameters off 16-byte boundaries."""
+import pytest
+import torch
+
+from mgpt_b200 import MoELayer, synth
+from oracle import oracle
+from tests.util import assert_routing_exact, assert_values, dims_of, rel_l2, run_layer
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,C,H,E,k", [
+    (30, 64, 1032, 2, 2),       # one tile of columns: eight CTAs
+    (64, 264, 1024, 8, 2),      # four; C ends inside a tile
+    (500, 128, 520, 8, 2),      # two in dXg; the shortest k that is shared
+])
+def test_shared_k_loops(n, C, H, E, k):
+    w = synth.Workload("clusters", n, C, H, E, k, "fp32")
+    x, params, dy = synth.make_inputs(w, seed=n + C, bias_std=0.02)
+    ref = oracle.run(dims_of(w), x, params, dy, threads=8)
+    got = run_layer(w, x, params, dy, mode="fp32")
+    assert_routing_exact(got, ref)
+    assert_values(got, ref, 1e-5, w)
+
+    # the same from parameters that allow single accesses only: the same sums in the same order
+    layer = MoELayer(C, H, E, k, mode="fp32", lb_alpha=w.alpha)
+    layer.params = [torch.empty(p.numel() + 1, device="cuda")[1:].view(p.shape) for p in layer.params]
+    for p in layer.params:
+        p.grad = torch.zeros(p.numel() + 1, device="cuda")[1:].view(p.shape)
+    layer._bind()
+    layer.load_parameters(params)
+    y = layer.forward(torch.from_numpy(x).cuda())
+    dx = layer.backward(torch.from_numpy(dy).cuda())
+    layer.check_status()
+    assert rel_l2(y.cpu().numpy(), got["y"]) <= 1e-6 and rel_l2(dx.cpu().numpy(), got["dx"]) <= 1e-6
+    layer.close()
+    got["layer"].close()
