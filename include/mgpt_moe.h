@@ -273,7 +273,8 @@ int  mgpt_moe_selftest_bounded_wait(mgpt_moe_layer* layer, mgpt_stream_t stream)
 int  mgpt_moe_set_weight_grad_overwrite(mgpt_moe_layer* layer, int enabled);
 
 /* Upper bound on the CTAs of the persistent tensor-core kernels of this layer
- * (one CTA per SM; 0 = every SM, the default). A caller that overlaps these
+ * (one CTA per SM; 0 = every SM, the default; the weight gradients of many rows per expert
+ * run on pairs of CTAs and leave one of an odd number free). A caller that overlaps these
  * kernels with communication kernels on another stream leaves SMs free for
  * them this way; results do not depend on the value. No reference counterpart. */
 int  mgpt_moe_set_sm_budget(mgpt_moe_layer* layer, int n_sms);

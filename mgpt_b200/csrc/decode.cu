@@ -245,7 +245,8 @@ int launch_phase(const DecP& p, int sms, cudaStream_t st)
 // weight bytes times rows.  These kernels save about 15 us of a call (no dispatch where nothing is kept, no first tile to
 // wait for) and lose the more, the more weights stream by and the more rows meet each of them (B fragments and MMAs per
 // weight, and a crowded expert's weights again for every 16 rows).  Inference calls, us with tiles / with these kernels, L2
-// flushed (training steps at the same sizes: up to 11 % faster where few tiles decide, within 3 % of each other elsewhere):
+// flushed (training steps at the same sizes: up to 11 % faster where few tiles decide, within 3 % of each other elsewhere;
+// measured before the tiles' products requested their first weights early, which took 3-4 us off their calls):
 //   tokens                           1        8       16        32        64       128
 //   C=1024 H=2816 E=32 top-2     66/46    90/77  121/116   137/136   141/144   145/159
 //     a few experts take most    66/46    68/48    68/50     68/56     72/69    74/108
