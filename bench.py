@@ -30,10 +30,10 @@ METRIC = "moe_layer_fwd_bwd_tokens_per_sec"
 TRAFFIC = {
     ("c3", "wgrad_gemm"): 822.7e6, ("c3", "gateup_gemm"): 338.8e6, ("c3", "dhh_gemm"): 396.5e6,
     ("c3", "down_gemm"): 176.1e6, ("c3", "dxg_gemm"): 281.1e6,
-    ("c4q", "wgrad_gemm"): 1410.0e6, ("c4q", "gateup_gemm"): 369.5e6, ("c4q", "dhh_gemm"): 343.0e6,
-    ("c4q", "down_gemm"): 184.7e6, ("c4q", "dxg_gemm"): 335.5e6,
-    ("c4", "wgrad_gemm"): 4 * 1410.0e6, ("c4", "gateup_gemm"): 4 * 369.5e6, ("c4", "dhh_gemm"): 4 * 343.0e6,
-    ("c4", "down_gemm"): 4 * 184.7e6, ("c4", "dxg_gemm"): 4 * 335.5e6,
+    ("c4q", "wgrad_gemm"): 1336.1e6, ("c4q", "gateup_gemm"): 370.7e6, ("c4q", "dhh_gemm"): 331.3e6,
+    ("c4q", "down_gemm"): 184.4e6, ("c4q", "dxg_gemm"): 334.4e6,
+    ("c4", "wgrad_gemm"): 4 * 1336.1e6, ("c4", "gateup_gemm"): 4 * 370.7e6, ("c4", "dhh_gemm"): 4 * 331.3e6,
+    ("c4", "down_gemm"): 4 * 184.4e6, ("c4", "dxg_gemm"): 4 * 334.4e6,
 }
 UNIT = "tokens/s"
 
