@@ -25,6 +25,7 @@ if ROOT not in sys.path:
 
 METRIC = "moe_layer_fwd_bwd_tokens_per_sec"
 # DRAM bytes (read + write) per launch from ncu captures, keyed by (workload, stage); see profiles/.
+# c3's are from before the weight gradients' CTA pairs.
 # c4 is too large to capture with many passes: its figures are those of c4q (a quarter of the tokens and of the
 # experts, same rows per expert) times four -- every term of the traffic is proportional to the number of experts.
 TRAFFIC = {
