@@ -76,8 +76,8 @@ inline int check_aligned(const void* p, const char* what, uintptr_t bytes = 16)
 // addresses) while that kernel's writes are still being flushed, and wait in pdl_wait() until all of it has finished
 // and is visible.  EVERY block of EVERY kernel launched this way goes through pdl_wait(), also one that has nothing to do: "the kernel
 // before has finished" then implies the same for all kernels before that one.  Takes the ~2 us between two kernels of
-// a step to ~1 us.  A kernel whose successor can request weights meanwhile (dispatch and gate/up: the next product's first)
-// releases it early (pdl_release), after its own wait: what an earlier kernel wrote -- the plan, the weights -- is complete by
+// a step to ~1 us.  A kernel whose successor can request weights meanwhile (dispatch and, without an SM budget, gate/up: the next
+// product's first) releases it early (pdl_release), after its own wait: what an earlier kernel wrote -- the plan, the weights -- is complete by
 // then, so that the successor may read it before it waits.  With an early release at the top of every kernel the waiting
 // blocks pile up several kernels deep and spread the next kernel's blocks unevenly over the SMs (a 256-token decode call:
 // 155 us without any of this, 144 us with the wait alone, 194 us with that).

@@ -44,6 +44,7 @@ struct DecP {
     const bf16* A;                     // down: Hh
     bf16 *out, *G, *U;
     int C, H, k, hb, cb, kb1, kb2;
+    int release;                       // phase 1: let phase 2's blocks in early
 };
 
 __device__ __forceinline__ uint4 ld_weights(const bf16* p)
@@ -126,11 +127,11 @@ __global__ void __launch_bounds__(32 * DW, 1) decode_kernel(const DecP p)
     constexpr int ROWS = PHASE == 1 ? 8 : 16;              // weight rows (of each matrix) per task
     const int per = (width + ROWS - 1) / ROWS, blocks = PHASE == 1 ? p.hb : p.cb;
     const int k0 = kbs * ks / KS, k1 = kbs * (ks + 1) / KS;
-    // Phase 1 lets phase 2's blocks in as SMs run out of work: those request their first weights and wait.  (They may
+    // Without an SM budget phase 1 lets phase 2's blocks in as SMs run out of work: those request their first weights and wait.  (They may
     // read the plan before they wait: it was complete before phase 1 came this far.)
     if (PHASE == 1) {
         pdl_wait();
-        pdl_release();
+        if (p.release) pdl_release();
     }
     const int total = __ldcg(p.n_groups) * per;
     bool waited = PHASE == 1;
@@ -282,7 +283,11 @@ int launch_decode_forward(mgpt_moe_layer* L, const Workspace& w, char* ws, const
     p.hb = (d.H + 127) / 128; p.cb = (d.C + 127) / 128; p.kb1 = (d.C + 63) / 64; p.kb2 = (d.H + 63) / 64;
     int sms = 0;
     MGPT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, L->device));
-    if (L->sm_budget > 0 && L->sm_budget < sms) sms = L->sm_budget;
+    p.release = 1;
+    if (L->sm_budget > 0 && L->sm_budget < sms) {
+        sms = L->sm_budget;
+        p.release = 0;
+    }
     p.x = from_rows ? (const void*)(ws + w.Xg) : x;
     p.row_src = from_rows ? nullptr : (const int32_t*)(ws + w.row_src);
     p.out = (bf16*)(ws + w.Hh);

@@ -272,6 +272,7 @@ struct RowsP {
     int n_out;              // output columns (H or C)
     int n_col_tiles;        // column tiles per row tile
     int early;              // plan and weights were complete before the kernel before this one on the stream went past its pdl_wait
+    int release;            // MODE_GATEUP: let the next kernel's CTAs in early
     bf16 *G, *U;            // P and Q (see the gate/up epilogue) in the blocked layout (written by MODE_GATEUP, read by MODE_DHH)
     const float* const* bias0;
     const float* const* bias1;
@@ -636,7 +637,7 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
     // The setup above overlaps the end of the kernel before, and so do the producer's first loads of weights.
     if (warp > 0) {
         pdl_wait();
-        if (MODE == MODE_GATEUP) pdl_release();
+        if (MODE == MODE_GATEUP && p.release) pdl_release();
     }
 
     auto consume = [&](uint32_t n, RowsItem& w) -> bool {
@@ -687,7 +688,7 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
                     }
             }
             pdl_wait();
-            if (MODE == MODE_GATEUP) pdl_release();
+            if (MODE == MODE_GATEUP && p.release) pdl_release();
             if (!p.early) {
                 total_items = *p.n_tiles * p.n_col_tiles;
                 decode(blockIdx.x);
@@ -1798,6 +1799,8 @@ int tc_experts_forward(mgpt_moe_layer* L, const Workspace& w, char* ws, cudaStre
     p.b_row_blocks = cdiv(d.H, 128); p.b_col_blocks = cdiv(d.C, BK);
     p.bias0 = L->master.bg; p.bias1 = L->master.bu;
     p.early = L->ext_Xg == nullptr;                     // behind dispatch (an expert side's tiles are the kernel's before)
+    // Under an SM budget down's CTAs, an SM each, would wait on the very SMs that the caller keeps free.
+    p.release = grid_sms(L, s) == s->sms;
     p.G = w.inference ? nullptr : (bf16*)(ws + w.G);
     p.U = w.inference ? nullptr : (bf16*)(ws + w.U);
     L->stage_begin(ST_GATEUP, st);
