@@ -115,9 +115,9 @@ __device__ __forceinline__ void router_finish(const float (&acc)[TPW][EPL], cons
 // The exact router.  What bounds it at scale is FP32 issue (one multiply and one add per token, expert and channel) and
 // for small batches the addition chain of one (token, expert) pair, C additions of four cycles.
 //
-// RS: experts rounded up to 16, 32, 64 or 128, the row length of the staged Wr, so that a thread's operands lie at constant
-// offsets; ET = RS / TE lanes of one warp share a token, each with TE neighbouring experts of TM tokens, and read the next
-// operands while they work on these.  Wr and the tokens' rows stream through a ring that four warps fill with cp.async (one
+// ET lanes of one warp share a token, each with TE neighbouring experts of up to TM tokens (rows tt, tt + 256 / ET, ...: a
+// warp works on the rows that it has tokens for), and read the next operands while they work on these.  RS = ET * TE, the
+// experts rounded up, is the row length of the staged Wr, so that a thread's operands lie at constant offsets.  Wr and the tokens' rows stream through a ring that four warps fill with cp.async (one
 // bulk copy per stage cost its issuing thread ~500 cycles, more than a small batch spends on the stage); the eight
 // compute warps never wait for each other.  Softmax and top-k stay with the lanes that hold the logits: maximum and
 // arg-max by shuffles, the sum -- sequential in the reference -- by every lane of the token from shared memory.  With
@@ -128,6 +128,11 @@ __device__ __forceinline__ void router_finish(const float (&acc)[TPW][EPL], cons
 // 17000.  Stage times before -> now, us: 1 token, C=1024, E=32, with the plan 22.4 -> 16.2; 64 tokens 28.7 -> 18.5; 256 tokens,
 // without, 18.6 -> 15; 1777 tokens 26.4 -> 22.6; 5003 FP32 tokens, C=512, E=16 28.5 -> 20.7; both passes of the screened
 // router, 16384 skewed tokens, C=1024, E=64, 91 -> 79.
+//
+// With RS a power of two from 16 on, numbers of experts between two of them paid for up to twice theirs, and rows of Wr off 16-byte
+// boundaries were copied with two divisions per element: slower than the kernel of 128 threads.  FP32 tokens, C=512, us, that
+// kernel / RS a power of two / now: 8 experts 32851 tokens 38 / 47 / 35; 24 experts 5619 tokens 18 / 21 / 16; 31 experts 291 tokens
+// 8.9 / 11.8 / 6.4; 48 experts 5619 tokens 25 / 38 / 21; 80 experts 32851 tokens 265 / 266 / 163; 127 experts 504 / 572 / 235.
 struct RouterArgs {
     const void* x;
     const float *Wr, *br;
@@ -142,13 +147,14 @@ struct RouterArgs {
     PlanArgs plan;
 };
 
+constexpr int pow2_from(int n) { return n <= 1 ? 1 : 2 * pow2_from((n + 1) / 2); }
 constexpr int RX_COMPUTE = 256, RX_PRODUCE = 128, RX_THREADS = RX_COMPUTE + RX_PRODUCE, RX_MAX_STAGES = 16;
 __host__ __device__ inline uint32_t rx_x_row(int ck, int elt) { return (uint32_t)(ck * elt + 16); }      // padded: rows in distinct banks
 __host__ __device__ inline uint32_t rx_stage(int ck, int rs, int tok, int elt)
 {
     return ((uint32_t)ck * rs * 4 + tok * rx_x_row(ck, elt) + 127u) & ~127u;
 }
-constexpr uint32_t rx_tail(int te, int tm, int rs) { return (uint32_t)(RX_COMPUTE * te / rs) * tm * (rs + 4) * 4; }      // exponentials, a row per token
+constexpr uint32_t rx_tail(int et, int te, int tm) { return (uint32_t)(RX_COMPUTE / et) * tm * (et * te + 4) * 4; }      // exponentials, a row per token
 
 // Loads with a 32-bit shared address: through pointers into the ring the compiler lost the address space, and a channel of one
 // pair took 13 cycles instead of 8.
@@ -162,28 +168,34 @@ template <int TE> __device__ __forceinline__ void lds_weights(float (&w)[TE], ui
 {
     if constexpr (TE == 4)
         asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(w[0]), "=f"(w[1]), "=f"(w[2]), "=f"(w[3]) : "r"(a));
-    else if constexpr (TE == 2)
-        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(w[0]), "=f"(w[1]) : "r"(a));
+    else if constexpr (TE % 2 == 0)
+#pragma unroll
+        for (int j = 0; j < TE; j += 2) asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(w[j]), "=f"(w[j + 1]) : "r"(a + 4 * j));
     else
-        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(w[0]) : "r"(a));
+#pragma unroll
+        for (int j = 0; j < TE; ++j) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(w[j]) : "r"(a + 4 * j));
 }
-// 8 consecutive channels of a staged row
-template <typename TIn> struct Row8;
-template <> struct Row8<bf16> {
-    uint4 u;
-    __device__ __forceinline__ void load(uint32_t a) { u = lds128(a); }
-    __device__ __forceinline__ float get(int i) const
-    {
-        const uint32_t w = i < 2 ? u.x : i < 4 ? u.y : i < 6 ? u.z : u.w;
-        return __uint_as_float((i & 1) ? w & 0xffff0000u : w << 16);
-    }
-};
-template <> struct Row8<float> {
-    uint4 u[2];
+// L consecutive channels (4 or 8) of a staged row
+template <typename TIn, int L> struct Row;
+template <int L> struct Row<bf16, L> {
+    uint32_t u[L / 2];
     __device__ __forceinline__ void load(uint32_t a)
     {
-        u[0] = lds128(a);
-        u[1] = lds128(a + 16);
+        if constexpr (L == 8) {
+            const uint4 v = lds128(a);
+            u[0] = v.x; u[1] = v.y; u[2] = v.z; u[3] = v.w;
+        } else {
+            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(u[0]), "=r"(u[1]) : "r"(a));
+        }
+    }
+    __device__ __forceinline__ float get(int i) const { return __uint_as_float((i & 1) ? u[i >> 1] & 0xffff0000u : u[i >> 1] << 16); }
+};
+template <int L> struct Row<float, L> {
+    uint4 u[L / 4];
+    __device__ __forceinline__ void load(uint32_t a)
+    {
+#pragma unroll
+        for (int i = 0; i < L / 4; ++i) u[i] = lds128(a + 16 * i);
     }
     __device__ __forceinline__ float get(int i) const
     {
@@ -192,14 +204,15 @@ template <> struct Row8<float> {
     }
 };
 
-template <typename TIn, int RS, int TE, int TM>
+template <typename TIn, int ET, int TE, int TM>
 __global__ void __launch_bounds__(RX_THREADS, 1) router_exact_kernel(const RouterArgs p)
 {
     extern __shared__ __align__(128) uint8_t rx_smem[];
     __shared__ __align__(8) uint64_t bars[2 * RX_MAX_STAGES];
     __shared__ int last;
-    constexpr int ET = RS / TE, GROUPS = RX_COMPUTE / ET;
-    static_assert(ET <= 32, "a token's lanes lie in one warp");
+    constexpr int RS = ET * TE, GROUPS = RX_COMPUTE / ET;
+    static_assert(TM >= 1 && TM <= 4, "rows of a warp");
+    static_assert((ET & (ET - 1)) == 0 && ET <= 32 && RS % 4 == 0, "a token's lanes lie in one warp");
     const int tid = threadIdx.x, lane = tid & 31;
     const int C = p.C, E = p.E, CK = p.ck, ST = p.stages;
     const uint32_t x_row = rx_x_row(CK, sizeof(TIn)), x_off = (uint32_t)CK * RS * 4, stage = rx_stage(CK, RS, p.tok, sizeof(TIn));
@@ -242,17 +255,22 @@ __global__ void __launch_bounds__(RX_THREADS, 1) router_exact_kernel(const Route
                 const int len = min(CK, C - c0), pieces = len / XV;
                 const uint32_t dst = ring0 + s * stage;
                 const float* src = p.Wr + (size_t)c0 * E;
+                // (a row of Wr is shorter than the staged one: some threads have nothing to copy, and none divides)
                 if (E == RS) {
                     for (int v = pt; v < len * (RS / 4); v += RX_PRODUCE)
                         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + v * 16), "l"(src + v * 4) : "memory");
                 } else if ((E & 3) == 0) {
-                    const int per = E / 4;
-                    for (int v = pt; v < len * per; v += RX_PRODUCE)
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
-                                     ::"r"(dst + v / per * (RS * 4) + v % per * 16), "l"(src + v * 4) : "memory");
+                    constexpr int P = pow2_from(RS / 4);
+                    const int q = pt % P * 4;
+                    if (q < E)
+                        for (int r = pt / P; r < len; r += RX_PRODUCE / P)
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (r * RS + q) * 4), "l"(src + r * E + q) : "memory");
                 } else {
-                    for (int v = pt; v < len * E; v += RX_PRODUCE)
-                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + v / E * (RS * 4) + v % E * 4), "l"(src + v) : "memory");
+                    constexpr int P = pow2_from(RS);
+                    const int q = pt % P;
+                    if (q < E)
+                        for (int r = pt / P; r < len; r += RX_PRODUCE / P)
+                            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + (r * RS + q) * 4), "l"(src + r * E + q) : "memory");
                 }
                 for (int v = pt; v < n << per_log; v += RX_PRODUCE) {
                     const int i = v >> per_log, q = v & ((1 << per_log) - 1);
@@ -277,15 +295,15 @@ __global__ void __launch_bounds__(RX_THREADS, 1) router_exact_kernel(const Route
         for (int j = 0; j < TE; ++j) bias[j] = e0 + j < E ? p.br[e0 + j] : 0.0f;
         int s = 0;
         uint32_t round = 0;
-        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-            const int n = min(TOK, n_active - tile * TOK);
-            const bool works = (tid & ~31) / ET < n;        // some lane of this warp has a token
-            uint32_t xr[TM];
+        // one tile of n tokens, of which this warp has R rows (tt, tt + GROUPS, ...), or none
+        auto work_tile = [&](auto rows, bool works, int tile, int n) {
+            constexpr int R = decltype(rows)::value;
+            uint32_t xr[R];
 #pragma unroll
-            for (int t = 0; t < TM; ++t) xr[t] = x_off + min(tt + t * GROUPS, p.tok - 1) * x_row;      // (past the end: not stored)
-            float acc[TM][TE];
+            for (int t = 0; t < R; ++t) xr[t] = x_off + min(tt + t * GROUPS, p.tok - 1) * x_row;      // (past the end: not stored)
+            float acc[R][TE];
 #pragma unroll
-            for (int t = 0; t < TM; ++t)
+            for (int t = 0; t < R; ++t)
 #pragma unroll
                 for (int j = 0; j < TE; ++j) acc[t][j] = 0.0f;
             for (int c0 = 0; c0 < C; c0 += CK) {
@@ -293,18 +311,19 @@ __global__ void __launch_bounds__(RX_THREADS, 1) router_exact_kernel(const Route
                 wait(full(s), round & 1);
                 if (works) {
                     const uint32_t base = ring0 + s * stage, ws = base + e0 * 4;
-                    // U channels' operands at a time; two sets, the next one on its way
-                    constexpr int U = TE * TM <= 2 ? 16 : 8;
+                    // U channels' operands at a time; two sets, the next one on its way.  (More pairs need fewer channels to hide a
+                    // load behind, and longer sets cost them registers: 16 x 3 x 4 BF16 tokens 57 -> 50 us with 4.)
+                    constexpr int U = TE * R <= 2 ? 16 : TE * R <= (sizeof(TIn) == 2 ? 8 : 4) ? 8 : 4, L = U < 8 ? U : 8;
                     struct Ops {
                         float w[U][TE];
-                        Row8<TIn> x[TM][U / 8];
+                        Row<TIn, L> x[R][U / L];
                     };
                     auto load = [&](Ops& o, int c) {
                         const uint32_t wc = ws + c * (RS * 4);
 #pragma unroll
-                        for (int t = 0; t < TM; ++t)
+                        for (int t = 0; t < R; ++t)
 #pragma unroll
-                            for (int i = 0; i < U / 8; ++i) o.x[t][i].load(base + xr[t] + (c + 8 * i) * sizeof(TIn));
+                            for (int i = 0; i < U / L; ++i) o.x[t][i].load(base + xr[t] + (c + L * i) * sizeof(TIn));
 #pragma unroll
                         for (int u = 0; u < U; ++u) lds_weights<TE>(o.w[u], wc + u * (RS * 4));
                     };
@@ -313,19 +332,19 @@ __global__ void __launch_bounds__(RX_THREADS, 1) router_exact_kernel(const Route
                     auto work = [&](const Ops& o) {
 #pragma unroll
                         for (int h = 0; h < U; h += 4) {
-                            float pr[4][TM][TE];
+                            float pr[4][R][TE];
 #pragma unroll
                             for (int u = 0; u < 4; ++u)
 #pragma unroll
-                                for (int t = 0; t < TM; ++t) {
-                                    const float xv = o.x[t][(h + u) / 8].get((h + u) & 7);
+                                for (int t = 0; t < R; ++t) {
+                                    const float xv = o.x[t][(h + u) / L].get((h + u) % L);
 #pragma unroll
                                     for (int j = 0; j < TE; ++j) pr[u][t][j] = __fmul_rn(xv, o.w[h + u][j]);
                                 }
 #pragma unroll
                             for (int u = 0; u < 4; ++u)
 #pragma unroll
-                                for (int t = 0; t < TM; ++t)
+                                for (int t = 0; t < R; ++t)
 #pragma unroll
                                     for (int j = 0; j < TE; ++j) acc[t][j] = __fadd_rn(acc[t][j], pr[u][t][j]);
                         }
@@ -348,8 +367,8 @@ __global__ void __launch_bounds__(RX_THREADS, 1) router_exact_kernel(const Route
 #pragma unroll
                         for (int u = 0; u < 8; ++u) lds_weights<TE>(w[u], ws + (c + u) * (RS * 4));
 #pragma unroll
-                        for (int t = 0; t < TM; ++t) {
-                            Row8<TIn> x;
+                        for (int t = 0; t < R; ++t) {
+                            Row<TIn, 8> x;
                             x.load(base + xr[t] + c * sizeof(TIn));
 #pragma unroll
                             for (int u = 0; u < 8; ++u)
@@ -365,76 +384,85 @@ __global__ void __launch_bounds__(RX_THREADS, 1) router_exact_kernel(const Route
                     ++round;
                 }
             }
-            if (!works) continue;
-            // clamped softmax (utils/Tensor.cpp:850-883) and top-k, strict '>' (utils/Tensor.cpp:1296-1334)
-            const unsigned all = 0xffffffffu;
-            float lg[TM][TE], pr[TM][TE];
+            if (works) {
+                // clamped softmax (utils/Tensor.cpp:850-883) and top-k, strict '>' (utils/Tensor.cpp:1296-1334)
+                const unsigned all = 0xffffffffu;
+                float lg[R][TE], pr[R][TE];
 #pragma unroll
-            for (int t = 0; t < TM; ++t) {
-                float mx = -INFINITY;
+                for (int t = 0; t < R; ++t) {
+                    float mx = -INFINITY;
 #pragma unroll
-                for (int j = 0; j < TE; ++j) {
-                    lg[t][j] = __fadd_rn(acc[t][j], bias[j]);
-                    if (e0 + j < E) mx = fmaxf(mx, lg[t][j]);
-                }
-#pragma unroll
-                for (int o = ET / 2; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(all, mx, o));
-                // exp through double and one rounding: agrees with a correctly rounded expf
-#pragma unroll
-                for (int j = 0; j < TE; ++j) pr[t][j] = e0 + j < E ? (float)exp((double)__fsub_rn(lg[t][j], mx)) : 0.0f;
-#pragma unroll
-                for (int j = 0; j < TE; ++j) ex[t * (RS + 4) + e0 + j] = pr[t][j];
-            }
-            __syncwarp();
-            float sum[TM] = {};
-            for (int e = 0; e < E; e += 4)                          // in index order (zeros past the last: they add nothing)
-#pragma unroll
-                for (int t = 0; t < TM; ++t) {
-                    const float4 v = *reinterpret_cast<const float4*>(ex + t * (RS + 4) + e);
-                    sum[t] = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum[t], v.x), v.y), v.z), v.w);
-                }
-            __syncwarp();
-#pragma unroll
-            for (int t = 0; t < TM; ++t) {
-                const int i = tt + t * GROUPS;
-                const bool live = i < n;
-                const size_t tok = live ? (p.list ? p.list[tile * TOK + i] : tile * TOK + i) : 0;
-                const float inv = __fdiv_rn(1.0f, fmaxf(sum[t], 1e-15f));
-#pragma unroll
-                for (int j = 0; j < TE; ++j) {
-                    pr[t][j] = fminf(fmaxf(__fmul_rn(pr[t][j], inv), 1e-7f), 1.0f);
-                    if (live && e0 + j < E) {
-                        p.probs[tok * E + e0 + j] = pr[t][j];
-                        if (p.logits) p.logits[tok * E + e0 + j] = lg[t][j];
+                    for (int j = 0; j < TE; ++j) {
+                        lg[t][j] = __fadd_rn(acc[t][j], bias[j]);
+                        if (e0 + j < E) mx = fmaxf(mx, lg[t][j]);
                     }
+#pragma unroll
+                    for (int o = ET / 2; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(all, mx, o));
+                    // exp through double and one rounding: agrees with a correctly rounded expf
+#pragma unroll
+                    for (int j = 0; j < TE; ++j) pr[t][j] = e0 + j < E ? (float)exp((double)__fsub_rn(lg[t][j], mx)) : 0.0f;
+#pragma unroll
+                    for (int j = 0; j < TE; ++j) ex[t * (RS + 4) + e0 + j] = pr[t][j];
                 }
-                // k rounds of (value desc, index asc) arg-max == the reference's stable insertion
-                unsigned taken = 0;
-                for (int r = 0; r < p.k; ++r) {
-                    float bv = -INFINITY;
-                    int bi = 0x7fffffff;
+                __syncwarp();
+                float sum[R] = {};
+                for (int e = 0; e < E; e += 4)                      // in index order (zeros past the last: they add nothing)
 #pragma unroll
-                    for (int j = 0; j < TE; ++j)
-                        if (e0 + j < E && !(taken >> j & 1u) && pr[t][j] > bv) {
-                            bv = pr[t][j];
-                            bi = e0 + j;
-                        }
+                    for (int t = 0; t < R; ++t) {
+                        const float4 v = *reinterpret_cast<const float4*>(ex + t * (RS + 4) + e);
+                        sum[t] = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum[t], v.x), v.y), v.z), v.w);
+                    }
+                __syncwarp();
 #pragma unroll
-                    for (int o = ET / 2; o > 0; o >>= 1) {
-                        const float ov = __shfl_xor_sync(all, bv, o);
-                        const int oi = __shfl_xor_sync(all, bi, o);
-                        if (ov > bv || (ov == bv && oi < bi)) {
-                            bv = ov;
-                            bi = oi;
+                for (int t = 0; t < R; ++t) {
+                    const int i = tt + t * GROUPS;
+                    const bool live = i < n;
+                    const size_t tok = live ? (p.list ? p.list[tile * TOK + i] : tile * TOK + i) : 0;
+                    const float inv = __fdiv_rn(1.0f, fmaxf(sum[t], 1e-15f));
+#pragma unroll
+                    for (int j = 0; j < TE; ++j) {
+                        pr[t][j] = fminf(fmaxf(__fmul_rn(pr[t][j], inv), 1e-7f), 1.0f);
+                        if (live && e0 + j < E) {
+                            p.probs[tok * E + e0 + j] = pr[t][j];
+                            if (p.logits) p.logits[tok * E + e0 + j] = lg[t][j];
                         }
                     }
-                    if (bi / TE == te) taken |= 1u << (bi % TE);
-                    if (live && te == 0) {
-                        p.top_idx[tok * p.k + r] = bi;
-                        p.top_p[tok * p.k + r] = bv;
+                    // k rounds of (value desc, index asc) arg-max == the reference's stable insertion
+                    unsigned taken = 0;
+                    for (int r = 0; r < p.k; ++r) {
+                        float bv = -INFINITY;
+                        int bi = 0x7fffffff;
+#pragma unroll
+                        for (int j = 0; j < TE; ++j)
+                            if (e0 + j < E && !(taken >> j & 1u) && pr[t][j] > bv) {
+                                bv = pr[t][j];
+                                bi = e0 + j;
+                            }
+#pragma unroll
+                        for (int o = ET / 2; o > 0; o >>= 1) {
+                            const float ov = __shfl_xor_sync(all, bv, o);
+                            const int oi = __shfl_xor_sync(all, bi, o);
+                            if (ov > bv || (ov == bv && oi < bi)) {
+                                bv = ov;
+                                bi = oi;
+                            }
+                        }
+                        if (bi / TE == te) taken |= 1u << (bi % TE);
+                        if (live && te == 0) {
+                            p.top_idx[tok * p.k + r] = bi;
+                            p.top_p[tok * p.k + r] = bv;
+                        }
                     }
                 }
             }
+        };
+        const int first = (tid & ~31) / ET;                 // the warp's first token
+        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+            const int n = min(TOK, n_active - tile * TOK), rows = n > first ? (n - first + GROUPS - 1) / GROUPS : 0;       // (warp-uniform)
+            if (TM == 1 || rows <= 1) work_tile(std::integral_constant<int, 1>(), rows > 0, tile, n);
+            else if (TM == 2 || rows == 2) work_tile(std::integral_constant<int, (TM >= 2 ? 2 : 1)>(), true, tile, n);
+            else if (TM == 3 || rows == 3) work_tile(std::integral_constant<int, (TM >= 3 ? 3 : 1)>(), true, tile, n);
+            else work_tile(std::integral_constant<int, (TM >= 4 ? 4 : 1)>(), true, tile, n);
         }
     }
     if (!p.plan.top_idx) return;
@@ -846,19 +874,29 @@ router_wgrad_reduce_kernel(const float* part, const float* partb, int n_chunks, 
     }
 }
 
-template <typename TIn, int RS, int TE, int TM>
+template <typename TIn, int ET, int TE, int TM>
 int router_exact_launch(RouterArgs p, int device, cudaStream_t st)
 {
-    auto* kernel = router_exact_kernel<TIn, RS, TE, TM>;
-    // every SM its share of the tokens, up to what the compute threads hold at a time (a list's length is only known on the device)
-    constexpr int most = RX_COMPUTE * TE / RS * TM;
-    const int share = (p.N + 147) / 148;
-    p.tok = p.list || share > most ? most : share;
+    auto* kernel = router_exact_kernel<TIn, ET, TE, TM>;
+    constexpr int RS = ET * TE;
+    // Every SM its share of the tokens (a list's length is only known on the device: two rows per warp), in the rounds that cost
+    // least (one of 1, 2, 3, 4 rows of 16 tokens x 64 experts x 1024 channels: 20, 28, 41, 55 us; the other forms alike).
+    constexpr int GROUPS = RX_COMPUTE / ET;
+    const int share = p.list ? GROUPS * (TM < 2 ? TM : 2) : (p.N + 147) / 148;
+    int rounds = 0, least = 0;
+    for (int r = 1; r <= TM; ++r) {
+        const int n = (share + GROUPS * r - 1) / (GROUPS * r), cost = n * (r == 1 ? 10 : 6 * r + 3);
+        if (!rounds || cost < least) {
+            rounds = n;
+            least = cost;
+        }
+    }
+    p.tok = (share + rounds - 1) / rounds;
     // A stage's beginning and end cost 650 cycles (one warp per scheduler hides no instruction fetch), so stages are long: 512
     // channels with a few tokens, whose loads are all on their way at once, 256 with more; two of them fit.
     for (p.ck = p.tok <= 4 ? 512 : 256; p.ck > 16 && rx_stage(p.ck, RS, p.tok, sizeof(TIn)) > 90u * 1024u;) p.ck /= 2;
     const int ctas = (p.N + p.tok - 1) / p.tok, grid = ctas < 148 ? ctas : 148;
-    const uint32_t stage = rx_stage(p.ck, RS, p.tok, sizeof(TIn)), tail = rx_tail(TE, TM, RS);
+    const uint32_t stage = rx_stage(p.ck, RS, p.tok, sizeof(TIn)), tail = rx_tail(ET, TE, TM);
     int stages = (int)((200u * 1024u - tail) / stage);
     const int chunks = (p.C + p.ck - 1) / p.ck;
     if (stages > RX_MAX_STAGES) stages = RX_MAX_STAGES;
@@ -876,31 +914,53 @@ int router_exact_launch(RouterArgs p, int device, cudaStream_t st)
     return 0;
 }
 
-// (Token, expert) pairs per thread: as few as hold an SM's share of the tokens in eight warps, for a channel's step is bound by
-// latency (one pair 7.5 cycles, two 15-18, four 22-30).  Not four experts of one token: shared memory then delivers a
-// step's weights no faster than 1.1 cycles per 32 pairs (two of two tokens 0.83, four of two 0.72, issue alone 0.5).
-template <typename TIn, int RS>
-int router_exact_pick(const RouterArgs& p, int device, cudaStream_t st)
-{
-    constexpr int one = RX_COMPUTE / RS;               // tokens held with one pair per thread
-    const int share = p.list ? 1 << 30 : (p.N + 147) / 148;
-    if constexpr (RS <= 32)
-        if (share <= one) return router_exact_launch<TIn, RS, 1, 1>(p, device, st);
-    if constexpr (RS <= 64) {
-        if (share <= 2 * one) return router_exact_launch<TIn, RS, 2, 1>(p, device, st);
-        if (share <= 4 * one) return router_exact_launch<TIn, RS, 2, 2>(p, device, st);
-    } else {
-        if (share <= 4 * one) return router_exact_launch<TIn, RS, 4, 1>(p, device, st);
-    }
-    return router_exact_launch<TIn, RS, 4, 2>(p, device, st);
-}
+// Lanes per token x experts per lane x most rows per warp, by the experts and by an SM's share of the tokens: few pairs per
+// thread while an SM has few tokens (a channel's step is bound by latency), more where it is bound by issue, and as few idle
+// experts as possible.  The lines lie where the forms cross, us for C=1024, BF16 tokens, by the share:
+//   16 experts   16x1 8.5, 8x2 9.6 at 8; 10.9, 10.2 at 12; 8x2 33, 4x4 35 at 96; 40, 36 at 112
+//   32           32x1 8.9, 16x2 9.2 at 4; 11.3, 10.9 at 8; 16x2 30, 8x4 33 at 48; 39, 34 at 64
+//   64           32x2 29, 16x4 32 at 24; 40, 32 at 28
+//    8           8x1 11.6, 2x4 14 at 32; 20, 16 at 40
+//   20           8x3 32, 4x5 32 at 64; 49, 45 at 104; 70, 55 at 144
+//   40           16x3 31, 8x5 32 at 32; 41, 39 at 46; 68, 54 at 72
+//   80           32x3 29, 16x5 30 at 12; 53, 49 at 32; 120, 107 at 72
+// One row has a kernel of its own for small shares: in a call whose instructions come from HBM the kernels for several rows cost
+// up to 4 us more.
 template <typename TIn>
 int router_exact_dispatch(const RouterArgs& p, int device, cudaStream_t st)
 {
-    if (p.E <= 16) return router_exact_pick<TIn, 16>(p, device, st);
-    if (p.E <= 32) return router_exact_pick<TIn, 32>(p, device, st);
-    if (p.E <= 64) return router_exact_pick<TIn, 64>(p, device, st);
-    return router_exact_pick<TIn, 128>(p, device, st);
+    const int E = p.E, share = p.list ? 1 << 30 : (p.N + 147) / 148;
+    if (E <= 8) {
+        if (share <= 32) return router_exact_launch<TIn, 8, 1, 1>(p, device, st);
+        if (E <= 4) return router_exact_launch<TIn, 1, 4, 2>(p, device, st);
+        return router_exact_launch<TIn, 2, 4, 2>(p, device, st);
+    }
+    if (E <= 16) {
+        if (share <= 8) return router_exact_launch<TIn, 16, 1, 1>(p, device, st);
+        if (share <= (E > 12 ? 32 : 16)) return router_exact_launch<TIn, 8, 2, 1>(p, device, st);
+        if (E <= 12) return router_exact_launch<TIn, 4, 3, 3>(p, device, st);
+        if (share <= 96) return router_exact_launch<TIn, 8, 2, 3>(p, device, st);
+        return router_exact_launch<TIn, 4, 4, 3>(p, device, st);
+    }
+    if (E <= 32) {
+        if (share <= (E > 24 ? 8 : 4)) return router_exact_launch<TIn, 32, 1, 1>(p, device, st);
+        if (share <= (E > 24 ? 16 : 8)) return router_exact_launch<TIn, 16, 2, 1>(p, device, st);
+        if (E <= 20 && share > 64) return router_exact_launch<TIn, 4, 5, 3>(p, device, st);
+        if (E <= 24) return router_exact_launch<TIn, 8, 3, 4>(p, device, st);
+        if (share <= 48) return router_exact_launch<TIn, 16, 2, 3>(p, device, st);
+        return router_exact_launch<TIn, 8, 4, 3>(p, device, st);
+    }
+    if (E <= 64) {
+        if (share <= (E > 48 ? 8 : 4)) return router_exact_launch<TIn, 32, 2, 1>(p, device, st);
+        if (E <= 40 && share > 40) return router_exact_launch<TIn, 8, 5, 3>(p, device, st);
+        if (E <= 48) return router_exact_launch<TIn, 16, 3, 4>(p, device, st);
+        if (share <= 24) return router_exact_launch<TIn, 32, 2, 3>(p, device, st);
+        return router_exact_launch<TIn, 16, 4, 3>(p, device, st);
+    }
+    if (share <= (E > 96 ? 8 : 4)) return router_exact_launch<TIn, 32, 4, 1>(p, device, st);
+    if (E <= 80 && share > 16) return router_exact_launch<TIn, 16, 5, 3>(p, device, st);
+    if (E <= 96) return router_exact_launch<TIn, 32, 3, 4>(p, device, st);
+    return router_exact_launch<TIn, 32, 4, 4>(p, device, st);
 }
 
 template <typename TIn, int EL, int EPL, int TPW>
