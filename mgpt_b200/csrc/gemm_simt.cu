@@ -171,7 +171,6 @@ struct RowsArgs {
     // reads them: the weight gradients below stop at the last real row).  Null where rows come in segments.
     const int32_t* counts; const int32_t* padded_offsets;
     int K, Nout;
-    int ctas;                                  // CTAs of a cluster that share a tile's k loop
 };
 
 template <int EPI, int KS> constexpr size_t rows_smem()
@@ -182,7 +181,7 @@ template <int EPI, int KS> constexpr size_t rows_smem()
 }
 
 // VEC: weights and their gradients, AVEC: rows, start on boundaries of four elements.
-// CL: a cluster of a.ctas CTAs per tile.
+// CL: a cluster of CTAs per tile.
 template <typename TAct, typename TW, int EPI, int KS, bool VEC, bool AVEC, bool CL>
 __global__ void __launch_bounds__(GT * KS) simt_rows_kernel(RowsArgs a)
 {
@@ -190,8 +189,7 @@ __global__ void __launch_bounds__(GT * KS) simt_rows_kernel(RowsArgs a)
     pdl_wait();
     constexpr bool BK_MAJOR = EPI == EPI_DHH || EPI == EPI_DXG;      // B(k, n) at n*K + k
     constexpr int NOP = EPI == EPI_GATEUP ? 3 : 2;
-    const int ctas = CL ? a.ctas : 1, rank = CL ? (int)tcx::cluster_ctarank() : 0;
-    const int m0 = (int)blockIdx.x / ctas * TM, n0 = blockIdx.y * TN;
+    const int m0 = (CL ? blockIdx.x / tcx::cluster_size() : blockIdx.x) * TM, n0 = blockIdx.y * TN;
     const int rows = *a.n_tiles * ROW_TILE;
     if (m0 >= rows) return;
     const int e = a.tile_expert[m0 / ROW_TILE];
@@ -203,8 +201,13 @@ __global__ void __launch_bounds__(GT * KS) simt_rows_kernel(RowsArgs a)
     float acc[8][4] = {}, acc2[8][4] = {};
     // this group's steps of TK; EPI_DXG runs through dG*Wg^T and then dU*Wu^T
     const int per = (K + TK - 1) / TK, steps = EPI == EPI_DXG ? 2 * per : per;
-    const int part = rank * KS + group, parts = KS * ctas;
-    const int s0 = (int)((long)steps * part / parts), s1 = (int)((long)steps * (part + 1) / parts);
+    int s0 = (int)((long)steps * group / KS), s1 = (int)((long)steps * (group + 1) / KS), rank = 0;
+    if constexpr (CL) {
+        rank = (int)tcx::cluster_ctarank();
+        const int part = rank * KS + group, parts = KS * (int)tcx::cluster_size();
+        s0 = (int)((long)steps * part / parts);
+        s1 = (int)((long)steps * (part + 1) / parts);
+    }
     const TW *B1 = (const TW*)a.B[e], *B2 = NOP == 3 || EPI == EPI_DXG ? (const TW*)a.B2[e] : nullptr;
     float4 ra[2], rb[2], rc[2];
     auto gload = [&](int s) {
@@ -237,11 +240,12 @@ __global__ void __launch_bounds__(GT * KS) simt_rows_kernel(RowsArgs a)
     fold<KS>(sm, group, t, acc);
     if (NOP == 3) fold<KS>(sm + (KS - 1) * TM * TN, group, t, acc2);
     if constexpr (CL) {
-        fold_cluster(sm, ctas, rank, group == 0, t, acc);
-        if (NOP == 3) fold_cluster(sm, ctas, rank, group == 0, t, acc2);
+        fold_cluster(sm, tcx::cluster_size(), rank, group == 0, t, acc);
+        if (NOP == 3) fold_cluster(sm, tcx::cluster_size(), rank, group == 0, t, acc2);
+        if (rank > 0) return;
     }
     const int n = n0 + tx * 4;
-    if (rank > 0 || group > 0 || n >= N) return;
+    if (group > 0 || n >= N) return;
     float b1[4] = {}, b2[4] = {};
     if (EPI == EPI_GATEUP || EPI == EPI_DOWN)
 #pragma unroll
@@ -420,30 +424,29 @@ template <typename TAct> bool rows_aligned(const mgpt_moe_layer* L)
 }
 
 template <typename TAct, typename TW, int EPI, int KS, bool CL>
-int launch_rows_ks(const mgpt_moe_layer* L, const RowsArgs& a, dim3 grid, cudaStream_t st)
+int launch_rows_ks(const mgpt_moe_layer* L, const RowsArgs& a, dim3 grid, int ctas, cudaStream_t st)
 {
     constexpr size_t smem = rows_smem<EPI, KS>();
     auto* kernel = !rows_aligned<TAct>(L) ? simt_rows_kernel<TAct, TW, EPI, KS, false, false, CL>
                    : L->masters_aligned   ? simt_rows_kernel<TAct, TW, EPI, KS, true, true, CL>
                                           : simt_rows_kernel<TAct, TW, EPI, KS, false, true, CL>;
     if (smem > 48 * 1024) MGPT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    if (CL) MGPT_CUDA(launch_pdl_cluster(kernel, grid, a.ctas, GT * KS, smem, st, a));
+    if (CL) MGPT_CUDA(launch_pdl_cluster(kernel, grid, ctas, GT * KS, smem, st, a));
     else MGPT_CUDA(launch_pdl(kernel, grid, GT * KS, smem, st, a));
     return 0;
 }
 template <typename TAct, typename TW, int EPI>
-int launch_rows(const mgpt_moe_layer* L, const Workspace& w, RowsArgs a, cudaStream_t st, const char* what)
+int launch_rows(const mgpt_moe_layer* L, const Workspace& w, const RowsArgs& a, cudaStream_t st, const char* what)
 {
     const int cols = (a.Nout + TN - 1) / TN;
     // tiles with real rows: about R/64 and half a tile per expert
     const int tiles = (w.R / TM + (L->d.E + 1) / 2) * cols, k = EPI == EPI_DXG ? 2 * a.K : a.K;
-    const int ks = split_k(tiles, k);
-    a.ctas = ks == 4 ? split_ctas(tiles, k) : 1;
-    const dim3 grid(w.row_cap / TM * a.ctas, cols);
-    if (a.ctas > 1) MGPT_TRY((launch_rows_ks<TAct, TW, EPI, 4, true>(L, a, grid, st)));
-    else if (ks == 4) MGPT_TRY((launch_rows_ks<TAct, TW, EPI, 4, false>(L, a, grid, st)));
-    else if (ks == 2) MGPT_TRY((launch_rows_ks<TAct, TW, EPI, 2, false>(L, a, grid, st)));
-    else MGPT_TRY((launch_rows_ks<TAct, TW, EPI, 1, false>(L, a, grid, st)));
+    const int ks = split_k(tiles, k), ctas = ks == 4 ? split_ctas(tiles, k) : 1;
+    const dim3 grid(w.row_cap / TM * ctas, cols);
+    if (ctas > 1) MGPT_TRY((launch_rows_ks<TAct, TW, EPI, 4, true>(L, a, grid, ctas, st)));
+    else if (ks == 4) MGPT_TRY((launch_rows_ks<TAct, TW, EPI, 4, false>(L, a, grid, ctas, st)));
+    else if (ks == 2) MGPT_TRY((launch_rows_ks<TAct, TW, EPI, 2, false>(L, a, grid, ctas, st)));
+    else MGPT_TRY((launch_rows_ks<TAct, TW, EPI, 1, false>(L, a, grid, ctas, st)));
     MGPT_LAUNCHED(what);
     return 0;
 }

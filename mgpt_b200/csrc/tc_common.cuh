@@ -175,6 +175,12 @@ __device__ __forceinline__ uint32_t cluster_ctarank()
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
+__device__ __forceinline__ uint32_t cluster_size()
+{
+    uint32_t n;
+    asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
+    return n;
+}
 // shared::cluster address of the same shared-memory location in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank)
 {
