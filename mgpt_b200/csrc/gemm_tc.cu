@@ -366,7 +366,7 @@ __device__ __forceinline__ void rows_epilogue(const RowsP& p, RowsShared& sh, ui
                         const uint64_t sig = pk2(rcp(d0), rcp(d1)), qv = mul2(g, sig), us = mul2(u, sig);
                         hp[4 * c + j] = bf2(mul2(qv, u));
                         qp[j] = bf2(qv);
-                        pp[j] = bf2(fma2(us, fma2(qv, pk2(-1.0f, -1.0f), g), us));
+                        pp[j] = bf2(mul2(us, add2(fma2(qv, pk2(-1.0f, -1.0f), g), one)));      // (not us + us*(..): NaN where us is infinite)
                     }
                     if (p.G && c * 8 < valid) {            // inference keeps nothing for a backward pass
                         gp[c * BM] = make_uint4(pp[0], pp[1], pp[2], pp[3]);
