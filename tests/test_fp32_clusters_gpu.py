@@ -14,6 +14,9 @@ pytestmark = pytest.mark.gpu
     (30, 64, 1032, 2, 2),       # one tile of columns: eight CTAs
     (64, 264, 1024, 8, 2),      # four; C ends inside a tile
     (500, 128, 520, 8, 2),      # two in dXg; the shortest k that is shared
+    # gate/up (both sums through the same shared memory) and dHh share theirs from C = 256 on: eight, four and two CTAs, H ends
+    # inside a second and a third tile of columns
+    (30, 1032, 72, 2, 2), (64, 520, 136, 4, 2), (64, 264, 136, 4, 2),
 ])
 def test_shared_k_loops(n, C, H, E, k):
     w = synth.Workload("clusters", n, C, H, E, k, "fp32")
