@@ -408,8 +408,10 @@ int split_k(int tiles, int k)
 // CTAs per tile where four groups each leave SMs without one: a cluster of two, four or eight, no group with less than two steps.
 // Stage times without -> with, us: 1024 tokens, C=128, H=512, E=8, top-2 (two CTAs) down 23 -> 19, dXg 37 -> 27, the step 149 ->
 // 135; 64 tokens, C=256, H=1024 (four) 35 -> 20 and 66 -> 29, the step 172 -> 120; 256 tokens, C=256, H=1024, E=16, top-1 234
-// -> 203.
-int split_ctas(int tiles, int k)
+// -> 203.  A few clusters more than the SMs hold are a second round, which takes the gain and more (the step of 564 tokens,
+// C=192, H=152, E=13, top-2, 108 without, 113 with 25 row tiles instead of the 24 that were expected), so `tiles` is a number that
+// the routing seldom exceeds.
+int split_ctas(double tiles, int k)
 {
     int ctas = 1;
     while (ctas < 8 && tiles * ctas * 2 <= 148 && k >= ctas * 2 * 4 * 2 * TK) ctas *= 2;
@@ -441,7 +443,9 @@ int launch_rows(const mgpt_moe_layer* L, const Workspace& w, const RowsArgs& a, 
     const int cols = (a.Nout + TN - 1) / TN;
     // tiles with real rows: about R/64 and half a tile per expert
     const int tiles = (w.R / TM + (L->d.E + 1) / 2) * cols, k = EPI == EPI_DXG ? 2 * a.K : a.K;
-    const int ks = split_k(tiles, k), ctas = ks == 4 ? split_ctas(tiles, k) : 1;
+    // (each expert's last tile is filled by chance: that half has a standard deviation of sqrt(E / 12))
+    const double most = (w.R / (double)TM + L->d.E / 2.0 + sqrt(L->d.E / 12.0)) * cols;
+    const int ks = split_k(tiles, k), ctas = ks == 4 ? split_ctas(most, k) : 1;
     const dim3 grid(w.row_cap / TM * ctas, cols);
     if (ctas > 1) MGPT_TRY((launch_rows_ks<TAct, TW, EPI, 4, true>(L, a, grid, ctas, st)));
     else if (ks == 4) MGPT_TRY((launch_rows_ks<TAct, TW, EPI, 4, false>(L, a, grid, ctas, st)));
