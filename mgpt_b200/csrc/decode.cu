@@ -246,16 +246,18 @@ int launch_phase(const DecP& p, int sms, cudaStream_t st)
 // weight bytes times rows.  These kernels save about 15 us of a call (no dispatch where nothing is kept, no first tile to
 // wait for) and lose the more, the more weights stream by and the more rows meet each of them (B fragments and MMAs per
 // weight, and a crowded expert's weights again for every 16 rows).  Inference calls, us with tiles / with these kernels, L2
-// flushed (training steps at the same sizes: up to 11 % faster where few tiles decide, within 3 % of each other elsewhere;
-// measured before the tiles' products requested their first weights early, which took 3-4 us off their calls):
-//   tokens                           1        8       16        32        64       128
-//   C=1024 H=2816 E=32 top-2     66/46    90/77  121/116   137/136   141/144   145/159
-//     a few experts take most    66/46    68/48    68/50     68/56     72/69    74/108
-//   C=2048 H=1408 E=64 top-2     80/60  121/106  157/147   199/194   232/241   250/271
-//     a few experts take most    82/59    84/61    88/75     88/81     92/95    96/130
-//   C=1024 H= 512 E=64 top-4     64/46    76/65    92/78     98/87    102/95     95/92
-//   C=2048 H=2816 E= 8 top-2     82/58   113/95   113/95    113/99         .         .
-//   C= 768 H=2048 E=16 top-2     57/38    72/54    78/65     78/67     78/71         .
+// flushed (training steps at the same sizes, for which the rows are copied all the same: with these kernels up to 5 % slower where
+// the routing is even, 3 % faster to 7 % slower where it is crowded):
+//   tokens                           1       8       16       24       32       48       64      128
+//   C=1024 H=2816 E=32 top-2     51/34   78/67   102/97  121/120  127/130  130/134  129/136  131/146
+//     a few experts take most    51/36   55/38    54/40    54/42    57/48    57/52    57/65    61/97
+//   C=2048 H=1408 E=64 top-2     57/40   98/87  134/124  143/146  173/174  186/202  213/224  227/254
+//     a few experts take most    57/40   62/44    65/52    65/56    68/62    68/66    70/77   73/106
+//   C=1024 H= 512 E=64 top-4     41/30   53/46    68/58    72/60    74/71    76/75    76/76    78/80
+//   C=2048 H=2816 E= 8 top-2     65/46   98/83    98/83    97/85    97/87        .        .        .
+//   C= 768 H=2048 E=16 top-2     43/29   64/52    64/56    66/58    66/58    66/59    66/60        .
+// At the line in weight bytes times rows (32 tokens of the first width) an even routing loses 2 % and a crowded one gains 16 %;
+// further on (64) both lose.  Which of the two a call has is not known here.
 bool decode_usable(const Dims& d, int n_tokens)
 {
     const double rows = (double)n_tokens * d.k, experts = rows < d.E ? rows : d.E;

@@ -276,10 +276,10 @@ struct RowsP {
     bf16 *G, *U;            // P and Q (see the gate/up epilogue) in the blocked layout (written by MODE_GATEUP, read by MODE_DHH)
     const float* const* bias0;
     const float* const* bias1;
-    // MODE_DX only: row tiles are token tiles (no experts); the epilogue adds the expert rows of each token
+    // tc_dx_kernel only: row tiles are token tiles (no experts); the epilogue adds the expert rows of each token
     int fixed_tiles;            // number of 128-token tiles
     int n_valid_rows;           // tokens
-    // The B operand (MODE_DX apart) is a tile-major weight copy (common.cuh): block (expert e, row block rb, column block
+    // The B operand of the expert products is a tile-major weight copy (common.cuh): block (expert e, row block rb, column block
     // cb) is block (e * b_row_blocks + rb) * b_col_blocks + cb of the copy.
     // MODE_GATEUP / MODE_DOWN: rows are output columns, block columns the reduction (whole blocks of 128 rows, K-major);
     // MODE_DHH / MODE_DXG: rows are the reduction, block columns output columns (half blocks of 64 rows, MN-major).
@@ -287,7 +287,7 @@ struct RowsP {
     const bf16* gather_src;     // dXg rows [*, n_out]
     const int32_t* gather_pos;  // [tokens, gather_k] row of dXg for (token, j)
     int gather_k;
-    bf16* dx;                   // MODE_DX: the output
+    bf16* dx;                   // tc_dx_kernel: the output
 };
 
 // What follows the operand ring and the staging tiles of the four expert products.
@@ -804,7 +804,7 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
     cta_teardown(tmem_base, warp);
 }
 
-// MODE_DX: dlogits * Wr^T, an item of one or two k-blocks; one stage, and the epilogue's staging lies where the others would.
+// dx: dlogits * Wr^T, an item of one or two k-blocks; one stage, and the epilogue's staging lies where the others would.
 // Its items are all alike: by stride, no queue.
 __global__ void __launch_bounds__(TC_THREADS, 1)
 tc_dx_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const RowsP p)
@@ -1230,6 +1230,9 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant_
 //   C=1024 H= 512 E=64   166/121      189/162      228/201      263/240        .
 //                        172/125      191/152      211/181      236/207        .
 // Few rows leave nothing for a pair to save, and its CTAs wait for one another; hence the line at 512 (pair_wgrad_usable).
+// The line is drawn for evenly spread rows.  Where a few experts take most rows pairs are faster on both sides of it, for their
+// longest items come first; the step, this kernel / the other one: C=2048 H=1408 E=64 256 rows on average 979/1061, 768
+// 2412/2475; C=1024 H=1408 E=32 512 495/513, 768 678/706; C=512 H=1376 E=16 512 184/193, 768 248/256.
 //
 // The bias gradients are column sums of the A tiles.  Two warps of the LEADER add them up (the peer has no barrier that
 // says when its tiles are there: all bytes are counted on the leader's); the pair swaps its two A tiles from one column
