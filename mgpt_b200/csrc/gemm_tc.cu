@@ -93,6 +93,24 @@ __device__ __forceinline__ float rcp(float x)
     return y;
 }
 
+__device__ __forceinline__ uint64_t sigmoid2(uint64_t g)
+{
+    float e0, e1, d0, d1;
+    unpk2(mul2(g, pk2(-1.4426950408889634f, -1.4426950408889634f)), e0, e1);
+    unpk2(add2(pk2(ex2(e0), ex2(e1)), pk2(1.0f, 1.0f)), d0, d1);
+    return pk2(rcp(d0), rcp(d1));
+}
+
+// per half: a where x is infinite, else b
+__device__ __forceinline__ uint64_t where_infinite(uint64_t x, uint64_t a, uint64_t b)
+{
+    float x0, x1, a0, a1, b0, b1;
+    unpk2(x, x0, x1);
+    unpk2(a, a0, a1);
+    unpk2(b, b0, b1);
+    return pk2(isinf(x0) ? a0 : b0, isinf(x1) ? a1 : b1);
+}
+
 // Shared memory of one CTA: operand ring, one 2 KiB staging tile per epilogue warp, barriers.
 struct Pipe {
     uint32_t bars, tmem_slot;          // shared-space addresses
@@ -353,26 +371,37 @@ __device__ __forceinline__ void rows_epilogue(const RowsP& p, RowsShared& sh, ui
                 uint32_t hp[16];
                 const size_t o = blocked_index(w.row_tile, ld, n, q * 32 + lane);
                 uint4 *gp = reinterpret_cast<uint4*>(p.G) + o, *up = reinterpret_cast<uint4*>(p.U) + o;
+                auto work = [&](auto infinite) {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {              // 8 hidden units at a time
-                    uint32_t pp[4], qp[4];
+                    for (int c = 0; c < 4; ++c) {          // 8 hidden units at a time
+                        uint32_t pp[4], qp[4];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const uint64_t g = g2[4 * c + j], u = u2[4 * c + j], one = pk2(1.0f, 1.0f);
-                        float e0, e1;
-                        unpk2(mul2(g, pk2(-1.4426950408889634f, -1.4426950408889634f)), e0, e1);
-                        float d0, d1;
-                        unpk2(add2(pk2(ex2(e0), ex2(e1)), one), d0, d1);
-                        const uint64_t sig = pk2(rcp(d0), rcp(d1)), qv = mul2(g, sig), us = mul2(u, sig);
-                        hp[4 * c + j] = bf2(mul2(qv, u));
-                        qp[j] = bf2(qv);
-                        pp[j] = bf2(mul2(us, add2(fma2(qv, pk2(-1.0f, -1.0f), g), one)));      // (not us + us*(..): NaN where us is infinite)
+                        for (int j = 0; j < 4; ++j) {
+                            const uint64_t g = g2[4 * c + j], u = u2[4 * c + j], sig = sigmoid2(g), qv = mul2(g, sig), us = mul2(u, sig);
+                            const uint64_t d = fma2(qv, pk2(-1.0f, -1.0f), g), v = fma2(us, d, us);
+                            hp[4 * c + j] = bf2(mul2(qv, u));
+                            qp[j] = bf2(qv);
+                            pp[j] = bf2(decltype(infinite)::value ? where_infinite(us, mul2(us, add2(d, pk2(1.0f, 1.0f))), v) : v);
+                        }
+                        if (p.G && c * 8 < valid) {        // inference keeps nothing for a backward pass
+                            gp[c * BM] = make_uint4(pp[0], pp[1], pp[2], pp[3]);
+                            up[c * BM] = make_uint4(qp[0], qp[1], qp[2], qp[3]);
+                        }
                     }
-                    if (p.G && c * 8 < valid) {            // inference keeps nothing for a backward pass
-                        gp[c * BM] = make_uint4(pp[0], pp[1], pp[2], pp[3]);
-                        up[c * BM] = make_uint4(qp[0], qp[1], qp[2], qp[3]);
-                    }
+                };
+                // us + us * (g - q) is NaN where us is infinite and g - q negative or zero.  (The sum of products is finite unless
+                // a value is not, or values are huge: 8 instructions for the 32 that a test of each took.)
+                bool infinite = false;
+                if (p.G) {
+                    uint64_t sum[2] = {};
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) sum[i & 1] = fma2(u2[2 * i], u2[2 * i + 1], sum[i & 1]);
+                    float s0, s1;
+                    unpk2(add2(sum[0], sum[1]), s0, s1);
+                    infinite = !(fabsf(s0) + fabsf(s1) < INFINITY);
                 }
+                if (__any_sync(0xffffffffu, infinite)) work(std::true_type());
+                else work(std::false_type());
                 store(hp, tmD0, n);
             }
         }
