@@ -147,7 +147,6 @@ struct RouterArgs {
     PlanArgs plan;
 };
 
-constexpr int pow2_from(int n) { return n <= 1 ? 1 : 2 * pow2_from((n + 1) / 2); }
 constexpr int RX_COMPUTE = 256, RX_PRODUCE = 128, RX_THREADS = RX_COMPUTE + RX_PRODUCE, RX_MAX_STAGES = 16;
 __host__ __device__ inline uint32_t rx_x_row(int ck, int elt) { return (uint32_t)(ck * elt + 16); }      // padded: rows in distinct banks
 __host__ __device__ inline uint32_t rx_stage(int ck, int rs, int tok, int elt)
@@ -246,6 +245,19 @@ __global__ void __launch_bounds__(RX_THREADS, 1) router_exact_kernel(const Route
         // fills the ring
         constexpr int XV = 16 / sizeof(TIn);
         const int per_log = __ffs(CK / XV) - 1, pt = tid - RX_COMPUTE;        // 16-byte pieces per row and chunk
+        // A row of Wr may be shorter than the staged one: piece pt, pt + 128, ... of the rows, column and row by addition.  (A column
+        // per thread leaves up to half of them without: 296 tokens, C=1024, 4 experts 10.7 us; two divisions per element before
+        // that, 127 experts 572 us for 32851 tokens.)
+        const bool wide = (E & 3) == 0;
+        const int per = wide ? E >> 2 : E, r0 = pt / per, q0 = pt % per, dr = RX_PRODUCE / per, dq = RX_PRODUCE % per;
+        auto step = [&](int& r, int& q) {
+            r += dr;
+            q += dq;
+            if (q >= per) {
+                q -= per;
+                ++r;
+            }
+        };
         int s = 0;
         uint32_t round = 0;
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
@@ -255,22 +267,19 @@ __global__ void __launch_bounds__(RX_THREADS, 1) router_exact_kernel(const Route
                 const int len = min(CK, C - c0), pieces = len / XV;
                 const uint32_t dst = ring0 + s * stage;
                 const float* src = p.Wr + (size_t)c0 * E;
-                // (a row of Wr is shorter than the staged one: some threads have nothing to copy, and none divides)
                 if (E == RS) {
                     for (int v = pt; v < len * (RS / 4); v += RX_PRODUCE)
                         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + v * 16), "l"(src + v * 4) : "memory");
-                } else if ((E & 3) == 0) {
-                    constexpr int P = pow2_from(RS / 4);
-                    const int q = pt % P * 4;
-                    if (q < E)
-                        for (int r = pt / P; r < len; r += RX_PRODUCE / P)
-                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (r * RS + q) * 4), "l"(src + r * E + q) : "memory");
+                } else if (wide) {
+                    for (int v = pt, r = r0, q = q0; v < len * per; v += RX_PRODUCE) {
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (r * RS + q * 4) * 4), "l"(src + v * 4) : "memory");
+                        step(r, q);
+                    }
                 } else {
-                    constexpr int P = pow2_from(RS);
-                    const int q = pt % P;
-                    if (q < E)
-                        for (int r = pt / P; r < len; r += RX_PRODUCE / P)
-                            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + (r * RS + q) * 4), "l"(src + r * E + q) : "memory");
+                    for (int v = pt, r = r0, q = q0; v < len * per; v += RX_PRODUCE) {
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + (r * RS + q) * 4), "l"(src + v) : "memory");
+                        step(r, q);
+                    }
                 }
                 for (int v = pt; v < n << per_log; v += RX_PRODUCE) {
                     const int i = v >> per_log, q = v & ((1 << per_log) - 1);
