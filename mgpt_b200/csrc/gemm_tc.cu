@@ -324,7 +324,8 @@ static_assert(ROWS_SMEM <= 232448, "shared memory of one CTA");
 
 // The epilogue of every second item of a CTA for one of the eight warps of its group: TMEM lane quarter q (rows q*32..+31 of
 // the row tile), column half h.  `next(n, w)`: the CTA's n-th item, false: no more.
-template <int MODE, class Next>
+// KEEP (gate/up): a backward pass follows, which needs the saved factors; inference keeps nothing.
+template <int MODE, bool KEEP, class Next>
 __device__ __forceinline__ void rows_epilogue(const RowsP& p, RowsShared& sh, uint32_t tmem_base, int group, int q, int h, int lane,
                                               uint8_t* stage, const CUtensorMap* tmD0, const CUtensorMap* tmD1, Next next)
 {
@@ -383,25 +384,25 @@ __device__ __forceinline__ void rows_epilogue(const RowsP& p, RowsShared& sh, ui
                             qp[j] = bf2(qv);
                             pp[j] = bf2(decltype(infinite)::value ? where_infinite(us, mul2(us, add2(d, pk2(1.0f, 1.0f))), v) : v);
                         }
-                        if (p.G && c * 8 < valid) {        // inference keeps nothing for a backward pass
+                        if (KEEP && c * 8 < valid) {
                             gp[c * BM] = make_uint4(pp[0], pp[1], pp[2], pp[3]);
                             up[c * BM] = make_uint4(qp[0], qp[1], qp[2], qp[3]);
                         }
                     }
                 };
-                // us + us * (g - q) is NaN where us is infinite and g - q negative or zero.  (The sum of products is finite unless
-                // a value is not, or values are huge: 8 instructions for the 32 that a test of each took.)
-                bool infinite = false;
-                if (p.G) {
+                if constexpr (KEEP) {
+                    // us + us * (g - q) is NaN where us is infinite and g - q negative or zero.  (The sum of products is finite
+                    // unless a value is not, or values are huge: 8 instructions for the 32 that a test of each took.)
                     uint64_t sum[2] = {};
 #pragma unroll
                     for (int i = 0; i < 8; ++i) sum[i & 1] = fma2(u2[2 * i], u2[2 * i + 1], sum[i & 1]);
                     float s0, s1;
                     unpk2(add2(sum[0], sum[1]), s0, s1);
-                    infinite = !(fabsf(s0) + fabsf(s1) < INFINITY);
+                    if (__builtin_expect(__any_sync(0xffffffffu, !(fabsf(s0) + fabsf(s1) < INFINITY)), 0)) work(std::true_type());
+                    else work(std::false_type());
+                } else {
+                    work(std::false_type());
                 }
-                if (__any_sync(0xffffffffu, infinite)) work(std::true_type());
-                else work(std::false_type());
                 store(hp, tmD0, n);
             }
         }
@@ -627,7 +628,7 @@ __device__ __forceinline__ void dx_epilogue(const RowsP& p, const Pipe& pipe, ui
 // tiles: no gain.  dHh's results through 16-byte stores from registers instead of TMA: 54 -> 70 us.  Its factors sent to L2
 // an item ahead: 54 -> 56.  More weights sent to L2 before pdl_wait (8 or 16 k-blocks behind the ring): 120.0 -> 120.7 and
 // 121.2 us for 256 tokens, C=1024, H=2816, E=32.
-template <int MODE>
+template <int MODE, bool KEEP = true>
 __global__ void __launch_bounds__(ROWS_THREADS, 1)
 tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                const __grid_constant__ CUtensorMap tmB0, const __grid_constant__ CUtensorMap tmB1,
@@ -823,7 +824,7 @@ tc_rows_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
         // TMEM lane quarter q = warp % 4, column half h
         constexpr int PER = EPI_WARPS / rows_groups(MODE);
         const int i = warp - 2;
-        rows_epilogue<MODE>(p, sh, tmem_base, i / PER, warp & 3, i % PER / 4, lane, smem_raw + STAGES * STAGE_BYTES + i * STAGING_BYTES, &tmD0, &tmD1,
+        rows_epilogue<MODE, KEEP>(p, sh, tmem_base, i / PER, warp & 3, i % PER / 4, lane, smem_raw + STAGES * STAGE_BYTES + i * STAGING_BYTES, &tmD0, &tmD1,
                             [&](uint32_t n, RowsItem& w) -> bool {
                                 const bool more = __any_sync(0xffffffffu, consume(n, w));       // (warp-uniform)
                                 if (more && lane == 0) release(n);
@@ -1775,6 +1776,7 @@ int prepare_attrs(mgpt_moe_layer* L)
     TcState* s = (TcState*)L->tc_state;
     if (!s->attr_set) {
         MGPT_CUDA(cudaFuncSetAttribute(tc_rows_kernel<MODE_GATEUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROWS_SMEM));
+        MGPT_CUDA(cudaFuncSetAttribute((tc_rows_kernel<MODE_GATEUP, false>), cudaFuncAttributeMaxDynamicSharedMemorySize, ROWS_SMEM));
         MGPT_CUDA(cudaFuncSetAttribute(tc_rows_kernel<MODE_DOWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROWS_SMEM));
         MGPT_CUDA(cudaFuncSetAttribute(tc_rows_kernel<MODE_DHH>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROWS_SMEM));
         MGPT_CUDA(cudaFuncSetAttribute(tc_rows_kernel<MODE_DXG>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROWS_SMEM));
@@ -1805,11 +1807,11 @@ bool tc_fused_bias_grads(const Dims& d) { return cdiv(d.H, BM) >= 2; }
 
 namespace {
 // One of the four token-major products.
-template <int MODE>
+template <int MODE, bool KEEP = true>
 int launch_rows(mgpt_moe_layer* L, TcState* s, const Workspace& w, const RowsP& p, const CUtensorMap& a0, const CUtensorMap& a1,
                 const CUtensorMap& b0, const CUtensorMap& b1, const CUtensorMap& d0, const CUtensorMap& d1, cudaStream_t st, const char* what)
 {
-    MGPT_CUDA(launch_pdl(tc_rows_kernel<MODE>, imin(grid_sms(L, s), w.max_tiles * p.n_col_tiles), ROWS_THREADS, ROWS_SMEM, st, a0, a1, b0, b1, d0, d1, p));
+    MGPT_CUDA(launch_pdl(tc_rows_kernel<MODE, KEEP>, imin(grid_sms(L, s), w.max_tiles * p.n_col_tiles), ROWS_THREADS, ROWS_SMEM, st, a0, a1, b0, b1, d0, d1, p));
     MGPT_LAUNCHED(what);
     return 0;
 }
@@ -1837,7 +1839,8 @@ int tc_experts_forward(mgpt_moe_layer* L, const Workspace& w, char* ws, cudaStre
     p.U = w.inference ? nullptr : (bf16*)(ws + w.U);
     L->stage_begin(ST_GATEUP, st);
     p.sched = s->sched + 0;
-    MGPT_TRY(launch_rows<MODE_GATEUP>(L, s, w, p, s->Xg, s->Xg, s->WguT, s->WguT, s->Hh_s, s->Hh_s, st, "tc_rows<gateup>"));
+    if (w.inference) MGPT_TRY((launch_rows<MODE_GATEUP, false>(L, s, w, p, s->Xg, s->Xg, s->WguT, s->WguT, s->Hh_s, s->Hh_s, st, "tc_rows<gateup>")));
+    else MGPT_TRY(launch_rows<MODE_GATEUP>(L, s, w, p, s->Xg, s->Xg, s->WguT, s->WguT, s->Hh_s, s->Hh_s, st, "tc_rows<gateup>"));
     L->stage_end(ST_GATEUP, st);
     // down: K = H
     p.kblocks = cdiv(d.H, BK); p.n_out = d.C; p.n_col_tiles = cdiv(d.C, BN);
