@@ -25,16 +25,15 @@ if ROOT not in sys.path:
 
 METRIC = "moe_layer_fwd_bwd_tokens_per_sec"
 # DRAM bytes (read + write) per launch from ncu captures, keyed by (workload, stage); see profiles/.
-# c3's are from before the weight gradients' CTA pairs.
 # c4 is too large to capture with many passes: its figures are those of c4q (a quarter of the tokens and of the
 # experts, same rows per expert) times four -- every term of the traffic is proportional to the number of experts.
 TRAFFIC = {
-    ("c3", "wgrad_gemm"): 822.7e6, ("c3", "gateup_gemm"): 338.8e6, ("c3", "dhh_gemm"): 396.5e6,
-    ("c3", "down_gemm"): 176.1e6, ("c3", "dxg_gemm"): 281.1e6,
-    ("c4q", "wgrad_gemm"): 1336.1e6, ("c4q", "gateup_gemm"): 370.7e6, ("c4q", "dhh_gemm"): 331.3e6,
-    ("c4q", "down_gemm"): 184.4e6, ("c4q", "dxg_gemm"): 334.4e6,
-    ("c4", "wgrad_gemm"): 4 * 1336.1e6, ("c4", "gateup_gemm"): 4 * 370.7e6, ("c4", "dhh_gemm"): 4 * 331.3e6,
-    ("c4", "down_gemm"): 4 * 184.4e6, ("c4", "dxg_gemm"): 4 * 334.4e6,
+    ("c3", "wgrad_gemm"): 661.1e6, ("c3", "gateup_gemm"): 338.8e6, ("c3", "dhh_gemm"): 392.7e6,
+    ("c3", "down_gemm"): 175.5e6, ("c3", "dxg_gemm"): 279.1e6,
+    ("c4q", "wgrad_gemm"): 1336.1e6, ("c4q", "gateup_gemm"): 375.1e6, ("c4q", "dhh_gemm"): 329.5e6,
+    ("c4q", "down_gemm"): 183.5e6, ("c4q", "dxg_gemm"): 335.3e6,
+    ("c4", "wgrad_gemm"): 4 * 1336.1e6, ("c4", "gateup_gemm"): 4 * 375.1e6, ("c4", "dhh_gemm"): 4 * 329.5e6,
+    ("c4", "down_gemm"): 4 * 183.5e6, ("c4", "dxg_gemm"): 4 * 335.3e6,
 }
 UNIT = "tokens/s"
 
