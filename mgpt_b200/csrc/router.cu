@@ -249,7 +249,14 @@ __global__ void __launch_bounds__(RX_THREADS, 1) router_exact_kernel(const Route
         // per thread leaves up to half of them without: 296 tokens, C=1024, 4 experts 10.7 us; two divisions per element before
         // that, 127 experts 572 us for 32851 tokens.)
         const bool wide = (E & 3) == 0;
-        const int per = wide ? E >> 2 : E, r0 = pt / per, q0 = pt % per, dr = RX_PRODUCE / per, dq = RX_PRODUCE % per;
+        int per = 1, r0 = 0, q0 = 0, dr = 0, dq = 0;
+        if (E != RS) {
+            per = wide ? E >> 2 : E;
+            r0 = pt / per;
+            q0 = pt % per;
+            dr = RX_PRODUCE / per;
+            dq = RX_PRODUCE % per;
+        }
         auto step = [&](int& r, int& q) {
             r += dr;
             q += dq;
@@ -321,8 +328,9 @@ __global__ void __launch_bounds__(RX_THREADS, 1) router_exact_kernel(const Route
                 if (works) {
                     const uint32_t base = ring0 + s * stage, ws = base + e0 * 4;
                     // U channels' operands at a time; two sets, the next one on its way.  (More pairs need fewer channels to hide a
-                    // load behind, and longer sets cost them registers: 16 x 3 x 4 BF16 tokens 57 -> 50 us with 4.)
-                    constexpr int U = TE * R <= 2 ? 16 : TE * R <= (sizeof(TIn) == 2 ? 8 : 4) ? 8 : 4, L = U < 8 ? U : 8;
+                    // load behind, and longer sets cost them registers: 16 x 3 x 4 BF16 tokens 57 -> 50 us with 4.  One pair of
+                    // BF16 tokens: 8.2 -> 7.9 us for 100 tokens, C=1024, 16 experts with 32; FP32 tokens 3 % slower.)
+                    constexpr int U = TE * R == 1 && sizeof(TIn) == 2 ? 32 : TE * R <= 2 ? 16 : TE * R <= (sizeof(TIn) == 2 ? 8 : 4) ? 8 : 4, L = U < 8 ? U : 8;
                     struct Ops {
                         float w[U][TE];
                         Row<TIn, L> x[R][U / L];
