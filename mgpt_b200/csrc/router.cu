@@ -329,8 +329,9 @@ __global__ void __launch_bounds__(RX_THREADS, 1) router_exact_kernel(const Route
                     const uint32_t base = ring0 + s * stage, ws = base + e0 * 4;
                     // U channels' operands at a time; two sets, the next one on its way.  (More pairs need fewer channels to hide a
                     // load behind, and longer sets cost them registers: 16 x 3 x 4 BF16 tokens 57 -> 50 us with 4.  One pair of
-                    // BF16 tokens: 8.2 -> 7.9 us for 100 tokens, C=1024, 16 experts with 32; FP32 tokens 3 % slower.)
-                    constexpr int U = TE * R == 1 && sizeof(TIn) == 2 ? 32 : TE * R <= 2 ? 16 : TE * R <= (sizeof(TIn) == 2 ? 8 : 4) ? 8 : 4, L = U < 8 ? U : 8;
+                    // BF16 tokens: 8.2 -> 7.9 us for 100 tokens, C=1024, 16 experts with 32; FP32 tokens 3 % slower,
+                    // 32 experts no faster, and 1 us slower in a call whose instructions come from HBM.)
+                    constexpr int U = TE * R == 1 && sizeof(TIn) == 2 && ET <= 16 ? 32 : TE * R <= 2 ? 16 : TE * R <= (sizeof(TIn) == 2 ? 8 : 4) ? 8 : 4, L = U < 8 ? U : 8;
                     struct Ops {
                         float w[U][TE];
                         Row<TIn, L> x[R][U / L];
